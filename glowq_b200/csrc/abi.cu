@@ -18,6 +18,8 @@ cudaError_t launch_generic(const __half* x, const MemberDev& mb, const float* r3
                            int group_size, int x_stride, cudaStream_t stream);
 cudaError_t launch_dequant(const int32_t* qweight, const __half* scales, const int32_t* qzeros, __half* out, int OC, int IC,
                            int group_size, int wstride, int zstride, int sstride, cudaStream_t stream);
+cudaError_t launch_quantize(const __half* w, int32_t* qweight, int32_t* qzeros, __half* scales, int OC, int IC,
+                            long long w_stride, cudaStream_t stream);
 bool gemm_supported(const glowq_w4a16_group_t& g);
 size_t gemm_workspace_bytes(int M, int IC, int OC_total, int rank, int n_members);
 unsigned allreduce_spin_limit();
@@ -552,6 +554,20 @@ int glowq_w4a16_dequant(const int32_t* qweight, const void* scales, const int32_
   cudaError_t e = launch_dequant(qweight, static_cast<const __half*>(scales), qzeros, static_cast<__half*>(out_w), OC, IC,
                                  group_size, weight_stride_i32, zero_stride_i32, scale_stride,
                                  static_cast<cudaStream_t>(stream));
+  return e == cudaSuccess ? GLOWQ_OK : fail_cuda(e);
+}
+
+int glowq_w4a16_quantize(const void* weight, int32_t* qweight, int32_t* qzeros, void* scales, int OC, int IC, int group_size,
+                         long long weight_stride, void* stream) {
+  if (!weight || !qweight || !qzeros || !scales || OC <= 0 || IC <= 0) return GLOWQ_ERR_BAD_ARGUMENT;
+  if (group_size <= 0 || group_size % 8 != 0) return GLOWQ_ERR_BAD_GROUP_SIZE;
+  if (group_size != kGroup) return GLOWQ_ERR_UNSUPPORTED_SHAPE;
+  if (weight_stride < IC) return GLOWQ_ERR_BAD_STRIDE;
+  const DeviceInfo* dev = nullptr;
+  int rc = device_info(&dev);
+  if (rc != GLOWQ_OK) return rc;
+  const cudaError_t e = launch_quantize(static_cast<const __half*>(weight), qweight, qzeros, static_cast<__half*>(scales), OC, IC,
+                                        weight_stride, static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? GLOWQ_OK : fail_cuda(e);
 }
 

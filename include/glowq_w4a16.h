@@ -147,6 +147,12 @@ int glowq_w4a16_dequant(const int32_t* qweight, const void* scales, const int32_
                         int OC, int IC, int group_size, int weight_stride_i32, int zero_stride_i32,
                         int scale_stride, void* stream);
 
+/* RTN uint4 quantiser and packer: weight[OC, IC] fp16 (row stride weight_stride elements) -> qweight[OC, G * 16],
+ * qzeros[OC, ceil(G / 8)], scales[OC, G] (dense, G = ceil(IC / 128)); groups of 128 columns only.  The same bits as
+ * _quantize_per_group_w4 (src/cuda_w4a16/linear.py:57-88) in fp16 arithmetic. */
+int glowq_w4a16_quantize(const void* weight, int32_t* qweight, int32_t* qzeros, void* scales, int OC, int IC,
+                         int group_size, long long weight_stride, void* stream);
+
 /* Plain W4A16 product out[M, OC] (fp16) = x[M, IC] . dequant(Q)^T with the weight-streaming kernel.
  * Replaces w4a16_gemv_forward_cuda / gemv_w4a16_asym (csrc/gemv_w4a16.cu:146-214, csrc/pybind.cpp:19-34).
  * The caller allocates `out`; `workspace` as for a group call. */
