@@ -879,7 +879,9 @@ inline size_t main_slot_bytes_bound(int M, int IC, int OC_total, int n_members) 
 size_t gemm_workspace_bytes(int M, int IC, int OC_total, int rank, int n_members) {
   size_t slots = std::max(rank > 0 ? r_slot_bytes(M, IC, rank) : 0, main_slot_bytes_bound(M, IC, OC_total, n_members));
   if (rank > 0 && M <= kRProductMaxM) slots = std::max(slots, r_product_slot_bytes(M, IC, rank));
-  if (M > 8 && M <= 2 * BM) slots = std::max(slots, kTmemSlotBytes);   // K slices of the tensor-memory form
+  // K slices of the tensor-memory form, unless whole tiles fill the SMs and the last round of them is nearly full too
+  const int tmem_tiles = cdiv(OC_total, BN), tmem_rest = tmem_tiles % kPlanSms;
+  if (M > 8 && M <= kTmemMaxM && !(tmem_tiles >= kPlanSms && tmem_rest * 4 >= 3 * kPlanSms)) slots = std::max(slots, kTmemSlotBytes);
   if (M > 2 * BM) slots = std::max(slots, static_cast<size_t>(kMaxTailSlots) * 2 * 2 * BM * BN * 4);  // sliced last wave
   if (slots == 0) return kWsHeaderBytes;
   return counters_end(OC_total, n_members) + slots + 256;
