@@ -44,8 +44,9 @@ cudaError_t launch_r_product(const __half* x, const __half* R, __half* r_buf, fl
 int tensor_map_2d_ex(CUtensorMap* out, CUtensorMapDataType dtype, const void* ptr, uint64_t dim0, uint64_t dim1,
                      uint64_t stride_bytes, uint32_t box0, uint32_t box1, int swizzle128);
 
-int gemm_tmem_forward(const glowq_w4a16_group_t& g, bool any_corr, bool any_separate, uint32_t* status, uint32_t* tile_ctr,
-                      int n_ctr, float* slots, size_t slot_bytes, int sms, cudaStream_t stream, cudaError_t* cuda_err);
+size_t gemm_tmem_r_bytes(int M, int IC, int rank);
+int gemm_tmem_forward(const glowq_w4a16_group_t& g, bool compute_r, bool any_corr, bool any_separate, uint32_t* status,
+                      uint32_t* r_ctr, uint32_t* tile_ctr, int n_ctr, float* slots, size_t slot_bytes, int sms, cudaStream_t stream, cudaError_t* cuda_err);
 
 namespace {
 
@@ -883,6 +884,7 @@ size_t gemm_workspace_bytes(int M, int IC, int OC_total, int rank, int n_members
   const int tmem_tiles = cdiv(OC_total, BN), tmem_rest = tmem_tiles % kPlanSms;
   if (M > 8 && M <= kTmemMaxM && !(tmem_tiles >= kPlanSms && tmem_rest * 4 >= 3 * kPlanSms)) slots = std::max(slots, kTmemSlotBytes);
   if (M > 2 * BM) slots = std::max(slots, static_cast<size_t>(kMaxTailSlots) * 2 * 2 * BM * BN * 4);  // sliced last wave
+  if (rank > 0 && M > 8 && M <= kTmemMaxM) slots = std::max(slots, gemm_tmem_r_bytes(M, IC, rank));
   if (slots == 0) return kWsHeaderBytes;
   return counters_end(OC_total, n_members) + slots + 256;
 }
@@ -904,10 +906,17 @@ int gemm_group_forward(const glowq_w4a16_group_t& g, cudaStream_t stream, cudaEr
   if ((rc = map(&tm_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, g.x, g.IC, g.M, static_cast<uint64_t>(g.x_stride) * 2, BK, BM, 1)))
     return rc;
 
-  // r = X . R^T, once per group, into r_buf.  Up to 128 tokens: one small launch (r_product.cu); the K-sliced GEMM
+  int oc_sum = 0;
+  for (int i = 0; i < g.n_members; ++i) oc_sum += g.members[i].OC;
+  const size_t scratch = counters_end(oc_sum, g.n_members);
+  const bool use_tmem = g.M <= kTmemMaxM;
+  const bool r_in_launch = use_tmem && g.r_mode == GLOWQ_R_COMPUTE &&
+                           g.workspace_bytes >= scratch + gemm_tmem_r_bytes(g.M, g.IC, g.rank);
+
+  // r = X . R^T, once per group, into r_buf: up to 64 tokens inside the group launch (gemm_tmem.cu).  Up to 128 tokens: one small launch (r_product.cu); the K-sliced GEMM
   // below plus its slot sum take about twenty microseconds.
-  bool r_done = false;
-  if (g.r_mode == GLOWQ_R_COMPUTE && g.M <= kRProductMaxM && cdiv(g.rank, 16) * cdiv(g.M, 64) <= kRpCtrWords) {
+  bool r_done = r_in_launch;
+  if (g.r_mode == GLOWQ_R_COMPUTE && !r_done && g.M <= kRProductMaxM && cdiv(g.rank, 16) * cdiv(g.M, 64) <= kRpCtrWords) {
     int oc_total = 0;
     for (int i = 0; i < g.n_members; ++i) oc_total += g.members[i].OC;
     const size_t need = r_product_slot_bytes(g.M, g.IC, g.rank);
@@ -979,18 +988,15 @@ int gemm_group_forward(const glowq_w4a16_group_t& g, cudaStream_t stream, cudaEr
     const auto& m = g.members[i];
     any_separate = any_separate || (g.r_mode != GLOWQ_R_NONE && m.L && m.alpha != 0.f && m.alpha != 1.f);
   }
-  static const int tmem_max = [] { const char* e = std::getenv("GLOWQ_TS_MAX"); return e ? std::atoi(e) : kTmemMaxM; }();
-  if (g.M <= tmem_max) {
-    int sms = kPlanSms, dev = 0, oc_total = 0;
+  if (use_tmem) {
+    int sms = kPlanSms, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    for (int i = 0; i < g.n_members; ++i) oc_total += g.members[i].OC;
-    const size_t begin = counters_end(oc_total, g.n_members);
     unsigned char* ws = static_cast<unsigned char*>(g.workspace);
-    const bool room = g.workspace_bytes > begin;
-    return gemm_tmem_forward(g, any_corr, any_separate, status, reinterpret_cast<uint32_t*>(ws + kWsTileCtrOffset),
-                             room ? cdiv(oc_total, kTileRows) : 0, reinterpret_cast<float*>(ws + begin),
-                             room ? g.workspace_bytes - begin : 0, sms, stream, cuda_err);
+    const bool room = g.workspace_bytes > scratch;
+    return gemm_tmem_forward(g, r_in_launch, any_corr, any_separate, status, reinterpret_cast<uint32_t*>(ws + kWsHeaderBytes),
+                             reinterpret_cast<uint32_t*>(ws + kWsTileCtrOffset), room ? cdiv(oc_sum, kTileRows) : 0,
+                             reinterpret_cast<float*>(ws + scratch), room ? g.workspace_bytes - scratch : 0, sms, stream, cuda_err);
   }
   // Tile shape: the 256 x 256 CTA tile has the best operand reuse, but a problem that fills the SMs badly in whole
   // waves is faster with narrower (nn = 1) or shorter (mt = 1) tiles.  A separate correction accumulator needs nn = 1.

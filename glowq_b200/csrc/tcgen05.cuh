@@ -6,7 +6,9 @@
 
 namespace glowq {
 
-constexpr uint32_t kGemmSpin = 1u << 18;   // polls of one wait before the kernel gives up (status 3)
+// Polls of one wait before the kernel gives up (status 3): seconds, because warps that run ahead of the dependency wait sit in
+// these waits until the kernels before are complete.
+constexpr uint32_t kGemmSpin = 1u << 20;
 
 __device__ __forceinline__ uint32_t sm_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ void g_mbar_init(uint32_t a, uint32_t count) {

@@ -45,3 +45,29 @@ def test_strided_output_and_a_scarce_workspace():
         assert run_group(g) == 0 and status_ok(g) == 0
         assert_close(wide[:, :200], lin.oracle(x))
         assert wide[:, 200:].isnan().all()
+
+
+@pytest.mark.parametrize("M,ocs,ic,rank", [(16, [3072, 1024, 1024], 3072, 64), (64, [640], 18944, 128), (32, [2048], 2048, 256)])
+def test_launches_back_to_back_on_one_workspace(M, ocs, ic, rank):
+    """Counters, slots and r of one workspace through launches that overlap (short slices reach their epilogue before the launch
+    before is complete; at 64 tokens the packed ring is shorter than the stages): every launch gives the same bits."""
+    rng = np.random.default_rng(M)
+    lins = [Linear(rng, oc, ic, rank=rank, quantize=False) for oc in ocs]
+    R_d = dev((rng.standard_normal((rank, ic)) * 0.01).astype(np.float16))
+    x_d = dev(rng.standard_normal((M, ic)).astype(np.float16))
+    ws, groups = None, []
+    for _ in range(24):
+        outs = [new_out(M, l) for l in lins]
+        g = make_group(x_d, lins, outs, R_d=R_d, r_buf=torch.zeros(M, rank, dtype=torch.float16, device="cuda"), r_mode=K.R_COMPUTE,
+                       ws=ws)
+        ws = g._keep[5]
+        groups.append((g, outs))
+    many = (K.Group * len(groups))(*[g for g, _ in groups])
+    assert K.load_w4a16_extension().lib.glowq_w4a16_group_forward_many(many, len(groups)) == 0
+    torch.cuda.synchronize()
+    assert status_ok(groups[0][0]) == 0
+    for l, o in zip(lins, groups[0][1]):
+        assert_close(o, l.oracle(x_d.cpu().numpy(), R_d.cpu().numpy()), tol_abs=5e-2)   # K = 18944: outputs of 3.7 rms, fp16 ulp 2^-8
+    for g, outs in groups[1:]:
+        assert torch.equal(g._keep[4], groups[0][0]._keep[4])
+        assert all(torch.equal(a, b) for a, b in zip(outs, groups[0][1]))
