@@ -860,7 +860,7 @@ inline size_t counters_end(int OC_total, int n_members) {
 // depend on the device.
 constexpr int kPlanSms = 148;
 constexpr int kTmemMaxM = 64;                  // tokens up to which the weights go through tensor memory (gemm_tmem.cu)
-constexpr size_t kTmemSlotBytes = 16u << 20;   // its fp32 slots: 512 slices of a 64-token tile
+constexpr int kTmemSlices = 304;               // its K slices at most (two CTAs per SM), a tile of 32 or 64 tokens x 128 fp32 each
 constexpr int kMaxTailSlots = 64;   // tiles x slices of a sliced last wave (256 KB of fp32 each for a 256 x 256 tile)
 inline int main_ksplit(int tiles, int nk, int sms) {
   if (tiles * 2 > sms) return 1;
@@ -882,9 +882,10 @@ size_t gemm_workspace_bytes(int M, int IC, int OC_total, int rank, int n_members
   if (rank > 0 && M <= kRProductMaxM) slots = std::max(slots, r_product_slot_bytes(M, IC, rank));
   // K slices of the tensor-memory form, unless whole tiles fill the SMs and the last round of them is nearly full too
   const int tmem_tiles = cdiv(OC_total, BN), tmem_rest = tmem_tiles % kPlanSms;
-  if (M > 8 && M <= kTmemMaxM && !(tmem_tiles >= kPlanSms && tmem_rest * 4 >= 3 * kPlanSms)) slots = std::max(slots, kTmemSlotBytes);
+  if (M > 8 && M <= kTmemMaxM && !(tmem_tiles >= kPlanSms && tmem_rest * 4 >= 3 * kPlanSms))
+    slots = std::max(slots, static_cast<size_t>(kTmemSlices) * (M <= 32 ? 32 : 64) * BN * 4);
   if (M > 2 * BM) slots = std::max(slots, static_cast<size_t>(kMaxTailSlots) * 2 * 2 * BM * BN * 4);  // sliced last wave
-  if (rank > 0 && M > 8 && M <= kTmemMaxM) slots = std::max(slots, gemm_tmem_r_bytes(M, IC, rank));
+  if (rank > 0 && M > 8 && M <= kTmemMaxM) slots += gemm_tmem_r_bytes(M, IC, rank);
   if (slots == 0) return kWsHeaderBytes;
   return counters_end(OC_total, n_members) + slots + 256;
 }

@@ -19,11 +19,16 @@
 // the other's steps.
 //   r = X . R^T is computed inside the launch by the lowest block indices (placed first): a CTA multiplies 128 rows of R with a
 // slice of K - the correction steps' loop with R in the place of L and X in the place of r - parks an fp32 slot, and the CTAs
-// of an R tile, once all have arrived, add each a share of its elements in slice order, round to fp16 and write r_buf.  The
+// of an R tile, once all have arrived, add each a share of its elements in a fixed order, round to fp16 and write r_buf.  The
 // activation producers poll the count of finished CTAs before their first correction step.  As a launch of its own in front,
 // r cost 6 to 11 microseconds per group.
 // K may be sliced over CTAs; the CTA of a tile's last slice adds the others' fp32 slots in slice order (deterministic).
-// Every mbarrier wait is bounded; on expiry a status word is set and the CTA drains and frees its tensor memory.
+// Every wait is bounded; on expiry a status word is set and the CTA drains and frees its tensor memory.
+//
+// Measured (B200, corrected group calls of the 13B shapes, microseconds at 16 / 32 / 64 tokens; before: weights through
+// shared memory, r and slot sum as launches of their own): q/k/v 38.7 / 39.4 / 44.5 -> 23.6 / 24.3 / 28.7, o_proj 22.2 /
+// 22.9 / 25.0 -> 15.5 / 16.1 / 21.6, gate/up 58.1 / 58.6 / 60.5 -> 36.7 / 37.5 / 42.3 (1.9 TB/s of packed weights), down_proj
+// 38.8 / 38.1 / 40.7 -> 22.8 / 23.7 / 29.0.  Left: about 8 microseconds of dependent chain per launch, and 0.33 per step and SM.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -50,6 +55,9 @@ constexpr int kDequantWarps = 4 * kTeams, kCtrlWarps = 3, kThreads = 32 * (kCtrl
 constexpr int kTmemCols = 256;                // per CTA: two share an SM
 constexpr int kSmemBytes = 112 * 1024;
 constexpr int kMaxRCtas = 48;                 // CTAs that compute r
+// Polls of a count of finished CTAs: seconds, because another stream's kernel may hold the SMs that the rest of the CTAs
+// of r need (they are placed first, so that nothing of this launch does).
+constexpr unsigned kCountSpin = 1u << 22;
 enum : int { kRCnt = 0, kRFlag = 64, kRExit = 65 };   // words of the r counters: arrivals per R tile, finished CTAs, exits
 
 struct TsMember {
@@ -276,7 +284,7 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
         uint32_t spins = 0;
         while (ld_acquire_u32(p.r_ctr + kRFlag) != static_cast<uint32_t>(p.n_r)) {
           __nanosleep(32);
-          if (++spins > kSpinLimit || *abort_flag) {
+          if (++spins > kCountSpin || *abort_flag) {
             *abort_flag = 1;
             atomicExch(p.status, 1u);
             ok = false;
@@ -439,9 +447,6 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
     // ---- epilogue.  Of a sliced tile, the CTAs of all slices but the last park fp32 slots; the last one - which holds the
     // correction steps, so that it is the late one - adds them, in slice order, to its own accumulators and stores.  (Its
     // block index is the highest of the tile's: the others are resident or done.)
-    // The counters and slots are the previous launch's until it is complete, and a short slice gets here without having
-    // waited for an MMA.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int et = threadIdx.x - 32 * kCtrlWarps;
     const int ntok = min(p.N, p.M - m0);
     const size_t slot_floats = static_cast<size_t>(p.N) * kRows;
@@ -452,14 +457,17 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
     auto await_count = [&](uint32_t* ctr, uint32_t n) {   // one thread; acquires the slots of the CTAs that counted
       uint32_t spins = 0;
       while (ld_acquire_u32(ctr) != n) {
-        if (++spins > kSpinLimit || *abort_flag) {
+        if (++spins > kCountSpin || *abort_flag) {
           atomicExch(p.status, 1u);
           break;
         }
       }
     };
     if (finish) {
+      // The counters and slots are the previous launch's until it is complete, and a short slice gets here without having
+      // waited for an MMA.
       if (et == 0) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
         await_count(p.tile_ctr + sl_tile, static_cast<uint32_t>(ks - 1));
         p.tile_ctr[sl_tile] = 0u;
       }
@@ -616,11 +624,6 @@ cudaError_t launch(const TsParams& p, const TsMaps& tm, int ctas, cudaStream_t s
   return cudaLaunchKernelEx(&cfg, gemm_tmem_kernel, p, tm);
 }
 
-int env_or(const char* name, int dflt) {
-  const char* v = std::getenv(name);
-  return (v && *v) ? std::atoi(v) : dflt;
-}
-
 inline int tile_tokens(int M) { return cdiv(M, 16) * 16; }   // tokens of the one tile (M <= 64)
 // K slices of an R tile: about four 64-column steps each, at most kMaxRCtas CTAs in all.
 inline int r_slices_for(int IC, int rank) { return std::max(1, std::min(cdiv(cdiv(IC, 64), 4), kMaxRCtas / cdiv(rank, kRows))); }
@@ -637,7 +640,6 @@ size_t gemm_tmem_r_bytes(int M, int IC, int rank) {
 // `tile_ctr`: n_ctr zeroed counters, `r_ctr`: kRpCtrWords of them.
 int gemm_tmem_forward(const glowq_w4a16_group_t& g, bool compute_r, bool any_corr, bool any_separate, uint32_t* status,
                       uint32_t* r_ctr, uint32_t* tile_ctr, int n_ctr, float* slots, size_t slot_bytes, int sms, cudaStream_t stream, cudaError_t* cuda_err) {
-  static const int env_f = env_or("GLOWQ_TS_F", -1), env_ks = env_or("GLOWQ_TS_KS", 0);   // tuning overrides
   const int G = cdiv(g.IC, kGroup);
   TsParams p{};
   p.N = tile_tokens(g.M);
@@ -712,25 +714,24 @@ int gemm_tmem_forward(const glowq_w4a16_group_t& g, bool compute_r, bool any_cor
   p.n_x = n_x;
   const int total = n_x, units = sms, resident = 2 * sms;
   const size_t item_bytes = static_cast<size_t>(p.N) * kRows * 4;
-  // Work partition: f rounds of whole tiles, the rest cut into ks slices of K.  Cost in microseconds, fitted on B200: an
-  // SM takes 0.33 per step while two CTAs share it (0.5 alone), 2.5 per wave of items for prologue
-  // and epilogue, and the slices of a tile are added through memory.  Measured at 16 tokens on the 13B shapes: q/k/v
-  // 31.5 us whole, 21.7 in two slices, 28.0 in four; o_proj 24.8 / 17.5 / 13.3, 12.7 in six; gate/up 35.5 whole, 41.4 in two
-  // slices, 33.8 with one round whole and the other 68 tiles in two slices.
+  // Work partition: f rounds of whole tiles, the rest cut into ks slices of K.  Cost in microseconds, fitted on B200: an SM
+  // takes 0.33 per step while two CTAs share it (0.5 alone), 2.5 per wave of items for prologue and epilogue (the CTAs of r
+  // take slots, but are gone before a whole tile is done), and the slices of a tile are added through memory.  Measured at
+  // 16 tokens on the 13B shapes: q/k/v 30.2 whole, 22.8 in two slices, 30.5 in three; o_proj 24.8 whole, 19.1 / 15.8 /
+  // 15.5 in two / three / five, 19.1 in seven (a second wave behind the CTAs of r); gate/up 35.5 whole, 43.2 in two slices,
+  // 33.8 with one round whole and the other 68 tiles in two slices.
   p.full_tiles = total;
   p.n_tail = 0;
   p.ksplit = 1;
   const int nk = G + nu;
   double best = 1e30;
   for (int f = 0; f <= total / units; ++f) {
-    if (env_f >= 0 && f != env_f) continue;
     const int full = f * units, tail = total - full;
     for (int ks = 1; ks <= 16 && (ks == 1 || ks * 4 <= nk); ++ks) {
-      if (env_ks > 0 && ks != env_ks) continue;
       if (ks > 1 && (tail == 0 || tail > n_ctr || static_cast<size_t>(tail) * ks * item_bytes > slot_bytes)) break;
       const int items = full + tail * ks;
       const double load = static_cast<double>(f) * nk + static_cast<double>(cdiv(tail * ks, units)) * nk / ks;
-      const double cost = load * (items > units ? 0.33 : 0.5) + 2.5 * cdiv(items, resident) +
+      const double cost = load * (items > units ? 0.33 : 0.5) + 2.5 * cdiv(items, f > 0 ? resident : std::max(units, resident - p.n_r)) +
                           (ks > 1 ? 1.5 + 0.006 * p.N * ks : 0.0);
       if (cost < best) {
         best = cost;
