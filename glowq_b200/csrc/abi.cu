@@ -24,6 +24,7 @@ bool gemm_supported(const glowq_w4a16_group_t& g);
 size_t gemm_workspace_bytes(int M, int IC, int OC_total, int rank, int n_members);
 unsigned allreduce_spin_limit();
 int gemm_group_forward(const glowq_w4a16_group_t& g, cudaStream_t stream, cudaError_t* cuda_err);
+void gemm_workspace_map(const glowq_w4a16_group_t& g, int sms, WorkspaceMap* map);
 }  // namespace glowq
 
 using namespace glowq;
@@ -192,7 +193,8 @@ int env_int(const char* name, int dflt) {
 struct GemvPlan {
   int NT, G, n_tiles, SK, gps, n_r_tiles, SKr, gpr, stages, ctas_per_sm, meta_gp, meta_gw, xs_stride;
   size_t smem;
-  size_t off_r_ctr, off_tile_ctr, off_r_partial, off_sk_partial, off_r32, total;
+  bool own_ctr;   // more sliced tiles than the workspace has counters for: they lie among the slots, cleared by the launch
+  size_t off_tile_ctr, off_r_partial, off_sk_partial, off_r32, total;
 };
 
 size_t plan_smem(const GemvPlan& pl, int Mc, int stages) {
@@ -250,10 +252,12 @@ GemvPlan make_plan(int M, int IC, int n_tiles, int rank, int sms, int split_k) {
   pl.n_r_tiles = ceil_div(std::max(rank, 0), kRTileRows);
   pl.SKr = chunks;   // one quantisation group per warp and R unit: a single round of loads per unit
   const size_t tile_elems = static_cast<size_t>(kRowTiles) * pl.NT * 128;
-  pl.off_r_ctr = kWsHeaderBytes;
-  size_t off = kWsTileCtrOffset;
-  pl.off_tile_ctr = off;
-  off = align_up(off + static_cast<size_t>(n_tiles) * 4, 256);
+  // (room for counters among the slots whether or not K is sliced: the size a call needs grows with its rows, as the callers'
+  // checks against their scratch expect)
+  pl.own_ctr = n_tiles > kTileCtrWords;
+  pl.off_tile_ctr = pl.own_ctr ? kWsSlotsOffset : kWsTileCtrOffset;
+  size_t off = kWsSlotsOffset;
+  if (pl.own_ctr) off = align_up(off + static_cast<size_t>(n_tiles) * 4, 256);
   pl.off_r_partial = off;
   pl.gpr = ceil_div(pl.G, pl.SKr);
   pl.SKr = ceil_div(pl.G, pl.gpr);
@@ -340,6 +344,14 @@ int n_tiles_of(const glowq_w4a16_group_t& g) {
   int n = 0;
   for (int i = 0; i < g.n_members; ++i) n += ceil_div(g.members[i].OC, kTileRows);
   return n;
+}
+
+// Measured on B200: up to 8 tokens fit one streaming launch (one MMA N tile); 9..16 tokens would take two, and at
+// 16 tokens the tcgen05 GEMM (K-sliced over all SMs when it has few tiles) is ahead on every Llama-2-13B shape
+// (q/k/v 44 vs 47 us, gate/up 65 vs 70, down_proj 43 vs 64, o_proj 26 vs 33, corrected), so it takes over from 9.
+bool takes_gemm(const glowq_w4a16_group_t& g) {
+  const bool use_gemm = g.kernel == GLOWQ_KERNEL_GEMM || (g.kernel == GLOWQ_KERNEL_AUTO && g.M > kGemvAutoMaxM);
+  return use_gemm && gemm_supported(g);
 }
 
 int gemv_group_forward(const glowq_w4a16_group_t& g, const DeviceInfo& dev, cudaStream_t stream) {
@@ -501,6 +513,10 @@ int gemv_group_forward(const glowq_w4a16_group_t& g, const DeviceInfo& dev, cuda
           }
         }
       }
+      if (pl.own_ctr && pl.SK > 1) {
+        e = cudaMemsetAsync(p.tile_ctr, 0, static_cast<size_t>(n_tiles) * 4, stream);
+        if (e != cudaSuccess) return fail_cuda(e);
+      }
       e = launch_gemv_stream(p, tm, pl.NT, grid, stream);
       if (e != cudaSuccess) return fail_cuda(e);
     } else {
@@ -593,18 +609,41 @@ int glowq_w4a16_group_forward(const glowq_w4a16_group_t* group) {
   if (rc != GLOWQ_OK) return rc;
   if (g.M == 0) return GLOWQ_OK;
   cudaStream_t stream = static_cast<cudaStream_t>(g.stream);
-  // Measured on B200: up to 8 tokens fit one streaming launch (one MMA N tile); 9..16 tokens would take two, and at
-  // 16 tokens the tcgen05 GEMM (K-sliced over all SMs when it has few tiles) is ahead on every Llama-2-13B shape
-  // (q/k/v 44 vs 47 us, gate/up 65 vs 70, down_proj 43 vs 64, o_proj 26 vs 33, corrected), so it takes over from 9.
-  bool use_gemm = g.kernel == GLOWQ_KERNEL_GEMM;
-  if (g.kernel == GLOWQ_KERNEL_AUTO) use_gemm = g.M > kGemvAutoMaxM;
-  if (use_gemm && gemm_supported(g)) {
+  if (takes_gemm(g)) {
     cudaError_t ce = cudaSuccess;
     rc = gemm_group_forward(g, stream, &ce);
     if (rc == GLOWQ_ERR_CUDA) return fail_cuda(ce);
     return rc;
   }
   return gemv_group_forward(g, *dev, stream);
+}
+
+// Where in its workspace a launch of this group keeps what (host arithmetic, for the tests of the layout; not part of the
+// ABI).  `sms`: streaming multiprocessors to plan for.
+int glowq_internal_workspace_map(const glowq_w4a16_group_t* group, int sms, WorkspaceMap* map) {
+  if (!group || !map) return GLOWQ_ERR_BAD_ARGUMENT;
+  const glowq_w4a16_group_t& g = *group;
+  const int rc = validate_group(g);
+  if (rc != GLOWQ_OK) return rc;
+  *map = WorkspaceMap{};
+  if (g.M == 0) return GLOWQ_OK;
+  if (takes_gemm(g)) {
+    gemm_workspace_map(g, sms, map);
+    return GLOWQ_OK;
+  }
+  const int n_tiles = n_tiles_of(g);
+  const GemvPlan pl = make_plan(std::min(g.M, kGemvMaxM), g.IC, n_tiles, g.r_mode != GLOWQ_R_NONE ? g.rank : 0, sms, g.split_k);
+  if (pl.total > g.workspace_bytes) return GLOWQ_ERR_WORKSPACE_TOO_SMALL;
+  map->kernel = 0;
+  if (pl.SK > 1 && !pl.own_ctr) {
+    map->ctr_begin = pl.off_tile_ctr;
+    map->ctr_end = pl.off_tile_ctr + static_cast<size_t>(n_tiles) * 4;
+  }
+  map->slots_begin = pl.own_ctr ? pl.off_tile_ctr : pl.off_r_partial;
+  map->slots_end = pl.total;
+  map->ksplit = pl.SK;
+  map->sliced_tiles = pl.SK > 1 ? n_tiles : 0;
+  return GLOWQ_OK;
 }
 
 int glowq_w4a16_group_forward_many(const glowq_w4a16_group_t* groups, int n) {

@@ -45,8 +45,9 @@ int tensor_map_2d_ex(CUtensorMap* out, CUtensorMapDataType dtype, const void* pt
                      uint64_t stride_bytes, uint32_t box0, uint32_t box1, int swizzle128);
 
 size_t gemm_tmem_r_bytes(int M, int IC, int rank);
-int gemm_tmem_forward(const glowq_w4a16_group_t& g, bool compute_r, bool any_corr, bool any_separate, uint32_t* status,
-                      uint32_t* r_ctr, uint32_t* tile_ctr, int n_ctr, float* slots, size_t slot_bytes, int sms, cudaStream_t stream, cudaError_t* cuda_err);
+int gemm_tmem_forward(const glowq_w4a16_group_t& g, bool compute_r, bool any_corr, bool any_separate, int sms, cudaStream_t stream,
+                      cudaError_t* cuda_err);
+void gemm_tmem_workspace_map(const glowq_w4a16_group_t& g, bool compute_r, bool any_corr, bool any_separate, int sms, WorkspaceMap* map);
 
 namespace {
 
@@ -849,12 +850,7 @@ inline size_t r_slot_bytes(int M, int IC, int rank) {
   const int ks = r_ksplit(M, IC, rank);
   return ks > 1 ? static_cast<size_t>(ks) * cdiv(rank, BN) * cdiv(M, BM) * kRSlotBytes : 0;
 }
-// The slots sit at the END of the workspace, clear of the counters that the weight-streaming kernel keeps (zeroed)
-// at its start: one workspace may serve launches of both kernels in turn.
-inline size_t counters_end(int OC_total, int n_members) {
-  const size_t n = kWsTileCtrOffset + (static_cast<size_t>(cdiv(OC_total, kTileRows)) + n_members) * 4;
-  return (n + 255) & ~static_cast<size_t>(255);
-}
+// The slots of the kernels of this file sit at the end of the workspace, behind kWsSlotsOffset.
 
 // K slices of a group GEMM with few tiles (up to 128 tokens): planned for 148 SMs so that the workspace size does not
 // depend on the device.
@@ -887,19 +883,44 @@ size_t gemm_workspace_bytes(int M, int IC, int OC_total, int rank, int n_members
   if (M > 2 * BM) slots = std::max(slots, static_cast<size_t>(kMaxTailSlots) * 2 * 2 * BM * BN * 4);  // sliced last wave
   if (rank > 0 && M > 8 && M <= kTmemMaxM) slots += gemm_tmem_r_bytes(M, IC, rank);
   if (slots == 0) return kWsHeaderBytes;
-  return counters_end(OC_total, n_members) + slots + 256;
+  return kWsSlotsOffset + slots + 256;
+}
+
+namespace {
+// What the routes of a group call hang on.
+struct GemmRoute {
+  bool any_corr, any_separate;   // some member is corrected; with a factor other than 1 (an accumulator of its own)
+  bool tmem, r_in_launch;        // the tensor-memory form (gemm_tmem.cu); r computed by its launch
+};
+GemmRoute gemm_route(const glowq_w4a16_group_t& g) {
+  GemmRoute rt{};
+  for (int i = 0; i < g.n_members && g.r_mode != GLOWQ_R_NONE; ++i) {
+    const bool corr = g.members[i].L && g.members[i].alpha != 0.f;
+    rt.any_corr = rt.any_corr || corr;
+    rt.any_separate = rt.any_separate || (corr && g.members[i].alpha != 1.f);
+  }
+  rt.tmem = g.M <= kTmemMaxM;
+  rt.r_in_launch = rt.tmem && g.r_mode == GLOWQ_R_COMPUTE &&
+                   g.workspace_bytes >= kWsSlotsOffset + gemm_tmem_r_bytes(g.M, g.IC, g.rank);
+  return rt;
+}
+}  // namespace
+
+// (host arithmetic: see glowq_internal_workspace_map)
+void gemm_workspace_map(const glowq_w4a16_group_t& g, int sms, WorkspaceMap* map) {
+  const GemmRoute rt = gemm_route(g);
+  if (rt.tmem) return gemm_tmem_workspace_map(g, rt.r_in_launch, rt.any_corr, rt.any_separate, sms, map);
+  map->kernel = 2;   // no tile counters; slots at the end, wherever they begin
+  map->slots_begin = kWsSlotsOffset;
+  map->slots_end = std::max<unsigned long long>(kWsSlotsOffset, g.workspace_bytes);
 }
 
 int gemm_group_forward(const glowq_w4a16_group_t& g, cudaStream_t stream, cudaError_t* cuda_err) {
   if (g.workspace_bytes < kWsHeaderBytes) return GLOWQ_ERR_WORKSPACE_TOO_SMALL;
   uint32_t* status = static_cast<uint32_t*>(g.workspace) + WS_STATUS;
   const int G = (g.IC + kGroup - 1) / kGroup;
-  const bool any_corr = [&] {
-    if (g.r_mode == GLOWQ_R_NONE) return false;
-    for (int i = 0; i < g.n_members; ++i)
-      if (g.members[i].L && g.members[i].alpha != 0.f) return true;
-    return false;
-  }();
+  const GemmRoute route = gemm_route(g);
+  const bool any_corr = route.any_corr, any_separate = route.any_separate;
   auto map = [&](CUtensorMap* out, CUtensorMapDataType dt, const void* ptr, uint64_t d0, uint64_t d1, uint64_t stride,
                  uint32_t b0, uint32_t b1, int sw) { return tensor_map_2d_ex(out, dt, ptr, d0, d1, stride, b0, b1, sw); };
   int rc;
@@ -907,22 +928,13 @@ int gemm_group_forward(const glowq_w4a16_group_t& g, cudaStream_t stream, cudaEr
   if ((rc = map(&tm_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, g.x, g.IC, g.M, static_cast<uint64_t>(g.x_stride) * 2, BK, BM, 1)))
     return rc;
 
-  int oc_sum = 0;
-  for (int i = 0; i < g.n_members; ++i) oc_sum += g.members[i].OC;
-  const size_t scratch = counters_end(oc_sum, g.n_members);
-  const bool use_tmem = g.M <= kTmemMaxM;
-  const bool r_in_launch = use_tmem && g.r_mode == GLOWQ_R_COMPUTE &&
-                           g.workspace_bytes >= scratch + gemm_tmem_r_bytes(g.M, g.IC, g.rank);
-
   // r = X . R^T, once per group, into r_buf: up to 64 tokens inside the group launch (gemm_tmem.cu).  Up to 128 tokens: one small launch (r_product.cu); the K-sliced GEMM
   // below plus its slot sum take about twenty microseconds.
-  bool r_done = r_in_launch;
+  bool r_done = route.r_in_launch;
   if (g.r_mode == GLOWQ_R_COMPUTE && !r_done && g.M <= kRProductMaxM && cdiv(g.rank, 16) * cdiv(g.M, 64) <= kRpCtrWords) {
-    int oc_total = 0;
-    for (int i = 0; i < g.n_members; ++i) oc_total += g.members[i].OC;
     const size_t need = r_product_slot_bytes(g.M, g.IC, g.rank);
     const size_t off = g.workspace_bytes >= need ? ((g.workspace_bytes - need) & ~static_cast<size_t>(255)) : 0;
-    if (off >= counters_end(oc_total, g.n_members)) {
+    if (off >= kWsSlotsOffset) {
       unsigned char* ws = static_cast<unsigned char*>(g.workspace);
       const cudaError_t e = launch_r_product(static_cast<const __half*>(g.x), static_cast<const __half*>(g.R),
                                              static_cast<__half*>(g.r_buf), reinterpret_cast<float*>(ws + off),
@@ -951,11 +963,9 @@ int gemm_group_forward(const glowq_w4a16_group_t& g, cudaStream_t stream, cudaEr
     p.n_members = 1;
     p.mt = 1;  // narrow output (rank columns): small tiles, more CTAs
     p.ksplit = r_ksplit(g.M, g.IC, g.rank);
-    int oc_total = 0;
-    for (int i = 0; i < g.n_members; ++i) oc_total += g.members[i].OC;
     const size_t slot_bytes = r_slot_bytes(g.M, g.IC, g.rank);
     size_t slot_off = g.workspace_bytes >= slot_bytes ? ((g.workspace_bytes - slot_bytes) & ~static_cast<size_t>(255)) : 0;
-    if (slot_off < counters_end(oc_total, g.n_members)) {  // workspace not sized for slicing: one CTA per tile walks all of K
+    if (slot_off < kWsSlotsOffset) {  // workspace not sized for slicing: one CTA per tile walks all of K
       p.ksplit = 1;
       slot_off = kWsHeaderBytes;
     }
@@ -984,20 +994,11 @@ int gemm_group_forward(const glowq_w4a16_group_t& g, cudaStream_t stream, cudaEr
     return rc;
 
   // All members in ONE launch: the grid's x index runs over the column tiles of member 0, then member 1, ...
-  bool any_separate = false;
-  for (int i = 0; i < g.n_members; ++i) {
-    const auto& m = g.members[i];
-    any_separate = any_separate || (g.r_mode != GLOWQ_R_NONE && m.L && m.alpha != 0.f && m.alpha != 1.f);
-  }
-  if (use_tmem) {
+  if (route.tmem) {
     int sms = kPlanSms, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    unsigned char* ws = static_cast<unsigned char*>(g.workspace);
-    const bool room = g.workspace_bytes > scratch;
-    return gemm_tmem_forward(g, r_in_launch, any_corr, any_separate, status, reinterpret_cast<uint32_t*>(ws + kWsHeaderBytes),
-                             reinterpret_cast<uint32_t*>(ws + kWsTileCtrOffset), room ? cdiv(oc_sum, kTileRows) : 0,
-                             reinterpret_cast<float*>(ws + scratch), room ? g.workspace_bytes - scratch : 0, sms, stream, cuda_err);
+    return gemm_tmem_forward(g, route.r_in_launch, any_corr, any_separate, sms, stream, cuda_err);
   }
   // Tile shape: the 256 x 256 CTA tile has the best operand reuse, but a problem that fills the SMs badly in whole
   // waves is faster with narrower (nn = 1) or shorter (mt = 1) tiles.  A separate correction accumulator needs nn = 1.
@@ -1120,11 +1121,9 @@ int gemm_group_forward(const glowq_w4a16_group_t& g, cudaStream_t stream, cudaEr
     ksplit = main_ksplit(static_cast<int>(tiles), cdiv(g.IC, BK), std::min(sms, kPlanSms));
     if (env_ks > 0) ksplit = std::min(env_ks, std::max(1, cdiv(g.IC, BK) / 2));
     if (ksplit > 1) {
-      int oc_total = 0;
-      for (int i = 0; i < g.n_members; ++i) oc_total += g.members[i].OC;
       const size_t need = static_cast<size_t>(ksplit) * tiles * nn * slot_rows_for(g.M) * BN * 4;
       main_slot_off = g.workspace_bytes >= need ? ((g.workspace_bytes - need) & ~static_cast<size_t>(255)) : 0;
-      if (main_slot_off < counters_end(oc_total, g.n_members)) ksplit = 1;  // workspace not sized for slicing
+      if (main_slot_off < kWsSlotsOffset) ksplit = 1;  // workspace not sized for slicing
     }
     if (ksplit > 1) mt = 1;
   }
@@ -1176,11 +1175,9 @@ int gemm_group_forward(const glowq_w4a16_group_t& g, cudaStream_t stream, cudaEr
       const int waves = total / sms, rest = total % sms;
       if (waves >= 1 && rest > 0 && rest * 2 <= sms) {
         const int ks = std::min({8, kMaxTailSlots / rest, cdiv(g.IC, BK) / 8});
-        int oc_total = 0;
-        for (int i = 0; i < g.n_members; ++i) oc_total += g.members[i].OC;
         const size_t need = static_cast<size_t>(ks) * rest * nn * mt * BM * BN * 4;
         const size_t off = g.workspace_bytes >= need ? ((g.workspace_bytes - need) & ~static_cast<size_t>(255)) : 0;
-        if (ks >= 2 && off >= counters_end(oc_total, g.n_members)) {
+        if (ks >= 2 && off >= kWsSlotsOffset) {
           p.ksplit = ks;
           p.full_tiles = waves * sms;
           p.n_tail = rest;

@@ -635,37 +635,115 @@ size_t gemm_tmem_r_bytes(int M, int IC, int rank) {
   return static_cast<size_t>(cdiv(rank, kRows)) * r_slices_for(IC, rank) * tile_tokens(M) * kRows * 4;
 }
 
-// Members' products and corrections of a group call of up to 64 tokens.  compute_r: r into g.r_buf as well (else it is
-// there).  `slots` .. `slots + slot_bytes`: scratch for the slots of r (gemm_tmem_r_bytes must fit) and for K slices;
-// `tile_ctr`: n_ctr zeroed counters, `r_ctr`: kRpCtrWords of them.
-int gemm_tmem_forward(const glowq_w4a16_group_t& g, bool compute_r, bool any_corr, bool any_separate, uint32_t* status,
-                      uint32_t* r_ctr, uint32_t* tile_ctr, int n_ctr, float* slots, size_t slot_bytes, int sms, cudaStream_t stream, cudaError_t* cuda_err) {
-  const int G = cdiv(g.IC, kGroup);
-  TsParams p{};
-  p.N = tile_tokens(g.M);
+namespace {
+// Rings, CTAs of r and the partition into work items of a group call; no CUDA calls.
+struct TmemPlan {
+  int N, ns, np;               // tokens per tile, ring depths
+  int n_r, r_slices;           // CTAs of r, K slices of an R tile
+  int ksplit, full_tiles, n_tail;
+  size_t off_slots;            // in the workspace: K slices' slots (those of r are at kWsSlotsOffset)
+};
+TmemPlan make_tmem_plan(const glowq_w4a16_group_t& g, bool compute_r, bool any_corr, bool any_separate, int sms) {
+  TmemPlan pl{};
+  pl.N = tile_tokens(g.M);
   {
     // stages: what tensor memory leaves beside the accumulators (a correction with its own doubles them), as far as shared
     // memory holds them and a few packed tiles
-    const int smem = kSmemBytes - 2048 - kA16Slots * kA16, bst = p.N * 256;
-    p.ns = std::min({kMaxS, (kTmemCols - (any_separate ? 2 : 1) * p.N) / 64, (smem - 3 * kPStage) / bst});
-    p.np = std::min(kMaxP, (smem - p.ns * bst) / kPStage);
-    p.a_col = kTmemCols - p.ns * 64;
+    const int smem = kSmemBytes - 2048 - kA16Slots * kA16, bst = pl.N * 256;
+    pl.ns = std::min({kMaxS, (kTmemCols - (any_separate ? 2 : 1) * pl.N) / 64, (smem - 3 * kPStage) / bst});
+    pl.np = std::min(kMaxP, (smem - pl.ns * bst) / kPStage);
   }
+  pl.off_slots = kWsSlotsOffset;
   if (compute_r) {
-    p.r_slices = r_slices_for(g.IC, g.rank);
-    p.n_r = cdiv(g.rank, kRows) * p.r_slices;
+    pl.r_slices = r_slices_for(g.IC, g.rank);
+    pl.n_r = cdiv(g.rank, kRows) * pl.r_slices;
+    pl.off_slots += gemm_tmem_r_bytes(g.M, g.IC, g.rank);
+  }
+  const size_t slot_bytes = g.workspace_bytes > pl.off_slots ? g.workspace_bytes - pl.off_slots : 0;
+  int total = 0, nu = 0;
+  for (int i = 0; i < g.n_members; ++i) {
+    total += cdiv(g.members[i].OC, kRows);
+    if (any_corr && g.members[i].L && g.members[i].alpha != 0.f) nu = cdiv(g.rank, 64);
+  }
+  const int units = sms, resident = 2 * sms;
+  const size_t item_bytes = static_cast<size_t>(pl.N) * kRows * 4;
+  // Work partition: f rounds of whole tiles, the rest cut into ks slices of K.  Cost in microseconds, fitted on B200: an SM
+  // takes 0.33 per step while two CTAs share it (0.5 alone), 2.5 per wave of items for prologue and epilogue (the CTAs of r
+  // take slots, but are gone before a whole tile is done), and the slices of a tile are added through memory.  Measured at
+  // 16 tokens on the 13B shapes: q/k/v 30.2 whole, 22.8 in two slices, 30.5 in three; o_proj 24.8 whole, 19.1 / 15.8 /
+  // 15.5 in two / three / five, 19.1 in seven (a second wave behind the CTAs of r); gate/up 35.5 whole, 43.2 in two slices,
+  // 33.8 with one round whole and the other 68 tiles in two slices.
+  pl.full_tiles = total;
+  pl.n_tail = 0;
+  pl.ksplit = 1;
+  const int nk = cdiv(g.IC, kGroup) + nu;
+  double best = 1e30;
+  for (int f = 0; f <= total / units; ++f) {
+    const int full = f * units, tail = total - full;
+    for (int ks = 1; ks <= 16 && (ks == 1 || ks * 4 <= nk); ++ks) {
+      if (ks > 1 && (tail == 0 || tail > kTileCtrWords || static_cast<size_t>(tail) * ks * item_bytes > slot_bytes)) break;
+      const int items = full + tail * ks;
+      const double load = static_cast<double>(f) * nk + static_cast<double>(cdiv(tail * ks, units)) * nk / ks;
+      const double cost = load * (items > units ? 0.33 : 0.5) + 2.5 * cdiv(items, f > 0 ? resident : std::max(units, resident - pl.n_r)) +
+                          (ks > 1 ? 1.5 + 0.006 * pl.N * ks : 0.0);
+      if (cost < best) {
+        best = cost;
+        pl.ksplit = ks;
+        pl.full_tiles = ks > 1 ? full : total;
+        pl.n_tail = ks > 1 ? tail : 0;
+      }
+    }
+  }
+  return pl;
+}
+}  // namespace
+
+// (host arithmetic: see glowq_internal_workspace_map)
+void gemm_tmem_workspace_map(const glowq_w4a16_group_t& g, bool compute_r, bool any_corr, bool any_separate, int sms, WorkspaceMap* map) {
+  const TmemPlan pl = make_tmem_plan(g, compute_r, any_corr, any_separate, sms);
+  map->kernel = 1;
+  map->ksplit = pl.ksplit;
+  map->whole_tiles = pl.full_tiles;
+  map->sliced_tiles = pl.n_tail;
+  map->r_ctas = pl.n_r;
+  map->shortest = 1 << 30;
+  for (int i = 0; i < g.n_members; ++i) {
+    const bool corr = any_corr && g.members[i].L && g.members[i].alpha != 0.f;
+    map->shortest = std::min(map->shortest, cdiv(g.IC, kGroup) + (corr ? cdiv(g.rank, 64) : 0));
+  }
+  map->ctr_begin = kWsTileCtrOffset;
+  map->ctr_end = kWsTileCtrOffset + static_cast<size_t>(pl.n_tail) * 4;
+  map->slots_begin = kWsSlotsOffset;
+  map->slots_end = pl.off_slots + static_cast<size_t>(pl.n_tail) * pl.ksplit * pl.N * kRows * 4;
+}
+
+// Members' products and corrections of a group call of up to 64 tokens.  compute_r: r into g.r_buf as well (else it is
+// there); the workspace must hold gemm_tmem_r_bytes for it behind kWsSlotsOffset.
+int gemm_tmem_forward(const glowq_w4a16_group_t& g, bool compute_r, bool any_corr, bool any_separate, int sms, cudaStream_t stream,
+                      cudaError_t* cuda_err) {
+  const int G = cdiv(g.IC, kGroup);
+  const TmemPlan pl = make_tmem_plan(g, compute_r, any_corr, any_separate, sms);
+  unsigned char* const ws = static_cast<unsigned char*>(g.workspace);
+  TsParams p{};
+  p.N = pl.N;
+  p.ns = pl.ns;
+  p.np = pl.np;
+  p.a_col = kTmemCols - p.ns * 64;
+  if (compute_r) {
+    p.r_slices = pl.r_slices;
+    p.n_r = pl.n_r;
     p.nkr = cdiv(g.IC, 64);
     p.rank = g.rank;
     p.r_buf = static_cast<__half*>(g.r_buf);
-    p.r_ctr = r_ctr;
-    p.r_slots = slots;
-    const size_t r_bytes = gemm_tmem_r_bytes(g.M, g.IC, g.rank);
-    slots += r_bytes / 4;
-    slot_bytes -= r_bytes;
+    p.r_ctr = reinterpret_cast<uint32_t*>(ws + kWsHeaderBytes);
+    p.r_slots = reinterpret_cast<float*>(ws + kWsSlotsOffset);
   }
-  p.status = status;
-  p.tile_ctr = tile_ctr;
-  p.slots = slots;
+  p.status = reinterpret_cast<uint32_t*>(ws) + WS_STATUS;
+  p.tile_ctr = reinterpret_cast<uint32_t*>(ws + kWsTileCtrOffset);
+  p.slots = reinterpret_cast<float*>(ws + pl.off_slots);
+  p.ksplit = pl.ksplit;
+  p.full_tiles = pl.full_tiles;
+  p.n_tail = pl.n_tail;
   p.M = g.M;
   p.G = G;
   p.out_fp32 = g.out_dtype == GLOWQ_OUT_F32;
@@ -684,7 +762,7 @@ int gemm_tmem_forward(const glowq_w4a16_group_t& g, bool compute_r, bool any_cor
   if (any_corr && (rc = tensor_map_2d_ex(&tm.r, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, g.r_buf, g.rank, g.M,
                                          static_cast<uint64_t>(g.rank) * 2, 64, p.N, 1)))
     return rc;
-  int n_x = 0, nu = 0;
+  int n_x = 0;
   for (int i = 0; i < g.n_members; ++i) {
     const auto& m = g.members[i];
     const bool corr = any_corr && m.L && m.alpha != 0.f;
@@ -702,7 +780,6 @@ int gemm_tmem_forward(const glowq_w4a16_group_t& g, bool compute_r, bool any_cor
     d.out = m.out;
     d.OC = m.OC;
     d.nu = corr ? cdiv(g.rank, 64) : 0;
-    nu = std::max(nu, d.nu);
     d.sstride = m.scale_stride;
     d.zstride = m.zero_stride_i32;
     d.out_stride = m.out_stride;
@@ -712,35 +789,6 @@ int gemm_tmem_forward(const glowq_w4a16_group_t& g, bool compute_r, bool any_cor
     n_x += cdiv(m.OC, kRows);
   }
   p.n_x = n_x;
-  const int total = n_x, units = sms, resident = 2 * sms;
-  const size_t item_bytes = static_cast<size_t>(p.N) * kRows * 4;
-  // Work partition: f rounds of whole tiles, the rest cut into ks slices of K.  Cost in microseconds, fitted on B200: an SM
-  // takes 0.33 per step while two CTAs share it (0.5 alone), 2.5 per wave of items for prologue and epilogue (the CTAs of r
-  // take slots, but are gone before a whole tile is done), and the slices of a tile are added through memory.  Measured at
-  // 16 tokens on the 13B shapes: q/k/v 30.2 whole, 22.8 in two slices, 30.5 in three; o_proj 24.8 whole, 19.1 / 15.8 /
-  // 15.5 in two / three / five, 19.1 in seven (a second wave behind the CTAs of r); gate/up 35.5 whole, 43.2 in two slices,
-  // 33.8 with one round whole and the other 68 tiles in two slices.
-  p.full_tiles = total;
-  p.n_tail = 0;
-  p.ksplit = 1;
-  const int nk = G + nu;
-  double best = 1e30;
-  for (int f = 0; f <= total / units; ++f) {
-    const int full = f * units, tail = total - full;
-    for (int ks = 1; ks <= 16 && (ks == 1 || ks * 4 <= nk); ++ks) {
-      if (ks > 1 && (tail == 0 || tail > n_ctr || static_cast<size_t>(tail) * ks * item_bytes > slot_bytes)) break;
-      const int items = full + tail * ks;
-      const double load = static_cast<double>(f) * nk + static_cast<double>(cdiv(tail * ks, units)) * nk / ks;
-      const double cost = load * (items > units ? 0.33 : 0.5) + 2.5 * cdiv(items, f > 0 ? resident : std::max(units, resident - p.n_r)) +
-                          (ks > 1 ? 1.5 + 0.006 * p.N * ks : 0.0);
-      if (cost < best) {
-        best = cost;
-        p.ksplit = ks;
-        p.full_tiles = ks > 1 ? full : total;
-        p.n_tail = ks > 1 ? tail : 0;
-      }
-    }
-  }
   const cudaError_t e = launch(p, tm, p.n_r + p.full_tiles + p.n_tail * p.ksplit, stream);
   if (e != cudaSuccess) {
     *cuda_err = e;

@@ -50,15 +50,30 @@ constexpr uint32_t kEpochMask = (1u << 20) - 1u;
 constexpr size_t kWsHeaderBytes = WS_HEADER_WORDS * 4;
 constexpr int kMaxRTiles = 64;      // rank <= 1024
 // After the header: 1 KB of arrival counters for the stand-alone r product, then r of the running launch as the row tiles read it - 8-byte words
-// {half2(r[tok][2j], r[tok][2j+1]), launch epoch}, up to 8 tokens x rank 1024 - then the tile counters.  Launches of
-// the other kernels keep clear of everything up to the end of the tile counters.
+// {half2(r[tok][2j], r[tok][2j+1]), launch epoch}, up to 8 tokens x rank 1024 - then the tile counters.  All of this lies at
+// the same place whatever a call's sizes are, and every slot and partial buffer of every kernel lies behind it
+// (kWsSlotsOffset): launches of different widths that take turns on one workspace find each other's counters at zero.
 constexpr int kRpCtrWords = 256;    // arrival counters of the stand-alone r product (rank / 16 x token blocks of 64)
 constexpr size_t kWsRllOffset = kWsHeaderBytes + kRpCtrWords * 4;
 constexpr size_t kWsRllBytes = 8 * 1024 * 4;
 constexpr size_t kWsTileCtrOffset = kWsRllOffset + kWsRllBytes;
+// Arrival counters of K-sliced tiles.  No plan of its own slices more tiles than this (at most 2 x 148 on B200); a launch
+// that has to (slices on request, or rows too long for shared memory, and more than 32768 output rows) keeps its counters
+// among its slots and clears them first.
+constexpr int kTileCtrWords = 1024;
+constexpr size_t kWsSlotsOffset = kWsTileCtrOffset + kTileCtrWords * 4;
+static_assert(kWsSlotsOffset % 256 == 0, "slots start on a 256-byte boundary");
 constexpr int kMaxPrefetch = kMaxMembers + 1;
 constexpr int kMaxRanks = 8;        // GLOWQ_MAX_RANKS
 constexpr unsigned kPrefetchSlice = 16u << 10;  // bytes per L2 prefetch request
+
+// Byte ranges of the workspace that a launch uses besides the fixed areas in front of the tile counters, and its partition.
+struct WorkspaceMap {
+  int kernel;                       // 0 weight streaming, 1 tensor-memory GEMM, 2 shared-memory GEMM
+  int ksplit, whole_tiles, sliced_tiles, r_ctas, shortest;   // shortest: K steps of the member with the fewest
+  unsigned long long ctr_begin, ctr_end;       // tile counters, zero between launches
+  unsigned long long slots_begin, slots_end;   // partial results: any bits before and after a launch
+};
 
 struct MemberDev {
   const int32_t* qweight;
@@ -87,7 +102,7 @@ struct GemvParams {
   uint32_t* ws_head;      // header words
   float* r_partial;       // [n_r_tiles][SKr][NT*128] fp32 partial products of r, one slot per R unit
   uint2* r_ll;            // [M][rank/2] words {two fp16 elements of r, launch epoch}: written by the CTA that completes r
-  uint32_t* tile_ctr;     // [n_tiles] arrival counters of the split-K partial sums
+  uint32_t* tile_ctr;     // [n_tiles] arrival counters of the split-K partial sums (zero between launches)
   float* sk_partial;      // [n_tiles][SK][kRowTiles*NT*128]
   int M, IC, x_stride, R_stride, G, rank, r_mode, out_fp32, n_members;
   int n_tiles, SK, gps;          // main work: tiles x K slices, groups per slice (multiple of kChunkGroups)

@@ -199,7 +199,7 @@ int glowq_w4a16_group_forward_host(const glowq_w4a16_group_t* group, const void*
  * counters at zero when they finish and this entry point re-zeroes the counter area on `stream` before every
  * launch, but two calls that overlap on the GPU (different streams, no ordering between them) race on it.
  * No cudaMalloc / cudaFree or other allocating routine is called. */
-#define GLOWQ_W4A16_STATIC_SCRATCH_BYTES (4u << 20)
+#define GLOWQ_W4A16_STATIC_SCRATCH_BYTES ((4u << 20) + 4096u)
 int glowq_w4a16_gemv_forward_static(const void* x, const int32_t* qweight, const void* scales, const int32_t* qzeros,
                                     void* out, int M, int IC, int OC, int group_size, int weight_stride_i32,
                                     int zero_stride_i32, int scale_stride, void* stream);

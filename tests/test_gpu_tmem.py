@@ -71,3 +71,54 @@ def test_launches_back_to_back_on_one_workspace(M, ocs, ic, rank):
     for g, outs in groups[1:]:
         assert torch.equal(g._keep[4], groups[0][0]._keep[4])
         assert all(torch.equal(a, b) for a, b in zip(outs, groups[0][1]))
+
+
+def test_narrow_and_wide_launches_take_turns_on_one_workspace():
+    """Calls of different widths, token counts and ranks share a workspace (and w4a16_*_forward_cuda share one per device): each
+    gives the bits it gives on a workspace of its own, whatever the one before left in its slots, and the counters stay zero."""
+    rng = np.random.default_rng(17)
+    lins = {oc: Linear(rng, oc, 5120, rank=128, quantize=False) for oc in (512, 1024, 5120, 18944)}
+    down = Linear(rng, 3584, 18944, quantize=False)           # at one token: K slices of the weight-streaming kernel
+    x = {ic: dev(rng.standard_normal((64, ic)).astype(np.float16)) for ic in (5120, 18944)}
+    R_d = dev((rng.standard_normal((128, 5120)) * 0.01).astype(np.float16))
+
+    def call(oc, M, corrected, ws):
+        lin = lins.get(oc, down)
+        out = new_out(M, lin)
+        kw = dict(R_d=R_d, r_buf=torch.zeros(M, 128, dtype=torch.float16, device="cuda"), r_mode=K.R_COMPUTE) if corrected else {}
+        g = make_group(x[lin.ic][:M], [lin], [out], ws=ws, **kw)
+        assert run_group(g) == 0 and status_ok(g) == 0, (oc, M, corrected)
+        return out
+
+    calls = [(18944, 16, False), (512, 16, False), (18944, 16, False), (1024, 64, True), (18944, 64, False), (512, 16, False),
+             (3584, 1, False), (5120, 1, True), (18944, 16, True), (5120, 8, True), (5120, 33, True), (1024, 16, False), (3584, 1, False),
+             (18944, 64, True)]
+    nbytes = max(K.load_w4a16_extension().workspace_bytes(M, lins.get(oc, down).ic, oc, 128, 1) for oc, M, _ in calls)
+    fresh = lambda: torch.zeros(nbytes, dtype=torch.uint8, device="cuda")
+    want = {c: call(*c, fresh()) for c in set(calls)}
+    ws = fresh()
+    for c in calls:
+        assert torch.equal(call(*c, ws), want[c]), c
+        assert int(ws[256:1280].count_nonzero()) == 0 and int(ws[34048:38144].count_nonzero()) == 0, c
+    e = K.load_w4a16_extension()
+    for oc, M in ((18944, 16), (512, 16), (18944, 16), (3584, 1), (1024, 16), (18944, 16), (512, 16), (3584, 1)):
+        lin = lins.get(oc, down)
+        fn = e.w4a16_gemv_forward_cuda if M == 1 else e.w4a16_gemm_forward_cuda
+        y = fn(x[lin.ic][:M], lin.d_qweight, lin.d_scales, lin.d_qzeros, 128)
+        torch.testing.assert_close(y, want[oc, M, False], rtol=2e-3, atol=4e-3)   # (scratch of another size: other slices; an fp16 ulp)
+    assert e.lib.glowq_w4a16_read_status(e._ws["cuda", 0].data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+
+
+def test_more_sliced_tiles_than_the_workspace_has_counters():
+    """Slices on request of more than 1024 row tiles: the launch brings counters of its own and clears them, also where the call
+    before left partial sums."""
+    rng = np.random.default_rng(18)
+    lin = Linear(rng, 33024, 4096, quantize=False)
+    x = rng.standard_normal((2, 4096)).astype(np.float16)
+    ws = torch.full((64 << 20,), 255, dtype=torch.uint8, device="cuda")
+    ws[:38144] = 0
+    for _ in range(2):
+        out = new_out(2, lin)
+        g = make_group(dev(x), [lin], [out], split_k=4, ws=ws)
+        assert run_group(g) == 0 and status_ok(g) == 0
+        assert_close(out, lin.oracle(x))

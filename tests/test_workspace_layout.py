@@ -1,0 +1,78 @@
+"""Where launches keep their counters and partial results in a workspace that calls of all widths may share (no GPU: the
+planner of the library is host arithmetic)."""
+import ctypes
+import itertools
+
+import pytest
+
+from glowq_b200.cuda_w4a16 import kernels as K
+
+
+class Map(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_int) for n in ("kernel", "ksplit", "whole_tiles", "sliced_tiles", "r_ctas", "shortest")] + [
+        (n, ctypes.c_ulonglong) for n in ("ctr_begin", "ctr_end", "slots_begin", "slots_end")]
+
+
+def workspace_map(M, ic, ocs, rank=0, alphas=None, nbytes=1 << 28, kernel=K.KERNEL_AUTO, split_k=0, sms=148, rc=0):
+    """The map of a call; every address is a placeholder."""
+    at, g = 1 << 20, K.Group()
+    g.x, g.M, g.IC, g.x_stride, g.group_size = at, M, ic, ic, 128
+    g.kernel, g.split_k, g.n_members = kernel, split_k, len(ocs)
+    g.workspace, g.workspace_bytes = at, nbytes
+    if rank:
+        g.r_mode, g.rank, g.r_buf, g.R, g.R_stride = K.R_COMPUTE, rank, at, at, ic
+    groups = -(-ic // 128)
+    for i, oc in enumerate(ocs):
+        m = g.members[i]
+        m.qweight = m.scales = m.qzeros = m.out = at
+        m.OC = m.out_stride = oc
+        m.weight_stride_i32, m.scale_stride, m.zero_stride_i32 = groups * 16, groups, -(-groups // 8)
+        m.alpha = 1.0 if alphas is None else alphas[i]
+        if rank:
+            m.L, m.L_stride = at, rank
+    out = Map()
+    fn = K.load_w4a16_extension().lib.glowq_internal_workspace_map
+    fn.argtypes = [ctypes.POINTER(K.Group), ctypes.c_int, ctypes.POINTER(Map)]
+    assert fn(g, sms, out) == rc
+    return out
+
+
+WIDTHS = [[128], [512], [1024], [3584], [5120], [18944], [65536], [151936], [5120] * 3, [3072, 1024, 1024], [17408] * 2]
+
+
+def test_counters_of_any_call_lie_in_front_of_the_slots_of_every_other():
+    """A call leaves bits of partial sums in its slots and takes its counters to be zero, so no call's counters may lie where
+    another one keeps slots: narrow before wide, 9 to 64 tokens before one token, and the other way around."""
+    counters = slots = 0
+    for ocs, ic, M, rank in itertools.product(WIDTHS, (128, 2048, 5120, 18944), (1, 5, 8, 9, 16, 33, 64, 100, 300), (0, 64, 1024)):
+        for split_k in ((0, 4) if M <= 8 else (0,)):
+            m = workspace_map(M, ic, ocs, rank, split_k=split_k)
+            tag = (ocs, ic, M, rank, split_k)
+            assert m.slots_begin <= m.slots_end and m.slots_begin >= 38144, tag
+            if m.ctr_end > m.ctr_begin:
+                counters += 1
+                assert m.ctr_begin == 34048 and m.ctr_end <= 38144, tag
+            slots += m.slots_end > m.slots_begin
+    assert counters > 100 and slots > 500
+
+
+def test_a_launch_with_more_sliced_tiles_than_counters_brings_its_own():
+    """Slices on request and more than 32768 output rows: the counters lie among the slots (the launch clears them)."""
+    m = workspace_map(1, 4096, [32768], split_k=4)
+    assert m.ksplit == 4 and m.sliced_tiles == 1024 and (m.ctr_begin, m.ctr_end) == (34048, 38144)
+    m = workspace_map(1, 4096, [32800], split_k=4)
+    assert m.ksplit == 4 and m.sliced_tiles == 1025 and m.ctr_end == 0 and m.slots_begin == 38144
+    # the size grows with the rows whether or not K is sliced: 2^26 of them do not fit the scratch of 4 MiB + 4 KiB that is
+    # part of the library
+    workspace_map(1, 128, [1 << 26], nbytes=(4 << 20) + 4096, rc=4)
+    workspace_map(1, 128, [(1 << 25) - (1 << 15)], nbytes=(4 << 20) + 38144)
+
+
+@pytest.mark.parametrize("M,ic,oc,rank", [(16, 5120, 5120, 128), (64, 5120, 15360, 128), (1, 18944, 3584, 128), (33, 8192, 3072, 64)])
+def test_the_reported_size_holds_the_slices(M, ic, oc, rank):
+    """With exactly the bytes glowq_w4a16_workspace_bytes asks for, a launch takes the slices it takes with any amount."""
+    e = K.load_w4a16_extension()
+    exact = workspace_map(M, ic, [oc], rank, nbytes=e.workspace_bytes(M, ic, oc, rank, 1))
+    ample = workspace_map(M, ic, [oc], rank)
+    assert (exact.ksplit, exact.whole_tiles, exact.sliced_tiles) == (ample.ksplit, ample.whole_tiles, ample.sliced_tiles)
+    assert exact.ksplit > 1
