@@ -641,6 +641,7 @@ struct TmemPlan {
   int N, ns, np;               // tokens per tile, ring depths
   int n_r, r_slices;           // CTAs of r, K slices of an R tile
   int ksplit, full_tiles, n_tail;
+  int nk_min;                  // K steps of the shortest member
   size_t off_slots;            // in the workspace: K slices' slots (those of r are at kWsSlotsOffset)
 };
 TmemPlan make_tmem_plan(const glowq_w4a16_group_t& g, bool compute_r, bool any_corr, bool any_separate, int sms) {
@@ -660,11 +661,15 @@ TmemPlan make_tmem_plan(const glowq_w4a16_group_t& g, bool compute_r, bool any_c
     pl.off_slots += gemm_tmem_r_bytes(g.M, g.IC, g.rank);
   }
   const size_t slot_bytes = g.workspace_bytes > pl.off_slots ? g.workspace_bytes - pl.off_slots : 0;
-  int total = 0, nu = 0;
+  int total = 0, nk = 0, nk_min = 1 << 30;   // K steps of the longest and of the shortest member
   for (int i = 0; i < g.n_members; ++i) {
+    const bool corr = any_corr && g.members[i].L && g.members[i].alpha != 0.f;
+    const int steps = cdiv(g.IC, kGroup) + (corr ? cdiv(g.rank, 64) : 0);
     total += cdiv(g.members[i].OC, kRows);
-    if (any_corr && g.members[i].L && g.members[i].alpha != 0.f) nu = cdiv(g.rank, 64);
+    nk = std::max(nk, steps);
+    nk_min = std::min(nk_min, steps);
   }
+  pl.nk_min = nk_min;
   const int units = sms, resident = 2 * sms;
   const size_t item_bytes = static_cast<size_t>(pl.N) * kRows * 4;
   // Work partition: f rounds of whole tiles, the rest cut into ks slices of K.  Cost in microseconds, fitted on B200: an SM
@@ -676,11 +681,11 @@ TmemPlan make_tmem_plan(const glowq_w4a16_group_t& g, bool compute_r, bool any_c
   pl.full_tiles = total;
   pl.n_tail = 0;
   pl.ksplit = 1;
-  const int nk = cdiv(g.IC, kGroup) + nu;
   double best = 1e30;
   for (int f = 0; f <= total / units; ++f) {
     const int full = f * units, tail = total - full;
-    for (int ks = 1; ks <= 16 && (ks == 1 || ks * 4 <= nk); ++ks) {
+    // (a member is cut by its own steps: a slice without any would add what nothing wrote)
+    for (int ks = 1; ks <= std::min(16, nk_min) && (ks == 1 || ks * 4 <= nk); ++ks) {
       if (ks > 1 && (tail == 0 || tail > kTileCtrWords || static_cast<size_t>(tail) * ks * item_bytes > slot_bytes)) break;
       const int items = full + tail * ks;
       const double load = static_cast<double>(f) * nk + static_cast<double>(cdiv(tail * ks, units)) * nk / ks;
@@ -706,11 +711,7 @@ void gemm_tmem_workspace_map(const glowq_w4a16_group_t& g, bool compute_r, bool 
   map->whole_tiles = pl.full_tiles;
   map->sliced_tiles = pl.n_tail;
   map->r_ctas = pl.n_r;
-  map->shortest = 1 << 30;
-  for (int i = 0; i < g.n_members; ++i) {
-    const bool corr = any_corr && g.members[i].L && g.members[i].alpha != 0.f;
-    map->shortest = std::min(map->shortest, cdiv(g.IC, kGroup) + (corr ? cdiv(g.rank, 64) : 0));
-  }
+  map->shortest = pl.nk_min;
   map->ctr_begin = kWsTileCtrOffset;
   map->ctr_end = kWsTileCtrOffset + static_cast<size_t>(pl.n_tail) * 4;
   map->slots_begin = kWsSlotsOffset;

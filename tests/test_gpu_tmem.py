@@ -122,3 +122,25 @@ def test_more_sliced_tiles_than_the_workspace_has_counters():
         g = make_group(dev(x), [lin], [out], split_k=4, ws=ws)
         assert run_group(g) == 0 and status_ok(g) == 0
         assert_close(out, lin.oracle(x))
+
+
+@pytest.mark.parametrize("M,ocs,ic,rank,alpha,use_L", [
+    (16, [128, 128], 128, 448, [1.0, 0.0], None), (9, [200, 136], 256, 1024, [0.5, 1.0], [True, False]),
+    (64, [512, 96, 128], 5120, 128, [1.0, 0.5, 0.0], None), (33, [640, 640], 2048, 64, [1.0, 1.0], [False, True])])
+def test_corrected_and_uncorrected_members_in_one_launch(M, ocs, ic, rank, alpha, use_L):
+    """K slices of members with different numbers of steps: a member without a correction (alpha 0, no L) is the shortest, down
+    to one step beside sixteen of the correction; with and without a second accumulator.  Two passes on one workspace."""
+    rng = np.random.default_rng(M + rank)
+    lins = [Linear(rng, oc, ic, rank=rank, bias=True) for oc in ocs]
+    R = (rng.standard_normal((rank, ic)) * 0.01).astype(np.float16)
+    x = rng.standard_normal((M, ic)).astype(np.float16)
+    ws = None
+    for _ in range(2):
+        outs = [new_out(M, l, K.OUT_F32) for l in lins]
+        g = make_group(dev(x), lins, outs, R_d=dev(R), r_buf=torch.zeros(M, rank, dtype=torch.float16, device="cuda"), ws=ws,
+                       r_mode=K.R_COMPUTE, alpha=alpha, use_L=use_L, out_dtype=K.OUT_F32)
+        ws = g._keep[5]
+        assert run_group(g) == 0 and status_ok(g) == 0
+        for i, (l, o) in enumerate(zip(lins, outs)):
+            on = alpha[i] != 0 and (use_L is None or use_L[i])
+            assert_close(o, l.oracle(x, R if on else None, alpha=alpha[i]), tag=f"member {i}")

@@ -76,3 +76,13 @@ def test_the_reported_size_holds_the_slices(M, ic, oc, rank):
     ample = workspace_map(M, ic, [oc], rank)
     assert (exact.ksplit, exact.whole_tiles, exact.sliced_tiles) == (ample.ksplit, ample.whole_tiles, ample.sliced_tiles)
     assert exact.ksplit > 1
+
+
+@pytest.mark.parametrize("ic,rank", [(128, 448), (128, 1024), (256, 1024), (640, 1024), (5120, 256)])
+@pytest.mark.parametrize("M", [9, 16, 33, 64])
+def test_no_slice_of_a_group_of_unlike_members_is_empty(M, ic, rank):
+    """Each member is cut by its own K steps: the one without a correction has the fewest, and no more slices than that."""
+    for ocs in ([128, 128], [1024, 1024], [5120, 5120, 5120], [128, 8192]):
+        for alphas in ([1.0, 0.0, 0.5], [0.0, 1.0, 1.0], [0.5, 0.0, 0.0]):
+            m = workspace_map(M, ic, ocs, rank, alphas=alphas[:len(ocs)])
+            assert m.kernel == 1 and m.shortest == -(-ic // 128) and m.ksplit <= m.shortest, (ocs, alphas, m.ksplit)
