@@ -58,6 +58,7 @@ constexpr int kMaxRCtas = 48;                 // CTAs that compute r
 // Polls of a count of finished CTAs: seconds, because another stream's kernel may hold the SMs that the rest of the CTAs
 // of r need (they are placed first, so that nothing of this launch does).
 constexpr unsigned kCountSpin = 1u << 22;
+constexpr unsigned kDrainSpin = 1u << 18;     // polls (tens of milliseconds) for one of this CTA's own copies or MMAs
 enum : int { kRCnt = 0, kRFlag = 64, kRExit = 65 };   // words of the r counters: arrivals per R tile, finished CTAs, exits
 
 struct TsMember {
@@ -244,18 +245,11 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const uint32_t tmem = s_tmem_base;
   volatile int* abort_flag = &s_abort;
-  auto drain = [&](uint32_t bars, int depth, int issued) {   // after a failed wait: let copies in flight land (bounded)
-    for (int j = (issued > depth ? issued - depth : 0); j < issued; ++j) {
-      uint32_t spins = 0;
-      while (!g_mbar_try_once(bars + 8 * (j % depth), (j / depth) & 1) && ++spins < kGemmSpin) {
-      }
-    }
-  };
+  int issued = 0, cissued = 0;   // copies of this thread, should they have to be waited for at the end
 
   if (warp == 0) {
     if (lane == 0) {
       Ring b{0, 0}, c{0, 0}, ca{0, 0};
-      int issued = 0, cissued = 0;
       bool ok = true;
       const CUtensorMap* const tb = r_cta ? &tm.x : &tm.r;
       const CUtensorMap* const ta = r_cta ? &tm.R : &tm.l[mi];
@@ -303,25 +297,18 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
         c.step(1, cdepth);
         b.step(1, p.ns);
       }
-      if (!ok || *abort_flag != 0) {
-        drain(full, p.ns, issued);
-        drain(cfull, cdepth, cissued);
-      }
     }
     __syncwarp();
   } else if (warp == 2) {
     if (lane == 0) {
       Ring s{0, 0};
-      int issued = 0;
-      bool ok = true;
       for (int it = it0; it < nkp; ++it) {
-        if (!(ok = g_mbar_wait(pempty + 8 * s.i, s.ph ^ 1, abort_flag, p.status) && *abort_flag == 0)) break;
+        if (!g_mbar_wait(pempty + 8 * s.i, s.ph ^ 1, abort_flag, p.status) || *abort_flag != 0) break;
         g_mbar_expect_tx(pfull + 8 * s.i, kPStage);
         g_tma_2d(pring + s.i * kPStage, &tm.w[mi], it * 16, n0, pfull + 8 * s.i);
         ++issued;
         s.step(1, p.np);
       }
-      if (!ok || *abort_flag != 0) drain(pfull, p.np, issued);
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -580,6 +567,25 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
 
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (s_abort != 0) {
+    // A wait of this CTA has run out, so copies may not have been consumed and accumulators not read: the thread that issued
+    // them lets its copies land, and its MMAs (which go on without waiting) and their commits finish, before another CTA
+    // gets the shared and tensor memory.  Bounded as well: a step that was announced and never issued does not complete.
+    auto drain = [&](uint32_t bars, int depth, int n) {
+      for (int j = max(n - depth, 0); j < n; ++j)
+        for (uint32_t spins = 0; spins < kDrainSpin && !test_bar(bars + 8 * (j % depth), (j / depth) & 1); ++spins) {
+        }
+    };
+    if (warp == 0 && lane == 0) {
+      drain(full, p.ns, issued);
+      drain(cfull, cdepth, cissued);
+    } else if (warp == 1 && lane == 0) {
+      drain(accum, 1, 1);
+    } else if (warp == 2 && lane == 0) {
+      drain(pfull, p.np, issued);
+    }
+    __syncthreads();
+  }
   if (p.n_r > 0 && threadIdx.x == 0) {   // the last CTA leaves the counters of r at zero
     if (atomicAdd(p.r_ctr + kRExit, 1u) == gridDim.x - 1) {
       for (int i = 0; i * p.r_slices < p.n_r; ++i) p.r_ctr[kRCnt + i] = 0u;

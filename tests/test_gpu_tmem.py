@@ -144,3 +144,21 @@ def test_corrected_and_uncorrected_members_in_one_launch(M, ocs, ic, rank, alpha
         for i, (l, o) in enumerate(zip(lins, outs)):
             on = alpha[i] != 0 and (use_L is None or use_L[i])
             assert_close(o, l.oracle(x, R if on else None, alpha=alpha[i]), tag=f"member {i}")
+
+
+def test_a_wait_that_runs_out_is_reported_and_leaves_the_device_usable():
+    """The count of finished parts of r starts at a value it cannot reach: the CTAs that wait for r give up, let what they have
+    in flight finish and return; the status word says so, and launches on another workspace are right."""
+    rng = np.random.default_rng(21)
+    lin = Linear(rng, 2048, 2048, rank=64)
+    R = (rng.standard_normal((64, 2048)) * 0.01).astype(np.float16)
+    x = rng.standard_normal((16, 2048)).astype(np.float16)
+    kw = dict(R_d=dev(R), r_mode=K.R_COMPUTE)
+    g = make_group(dev(x), [lin], [new_out(16, lin)], r_buf=torch.zeros(16, 64, dtype=torch.float16, device="cuda"), **kw)
+    g._keep[5][256:1280].view(torch.int32)[64] = 1 << 20
+    assert run_group(g) == 0                      # (the stream runs to its end)
+    assert status_ok(g) == 7 and status_ok(g) == 0
+    out = new_out(16, lin)
+    g = make_group(dev(x), [lin], [out], r_buf=torch.zeros(16, 64, dtype=torch.float16, device="cuda"), **kw)
+    assert run_group(g) == 0 and status_ok(g) == 0
+    assert_close(out, lin.oracle(x, R))
