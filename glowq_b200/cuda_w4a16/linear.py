@@ -65,14 +65,26 @@ def _unpack_int4_i32(packed_i32: torch.Tensor, total_vals: int) -> torch.Tensor:
     return torch.stack(cols, dim=-1).reshape(p.size(0), -1)[:, :total_vals].contiguous()
 
 
+def _device_quantises(device: torch.device) -> bool:
+    """The library's kernels run on compute capability 10.0 alone (sm_100a code).  Converting a model needs no library: where
+    it is missing or of another version, the forward call says so and the quantiser is the torch expression."""
+    if torch.cuda.get_device_capability(device) != (10, 0):
+        return False
+    try:
+        load_w4a16_extension()
+    except RuntimeError:
+        return False
+    return True
+
+
 def _kernel_quantises(weight: torch.Tensor, group_size: int) -> bool:
     """The one-launch quantiser takes what a conversion hands over: a plain fp16 matrix on an sm_100 device in groups of
-    128.  Everything else (CPU tensors, other types, group sizes and devices) is the torch expression, the same bits.
+    128.  Everything else (CPU tensors, other types, group sizes and devices, no library) is the torch expression, the same bits.
     Measured for the seven linears of a Llama-2-13B layer: 29.1 ms with the torch expression and the buffers of the
     module made on the host, 1.0 ms with this launch (0.32 ms on the GPU, the rest builds the modules)."""
     return (group_size == 128 and weight.is_cuda and weight.dtype == torch.float16 and type(weight) is torch.Tensor
             and not weight.requires_grad and weight.numel() > 0 and weight.stride(1) == 1
-            and weight.stride(0) >= weight.shape[1] and torch.cuda.get_device_capability(weight.device)[0] == 10)
+            and weight.stride(0) >= weight.shape[1] and _device_quantises(weight.device))
 
 
 def _quantize_per_group_w4(weight: torch.Tensor, group_size: int):

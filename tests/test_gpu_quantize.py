@@ -56,3 +56,16 @@ def test_from_float_keeps_everything_on_the_weights_device():
     assert {t.device.type for t in list(mod.buffers()) + list(mod.parameters())} == {"cuda"}
     assert mod.qweight_i32.shape == (24, 32) and mod.gid.shape == (200,) and torch.equal(mod.bias.data, lin.bias.data)
     assert set(mod.state_dict()) == {"qweight_i32", "qzeros_i32", "scales_f16", "bias"}
+
+
+def test_from_float_without_a_library(monkeypatch):
+    lin = torch.nn.Linear(300, 40, bias=False, device="cuda", dtype=torch.float16)
+    want = L.CudaW4A16Linear.from_float(lin, 128)
+
+    def missing():
+        raise RuntimeError("failed to load libglowq_w4a16.so")
+
+    monkeypatch.setattr(L, "load_w4a16_extension", missing)
+    got = L.CudaW4A16Linear.from_float(lin, 128)
+    for name, t in want.state_dict().items():
+        assert torch.equal(got.state_dict()[name], t), name

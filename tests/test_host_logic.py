@@ -67,6 +67,21 @@ def test_module_surface_and_state_dict():
         mod(torch.zeros(1, 100, dtype=torch.float16))
 
 
+def test_conversion_needs_no_library(monkeypatch):
+    """The one-launch quantiser is for capability 10.0 and a library that loads; anything else converts with the torch
+    expression instead of raising (which convert_to_cuda_w4a16 would turn into an fp16 layer)."""
+    from glowq_b200.cuda_w4a16 import linear as L
+
+    def missing():
+        raise RuntimeError("failed to load libglowq_w4a16.so")
+
+    for capability, load, want in (((10, 0), K.load_w4a16_extension, True), ((10, 0), missing, False),
+                                   ((10, 3), K.load_w4a16_extension, False), ((9, 0), missing, False)):
+        monkeypatch.setattr(torch.cuda, "get_device_capability", lambda *_: capability)
+        monkeypatch.setattr(L, "load_w4a16_extension", load)
+        assert L._device_quantises(torch.device("cuda")) is want
+
+
 def _describe(model):
     rows, caches = {}, {}
     for name, mod in model.named_modules():
