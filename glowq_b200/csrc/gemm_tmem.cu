@@ -245,11 +245,20 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const uint32_t tmem = s_tmem_base;
   volatile int* abort_flag = &s_abort;
-  int issued = 0, cissued = 0;   // copies of this thread, should they have to be waited for at the end
+  // A thread that issues copies or MMAs stays until the last of them are done, also when a wait of the CTA has run out and
+  // nobody else waits for them any more.  (Bounded: a step that was announced and never issued does not complete.)
+  auto drain = [&](uint32_t bars, int depth, int issued) {
+    for (int j = (issued > depth ? issued - depth : 0); j < issued; ++j) {
+      uint32_t spins = 0;
+      while (!g_mbar_try_once(bars + 8 * (j % depth), (j / depth) & 1) && ++spins < kDrainSpin) {
+      }
+    }
+  };
 
   if (warp == 0) {
     if (lane == 0) {
       Ring b{0, 0}, c{0, 0}, ca{0, 0};
+      int issued = 0, cissued = 0;
       bool ok = true;
       const CUtensorMap* const tb = r_cta ? &tm.x : &tm.r;
       const CUtensorMap* const ta = r_cta ? &tm.R : &tm.l[mi];
@@ -297,11 +306,14 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
         c.step(1, cdepth);
         b.step(1, p.ns);
       }
+      drain(full, p.ns, issued);
+      drain(cfull, cdepth, cissued);
     }
     __syncwarp();
   } else if (warp == 2) {
     if (lane == 0) {
       Ring s{0, 0};
+      int issued = 0;
       for (int it = it0; it < nkp; ++it) {
         if (!g_mbar_wait(pempty + 8 * s.i, s.ph ^ 1, abort_flag, p.status) || *abort_flag != 0) break;
         g_mbar_expect_tx(pfull + 8 * s.i, kPStage);
@@ -309,6 +321,7 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
         ++issued;
         s.step(1, p.np);
       }
+      drain(pfull, p.np, issued);
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -355,6 +368,7 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
         b.step(1, p.ns);
       }
       umma_commit_elect(accum);
+      if (lane == 0) drain(accum, 1, 1);
     }
     __syncwarp();
   } else {
@@ -567,25 +581,6 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
 
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (s_abort != 0) {
-    // A wait of this CTA has run out, so copies may not have been consumed and accumulators not read: the thread that issued
-    // them lets its copies land, and its MMAs (which go on without waiting) and their commits finish, before another CTA
-    // gets the shared and tensor memory.  Bounded as well: a step that was announced and never issued does not complete.
-    auto drain = [&](uint32_t bars, int depth, int n) {
-      for (int j = max(n - depth, 0); j < n; ++j)
-        for (uint32_t spins = 0; spins < kDrainSpin && !test_bar(bars + 8 * (j % depth), (j / depth) & 1); ++spins) {
-        }
-    };
-    if (warp == 0 && lane == 0) {
-      drain(full, p.ns, issued);
-      drain(cfull, cdepth, cissued);
-    } else if (warp == 1 && lane == 0) {
-      drain(accum, 1, 1);
-    } else if (warp == 2 && lane == 0) {
-      drain(pfull, p.np, issued);
-    }
-    __syncthreads();
-  }
   if (p.n_r > 0 && threadIdx.x == 0) {   // the last CTA leaves the counters of r at zero
     if (atomicAdd(p.r_ctr + kRExit, 1u) == gridDim.x - 1) {
       for (int i = 0; i * p.r_slices < p.n_r; ++i) p.r_ctr[kRCnt + i] = 0u;
