@@ -18,12 +18,14 @@
 // Two CTAs share an SM (256 tensor-memory columns and two teams each), so that one CTA's prologue and epilogue hide behind
 // the other's steps.
 //   r = X . R^T is computed inside the launch by the lowest block indices (placed first): a CTA multiplies 128 rows of R with a
-// slice of K - the correction steps' loop with R in the place of L and X in the place of r - parks an fp32 slot, and the CTAs
-// of an R tile, once all have arrived, add each a share of its elements in a fixed order, round to fp16 and write r_buf.  The
-// activation producers poll the count of finished CTAs before their first correction step.  As a launch of its own in front,
-// r cost 6 to 11 microseconds per group.
+// slice of K - the correction steps' loop with R in the place of L and X in the place of r - and parks an fp32 slot; once all
+// slices of an R tile have arrived, its CTAs add each a share of its elements (one also the shares of those that left early) in a
+// fixed order, round to fp16 and write r_buf.  The activation producers poll the count of finished shares before their first
+// correction step.  As a launch of its own in front, r cost 6 to 11 microseconds per group.
 // K may be sliced over CTAs; the CTA of a tile's last slice adds the others' fp32 slots in slice order (deterministic).
-// Every wait is bounded; on expiry a status word is set and the CTA drains and frees its tensor memory.
+// A CTA waits for CTAs with lower block indices only (r, the earlier slices of its tile), which are placed before it: a launch
+// gets through on any number of SMs.  Every wait is bounded; on expiry a status word is set, and the CTA drains and frees its
+// tensor memory.
 //
 // Measured (B200, corrected group calls of the 13B shapes, microseconds at 16 / 32 / 64 tokens; before: weights through
 // shared memory, r and slot sum as launches of their own): q/k/v 38.7 / 39.4 / 44.5 -> 23.6 / 24.3 / 28.7, o_proj 22.2 /
@@ -59,7 +61,13 @@ constexpr int kMaxRCtas = 48;                 // CTAs that compute r
 // of r need (they are placed first, so that nothing of this launch does).
 constexpr unsigned kCountSpin = 1u << 22;
 constexpr unsigned kDrainSpin = 1u << 18;     // polls (tens of milliseconds) for one of this CTA's own copies or MMAs
-enum : int { kRCnt = 0, kRFlag = 64, kRExit = 65 };   // words of the r counters: arrivals per R tile, finished CTAs, exits
+// Polls (some tens of microseconds) that a CTA of r spends on the others' arrival before it leaves the adding to them.
+constexpr unsigned kShareSpin = 64;
+// Words of the counters of r: per R tile 64 bits, of which 0..15 count the K slices that have arrived and 16 + z says that the CTA
+// of slice z left before all had; then finished shares and exits.
+enum : int { kRCnt = 0, kRFlag = 64, kRExit = 65 };
+constexpr unsigned kArrivals = 0xFFFFu;
+static_assert(kMaxRCtas <= 48 && kMaxRTiles * kRTileRows / kRows * 2 <= kRFlag, "the words of an R tile's count");
 
 struct TsMember {
   const __half* scales;
@@ -167,10 +175,57 @@ struct Ring {
   }
 };
 
+// One share of the sum over an R tile's slots: four lanes per four elements, each a quarter of the slots (up to 12 loads in
+// flight), added in a fixed order.
+struct ShareArgs {
+  const float* base;
+  __half* r_buf;
+  size_t slot_floats;
+  int r_slices, rank, n0, units;
+};
+__device__ __forceinline__ void add_share(const ShareArgs& a, int share, int et) {
+  const int quarter = (a.r_slices + 3) >> 2, zq = (et & 3) * quarter, stride = a.r_slices * (kDequantWarps * 8);
+  for (int i0 = 0; i0 < a.units; i0 += stride) {   // (the same number of rounds for all lanes: they exchange sums)
+    const int i = i0 + share * (kDequantWarps * 8) + (et >> 2);
+    const int tok = i >> 5, c4 = (i & 31) * 4, col = a.n0 + c4;
+    const float* src = a.base + static_cast<size_t>(tok) * kRows + c4;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f), u[kMaxRCtas / 4];
+#pragma unroll
+    for (int z = 0; z < kMaxRCtas / 4; ++z)
+      u[z] = (i < a.units && z < quarter && zq + z < a.r_slices) ? __ldcg(reinterpret_cast<const float4*>(src + (zq + z) * a.slot_floats))
+                                                                 : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int z = 0; z < kMaxRCtas / 4; ++z) {
+      s.x += u[z].x;
+      s.y += u[z].y;
+      s.z += u[z].z;
+      s.w += u[z].w;
+    }
+#pragma unroll
+    for (int o = 1; o <= 2; o <<= 1) {
+      s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+      s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+      s.z += __shfl_xor_sync(0xffffffffu, s.z, o);
+      s.w += __shfl_xor_sync(0xffffffffu, s.w, o);
+    }
+    if ((et & 3) == 0 && i < a.units && col < a.rank) {   // the rank is a multiple of 8
+      const __half2 lo = __floats2half2_rn(s.x, s.y), hi = __floats2half2_rn(s.z, s.w);
+      *reinterpret_cast<uint2*>(a.r_buf + static_cast<size_t>(tok) * a.rank + col) =
+          make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    }
+  }
+}
+// The shares of the CTAs in `left`, which could not wait.  Rare, and out of line: with this loop in the kernel the code that the
+// compiler makes of the main loop is slower (the half-corrected Qwen2.5-7B step at 64 tokens: 548 us so, 514 with the call).
+__device__ __noinline__ void add_shares(ShareArgs a, unsigned long long left, int et) {
+  for (; left != 0; left &= left - 1) add_share(a, __ffsll(left) - 1, et);
+}
+
 __global__ void __launch_bounds__(kThreads, 2)
 gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsMaps tm) {
   extern __shared__ unsigned char smem[];
   __shared__ int s_abort;
+  __shared__ unsigned long long s_word;
   __shared__ uint32_t s_tmem_base;
   const uint32_t smem0 = (sm_u32(smem) + 1023u) & ~1023u;
   // barriers in the first 1 KB.  full: a stage's A tile is in tensor memory and its activations have landed (ONE barrier
@@ -527,53 +582,41 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
     if (park) {
       epi_sync();
       const int rt = n0 / kRows;
-      uint32_t* const ctr = r_cta ? p.r_ctr + kRCnt + rt : p.tile_ctr + sl_tile;
       if (et == 0) {
         __threadfence();   // (cumulative over the CTA's stores, which the barrier ordered before it)
-        atomicAdd(ctr, 1u);
+        if (!r_cta) atomicAdd(p.tile_ctr + sl_tile, 1u);
       }
       if (r_cta) {
-        // once all K slices of this R tile have arrived, every CTA adds its share of the elements: four lanes per four
-        // elements, each a quarter of the slots (up to 12 loads in flight), added in a fixed order
-        if (et == 0) await_count(ctr, static_cast<uint32_t>(p.r_slices));
+        // Once all K slices of this R tile have arrived, every CTA adds its share of the elements.  No CTA depends on another
+        // one being resident: it polls for a little while and then leaves, which the word of the count records unless all have
+        // arrived by then.  Once they have, the word no longer changes, and the first of the CTAs that stayed - the last to
+        // arrive always does - adds the shares of those that left.
+        const ShareArgs sa{p.r_slots + static_cast<size_t>(rt) * p.r_slices * slot_floats, p.r_buf, slot_floats, p.r_slices, p.rank,
+                           n0, ntok * (kRows / 4)};
+        if (et == 0) {
+          unsigned long long* const ctr = reinterpret_cast<unsigned long long*>(p.r_ctr + kRCnt) + rt;
+          atomicAdd(ctr, 1ull);
+          unsigned long long v;
+          for (unsigned spins = 0; ((v = ld_acquire_u64(ctr)) & kArrivals) != static_cast<unsigned>(p.r_slices); ++spins)
+            if (spins >= kShareSpin && atomicCAS(ctr, v, v | 1ull << (16 + zslice)) == v) break;
+          s_word = v;
+        }
         epi_sync();
-        const float* base = p.r_slots + static_cast<size_t>(rt) * p.r_slices * slot_floats;
-        const int quarter = (p.r_slices + 3) >> 2, zq = (et & 3) * quarter;
-        const int units = ntok * (kRows / 4), stride = p.r_slices * (kDequantWarps * 8);
-        for (int i0 = 0; i0 < units; i0 += stride) {   // (the same number of rounds for all lanes: they exchange sums)
-          const int i = i0 + zslice * (kDequantWarps * 8) + (et >> 2);
-          const int tok = i >> 5, c4 = (i & 31) * 4, col = n0 + c4;
-          const float* src = base + static_cast<size_t>(tok) * kRows + c4;
-          float4 s = make_float4(0.f, 0.f, 0.f, 0.f), u[kMaxRCtas / 4];
-#pragma unroll
-          for (int z = 0; z < kMaxRCtas / 4; ++z)
-            u[z] = (i < units && z < quarter && zq + z < p.r_slices) ? __ldcg(reinterpret_cast<const float4*>(src + (zq + z) * slot_floats))
-                                                                     : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-          for (int z = 0; z < kMaxRCtas / 4; ++z) {
-            s.x += u[z].x;
-            s.y += u[z].y;
-            s.z += u[z].z;
-            s.w += u[z].w;
-          }
-#pragma unroll
-          for (int o = 1; o <= 2; o <<= 1) {
-            s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
-            s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
-            s.z += __shfl_xor_sync(0xffffffffu, s.z, o);
-            s.w += __shfl_xor_sync(0xffffffffu, s.w, o);
-          }
-          if ((et & 3) == 0 && i < units && col < p.rank) {   // the rank is a multiple of 8
-            const __half2 a = __floats2half2_rn(s.x, s.y), b = __floats2half2_rn(s.z, s.w);
-            *reinterpret_cast<uint2*>(p.r_buf + static_cast<size_t>(tok) * p.rank + col) =
-                make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+        const bool stayed = (s_word & kArrivals) == static_cast<unsigned>(p.r_slices);
+        int done = 0;
+        if (stayed) {
+          add_share(sa, zslice, et);
+          done = 1;
+          if (unsigned long long left = s_word >> 16; left != 0 && zslice == __ffsll(~left) - 1) {
+            add_shares(sa, left, et);
+            done += __popcll(left);
           }
         }
         asm volatile("fence.proxy.async;" ::: "memory");   // read by other CTAs' copies
         epi_sync();
-        if (et == 0) {
+        if (et == 0 && done != 0) {
           __threadfence();
-          atomicAdd(p.r_ctr + kRFlag, 1u);
+          atomicAdd(p.r_ctr + kRFlag, static_cast<unsigned>(done));
         }
       }
     }
@@ -583,7 +626,7 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
   __syncthreads();
   if (p.n_r > 0 && threadIdx.x == 0) {   // the last CTA leaves the counters of r at zero
     if (atomicAdd(p.r_ctr + kRExit, 1u) == gridDim.x - 1) {
-      for (int i = 0; i * p.r_slices < p.n_r; ++i) p.r_ctr[kRCnt + i] = 0u;
+      for (int i = 0; i * p.r_slices < p.n_r; ++i) reinterpret_cast<unsigned long long*>(p.r_ctr + kRCnt)[i] = 0u;
       p.r_ctr[kRFlag] = 0u;
       p.r_ctr[kRExit] = 0u;
     }

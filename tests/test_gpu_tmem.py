@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from glowq_b200.cuda_w4a16 import kernels as K
-from gpu_helpers import Linear, assert_close, dev, make_group, new_out, run_group, status_ok
+from gpu_helpers import Linear, assert_close, dev, ext, make_group, new_out, run_group, status_ok
 
 pytestmark = pytest.mark.gpu
 
@@ -162,3 +162,34 @@ def test_a_wait_that_runs_out_is_reported_and_leaves_the_device_usable():
     g = make_group(dev(x), [lin], [out], r_buf=torch.zeros(16, 64, dtype=torch.float16, device="cuda"), **kw)
     assert run_group(g) == 0 and status_ok(g) == 0
     assert_close(out, lin.oracle(x, R))
+
+
+def test_r_on_fewer_SMs_than_its_CTAs_need():
+    """A stream of 8 SMs holds 16 CTAs of the launch, of which 20 compute r (and a second R tile's 20 more): none of them may
+    wait for another one to be resident.  The same bits as on the whole device."""
+    green = pytest.importorskip("torch.cuda.green_contexts")
+    if not green.SUPPORTED:
+        pytest.skip("PyTorch without green contexts")
+    rng = np.random.default_rng(23)
+    for rank, M in ((128, 16), (256, 50)):
+        lin = Linear(rng, 2048, 5120, rank=rank, quantize=False)
+        x_d, R_d = dev(rng.standard_normal((M, 5120)).astype(np.float16)), dev((rng.standard_normal((rank, 5120)) * 0.01).astype(np.float16))
+        outs = [new_out(M, lin) for _ in range(2)]
+        rs = [torch.zeros(M, rank, dtype=torch.float16, device="cuda") for _ in range(2)]
+        ctx = green.GreenContext.create(8, 0)
+        few = ctx.Stream()
+        for i in range(2):
+            torch.cuda.synchronize()
+            g = make_group(x_d, [lin], [outs[i]], R_d=R_d, r_buf=rs[i], r_mode=K.R_COMPUTE)
+            torch.cuda.synchronize()
+            if i == 1:
+                g.stream = few.cuda_stream
+                ctx.set_context()
+            try:
+                rc = run_group(g)
+                assert rc == 0 and status_ok(g) == 0, (i, rc, ext().lib.glowq_w4a16_last_cuda_error())
+            finally:
+                if i == 1:
+                    ctx.pop_context()
+        assert_close(outs[0], lin.oracle(x_d.cpu().numpy(), R_d.cpu().numpy()))
+        assert torch.equal(outs[0], outs[1]) and torch.equal(rs[0], rs[1])
