@@ -346,9 +346,11 @@ int n_tiles_of(const glowq_w4a16_group_t& g) {
   return n;
 }
 
-// Measured on B200: up to 8 tokens fit one streaming launch (one MMA N tile); 9..16 tokens would take two, and at
-// 16 tokens the tcgen05 GEMM (K-sliced over all SMs when it has few tiles) is ahead on every Llama-2-13B shape
-// (q/k/v 44 vs 47 us, gate/up 65 vs 70, down_proj 43 vs 64, o_proj 26 vs 33, corrected), so it takes over from 9.
+// Up to 8 tokens fit one streaming launch (one MMA N tile), which multiplies the exact integer codes and applies the scales in
+// fp32; the tensor-core kernels round the scaled weights to fp16 first, as the reference does.  So 8 tokens stay here although
+// the tensor-memory kernel is ahead in time by then (a corrected Qwen3-14B layer: 129 us at 8 tokens here, 112 at 16 there).
+// 9 to 16 tokens would take two streaming launches: 47 / 70 / 64 / 33 us for q/k/v, gate/up, down_proj and o_proj of the
+// Llama-2-13B shapes at 16 tokens, corrected, against 23.6 / 36.7 / 22.8 / 15.5.
 bool takes_gemm(const glowq_w4a16_group_t& g) {
   const bool use_gemm = g.kernel == GLOWQ_KERNEL_GEMM || (g.kernel == GLOWQ_KERNEL_AUTO && g.M > kGemvAutoMaxM);
   return use_gemm && gemm_supported(g);

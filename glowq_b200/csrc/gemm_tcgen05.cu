@@ -107,9 +107,8 @@ struct GemmParams {
   // split-K (only the narrow r = X . R^T product uses it): gridDim.z CTAs share a tile's K steps, each writes its fp32
   // partial tile to its own slot; slot_sum_kernel then adds the slots in slice order
   int ksplit;
-  // swap: up to 128 tokens.  The dequantised weight tile becomes the M side of the MMA (A operand, 128 output columns
-  // per accumulator) and the activation tile its N side (nt = 32, 64 or 128 token rows, B operand): the activation
-  // tile written and re-read per K step shrinks from 128 rows to nt, which is what bounds small token counts.
+  // swap: 65 to 128 tokens.  The dequantised weight tile becomes the M side of the MMA (A operand, 128 output columns
+  // per accumulator) and the activation tile its N side (nt = 128 token rows, B operand).
   int swap, nt;
   int debug;         // used by the clock trace of -DGLOWQ_GEMM_TRACE builds only (bit 2048, bit 4096 = trace CTA 1)
   // Work items (blockIdx.x, single-CTA kernels): tiles [0, full_tiles) are computed whole; each of the n_tail tiles
@@ -852,8 +851,8 @@ inline size_t r_slot_bytes(int M, int IC, int rank) {
 }
 // The slots of the kernels of this file sit at the end of the workspace, behind kWsSlotsOffset.
 
-// K slices of a group GEMM with few tiles (up to 128 tokens): planned for 148 SMs so that the workspace size does not
-// depend on the device.
+// K slices of a group GEMM with few tiles (65 to 256 tokens; the size is asked for from 9 tokens on, where the tensor-memory form
+// uses the room for its own slices): planned for 148 SMs so that the workspace size does not depend on the device.
 constexpr int kPlanSms = 148;
 constexpr int kTmemMaxM = 64;                  // tokens up to which the weights go through tensor memory (gemm_tmem.cu)
 constexpr int kTmemSlices = 304;               // its K slices at most (two CTAs per SM), a tile of 32 or 64 tokens x 128 fp32 each
@@ -924,12 +923,14 @@ int gemm_group_forward(const glowq_w4a16_group_t& g, cudaStream_t stream, cudaEr
   auto map = [&](CUtensorMap* out, CUtensorMapDataType dt, const void* ptr, uint64_t d0, uint64_t d1, uint64_t stride,
                  uint32_t b0, uint32_t b1, int sw) { return tensor_map_2d_ex(out, dt, ptr, d0, d1, stride, b0, b1, sw); };
   int rc;
-  CUtensorMap tm_x;
-  if ((rc = map(&tm_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, g.x, g.IC, g.M, static_cast<uint64_t>(g.x_stride) * 2, BK, BM, 1)))
-    return rc;
+  CUtensorMap tm_x;   // 128-token boxes of the activations
+  auto map_x = [&] {
+    return map(&tm_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, g.x, g.IC, g.M, static_cast<uint64_t>(g.x_stride) * 2, BK, BM, 1);
+  };
 
-  // r = X . R^T, once per group, into r_buf: up to 64 tokens inside the group launch (gemm_tmem.cu).  Up to 128 tokens: one small launch (r_product.cu); the K-sliced GEMM
-  // below plus its slot sum take about twenty microseconds.
+  // r = X . R^T, once per group, into r_buf.  Up to 64 tokens: inside the group launch (gemm_tmem.cu).  Up to 128, and below
+  // where the workspace has no room for that: one small launch (r_product.cu).  The K-sliced GEMM plus its slot sum, which take
+  // about twenty microseconds, are for more tokens and for workspaces without any slots.
   bool r_done = route.r_in_launch;
   if (g.r_mode == GLOWQ_R_COMPUTE && !r_done && g.M <= kRProductMaxM && cdiv(g.rank, 16) * cdiv(g.M, 64) <= kRpCtrWords) {
     const size_t need = r_product_slot_bytes(g.M, g.IC, g.rank);
@@ -951,6 +952,7 @@ int gemm_group_forward(const glowq_w4a16_group_t& g, cudaStream_t stream, cudaEr
     GemmParams p{};
     GemmMaps tm;
     std::memset(&tm, 0, sizeof(tm));
+    if ((rc = map_x())) return rc;
     tm.a1 = tm.a2 = tm_x;
     if ((rc = map(&tm.b1[0], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, g.R, g.IC, g.rank, static_cast<uint64_t>(g.R_stride) * 2, BK, BN, 1)))
       return rc;
@@ -987,12 +989,6 @@ int gemm_group_forward(const glowq_w4a16_group_t& g, cudaStream_t stream, cudaEr
       return GLOWQ_ERR_CUDA;
     }
   }
-  CUtensorMap tm_r;
-  std::memset(&tm_r, 0, sizeof(tm_r));
-  if (any_corr &&
-      (rc = map(&tm_r, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, g.r_buf, g.rank, g.M, static_cast<uint64_t>(g.rank) * 2, BK, BM, 1)))
-    return rc;
-
   // All members in ONE launch: the grid's x index runs over the column tiles of member 0, then member 1, ...
   if (route.tmem) {
     int sms = kPlanSms, dev = 0;
@@ -1000,17 +996,23 @@ int gemm_group_forward(const glowq_w4a16_group_t& g, cudaStream_t stream, cudaEr
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     return gemm_tmem_forward(g, route.r_in_launch, any_corr, any_separate, sms, stream, cuda_err);
   }
+  CUtensorMap tm_r;
+  std::memset(&tm_r, 0, sizeof(tm_r));
+  if ((rc = map_x())) return rc;
+  if (any_corr &&
+      (rc = map(&tm_r, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, g.r_buf, g.rank, g.M, static_cast<uint64_t>(g.rank) * 2, BK, BM, 1)))
+    return rc;
   // Tile shape: the 256 x 256 CTA tile has the best operand reuse, but a problem that fills the SMs badly in whole
   // waves is faster with narrower (nn = 1) or shorter (mt = 1) tiles.  A separate correction accumulator needs nn = 1.
   int nn = 1, mt = 2;
   bool pair = false;
   static const int env_pair = [] { const char* e = std::getenv("GLOWQ_GEMM_PAIR"); return e ? std::atoi(e) : -1; }();
   static const int env_swap = [] { const char* e = std::getenv("GLOWQ_GEMM_SWAP"); return e ? std::atoi(e) : -1; }();
-  // Up to 128 tokens: weights on the M side of the MMA, tokens on its N side (see GemmParams::swap).  Measured no
-  // faster than tokens on the M side (31.5 vs 30.3 us for Llama-3.2-3B gate/up at 32 tokens): at these sizes the MMA
-  // thread's issue rate sets the pace, and N = 256 instructions need half as many issues per weight row.  Opt-in.
+  // 65 to 128 tokens: weights on the M side of the MMA, tokens on its N side (see GemmParams::swap).  Measured no faster than
+  // tokens on the M side: the MMA thread's issue rate sets the pace, and N = 256 instructions need half as many issues per
+  // weight row.  Opt-in.
   const bool swap = g.M <= BM && env_swap == 1;
-  const int nt = g.M <= 32 ? 32 : (g.M <= 64 ? 64 : BM);
+  const int nt = BM;
   {
     int sms = 148, dev = 0;
     cudaGetDevice(&dev);

@@ -1,4 +1,4 @@
-// Corrected W4A16 product for decode batches (9 tokens and more) with the dequantised weights in TENSOR MEMORY.
+// Corrected W4A16 product for decode batches (9 to 64 tokens; fewer on request) with the dequantised weights in TENSOR MEMORY.
 //
 //   D[128 output columns, N tokens] += W[128, 128 k] . X[N, 128 k]^T      (one quantisation group of K per step)
 //
@@ -57,7 +57,7 @@ constexpr int kDequantWarps = 4 * kTeams, kCtrlWarps = 3, kThreads = 32 * (kCtrl
 constexpr int kTmemCols = 256;                // per CTA: two share an SM
 constexpr int kSmemBytes = 112 * 1024;
 constexpr int kMaxRCtas = 48;                 // CTAs that compute r
-// Polls of a count of finished CTAs: seconds, because another stream's kernel may hold the SMs that the rest of the CTAs
+// Polls of a count of finished CTAs: some seconds, because another stream's kernel may hold the SMs that the rest of the CTAs
 // of r need (they are placed first, so that nothing of this launch does).
 constexpr unsigned kCountSpin = 1u << 22;
 constexpr unsigned kDrainSpin = 1u << 18;     // polls (tens of milliseconds) for one of this CTA's own copies or MMAs

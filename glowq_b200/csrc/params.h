@@ -49,11 +49,12 @@ constexpr uint32_t kEpochReaderMask = (1u << kEpochShift) - 1u;
 constexpr uint32_t kEpochMask = (1u << 20) - 1u;
 constexpr size_t kWsHeaderBytes = WS_HEADER_WORDS * 4;
 constexpr int kMaxRTiles = 64;      // rank <= 1024
-// After the header: 1 KB of arrival counters for the stand-alone r product, then r of the running launch as the row tiles read it - 8-byte words
+// After the header: 1 KB of counters for r = x . R^T (of the stand-alone product, or of the CTAs of a 9 to 64 token launch that
+// compute it), then r of the running streaming launch as its row tiles read it - 8-byte words
 // {half2(r[tok][2j], r[tok][2j+1]), launch epoch}, up to 8 tokens x rank 1024 - then the tile counters.  All of this lies at
 // the same place whatever a call's sizes are, and every slot and partial buffer of every kernel lies behind it
 // (kWsSlotsOffset): launches of different widths that take turns on one workspace find each other's counters at zero.
-constexpr int kRpCtrWords = 256;    // arrival counters of the stand-alone r product (rank / 16 x token blocks of 64)
+constexpr int kRpCtrWords = 256;    // at most rank / 16 x token blocks of 64 are used
 constexpr size_t kWsRllOffset = kWsHeaderBytes + kRpCtrWords * 4;
 constexpr size_t kWsRllBytes = 8 * 1024 * 4;
 constexpr size_t kWsTileCtrOffset = kWsRllOffset + kWsRllBytes;

@@ -6,8 +6,8 @@
 
 namespace glowq {
 
-// Polls of one wait before the kernel gives up (status 3): seconds, because warps that run ahead of the dependency wait sit in
-// these waits until the kernels before are complete.
+// Polls of one wait before the kernel gives up (status 3), measured as about a quarter of a second: warps that run ahead of the
+// dependency wait sit in these waits until the kernels before are complete, which are launches of this library as well.
 constexpr uint32_t kGemmSpin = 1u << 20;
 
 __device__ __forceinline__ uint32_t sm_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }

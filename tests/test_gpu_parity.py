@@ -247,9 +247,9 @@ def test_fused_residual_rmsnorm_prologue(ocs, ic, rank, M, with_res):
 @pytest.mark.parametrize("M,ic,rank", [(9, 1152, 8), (16, 2048, 64), (40, 3200, 24), (64, 1024, 136), (65, 2176, 64),
                                        (128, 5120, 128), (129, 2048, 64)])
 def test_r_for_few_tokens_and_the_group_gemm(M, ic, rank):
-    """9..128 tokens take the tensor-core GEMM, with r = x R^T from the small stand-alone launch (one CTA per 16 rows
-    of R x 1024 columns x 64 tokens, K slices added in order by the last CTA to arrive); 129 tokens take the K-sliced
-    GEMM for r.  Ranks that are not multiples of 16, K that is not a multiple of 1024, token counts that do not fill
+    """9..64 tokens compute r = x R^T inside the group launch; 65..128 take it from the small stand-alone launch (one CTA
+    per 16 rows of R x 1024 columns x 64 tokens, K slices added in order by the last CTA to arrive); 129 tokens take the
+    K-sliced GEMM for r.  Ranks that are not multiples of 16, K that is not a multiple of 1024, token counts that do not fill
     the 64-token blocks; run twice on the same workspace (the arrival counters must be back at zero)."""
     rng = np.random.default_rng(40 + M)
     lins = [Linear(rng, oc, ic, rank=rank) for oc in (384, 200)]
@@ -551,7 +551,7 @@ def test_gemm_with_a_sliced_last_wave():
 
 @pytest.mark.gpu
 def test_cta_pair_variant_in_subprocess():
-    """The two-CTA (cta_group::2) GEMM variant (above 128 tokens) and the swapped-operand variant (up to 128 tokens)
+    """The two-CTA (cta_group::2) GEMM variant (above 128 tokens) and the swapped-operand variant (65 to 128 tokens)
     are opt-in through environment variables that the library reads once, so they are exercised in a child
     interpreter: the GEMM parity tests must pass with both forced on."""
     import os

@@ -217,8 +217,10 @@ def test_workspace_sizes_cover_what_the_kernels_plan():
 
 
 def test_workspace_covers_every_k_sliced_plan():
-    """For 9..256 tokens the GEMM may cut K into slices whose fp32 partial tiles live at the end of the workspace; the
-    size the library reports must cover the plan for either column-tile width (restated here from the host code)."""
+    """For 65..256 tokens the GEMM may cut K into slices whose fp32 partial tiles live at the end of the workspace; the
+    size the library reports must cover the plan for either column-tile width (restated here from the host code).  Up to 64
+    tokens the tensor-memory form has a plan of its own, which takes the slices the room allows (test_workspace_layout.py);
+    the reported size covers the old plan there too."""
     from glowq_b200.cuda_w4a16 import kernels as K
     wb = K.load_w4a16_extension().workspace_bytes
     cdiv = lambda a, b: -(-a // b)
