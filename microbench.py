@@ -104,6 +104,7 @@ def main():
                 if not args.no_chain:   # every launch names the one that follows it on the stream
                     for i in range(n):
                         arr[i].next = ctypes.addressof(arr[(i + 1) % n])
+                torch.cuda.synchronize()   # weights are drawn and workspaces cleared on another stream
                 with torch.cuda.stream(st):
                     for _ in range(2):
                         ext.check(ext.lib.glowq_w4a16_group_forward_many(arr, n))
