@@ -3,8 +3,9 @@
 //   Y[M, OC] = X[M, IC] . dequant(Q)^T  +  alpha * r[M, rank] . L[OC, rank]^T  (+ bias),     r = X . R^T
 //
 // Up to 64 tokens one CTA per 128 output columns (gemm_tmem.cu), above a CTA pair per 256 (gemm_pair.cu).  Both keep the
-// dequantised weights in tensor memory, and both compute r inside the group launch.  The line: an MMA of the pair form has at least
-// 32 tokens per CTA and its items at least 64; the other one's two CTAs per SM hold 64 tokens at most.
+// dequantised weights in tensor memory, and both compute r inside the group launch.  The line lies where the first ends: two CTAs
+// share an SM's tensor memory there, which leaves an accumulator 64 tokens (13B gate/up 45 us at 64 tokens; the pair form, whose
+// tiles have 64 tokens at least, takes 14B gate/up from 71 to 63 us at 70).
 #include <algorithm>
 
 #include "../../include/glowq_w4a16.h"

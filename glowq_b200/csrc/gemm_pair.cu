@@ -15,6 +15,11 @@
 //   warps 8-15  dequantise, in two teams of four warps that take alternate steps (a thread owns one weight row)
 // r = X . R^T is the first items of the launch: R in the place of the weights (fp16 rows go to tensor memory as they are), the
 // output goes to r_buf; the producers wait for the count of finished r tiles before their first correction step.
+//   What bounds it: 256 tokens, the MMAs (1024 clocks a step; measured 1030) and the epilogue that only the next steps' dequantisation
+// runs under; narrower tiles, tensor memory's writes and the chain from a stage's release to its next MMAs (about 1100 clocks a step
+// whatever the width, also with four teams).  Long runs are bound by the 1 kW limit (1.35 to 1.45 GHz).  Corrected group calls, us,
+// before (fp16 weight tile in shared memory, r and slot sum as launches) / now: 14B gate/up 94 / 85 at 211 tokens, 688 / 556 at 2048,
+// 1330 / 1103 at 4096; 14B down_proj 97 / 67, 371 / 316, 742 / 627; 3B q/k/v 36 / 22, 86 / 77, 144 / 132.
 //   Items are taken in order from a ticket (or are the clusters themselves where they are few): a CTA waits for items in front of
 // its own only, so a launch gets through on any number of SMs.  K may be sliced; the CTAs of a tile's last slice add the other
 // slices' fp32 slots in slice order (deterministic).  Every wait is bounded; on expiry a status word is set and the CTAs drain.
@@ -37,7 +42,8 @@ namespace {
 constexpr int kRows = 128;                 // weight rows (output columns) per CTA
 constexpr int kPStage = kRows * 64;        // weight stage: 128 rows x 64 bytes
 constexpr int kMeta = 2 * kRows * 4;       // per weight stage and row: the scale twice (half2), the zero-point constants
-constexpr int kMaxP = 4;                   // weight stages per team at most (an fp16 step of 128 columns takes four)
+constexpr int kNP = 4;                     // weight stages per team: an fp16 step of 128 columns takes all four.  (With two the producer,
+                                           // which takes the steps in order, feeds one team at a time; 14B down_proj, 777 tokens: 220 -> 194 us.)
 constexpr int kMaxB = 8;                   // activation stages at most
 constexpr int kOStage = 2048;              // output stage of a warp: 32 tokens x 32 fp16 columns, or 16 x 32 fp32
 constexpr int kMaxO = 8;                   // output stages at most
@@ -72,7 +78,6 @@ struct PtParams {
   int n_tiles, n_x, n_y, band, full_tiles, n_tail, ksplit;
   int sep;                // a correction with a factor other than 1: an accumulator of its own
   int nbuf, nb, na, no;   // accumulators, activation stages, A stages (64 columns each, behind the accumulators), output stages
-  int np;                 // weight stages per team
   PtMember mem[kMaxMembers];
 };
 struct alignas(64) PtMaps {
@@ -252,17 +257,16 @@ __device__ __forceinline__ bool epi_vote(bool ok) {
 }
 __device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
-// Ring positions of the teams' weight stages (up to four each).
+// Ring positions of the teams' weight stages.
+static_assert(kNP == 4, "two bits per team");
 struct TeamRings {
-  uint32_t np, idx, ph;   // stages; four bits and one bit per team
-  __device__ __forceinline__ uint32_t at(uint32_t team) const { return team * np + ((idx >> (4 * team)) & 15u); }
+  uint32_t idx, ph;   // two bits and one bit per team
+  __device__ __forceinline__ uint32_t at(uint32_t team) const { return team * kNP + ((idx >> (2 * team)) & 3u); }
   __device__ __forceinline__ uint32_t phase(uint32_t team) const { return (ph >> team) & 1u; }
   __device__ __forceinline__ void step(uint32_t team) {
-    idx += 1u << (4 * team);
-    if (((idx >> (4 * team)) & 15u) == np) {
-      idx &= ~(15u << (4 * team));
-      ph ^= 1u << team;
-    }
+    const uint32_t i = (idx >> (2 * team)) & 3u;
+    idx ^= (i ^ ((i + 1) & 3u)) << (2 * team);
+    ph ^= static_cast<uint32_t>(i == 3u) << team;
   }
 };
 struct Ring {   // one ring position: index and phase parity
@@ -278,7 +282,7 @@ struct Ring {   // one ring position: index and phase parity
 // Barriers in the first KB of shared memory.
 constexpr uint32_t kBFull = 0;                    // [kMaxB] CTA 0: both CTAs' activations have landed and A tiles are written
 constexpr uint32_t kBDone = 64;                   // [kMaxB] each CTA: the MMAs of the step are done
-constexpr uint32_t kBPFull = 128;                 // [kTeams][np] weight stages
+constexpr uint32_t kBPFull = 128;                 // [kTeams][kNP] weight stages
 constexpr uint32_t kBPEmpty = 192;
 constexpr uint32_t kBAccFull = 256;               // [2] each CTA
 constexpr uint32_t kBAccEmpty = 272;              // [2] CTA 0: the epilogue warps of both CTAs
@@ -294,8 +298,8 @@ gemm_pair_kernel(const __grid_constant__ PtParams p, const __grid_constant__ PtM
   __shared__ uint32_t s_tmem_base;
   const uint32_t smem0 = (sm_u32(smem) + 1023u) & ~1023u;
   const uint32_t sub = static_cast<uint32_t>(p.N) * 64;        // 64 columns of this CTA's N / 2 tokens
-  const uint32_t ring = smem0 + 1024, pring = ring + p.nb * 2 * sub, meta = pring + kTeams * p.np * kPStage,
-                 ostage = meta + kTeams * p.np * kMeta;
+  const uint32_t ring = smem0 + 1024, pring = ring + p.nb * 2 * sub, meta = pring + kTeams * kNP * kPStage,
+                 ostage = meta + kTeams * kNP * kMeta;
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int rank = static_cast<int>(cluster_ctarank());
   const int pair = static_cast<int>(blockIdx.x >> 1);
@@ -306,7 +310,7 @@ gemm_pair_kernel(const __grid_constant__ PtParams p, const __grid_constant__ PtM
       g_mbar_init(smem0 + kBFull + 8 * i, 9);    // four dequant warps of either CTA, the announcement of the copies
       g_mbar_init(smem0 + kBDone + 8 * i, 1);
     }
-    for (int i = 0; i < kTeams * kMaxP; ++i) {
+    for (int i = 0; i < kTeams * kNP; ++i) {
       g_mbar_init(smem0 + kBPFull + 8 * i, 2);   // the copy and the scales
       g_mbar_init(smem0 + kBPEmpty + 8 * i, 4);
     }
@@ -405,7 +409,7 @@ gemm_pair_kernel(const __grid_constant__ PtParams p, const __grid_constant__ PtM
     __syncwarp();
   } else if (warp == 2) {
     if (lane == 0) {
-      TeamRings s{static_cast<uint32_t>(p.np), 0, 0};
+      TeamRings s{0, 0};
       uint32_t j = 0;
       bool ok = true;
       while (ok && next_item(t, true, false)) {
@@ -431,8 +435,8 @@ gemm_pair_kernel(const __grid_constant__ PtParams p, const __grid_constant__ PtM
         }
       }
       // the last copy of every stage has landed
-      for (uint32_t at = 0; at < kTeams * s.np; ++at) {
-        const uint32_t team = at / s.np, k = at % s.np, cur = (s.idx >> (4 * team)) & 15u;
+      for (uint32_t at = 0; at < kTeams * kNP; ++at) {
+        const uint32_t team = at / kNP, k = at % kNP, cur = (s.idx >> (2 * team)) & 3u;
         // (a stage of the present round, or of the round before; none at all: its barrier is in its first phase)
         const uint32_t par = k < cur ? s.phase(team) : s.phase(team) ^ 1;
         uint32_t spins = 0;
@@ -444,7 +448,7 @@ gemm_pair_kernel(const __grid_constant__ PtParams p, const __grid_constant__ PtM
   } else if (warp == 3) {
     // A lane loads four rows, eight groups at a time: with one group at a time (two bytes of each row) the loads of a step
     // take 256 wavefronts, and the shared-memory loads of the dequant warps wait behind them.
-    TeamRings s{static_cast<uint32_t>(p.np), 0, 0};
+    TeamRings s{0, 0};
     uint32_t j = 0;
     bool ok = true;
     while (ok && next_item(t, false, true)) {
@@ -592,10 +596,10 @@ gemm_pair_kernel(const __grid_constant__ PtParams p, const __grid_constant__ PtM
     // ================================================================ dequant warps
     const int team = (warp - 8) >> 2, q = warp & 3;   // q: the tensor-memory lanes this warp reaches
     const int rloc = q * 32 + lane;
-    const uint32_t na = p.na, nb = p.nb, np = p.np, dst0 = tmem + (static_cast<uint32_t>(q * 32) << 16) + kTmemCols - na * 64;
-    const uint32_t prow = pring + team * np * kPStage + static_cast<uint32_t>(rloc) * 64, psw = (static_cast<uint32_t>(rloc) >> 1) & 3u;
-    const uint32_t mrow = meta + team * np * kMeta + static_cast<uint32_t>(rloc) * 8;
-    const uint32_t pfull = smem0 + kBPFull + 8 * team * np, pempty = smem0 + kBPEmpty + 8 * team * np;
+    const uint32_t na = p.na, nb = p.nb, dst0 = tmem + (static_cast<uint32_t>(q * 32) << 16) + kTmemCols - na * 64;
+    const uint32_t prow = pring + team * kNP * kPStage + static_cast<uint32_t>(rloc) * 64, psw = (static_cast<uint32_t>(rloc) >> 1) & 3u;
+    const uint32_t mrow = meta + team * kNP * kMeta + static_cast<uint32_t>(rloc) * 8;
+    const uint32_t pfull = smem0 + kBPFull + 8 * team * kNP, pempty = smem0 + kBPEmpty + 8 * team * kNP;
     const uint32_t full0 = map_to_cta(smem0 + kBFull, 0);
     // this team's next step (of all tiles' together), its place in the ring of steps, that of the step na before (whose MMAs read
     // the same A stage), its A stage
@@ -641,7 +645,7 @@ gemm_pair_kernel(const __grid_constant__ PtParams p, const __grid_constant__ PtM
             }
             tmem_st32p(dst + half * 32, v);   // (after a failed wait the stores go on: the status word is set)
           }
-          s.step(np);
+          s.step(kNP);
         } else {   // fp16 rows (L, R), or zeros beside rows that are corrected
           const int h = halves(p, it);
           await_stage();
@@ -656,7 +660,7 @@ gemm_pair_kernel(const __grid_constant__ PtParams p, const __grid_constant__ PtM
                 for (int i = 0; i < 4; ++i) lds_v4(v + 16 * k + 4 * i, prow + s.i * kPStage + ((static_cast<uint32_t>(i) ^ psw) << 4));
                 __syncwarp();
                 if (lane == 0) g_mbar_arrive(pempty + 8 * s.i);
-                s.step(np);
+                s.step(kNP);
               } else {
 #pragma unroll
                 for (int i = 0; i < 16; ++i) v[16 * k + i] = 0u;
@@ -936,7 +940,7 @@ cudaError_t launch(const PtParams& p, const PtMaps& tm, int pairs, size_t smem, 
 
 // Tiles, slices and rings of a group call; no CUDA calls.
 struct PairPlan {
-  int N, n_y, nbuf, nb, na, no, np;
+  int N, n_y, nbuf, nb, na, no;
   int n_tiles, n_x, ksplit, full_tiles, n_tail, nk_min;
   int r_x, r_tiles, r_slices;
   size_t off_slots, end;       // in the workspace: slots of the K slices (those of r at kWsSlotsOffset), end of all slots
@@ -947,7 +951,7 @@ struct PairPlan {
 // what cutting a tile into K slices costs (partial tiles of N tokens through memory).
 inline double step_us(int N) { return 0.46 + 0.001 * N; }
 inline double tile_us(bool two) { return two ? 1.2 : 4.2; }
-constexpr double kRStepUs = 0.9;   // a step of r, whose fp16 rows come through four weight stages
+constexpr double kRStepUs = 0.8;   // a step of r, whose fp16 rows come through four weight stages
 inline double slices_us(int N, int ks) { return ks > 1 ? 3.0 + (ks - 1) * 0.010 * N : 0.0; }
 
 PairPlan make_pair_plan(const glowq_w4a16_group_t& g, bool compute_r, bool any_corr, bool sep, int sms) {
@@ -1011,11 +1015,10 @@ PairPlan make_pair_plan(const glowq_w4a16_group_t& g, bool compute_r, bool any_c
     }
   }
   const int stage = best.N * 128;
-  best.np = best.N > 192 ? 2 : kMaxP;
-  const int left = kSmemMax - 2048 - kTeams * best.np * (kPStage + kMeta);
+  const int left = kSmemMax - 2048 - kTeams * kNP * (kPStage + kMeta);
   // At least as many activation stages as teams (a team waits for the MMAs of every second step, and a parity wait must not be able
   // to meet the phase before the last) and as A stages (the barrier of a step is that of the step nb before, which must be done).
-  best.nb = std::max(4, std::min(6, (left - 24 * kOStage) / stage));
+  best.nb = std::max(3, std::min(6, (left - (best.N > 192 ? 16 : 24) * kOStage) / stage));
   best.no = std::min(kMaxO, (left - best.nb * stage) / (4 * kOStage));
   best.na = std::min({4, (kTmemCols - std::max(best.nbuf, sep ? 2 : 1) * best.N) / 64, best.nb});
   return best;
@@ -1065,7 +1068,6 @@ int gemm_pair_forward(const glowq_w4a16_group_t& g, bool compute_r, bool r_only,
   p.nb = pl.nb;
   p.na = pl.na;
   p.no = pl.no;
-  p.np = pl.np;
   p.sep = any_separate;
   p.n_x = pl.n_x;
   p.n_y = pl.n_y;
@@ -1136,7 +1138,7 @@ int gemm_pair_forward(const glowq_w4a16_group_t& g, bool compute_r, bool r_only,
   }
   const int pairs = std::max(1, sms / 2);
   p.tickets = have_ctr && p.n_items > pairs;
-  const size_t smem = 2048 + static_cast<size_t>(p.nb) * p.N * 128 + kTeams * p.np * (kPStage + kMeta) + 4 * p.no * kOStage;
+  const size_t smem = 2048 + static_cast<size_t>(p.nb) * p.N * 128 + kTeams * kNP * (kPStage + kMeta) + 4 * p.no * kOStage;
   const cudaError_t e = launch(p, tm, p.tickets ? pairs : p.n_items, smem, stream);
   if (e != cudaSuccess) {
     *cuda_err = e;
