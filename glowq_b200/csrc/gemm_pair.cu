@@ -223,7 +223,6 @@ __device__ __forceinline__ void tma_2d_pair(uint32_t dst, const CUtensorMap* tma
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* tmap, int x, int y, uint32_t src) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(tmap), "r"(x), "r"(y), "r"(src)
                : "memory");
-  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
 // A poll that does not block (mbarrier.try_wait may suspend the thread while the phase is open).
 __device__ __forceinline__ bool test_bar(uint32_t a, uint32_t parity) {
@@ -692,7 +691,8 @@ gemm_pair_kernel(const __grid_constant__ PtParams p, const __grid_constant__ PtM
     const uint32_t ow = ostage + static_cast<uint32_t>(q * p.no) * kOStage;
     uint32_t n = 0, ob = 0;
     // Output stages, each warp its own, handed to the copy engine two at a time (the fence takes some hundred clocks).  Behind the
-    // stores the oldest ones have been read, so that the next two stages are free.
+    // stores the oldest ones have been read, so that the next two stages are free: a stage has a group of its own, an empty one where
+    // the warp's columns lie past the end, so that the groups still to be waited for are the last stages written.
     auto store_stages = [&](const CUtensorMap* m, int x, int y, int rows, int count, bool inside) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
@@ -700,6 +700,7 @@ gemm_pair_kernel(const __grid_constant__ PtParams p, const __grid_constant__ PtM
         uint32_t o = ob;
         for (int c = 0; c < count; ++c) {
           if (inside) tma_store_2d(m, x, y + c * rows, ow + o * kOStage);
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           if (++o == static_cast<uint32_t>(p.no)) o = 0;
         }
         if (p.no >= 8)

@@ -39,6 +39,26 @@ def test_against_the_oracle(M, ocs, ic, rank, alpha, bias, f32):
     assert all(torch.equal(a, b) for a, b in zip(seen[1], seen[2]))     # slices are added in slice order: the same bits
 
 
+@pytest.mark.parametrize("M,ocs,ic,alpha,f32", [(15000, [384], 128, 1.0, False), (12000, [128, 200], 128, 0.5, False),
+                                                (15000, [330], 128, 1.0, True), (9000, [40, 300, 300], 256, 1.0, False)])
+def test_output_stages_of_warps_with_and_without_columns(M, ocs, ic, alpha, f32):
+    """Short tiles one after another, and warps whose columns lie inside the outputs in one tile and past the end in the next: a stage
+    is written again only when the copy engine has read it."""
+    rng = np.random.default_rng(M)
+    lins = [Linear(rng, oc, ic, rank=16, quantize=False) for oc in ocs]
+    x_d, R_d = dev(rng.standard_normal((M, ic)).astype(np.float16)), dev((rng.standard_normal((16, ic)) * 0.01).astype(np.float16))
+    dt, seen, want = K.OUT_F32 if f32 else K.OUT_F16, [], [l.oracle(x_d.cpu().numpy(), R_d.cpu().numpy(), alpha=alpha) for l in lins]
+    for _ in range(5):
+        outs = [new_out(M, l, dt) for l in lins]
+        g = make_group(x_d, lins, outs, R_d=R_d, r_buf=torch.zeros(M, 16, dtype=torch.float16, device="cuda"), r_mode=K.R_COMPUTE,
+                       alpha=alpha, out_dtype=dt)
+        assert run_group(g) == 0 and status_ok(g) == 0
+        for o, w in zip(outs, want):
+            assert_close(o, w)
+        seen.append([o.cpu() for o in outs])
+    assert all(torch.equal(a, b) for s in seen[1:] for a, b in zip(s, seen[0]))
+
+
 def test_other_layouts_and_scarce_workspaces():
     """Rows of a wider output (no copies of whole rows), a workspace without slots, one without counters (r in front of the members,
     every tile a cluster of its own)."""
