@@ -546,6 +546,7 @@ gemm_pair_kernel(const __grid_constant__ PtParams p, const __grid_constant__ PtM
         uint32_t d = tmem + buf * static_cast<uint32_t>(p.N), acc = 0;
         const uint32_t nk = t.nk, last = G + ((p.rank + 127) >> 7) - 1, last_both = (p.rank & 127) == 0 || (p.rank & 127) > 64;
         const uint32_t sep_at = p.sep ? G : 0xFFFFFFFFu;
+        if (static_cast<uint32_t>(t.it0) > sep_at) d += p.N;   // a K slice that starts behind the correction's first step
         for (uint32_t it = t.it0; it < nk; ++it) {
           if (it == sep_at) {
             d += p.N;

@@ -5,6 +5,7 @@ import torch
 
 from glowq_b200.cuda_w4a16 import kernels as K
 from gpu_helpers import Linear, assert_close, dev, ext, make_group, new_out, run_group, status_ok
+from test_workspace_layout import BEHIND_THE_WEIGHTS
 
 pytestmark = pytest.mark.gpu
 
@@ -57,6 +58,28 @@ def test_output_stages_of_warps_with_and_without_columns(M, ocs, ic, alpha, f32)
             assert_close(o, w)
         seen.append([o.cpu() for o in outs])
     assert all(torch.equal(a, b) for s in seen[1:] for a, b in zip(s, seen[0]))
+
+
+@pytest.mark.parametrize("M,oc,ic,rank,r_mode", BEHIND_THE_WEIGHTS)
+@pytest.mark.parametrize("alpha", [0.5, 1.0])
+def test_slices_that_start_behind_the_weights(M, oc, ic, rank, r_mode, alpha):
+    """K slices of nothing but correction steps, and not the first of them: with a factor other than 1 they accumulate beside the
+    weights' products, and with 1 among them."""
+    rng = np.random.default_rng(M + rank)
+    lin = Linear(rng, oc, ic, rank=rank, bias=True, quantize=False)
+    x = rng.standard_normal((M, ic)).astype(np.float16)
+    R = (rng.standard_normal((rank, ic)) * 0.01).astype(np.float16)
+    r_buf = torch.zeros(M, rank, dtype=torch.float16, device="cuda")
+    if r_mode == K.R_LOAD:
+        r_buf.copy_(dev(x.astype(np.float32) @ R.astype(np.float32).T))
+    want, seen = lin.oracle(x, R, alpha=alpha), []
+    for _ in range(2):
+        out = new_out(M, lin, K.OUT_F32)
+        g = make_group(dev(x), [lin], [out], R_d=dev(R), r_buf=r_buf, r_mode=r_mode, alpha=alpha, out_dtype=K.OUT_F32)
+        assert run_group(g) == 0 and status_ok(g) == 0
+        assert_close(out, want, tag=f"alpha {alpha}")
+        seen.append(out.cpu())
+    assert torch.equal(*seen)
 
 
 def test_other_layouts_and_scarce_workspaces():

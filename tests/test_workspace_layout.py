@@ -13,14 +13,15 @@ class Map(ctypes.Structure):
         (n, ctypes.c_ulonglong) for n in ("ctr_begin", "ctr_end", "slots_begin", "slots_end")]
 
 
-def workspace_map(M, ic, ocs, rank=0, alphas=None, nbytes=1 << 28, kernel=K.KERNEL_AUTO, split_k=0, sms=148, rc=0):
+def workspace_map(M, ic, ocs, rank=0, alphas=None, nbytes=1 << 28, kernel=K.KERNEL_AUTO, split_k=0, sms=148, rc=0,
+                  r_mode=K.R_COMPUTE):
     """The map of a call; every address is a placeholder."""
     at, g = 1 << 20, K.Group()
     g.x, g.M, g.IC, g.x_stride, g.group_size = at, M, ic, ic, 128
     g.kernel, g.split_k, g.n_members = kernel, split_k, len(ocs)
     g.workspace, g.workspace_bytes = at, nbytes
     if rank:
-        g.r_mode, g.rank, g.r_buf, g.R, g.R_stride = K.R_COMPUTE, rank, at, at, ic
+        g.r_mode, g.rank, g.r_buf, g.R, g.R_stride = r_mode, rank, at, at, ic
     groups = -(-ic // 128)
     for i, oc in enumerate(ocs):
         m = g.members[i]
@@ -86,3 +87,16 @@ def test_no_slice_of_a_group_of_unlike_members_is_empty(M, ic, rank):
         for alphas in ([1.0, 0.0, 0.5], [0.0, 1.0, 1.0], [0.5, 0.0, 0.0]):
             m = workspace_map(M, ic, ocs, rank, alphas=alphas[:len(ocs)])
             assert m.kernel == 1 and m.shortest == -(-ic // 128) and m.ksplit <= m.shortest, (ocs, alphas, m.ksplit)
+
+
+# calls of the CTA pairs with ranks above 512 against a short K: (tokens, columns, K, rank, how r comes)
+BEHIND_THE_WEIGHTS = [(65, 20224, 1152, 768, K.R_COMPUTE), (256, 20224, 1536, 1024, K.R_COMPUTE), (400, 5248, 2560, 920, K.R_COMPUTE),
+                      (100, 512, 1536, 1024, K.R_LOAD), (65, 128, 1152, 648, K.R_LOAD)]
+
+
+@pytest.mark.parametrize("M,oc,ic,rank,r_mode", BEHIND_THE_WEIGHTS)
+def test_the_plans_have_slices_that_start_behind_the_weights(M, oc, ic, rank, r_mode):
+    nbytes = K.load_w4a16_extension().workspace_bytes(M, ic, oc, rank, 1)
+    m = workspace_map(M, ic, [oc], rank, alphas=[0.5], nbytes=nbytes, r_mode=r_mode)
+    groups, steps = -(-ic // 128), -(-ic // 128) + -(-rank // 128)
+    assert m.kernel == 2 and m.ksplit > 1 and steps * (m.ksplit - 1) // m.ksplit > groups
