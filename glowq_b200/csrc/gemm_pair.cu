@@ -956,12 +956,28 @@ inline double tile_us(bool two) { return two ? 1.2 : 4.2; }
 constexpr double kRStepUs = 0.8;   // a step of r, whose fp16 rows come through four weight stages
 inline double slices_us(int N, int ks) { return ks > 1 ? 3.0 + (ks - 1) * 0.010 * N : 0.0; }
 
+// First column tile of each member; returns the tiles in all.  Members that share a pair of tiles are corrected both or neither: in one
+// accumulator the correction steps of a pair would reach the rows of the other member as zeros times r, which are not zero where r
+// overflowed.  (With an accumulator of its own the correction is left out of the rows that have none.)
+int member_tiles(const glowq_w4a16_group_t& g, bool any_corr, bool sep, int* begin) {
+  int tiles = 0;
+  bool before = false;
+  for (int i = 0; i < g.n_members; ++i) {
+    const bool corr = any_corr && g.members[i].L && g.members[i].alpha != 0.f;
+    if (corr != before && !sep) tiles = (tiles + 1) & ~1;
+    before = corr;
+    begin[i] = tiles;
+    tiles += cdiv(g.members[i].OC, kRows);
+  }
+  return tiles;
+}
+
 PairPlan make_pair_plan(const glowq_w4a16_group_t& g, bool compute_r, bool any_corr, bool sep, int sms) {
   const int G = cdiv(g.IC, kGroup), nu = any_corr ? cdiv(g.rank, 128) : 0, nk = G + nu, pairs = std::max(1, sms / 2);
   PairPlan best{};
   double best_cost = 1e300;
-  int n_tiles = 0;
-  for (int i = 0; i < g.n_members; ++i) n_tiles += cdiv(g.members[i].OC, kRows);
+  int begin[kMaxMembers];
+  const int n_tiles = member_tiles(g, any_corr, sep, begin);
   const int n_x = cdiv(n_tiles, 2);
   const size_t room = g.workspace_bytes > kWsSlotsOffset ? g.workspace_bytes - kWsSlotsOffset : 0;
   const int max_n = sep ? 192 : 256, y0 = cdiv(g.M, max_n), y1 = std::max(y0, std::min(cdiv(g.M, 64), y0 * 2 + 2));
@@ -1103,7 +1119,8 @@ int gemm_pair_forward(const glowq_w4a16_group_t& g, bool compute_r, bool r_only,
   if (any_corr && (rc = tensor_map_2d_ex(&tm.r, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, g.r_buf, g.rank, g.M,
                                          static_cast<uint64_t>(g.rank) * 2, 64, p.N / 2, 1)))
     return rc;
-  int tiles = 0;
+  int begin[kMaxMembers];
+  member_tiles(g, any_corr, any_separate, begin);
   for (int i = 0; i < g.n_members; ++i) {
     const auto& m = g.members[i];
     const bool corr = any_corr && m.L && m.alpha != 0.f;
@@ -1135,8 +1152,7 @@ int gemm_pair_forward(const glowq_w4a16_group_t& g, bool compute_r, bool r_only,
     d.zstride = m.zero_stride_i32;
     d.out_stride = m.out_stride;
     d.alpha = m.alpha;
-    d.tile_begin = tiles;
-    tiles += cdiv(m.OC, kRows);
+    d.tile_begin = begin[i];
   }
   const int pairs = std::max(1, sms / 2);
   p.tickets = have_ctr && p.n_items > pairs;

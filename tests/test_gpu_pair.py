@@ -115,6 +115,31 @@ def test_corrected_and_uncorrected_members_in_one_launch(M, alpha, use_L):
         assert_close(o, l.oracle(x, R if on else None, alpha=alpha[i]), tag=f"member {i}")
 
 
+@pytest.mark.parametrize("M,ocs,ic,use_L", [(100, [384, 200, 128], 4096, [True, False, True]), (300, [128, 640], 640, [False, True]),
+                                            (70, [100, 100, 300, 40], 1024, [True, False, False, True]),
+                                            (700, [384, 130], 2048, [False, True])])
+def test_an_overflow_of_r_stays_with_the_corrected_members(M, ocs, ic, use_L):
+    """r is fp16 and may hold infinities: the tokens' results of the members without a correction do not depend on it, wherever their
+    column tiles lie."""
+    rng = np.random.default_rng(M)
+    lins = [Linear(rng, oc, ic, rank=72, bias=True, quantize=False) for oc in ocs]
+    x = rng.standard_normal((M, ic)).astype(np.float16)
+    R = (rng.standard_normal((72, ic)) * 0.01).astype(np.float16)
+    r_buf = dev((x.astype(np.float32) @ R.astype(np.float32).T).astype(np.float16))
+    r_buf[3, 5], r_buf[M - 1, 71] = float("inf"), float("-inf")
+    outs = [new_out(M, l) for l in lins]
+    g = make_group(dev(x), lins, outs, R_d=dev(R), r_buf=r_buf, r_mode=K.R_LOAD, use_L=use_L)
+    assert run_group(g) == 0 and status_ok(g) == 0
+    finite = [t for t in range(M) if t not in (3, M - 1)]
+    for i, (l, o) in enumerate(zip(lins, outs)):
+        want = l.oracle(x, R if use_L[i] else None)
+        if use_L[i]:
+            assert not o[3].isfinite().any()
+            assert_close(o[finite], want[finite], tag=f"member {i}")
+        else:
+            assert_close(o, want, tag=f"member {i}")
+
+
 @pytest.mark.parametrize("M,ocs,ic,rank,launches", [(211, [5120], 5120, 256, 100), (600, [3072, 1024, 1024], 3072, 64, 60),
                                                     (1300, [2048], 8192, 64, 40), (90, [1024], 18944, 128, 100)])
 def test_launches_back_to_back_on_one_workspace(M, ocs, ic, rank, launches):
