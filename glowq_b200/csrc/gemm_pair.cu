@@ -364,7 +364,7 @@ gemm_pair_kernel(const __grid_constant__ PtParams p, const __grid_constant__ PtM
     sph ^= 1;
     return t.flags & kValid;
   };
-  Tile t;
+  Tile t{};   // (no member out of range when the first wait for an item runs out)
 
   if (warp == 0) {
     if (lane == 0) {
