@@ -24,6 +24,7 @@
 // its own only, so a launch gets through on any number of SMs.  K may be sliced; the CTAs of a tile's last slice add the other
 // slices' fp32 slots in slice order (deterministic).  Every wait is bounded; on expiry a status word is set and the CTAs drain.
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 
@@ -948,13 +949,42 @@ struct PairPlan {
   size_t off_slots, end;       // in the workspace: slots of the K slices (those of r at kWsSlotsOffset), end of all slots
 };
 
-// Microseconds, fitted on B200: a step of N tokens (tensor-memory writes and the chain from a stage's release to its next MMAs bound
-// narrow tiles, the MMAs the widest); what a tile costs beside its steps (with one accumulator nothing runs under its epilogue);
-// what cutting a tile into K slices costs (partial tiles of N tokens through memory).
-inline double step_us(int N) { return 0.46 + 0.001 * N; }
-inline double tile_us(bool two) { return two ? 1.2 : 4.2; }
-constexpr double kRStepUs = 0.8;   // a step of r, whose fp16 rows come through four weight stages
-inline double slices_us(int N, int ks) { return ks > 1 ? 3.0 + (ks - 1) * 0.010 * N : 0.0; }
+// Microseconds of a launch's parts, fitted on B200 to 638 group calls of 65 to 4096 tokens with some twenty plans each: the plans that
+// the fit takes are 1 % slower than the best ones on average, 12 % at worst.
+// A step of N tokens (tensor-memory writes and the chain from a stage's release to its next MMAs bound narrow tiles, the MMAs the
+// widest; slower the more pairs are busy); what a tile costs beside its steps; an item of r, whose fp16 rows come through four weight
+// stages a step; adding up K slices, three slots of 16 tokens a trip to memory.
+inline double step_us(int N, double busy) { return (N <= 192 ? 0.366 + 0.0004 * N : 0.00183 * N) * (1.0 + 0.366 * busy); }
+inline double tile_us(int N, bool two) { return two ? 4.25 : 4.2 + 0.004 * N; }
+inline double r_item_us(int N, double steps) { return 0.3 + steps * (0.834 + 0.0034 * N); }
+inline double r_sum_us(int N, int ks) { return ks > 1 ? 0.7 + (0.0216 * cdiv(ks - 1, 3) + 0.0018 * (ks - 1)) * N : 0.0; }
+inline double sum_us(int N, int ks, bool whole_before) {
+  return ks > 1 ? (whole_before ? 3.4 : 1.4) + (0.0349 * cdiv(ks - 1, 3) + 0.0003 * (ks - 1)) * N : 0.0;
+}
+constexpr double kTicketUs = 3.2;   // the first item by ticket: nothing of it runs ahead of the kernel before
+// When `items` of d microseconds each, taken in order, are done: n[i] pairs are through with their first at e[i].
+double rounds_us(int items, const int (&n)[4], const double (&e)[4], double d) {
+  double lo = 1e300, hi = 0.0, t = 0.0;
+  int pairs = 0, k[4];
+  for (int i = 0; i < 4; ++i)
+    if (n[i] > 0) {
+      pairs += n[i];
+      lo = std::min(lo, e[i]);
+      hi = std::max(hi, e[i]);
+    }
+  // (every pair does so many at least)
+  const int all = std::max(0, items / pairs - 1 - static_cast<int>(std::ceil((hi - lo) / d)));
+  std::fill(k, k + 4, all);
+  for (int done = all * pairs; done < items;) {
+    int b = -1;
+    for (int i = 0; i < 4; ++i)
+      if (n[i] > 0 && (b < 0 || e[i] + k[i] * d < e[b] + k[b] * d)) b = i;
+    t = e[b] + k[b] * d;
+    done += n[b];
+    ++k[b];
+  }
+  return t;
+}
 
 // First column tile of each member; returns the tiles in all.  Members that share a pair of tiles are corrected both or neither: in one
 // accumulator the correction steps of a pair would reach the rows of the other member as zeros times r, which are not zero where r
@@ -993,7 +1023,6 @@ PairPlan make_pair_plan(const glowq_w4a16_group_t& g, bool compute_r, bool any_c
     pl.nk_min = G;
     const size_t tile_bytes = static_cast<size_t>(pl.N) * (2 * kRows) * 4;
     const int total = n_x * pl.n_y, f_max = total / pairs;
-    const double step = step_us(pl.N);
     const bool two = pl.N <= 192 && !sep;
     if (compute_r) {
       pl.r_x = cdiv(g.rank, 2 * kRows);
@@ -1003,20 +1032,37 @@ PairPlan make_pair_plan(const glowq_w4a16_group_t& g, bool compute_r, bool any_c
       const size_t r_bytes = rks > 1 ? tile_bytes * pl.r_tiles * rks : 0;
       if (rks > 1 && (2 * pl.r_tiles > kTileCtrWords || r_bytes > room)) break;
       const int n_r = pl.r_tiles * rks, ctr_room = kTileCtrWords / 2 - (rks > 1 ? pl.r_tiles : 0);
-      // when r is ready, and its load on the pairs
-      const double r_us = compute_r ? (static_cast<double>(G) / rks + 2) * kRStepUs + 1.2 * slices_us(pl.N, rks) + 3.0 : 0.0;
-      const double r_load = n_r * (static_cast<double>(G) / rks + 3) * kRStepUs / pairs;
+      // an item of r (pairs take one, or several one after another), the sum of its slices, the pairs that add them
+      const double r_item = compute_r ? r_item_us(pl.N, static_cast<double>(G) / rks) * cdiv(n_r, pairs) : 0.0;
+      const double r_ready = r_item + r_sum_us(pl.N, rks);
+      const int r_pairs = std::min(n_r, pairs), r_last = r_pairs / rks, others = pairs - r_pairs;
       for (int f = std::max(0, f_max - 1); f <= f_max; ++f) {   // rounds of whole tiles, the rest in ks slices each
         const int full = f * pairs, tail = total - full;
         for (int ks = 1; ks <= std::min(16, G) && (ks == 1 || ks * 4 <= nk); ++ks) {
           if (ks > 1 && (tail == 0 || tail > ctr_room || tile_bytes * tail * ks + r_bytes > room)) break;
-          const double slice = static_cast<double>(nk) / ks * step + tile_us(two);
-          double main;
-          if (f == 0)   // r takes pairs of the first round of items, and the first tiles wait for it before their correction
-            main = cdiv(n_r + tail * ks, pairs) * slice + std::max(0.0, r_us - (static_cast<double>(nk) / ks - nu) * step);
-          else
-            main = f * (nk * step + tile_us(two)) + cdiv(tail * ks, pairs) * slice + r_load + std::max(0.0, r_us - G * step);
-          const double cost = main + slices_us(pl.N, ks) + (two ? 1.0 + 0.008 * pl.N : 0.0);
+          const int items = n_r + (ks > 1 ? full + tail * ks : total);
+          const double step = step_us(pl.N, std::min(1.0, static_cast<double>(items) / pairs)), beside = tile_us(pl.N, two);
+          const double tile = nk * step + beside, slice = static_cast<double>(nk) / ks * step + beside;
+          if (((ks > 1 ? f * pairs : total) * tile + (ks > 1 ? tail * ks * slice : 0.0)) / pairs >= best_cost) continue;
+          // first tiles, and last slices of sliced ones, wait for r before their correction; with one accumulator a pair goes on
+          // when it has added r's slices
+          const double with_r = compute_r ? r_ready + nu * step + beside : 0.0, r_free = two ? r_item : r_ready;
+          // (a pair asks for its next item early in one of r: those that add r's slices take tiles although they are through late)
+          double cost;
+          if (ks == 1) {
+            const double last_r = std::max(r_free + tile, with_r);
+            cost = rounds_us(total, {others, r_pairs - r_last, r_last, 0},
+                             {std::max(tile, with_r), std::max(r_item + tile, with_r), last_r, 0.0}, tile);
+            if (r_last > 0 && total > others) cost = std::max(cost, last_r);
+          } else if (f == 0) {
+            const int last = compute_r ? others / ks : 0;
+            cost = std::max(with_r, rounds_us(tail * ks, {others - last, last, r_pairs - r_last, r_last},
+                                              {slice, std::max(slice, with_r), r_item + slice, r_free + slice}, slice));
+            if (r_last > 0 && tail * ks > others) cost = std::max(cost, r_free + slice);
+          } else {
+            cost = std::max(tile, with_r) + (f - 1) * tile + cdiv(tail * ks + static_cast<int>(n_r * r_item / slice), pairs) * slice;
+          }
+          cost += sum_us(pl.N, ks, f > 0) + (items > pairs ? kTicketUs : 0.0);
           if (cost < best_cost) {
             best_cost = cost;
             best = pl;

@@ -90,8 +90,8 @@ def test_no_slice_of_a_group_of_unlike_members_is_empty(M, ic, rank):
 
 
 # calls of the CTA pairs with ranks above 512 against a short K: (tokens, columns, K, rank, how r comes)
-BEHIND_THE_WEIGHTS = [(65, 20224, 1152, 768, K.R_COMPUTE), (256, 20224, 1536, 1024, K.R_COMPUTE), (400, 5248, 2560, 920, K.R_COMPUTE),
-                      (100, 512, 1536, 1024, K.R_LOAD), (65, 128, 1152, 648, K.R_LOAD)]
+BEHIND_THE_WEIGHTS = [(65, 19200, 1408, 1016, K.R_COMPUTE), (128, 19072, 2560, 976, K.R_COMPUTE), (200, 10240, 2560, 960, K.R_COMPUTE),
+                      (256, 20224, 1536, 1024, K.R_LOAD), (100, 512, 1536, 1024, K.R_LOAD), (65, 128, 1152, 648, K.R_LOAD)]
 
 
 @pytest.mark.parametrize("M,oc,ic,rank,r_mode", BEHIND_THE_WEIGHTS)
