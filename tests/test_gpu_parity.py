@@ -247,10 +247,9 @@ def test_fused_residual_rmsnorm_prologue(ocs, ic, rank, M, with_res):
 @pytest.mark.parametrize("M,ic,rank", [(9, 1152, 8), (16, 2048, 64), (40, 3200, 24), (64, 1024, 136), (65, 2176, 64),
                                        (128, 5120, 128), (129, 2048, 64)])
 def test_r_for_few_tokens_and_the_group_gemm(M, ic, rank):
-    """9..64 tokens compute r = x R^T inside the group launch; 65..128 take it from the small stand-alone launch (one CTA
-    per 16 rows of R x 1024 columns x 64 tokens, K slices added in order by the last CTA to arrive); 129 tokens take the
-    K-sliced GEMM for r.  Ranks that are not multiples of 16, K that is not a multiple of 1024, token counts that do not fill
-    the 64-token blocks; run twice on the same workspace (the arrival counters must be back at zero)."""
+    """r = x R^T inside the group launch: up to 64 tokens by CTAs of their own, above as the first items of the CTA pairs, K slices
+    added in order.  Ranks that are not multiples of 16, K that is not a multiple of 1024, token counts that do not fill the
+    64-token blocks; run twice on the same workspace (the arrival counters must be back at zero)."""
     rng = np.random.default_rng(40 + M)
     lins = [Linear(rng, oc, ic, rank=rank) for oc in (384, 200)]
     R = (np.random.default_rng(41).standard_normal((rank, ic)) * 0.01).astype(np.float16)
@@ -295,9 +294,9 @@ def test_gemm_parity(M, oc, ic, rank, alpha, bias):
 @pytest.mark.parametrize("M,oc,ic,rank,alpha", [(64, 256, 2048, 1024, 1.0), (64, 256, 2048, 1024, 0.5),
                                                 (48, 384, 1024, 512, 1.0), (2560, 4096, 1024, 1024, 1.0)])
 def test_gemm_k_slices_that_start_inside_the_correction_steps(M, oc, ic, rank, alpha):
-    """Large rank against a short K: with the K steps of weights and correction cut into slices, some slices
-    begin (or lie wholly) in the correction steps.  Their first MMA must overwrite the accumulator, and an
-    accumulator a slice never touches must count as zero."""
+    """Large rank against a short K, where up to 64 tokens some K slices begin (or lie wholly) in the correction steps: their first MMA
+    must overwrite the accumulator, and an accumulator a slice never touches must count as zero.  (Above 64 tokens:
+    test_slices_that_start_behind_the_weights; 2560 tokens have whole tiles only.)"""
     rng = np.random.default_rng(M + rank)
     lin = Linear(rng, oc, ic, rank=rank, bias=True)
     x = rng.standard_normal((M, ic)).astype(np.float16)
@@ -529,10 +528,10 @@ def test_toy_model_through_wrappers_matches_reference(golden_toy, monkeypatch, f
 
 
 @pytest.mark.gpu
-def test_gemm_with_a_sliced_last_wave():
-    """160 tiles of 256 x 256 on 148 SMs: one whole wave, and a last wave of 12 tiles that is cut into K slices whose
-    fp32 partial tiles are added by the slot-sum kernel (bias and correction included)."""
-    M, oc, ic, rank = 2560, 4096, 1024, 64
+@pytest.mark.parametrize("M,oc,ic,rank", [(2560, 4096, 1024, 64), (2000, 2560, 5120, 64)])
+def test_gemm_with_a_sliced_last_wave(M, oc, ic, rank):
+    """Tiles that fill the SMs in whole rounds and a last, partly filled one: as whole tiles, and (2000 tokens) cut into K slices
+    whose fp32 partial tiles are added by the last slice (bias and correction included)."""
     rng = np.random.default_rng(7)
     lin = Linear(rng, oc, ic, rank=rank, bias=True)
     x = rng.standard_normal((M, ic)).astype(np.float16)
@@ -547,20 +546,3 @@ def test_gemm_with_a_sliced_last_wave():
         for _ in range(2):   # the second call reuses the slots
             assert run_group(g) == 0 and status_ok(g) == 0
         assert_close(out, lin.oracle(x, R if r_mode != K.R_NONE else None, alpha=1.0), tag="sliced last wave")
-
-
-@pytest.mark.gpu
-def test_cta_pair_variant_in_subprocess():
-    """The two-CTA (cta_group::2) GEMM variant (above 128 tokens) and the swapped-operand variant (65 to 128 tokens)
-    are opt-in through environment variables that the library reads once, so they are exercised in a child
-    interpreter: the GEMM parity tests must pass with both forced on."""
-    import os
-    import subprocess
-    import sys
-    env = dict(os.environ, GLOWQ_GEMM_PAIR="1", GLOWQ_GEMM_SWAP="1")
-    here = os.path.dirname(os.path.abspath(__file__))
-    r = subprocess.run([sys.executable, "-m", "pytest", os.path.join(here, "test_gpu_parity.py"), "-q", "-x", "-m", "gpu",
-                        "-k", "gemm_parity or gemm_group or shared_memory_weight_tile", "-p", "no:cacheprovider"],
-                       env=env, capture_output=True, text=True, timeout=600)
-    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
-    assert " passed" in r.stdout
