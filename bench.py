@@ -522,7 +522,7 @@ def measure_prefill(arm, stack, tokens, steps):
     stack.check_status(pplan)
     fl = stack.algorithmic_flops(tokens, corrected=True)
     out = {"tokens": tokens, "ms": ms_p, "tokens_per_s": tokens / (ms_p * 1e-3), "tflops": fl / (ms_p * 1e-3) / 1e12,
-           "kernel": "gemm_w4a16_kernel (tcgen05)", "flops_per_pass": fl}
+           "kernel": "gemm_pair_kernel (tcgen05)", "flops_per_pass": fl}
     try:
         with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
             mp_ = json.load(f)

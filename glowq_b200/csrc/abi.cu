@@ -285,7 +285,7 @@ int validate_group(const glowq_w4a16_group_t& g) {
   if (g.group_size <= 0 || g.group_size % 8 != 0) return GLOWQ_ERR_BAD_GROUP_SIZE;
   if (g.x_stride < g.IC) return GLOWQ_ERR_BAD_STRIDE;
   if (g.out_dtype != GLOWQ_OUT_F16 && g.out_dtype != GLOWQ_OUT_F32) return GLOWQ_ERR_BAD_ARGUMENT;
-#if !defined(GLOWQ_GEMV_TRACE) && !defined(GLOWQ_GEMM_TRACE)
+#ifndef GLOWQ_GEMV_TRACE
   // reserved fields must be zero: a struct that was not cleared is refused instead of steering anything
   if (g.reserved != 0 || g.reserved2 != 0 || g.reserved3 != 0) return GLOWQ_ERR_BAD_ARGUMENT;
   for (int i = 0; i < g.n_members; ++i)

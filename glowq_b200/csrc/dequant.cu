@@ -1,6 +1,6 @@
 // Whole-weight dequantisation: out[OC, IC] fp16 = half_rn((code - zero) * scale), bit-exact with the
-// reference definition.  The same unpack8_minus_zero + HMUL2 sequence produces the tensor-core
-// kernel's shared-memory weight tiles, so this entry point is the bit-exactness check for both.
+// reference definition.  The tensor-core kernels' weight tiles hold the same bits ((code - zero) exact, one
+// rounding by the product with the scale), so this entry point is the bit-exactness check for them too.
 #include "common.cuh"
 #include "params.h"
 

@@ -5,7 +5,7 @@
 // Up to 64 tokens one CTA per 128 output columns (gemm_tmem.cu), above a CTA pair per 256 (gemm_pair.cu).  Both keep the
 // dequantised weights in tensor memory, and both compute r inside the group launch.  The line lies where the first ends: two CTAs
 // share an SM's tensor memory there, which leaves an accumulator 64 tokens (13B gate/up 45 us at 64 tokens; the pair form, whose
-// tiles have 64 tokens at least, takes 14B gate/up from 71 to 63 us at 70).
+// tiles have 64 tokens at least, takes 14B gate/up at 65 tokens from 67 to 63 us).
 #include <algorithm>
 
 #include "../../include/glowq_w4a16.h"
@@ -70,6 +70,7 @@ inline size_t main_slot_bytes(int M, int OC_total, int n_members) {
 
 size_t gemm_workspace_bytes(int M, int IC, int OC_total, int rank, int n_members) {
   size_t slots = std::max(rank > 0 ? r_slot_bytes(M, IC, rank) : 0, main_slot_bytes(M, OC_total, n_members));
+  // r in a launch of its own (up to 64 tokens); up to 128 the room serves the pairs' slots, which for long rows it lets slice K finer
   if (rank > 0 && M <= 128) slots = std::max(slots, r_product_slot_bytes(M, IC, rank));
   // K slices of the one-CTA form, unless whole tiles fill the SMs and the last round of them is nearly full too
   const int tmem_tiles = cdiv(OC_total, 128), tmem_rest = tmem_tiles % kPlanSms;

@@ -17,9 +17,9 @@
 // output goes to r_buf; the producers wait for the count of finished r tiles before their first correction step.
 //   What bounds it: 256 tokens, the MMAs (1024 clocks a step; measured 1030) and the epilogue that only the next steps' dequantisation
 // runs under; narrower tiles, tensor memory's writes and the chain from a stage's release to its next MMAs (about 1100 clocks a step
-// whatever the width, also with four teams).  Long runs are bound by the 1 kW limit (1.35 to 1.45 GHz).  Corrected group calls, us,
-// before (fp16 weight tile in shared memory, r and slot sum as launches) / now: 14B gate/up 94 / 85 at 211 tokens, 688 / 556 at 2048,
-// 1330 / 1103 at 4096; 14B down_proj 97 / 67, 371 / 316, 742 / 627; 3B q/k/v 36 / 22, 86 / 77, 144 / 132.
+// whatever the width, also with four teams).  Long runs are bound by the 1 kW limit.  Corrected group calls at 211, 2048 and
+// 4096 tokens, us (behind the stroke the form with fp16 weight tiles in shared memory, r and the slot sum as launches): 14B gate/up 70,
+// 551, 1083 / 90, 690, 1328; 14B down_proj 61, 298, 562 / 95, 374, 749; 3B q/k/v 21, 72, 117 / 37, 85, 143.
 //   Items are taken in order from a ticket (or are the clusters themselves where they are few): a CTA waits for items in front of
 // its own only, so a launch gets through on any number of SMs.  K may be sliced; the CTAs of a tile's last slice add the other
 // slices' fp32 slots in slice order (deterministic).  Every wait is bounded; on expiry a status word is set and the CTAs drain.
@@ -72,7 +72,6 @@ struct PtParams {
   int tickets;            // items by ticket (0: every cluster has one)
   uint32_t* tile_ctr;     // [r tiles, then sliced tiles][2 CTAs] arrivals of K slices
   float *slots, *r_slots; // [slice][tile][token / 4][256][4]
-  __half* r_buf;
   int M, G, N, rank, out_fp32, n_members;
   int n_items, n_r, r_x, r_slices, r_tiles;     // items; r items, column tiles, K slices and tiles of r
   int ctr_base;           // tile counters of r in front of those of the sliced tiles
@@ -1145,7 +1144,6 @@ int gemm_pair_forward(const glowq_w4a16_group_t& g, bool compute_r, bool r_only,
   if (compute_r) {
     p.r_tiles = pl.r_tiles;
     p.n_r = pl.r_tiles * pl.r_slices;
-    p.r_buf = static_cast<__half*>(g.r_buf);
     p.ctr_base = pl.r_slices > 1 ? pl.r_tiles : 0;
   }
   p.n_items = p.n_r + (r_only ? 0 : pl.full_tiles + pl.n_tail * pl.ksplit);

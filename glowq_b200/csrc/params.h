@@ -70,7 +70,7 @@ constexpr unsigned kPrefetchSlice = 16u << 10;  // bytes per L2 prefetch request
 
 // Byte ranges of the workspace that a launch uses besides the fixed areas in front of the tile counters, and its partition.
 struct WorkspaceMap {
-  int kernel;                       // 0 weight streaming, 1 tensor-memory GEMM, 2 shared-memory GEMM
+  int kernel;                       // 0 weight streaming, 1 one CTA per tile (9 to 64 tokens), 2 CTA pairs
   int ksplit, whole_tiles, sliced_tiles, r_ctas, shortest;   // shortest: K steps of the member with the fewest
   unsigned long long ctr_begin, ctr_end;       // tile counters, zero between launches
   unsigned long long slots_begin, slots_end;   // partial results: any bits before and after a launch

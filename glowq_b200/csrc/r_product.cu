@@ -1,5 +1,5 @@
-// r = x . R^T (the shared right factor applied to the activations) for 65 to 128 tokens, as ONE small launch in front
-// of the tensor-core group GEMM (up to 64 tokens the group launch computes r itself, unless its workspace has no room).
+// r = x . R^T (the shared right factor applied to the activations) for 9 to 64 tokens, as ONE small launch in front of a group
+// launch whose workspace has no room to compute r itself.
 // The [M, rank] result is a handful of tiles, so the work is cut along K as well:
 // CTA (unit, by) multiplies 16 rows of R with one 1024-column slice of K for 64 tokens (one 8-token block per warp,
 // tokens on the N axis of m16n8k16 MMAs; the R tile is staged in shared memory once, before the wait for the previous
