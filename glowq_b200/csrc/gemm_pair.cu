@@ -1059,7 +1059,7 @@ PairPlan make_pair_plan(const glowq_w4a16_group_t& g, bool compute_r, bool any_c
                                               {slice, std::max(slice, with_r), r_item + slice, r_free + slice}, slice));
             if (r_last > 0 && tail * ks > others) cost = std::max(cost, r_free + slice);
           } else {
-            cost = std::max(tile, with_r) + (f - 1) * tile + cdiv(tail * ks + static_cast<int>(n_r * r_item / slice), pairs) * slice;
+            cost = std::max(tile, with_r) + (f - 1) * tile + cdiv(tail * ks + static_cast<int>(r_pairs * r_item / slice), pairs) * slice;
           }
           cost += sum_us(pl.N, ks, f > 0) + (items > pairs ? kTicketUs : 0.0);
           if (cost < best_cost) {
