@@ -185,6 +185,48 @@ def test_a_wait_that_runs_out_is_reported_and_leaves_the_device_usable():
     assert_close(out, lin.oracle(x, R))
 
 
+_LATE_SCRIPT = r"""
+import numpy as np, torch
+from glowq_b200.cuda_w4a16 import kernels as K
+from gpu_helpers import Linear, assert_close, dev, ext, make_group, new_out, status_ok
+lib, stream = ext().lib, torch.cuda.current_stream().cuda_stream
+p, mem, flags = K.Peers(), [torch.zeros(4096, dtype=torch.float16, device="cuda") for _ in range(2)], torch.zeros(64, dtype=torch.int32, device="cuda")
+for r in range(2):                           # "rank 1" is local memory that nobody ever writes flags into
+    p.buf[r], p.flag[r] = mem[r].data_ptr(), flags.data_ptr() + 16 * r
+p.epoch, p.status = flags.data_ptr() + 64, flags.data_ptr() + 128
+p.world, p.rank, p.sites, p.max_n = 2, 0, 2, 1024
+v = torch.ones(1024, dtype=torch.float16, device="cuda")
+rng = np.random.default_rng(5)
+lin = Linear(rng, 5120, 1024, quantize=False)
+x = rng.standard_normal((1000, 1024)).astype(np.float16)
+late, right = [make_group(dev(x), [lin], [new_out(1000, lin)]) for _ in range(2)]
+assert lib.glowq_w4a16_group_forward(right) == 0 and status_ok(right) == 0    # (the kernel is loaded)
+torch.cuda.synchronize()
+assert lib.glowq_w4a16_allreduce_f16(p, v.data_ptr(), 1024, 0, stream) == 0 and lib.glowq_w4a16_group_forward(late) == 0
+torch.cuda.synchronize()
+print("LATE", status_ok(late), int(flags[32]))
+assert lib.glowq_w4a16_group_forward(right) == 0
+torch.cuda.synchronize()
+assert_close(right._keep[2][0], lin.oracle(x))
+print("RIGHT", status_ok(right))
+"""
+
+
+def test_a_launch_whose_first_waits_run_out():
+    """The warps that run ahead of the kernel before wait for their first item, which comes by ticket when that kernel is complete.  One
+    that lasts longer than their waits (an all-reduce whose second rank never arrives, with a poll limit of some seconds) makes them
+    give up before they have read an item: status 7, nothing faults, and launches on another workspace are right."""
+    import os
+    import subprocess
+    import sys
+    here = os.path.dirname(os.path.abspath(__file__))
+    root = os.path.dirname(here)
+    env = dict(os.environ, GLOWQ_AR_SPIN_LIMIT="6000000", PYTHONPATH=os.pathsep.join((root, here, os.path.join(root, "oracle"))))
+    r = subprocess.run([sys.executable, "-c", _LATE_SCRIPT], env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-2000:]
+    assert "LATE 7 4" in r.stdout and "RIGHT 0" in r.stdout, r.stdout
+
+
 def test_on_a_few_SMs():
     """A stream of 8 SMs: items are taken in order, so no CTA waits for one that cannot start.  The same bits as on the whole device."""
     green = pytest.importorskip("torch.cuda.green_contexts")
