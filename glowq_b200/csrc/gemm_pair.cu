@@ -533,37 +533,35 @@ gemm_pair_kernel(const __grid_constant__ PtParams p, const __grid_constant__ PtM
       const uint32_t idesc = (1u << 4) | ((static_cast<uint32_t>(p.N) >> 3) << 17) | (static_cast<uint32_t>(2 * kRows >> 4) << 24);
       const uint64_t desc0 = smem_desc_sw128(ring);
       const uint32_t hi = static_cast<uint32_t>(desc0 >> 32), lo0 = static_cast<uint32_t>(desc0);
-      bool ok = true, ready = false;   // lane 0's poll
+      bool ok = true;
+      uint32_t ready = 0;   // the elected lane's poll
       const uint32_t acol = tmem + kTmemCols - p.na * 64, stage16 = (2 * sub) >> 4, sub16 = sub >> 4, G = p.G, nb = p.nb, na = p.na;
       uint32_t ai = 0;
-      while (ok && next_item(t, false, true)) {
+      while (ok && __all_sync(0xffffffffu, next_item(t, false, true))) {
         const uint32_t buf = p.nbuf == 2 ? n & 1 : 0, use = p.nbuf == 2 ? n >> 1 : n;
         ++n;
-        bool w = true;
-        if (lane == 0) w = await(kBAccEmpty + 8 * buf, (use & 1) ^ 1);
-        if (!(ok = __all_sync(0xffffffffu, w))) break;
+        if (!(ok = g_mbar_wait_warp<false>(smem0 + kBAccEmpty + 8 * buf, (use & 1) ^ 1, abort_flag, p.status))) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         uint32_t d = tmem + buf * static_cast<uint32_t>(p.N), acc = 0;
-        const uint32_t nk = t.nk, last = G + ((p.rank + 127) >> 7) - 1, last_both = (p.rank & 127) == 0 || (p.rank & 127) > 64;
+        // (what was read from shared memory is the same in all lanes: the compiler learns it from a reduction)
+        const uint32_t it0 = __reduce_or_sync(0xffffffffu, t.it0), nk = __reduce_or_sync(0xffffffffu, t.nk);
+        const uint32_t last = G + ((p.rank + 127) >> 7) - 1, last_both = (p.rank & 127) == 0 || (p.rank & 127) > 64;
         const uint32_t sep_at = p.sep ? G : 0xFFFFFFFFu;
-        if (static_cast<uint32_t>(t.it0) > sep_at) d += p.N;   // a K slice that starts behind the correction's first step
-        for (uint32_t it = t.it0; it < nk; ++it) {
+        if (it0 > sep_at) d += p.N;   // a K slice that starts behind the correction's first step
+        for (uint32_t it = it0; it < nk; ++it) {
           if (it == sep_at) {
             d += p.N;
             acc = 0;
           }
-          if (!__any_sync(0xffffffffu, ready)) {
-            w = true;
-            if (lane == 0) w = spin_bar(smem0 + kBFull + 8 * b.i, b.ph, abort_flag, p.status);
-            if (!(ok = __all_sync(0xffffffffu, w))) break;
-          }
+          if (!__any_sync(0xffffffffu, ready) &&
+              !(ok = g_mbar_wait_warp<true>(smem0 + kBFull + 8 * b.i, b.ph, abort_flag, p.status)))
+            break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           pair_step(d, acol + ai * 64, lo0 + b.i * stage16, hi, sub16, idesc, acc, it < G || it != last || last_both,
                     smem0 + kBDone + 8 * b.i);
           if (++ai == na) ai = 0;
           b.step(nb);
-          if (lane == 0) ready = test_bar(smem0 + kBFull + 8 * b.i, b.ph);
-          __syncwarp();
+          ready = g_mbar_test_elected(smem0 + kBFull + 8 * b.i, b.ph);
           acc = 1;
         }
         if (ok) pair_commit(smem0 + kBAccFull + 8 * buf);

@@ -391,18 +391,16 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
       // stage is still released, and the warp stays converged for the elections.
       bool ok = true;
       auto wait_slow = [&](uint32_t bar, uint32_t ph) {
-        if (lane == 0) ok = ok && g_mbar_wait(bar, ph, abort_flag, p.status);   // (a whole warp's wait: 32 barrier operations)
-        __syncwarp();
+        if (ok) ok = g_mbar_wait_warp<false>(bar, ph, abort_flag, p.status);
       };
       uint32_t acc = 0;
-      bool ready = false;   // lane 0's poll
+      uint32_t ready = 0;   // the elected lane's poll
       for (int it = it0; it < nkp; ++it) {
         if (!__any_sync(0xffffffffu, ready)) wait_slow(full + 8 * b.i, b.ph);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t cur = b.i;
         b.step(1, p.ns);
-        if (lane == 0) ready = test_bar(full + 8 * b.i, b.ph);   // answered while this stage's MMAs are issued
-        __syncwarp();
+        ready = g_mbar_test_elected(full + 8 * b.i, b.ph);   // answered while this stage's MMAs are issued
         umma_ts_step(tmem, tmem + p.a_col + cur * 64, lo0 + cur * ((2 * sub) >> 4), hi, sub >> 4, idesc, acc, empty + 8 * cur);
         acc = 1;
       }
