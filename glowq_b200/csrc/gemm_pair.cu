@@ -627,16 +627,8 @@ gemm_pair_kernel(const __grid_constant__ PtParams p, const __grid_constant__ PtM
           for (int k = 0; k < 4; ++k) lds_v4(w + 4 * k, prow + s.i * kPStage + ((static_cast<uint32_t>(k) ^ psw) << 4));
 #pragma unroll
           for (int half = 0; half < 2; ++half) {
-            // byte i of the word holds codes 2i, 2i + 1: as the low bytes of two halves with exponent byte 0x64 and the other
-            // nibble masked off they are (1024 + n, 1024 + 16 n'), in the order the MMA wants them; one FMA leaves the exact
-            // (n - z, n' - z) and the product with the scale rounds once
             uint32_t v[32];
-#pragma unroll
-            for (int k = 0; k < 8; ++k)
-#pragma unroll
-              for (int i = 0; i < 4; ++i)
-                v[4 * k + i] =
-                    hmul2(hfma2(prmt(w[8 * half + k], 0x64646464u, 0x4040u + 0x0101u * i) & 0x64F0640Fu, 0x2C003C00u, zc), s2);
+            dequant_words(v, w, 8 * half, zc, s2);
             if (half == 0) {
               if (lane == 0) g_mbar_arrive(pempty + 8 * s.i);   // the packed rows are in registers
               await_stage();

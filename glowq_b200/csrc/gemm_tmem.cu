@@ -472,15 +472,7 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
           uint32_t v[32];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            // byte i of the word holds codes 2i, 2i + 1: as the low bytes of two halves with exponent byte 0x64 and the
-            // other nibble masked off they are (1024 + n, 1024 + 16 n'), in the order the MMA wants them; one FMA leaves
-            // the exact (n - z, n' - z) and the product with the scale rounds once
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              v[4 * j + i] = hmul2(hfma2(prmt(w[8 * half + j], 0x64646464u, 0x4040u + 0x0101u * i) & 0x64F0640Fu, 0x2C003C00u, zc), s2);
-          }
+          dequant_words(v, w, 8 * half, zc, s2);
           if (half == 0) {   // the MMAs that read this stage's A tile before are done
             if (!have_e) ok = ok && g_mbar_wait(empty + 8 * a.i, a.ph ^ 1, abort_flag, p.status);
             __syncwarp();
