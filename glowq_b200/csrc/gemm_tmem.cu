@@ -84,7 +84,7 @@ struct TsParams {
   float* r_slots;       // [CTA of r][token][128] fp32
   __half* r_buf;
   int n_r, r_slices, rank, nkr;   // CTAs of r (the lowest block indices; 0: r is ready), K slices of an R tile, 64-column steps of K
-  float* slots;         // [ksplit][sliced tile][token][128] fp32
+  float* slots;         // [ksplit][sliced tile][token / 4][128][4] fp32
   int M, G, out_fp32, n_members;
   int N;                // tokens per tile (multiple of 16)
   int ns, np;           // ring depths: stages (an activation tile and a tensor-memory A tile each), packed weights
@@ -107,12 +107,10 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
       "r"(r[31])
       : "memory");
 }
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
 }
 
 // The MMAs of one step and the commit that releases its stage, issued by one elected lane of a converged warp.  The whole
@@ -497,8 +495,8 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
     const int ntok = min(p.N, p.M - m0);
     const size_t slot_floats = static_cast<size_t>(p.N) * kRows;
     const int sl_tile = tile_lin - p.full_tiles;
-    const size_t slice_floats = static_cast<size_t>(p.n_tail) * slot_floats;
-    float* const slot0 = (r_cta ? p.r_slots + blockIdx.x * slot_floats : p.slots + sl_tile * slot_floats) + rloc;
+    const size_t slice_v4 = static_cast<size_t>(p.n_tail) * (slot_floats / 4);
+    float4* const slot0 = reinterpret_cast<float4*>(p.slots + (r_cta ? 0 : sl_tile * slot_floats)) + rloc;
     const bool park = r_cta || zslice < ks - 1, finish = ks > 1 && zslice == ks - 1;
     auto await_count = [&](uint32_t* ctr, uint32_t n) {   // one thread; acquires the slots of the CTAs that counted
       uint32_t spins = 0;
@@ -521,23 +519,31 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
     }
     // With a separate correction accumulator, a K slice that lies wholly in one phase never writes the other's.
     const bool has_main = it0 < p.G || !sep, has_lr = sep && nk > p.G;
-    const float bias = (rvalid && !r_cta && mb.bias) ? __half2float(mb.bias[row]) : 0.f;
+    const float bias = (rvalid && !park && mb.bias) ? __half2float(mb.bias[row]) : 0.f;
+    // Eight tokens at a time, alternately by the teams; four slots in flight (their tokens past the last one are not used).
     bool waited = false;
-    for (int t0 = team * 16; t0 < ntok; t0 += 16 * kTeams) {
-      float sum[16];
+    for (int t0 = team * 8; t0 < ntok; t0 += 8 * kTeams) {
+      float sum[8];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) sum[j] = 0.f;
+      for (int j = 0; j < 8; ++j) sum[j] = bias;
+      float4* const at = slot0 + (t0 >> 2) * kRows;
       if (finish) {
-        const float* src = slot0 + static_cast<size_t>(t0) * kRows;
-        for (int z = 0; z < ks - 1; z += 2, src += 2 * slice_floats) {   // two slots in flight (rows past ntok: not used)
-          float u[2][16];
+        for (int z = 0; z < ks - 1; z += 4) {
+          float4 u[4][2];
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            u[0][j] = __ldcg(src + j * kRows);
-            u[1][j] = z + 1 < ks - 1 ? __ldcg(src + slice_floats + j * kRows) : 0.f;
-          }
+          for (int k = 0; k < 4; ++k)
 #pragma unroll
-          for (int j = 0; j < 16; ++j) sum[j] = (sum[j] + u[0][j]) + u[1][j];
+            for (int h = 0; h < 2; ++h)
+              u[k][h] = z + k < ks - 1 ? __ldcg(at + (z + k) * slice_v4 + h * kRows) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              sum[4 * h] += u[k][h].x;
+              sum[4 * h + 1] += u[k][h].y;
+              sum[4 * h + 2] += u[k][h].z;
+              sum[4 * h + 3] += u[k][h].w;
+            }
         }
       }
       if (!waited) {   // the first batch of slots is on its way while the last MMAs run
@@ -546,26 +552,41 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         waited = true;
       }
-      uint32_t acc[16], lr[16];
-      tmem_ld16(lane_base + t0, acc);
-      if (sep) tmem_ld16(lane_base + p.N + t0, lr);
+      uint32_t acc[8], lr[8];
+      tmem_ld8(lane_base + t0, acc);
+      if (has_lr) tmem_ld8(lane_base + p.N + t0, lr);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       if (!ok) continue;
+      if (has_main) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        if (t0 + j < ntok) {
-          float v = has_main ? __uint_as_float(acc[j]) : 0.f;
-          if (has_lr) v = fmaf(mb.alpha, __uint_as_float(lr[j]), v);
-          if (park) {
-            __stcg(slot0 + (r_cta ? 0 : zslice * slice_floats) + static_cast<size_t>(t0 + j) * kRows, v);
-          } else if (rvalid) {
-            const size_t idx = static_cast<size_t>(m0 + t0 + j) * mb.out_stride + row;
-            v += sum[j] + bias;
-            if (p.out_fp32)
-              static_cast<float*>(mb.out)[idx] = v;
-            else
-              static_cast<__half*>(mb.out)[idx] = __float2half_rn(v);
-          }
+        for (int j = 0; j < 8; ++j) sum[j] += __uint_as_float(acc[j]);
+      }
+      if (has_lr) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) sum[j] = fmaf(mb.alpha, __uint_as_float(lr[j]), sum[j]);
+      }
+      const int n = ntok - t0;
+      if (r_cta) {
+        float* o = p.r_slots + blockIdx.x * slot_floats + static_cast<size_t>(t0) * kRows + rloc;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (j < n) __stcg(o + j * kRows, sum[j]);
+      } else if (park) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          __stcg(at + zslice * slice_v4 + h * kRows, make_float4(sum[4 * h], sum[4 * h + 1], sum[4 * h + 2], sum[4 * h + 3]));
+      } else if (rvalid) {
+        const size_t idx = static_cast<size_t>(m0 + t0) * mb.out_stride + row;
+        if (p.out_fp32) {
+          float* o = static_cast<float*>(mb.out) + idx;
+#pragma unroll
+          for (int j = 0; j < 8; ++j, o += mb.out_stride)
+            if (j < n) *o = sum[j];
+        } else {
+          __half* o = static_cast<__half*>(mb.out) + idx;
+#pragma unroll
+          for (int j = 0; j < 8; ++j, o += mb.out_stride)
+            if (j < n) *o = __float2half_rn(sum[j]);
         }
       }
     }
