@@ -56,6 +56,7 @@ constexpr int kTeams = 2;
 constexpr int kDequantWarps = 4 * kTeams, kCtrlWarps = 3, kThreads = 32 * (kCtrlWarps + kDequantWarps);
 constexpr int kTmemCols = 256;                // per CTA: two share an SM
 constexpr int kSmemBytes = 112 * 1024;
+constexpr int kSlotsAhead = 4;                // slots of a tile that a thread has in flight (two 16-byte loads each)
 constexpr int kMaxRCtas = 48;                 // CTAs that compute r
 // Polls of a count of finished CTAs: some seconds, because another stream's kernel may hold the SMs that the rest of the CTAs
 // of r need (they are placed first, so that nothing of this launch does).
@@ -173,8 +174,8 @@ struct Ring {
   }
 };
 
-// One share of the sum over an R tile's slots: four lanes per four elements, each a quarter of the slots (up to 12 loads in
-// flight), added in a fixed order.
+// One share of the sum over an R tile's slots, added in a fixed order: a lane takes up to 12 slots of four elements, all in flight, and
+// where there are more, two or four lanes share them.
 struct ShareArgs {
   const float* base;
   __half* r_buf;
@@ -182,31 +183,32 @@ struct ShareArgs {
   int r_slices, rank, n0, units;
 };
 __device__ __forceinline__ void add_share(const ShareArgs& a, int share, int et) {
-  const int quarter = (a.r_slices + 3) >> 2, zq = (et & 3) * quarter, stride = a.r_slices * (kDequantWarps * 8);
-  for (int i0 = 0; i0 < a.units; i0 += stride) {   // (the same number of rounds for all lanes: they exchange sums)
-    const int i = i0 + share * (kDequantWarps * 8) + (et >> 2);
+  constexpr int kSlots = kMaxRCtas / 4;
+  const int log = a.r_slices <= kSlots ? 0 : a.r_slices <= 2 * kSlots ? 1 : 2;   // log2 of the lanes per four elements
+  const int part = (a.r_slices + (1 << log) - 1) >> log, zq = (et & ((1 << log) - 1)) * part, per = (kDequantWarps * 32) >> log;
+  for (int i0 = 0; i0 < a.units; i0 += a.r_slices * per) {   // (the same number of rounds for all lanes: they exchange sums)
+    const int i = i0 + share * per + (et >> log);
     const int tok = i >> 5, c4 = (i & 31) * 4, col = a.n0 + c4;
     const float* src = a.base + static_cast<size_t>(tok) * kRows + c4;
-    float4 s = make_float4(0.f, 0.f, 0.f, 0.f), u[kMaxRCtas / 4];
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f), u[kSlots];
 #pragma unroll
-    for (int z = 0; z < kMaxRCtas / 4; ++z)
-      u[z] = (i < a.units && z < quarter && zq + z < a.r_slices) ? __ldcg(reinterpret_cast<const float4*>(src + (zq + z) * a.slot_floats))
-                                                                 : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int z = 0; z < kSlots; ++z)
+      u[z] = (i < a.units && z < part && zq + z < a.r_slices) ? __ldcg(reinterpret_cast<const float4*>(src + (zq + z) * a.slot_floats))
+                                                              : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int z = 0; z < kMaxRCtas / 4; ++z) {
+    for (int z = 0; z < kSlots; ++z) {
       s.x += u[z].x;
       s.y += u[z].y;
       s.z += u[z].z;
       s.w += u[z].w;
     }
-#pragma unroll
-    for (int o = 1; o <= 2; o <<= 1) {
+    for (int o = 1; o < (1 << log); o <<= 1) {
       s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
       s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
       s.z += __shfl_xor_sync(0xffffffffu, s.z, o);
       s.w += __shfl_xor_sync(0xffffffffu, s.w, o);
     }
-    if ((et & 3) == 0 && i < a.units && col < a.rank) {   // the rank is a multiple of 8
+    if ((et & ((1 << log) - 1)) == 0 && i < a.units && col < a.rank) {   // the rank is a multiple of 8
       const __half2 lo = __floats2half2_rn(s.x, s.y), hi = __floats2half2_rn(s.z, s.w);
       *reinterpret_cast<uint2*>(a.r_buf + static_cast<size_t>(tok) * a.rank + col) =
           make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
@@ -528,15 +530,15 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
       for (int j = 0; j < 8; ++j) sum[j] = bias;
       float4* const at = slot0 + (t0 >> 2) * kRows;
       if (finish) {
-        for (int z = 0; z < ks - 1; z += 4) {
-          float4 u[4][2];
+        for (int z = 0; z < ks - 1; z += kSlotsAhead) {
+          float4 u[kSlotsAhead][2];
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
+          for (int k = 0; k < kSlotsAhead; ++k)
 #pragma unroll
             for (int h = 0; h < 2; ++h)
               u[k][h] = z + k < ks - 1 ? __ldcg(at + (z + k) * slice_v4 + h * kRows) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
+          for (int k = 0; k < kSlotsAhead; ++k)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
               sum[4 * h] += u[k][h].x;
@@ -727,12 +729,11 @@ TmemPlan make_tmem_plan(const glowq_w4a16_group_t& g, bool compute_r, bool any_c
   pl.nk_min = nk_min;
   const int units = sms, resident = 2 * sms;
   const size_t item_bytes = static_cast<size_t>(pl.N) * kRows * 4;
-  // Work partition: f rounds of whole tiles, the rest cut into ks slices of K.  Cost in microseconds, fitted on B200: an SM
-  // takes 0.33 per step while two CTAs share it (0.5 alone), 2.5 per wave of items for prologue and epilogue (the CTAs of r
-  // take slots, but are gone before a whole tile is done), and the slices of a tile are added through memory.  Measured at
-  // 16 tokens on the 13B shapes: q/k/v 30.2 whole, 22.8 in two slices, 30.5 in three; o_proj 24.8 whole, 19.1 / 15.8 /
-  // 15.5 in two / three / five, 19.1 in seven (a second wave behind the CTAs of r); gate/up 35.5 whole, 43.2 in two slices,
-  // 33.8 with one round whole and the other 68 tiles in two slices.
+  // Work partition: f rounds of whole tiles, the rest cut into ks slices of K.  Microseconds, fitted on B200 to every partition of 108
+  // group calls (the one taken is 1.2 % slower than the best on average): a step of an SM while two CTAs share it, or of a CTA alone; r,
+  // which the last steps wait for; a second wave of items (the CTAs of r take slots, but are gone before a whole tile is done); the
+  // slices of a tile, which go through memory.
+  const double r_us = compute_r ? 3.9 + 0.052 * pl.N : 0.0;
   pl.full_tiles = total;
   pl.n_tail = 0;
   pl.ksplit = 1;
@@ -744,8 +745,9 @@ TmemPlan make_tmem_plan(const glowq_w4a16_group_t& g, bool compute_r, bool any_c
       if (ks > 1 && (tail == 0 || tail > kTileCtrWords || static_cast<size_t>(tail) * ks * item_bytes > slot_bytes)) break;
       const int items = full + tail * ks;
       const double load = static_cast<double>(f) * nk + static_cast<double>(cdiv(tail * ks, units)) * nk / ks;
-      const double cost = load * (items > units ? 0.33 : 0.5) + 2.5 * cdiv(items, f > 0 ? resident : std::max(units, resident - pl.n_r)) +
-                          (ks > 1 ? 1.5 + 0.006 * pl.N * ks : 0.0);
+      const double cost = std::max(load * (items > units ? 0.283 + 0.0012 * pl.N : 0.492 + 0.0012 * pl.N), r_us) +
+                          5.1 * (cdiv(items, f > 0 ? resident : std::max(units, resident - pl.n_r)) - 1) +
+                          (ks > 1 ? 1.0 + 0.0122 * pl.N * ks + 0.0129 * pl.N : 0.0);
       if (cost < best) {
         best = cost;
         pl.ksplit = ks;
