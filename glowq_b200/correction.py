@@ -117,7 +117,7 @@ class GroupLauncher:
 
     def _plan(self, m: int, device) -> dict:
         first = self.members[0]
-        key = (m, device, first.inner._out_dtype)
+        key = (m, device, first._modules["inner"]._out_dtype)
         plan = self._plans.get(key)
         if plan is None:
             ext = first.inner._get_ext()
@@ -136,46 +136,58 @@ class GroupLauncher:
             oc_total = sum(w.inner.out_features for w in self.members)
             ws = ext.new_workspace(ext.workspace_bytes(m, grp.IC, oc_total, rank, len(self.members)), device)
             grp.workspace, grp.workspace_bytes = ws.data_ptr(), ws.numel()
-            plan = {"grp": grp, "r_buf": r_buf, "ws": ws, "ext": ext}
+            plan = {"grp": grp, "r_buf": r_buf, "ws": ws, "ext": ext, "address": ctypes.addressof(grp)}
             self._plans[key] = plan
         return plan
 
     def descriptor_address(self, m: int, device, dtype) -> Optional[int]:
         plan = self._plans.get((m, device, dtype))
-        return None if plan is None else ctypes.addressof(plan["grp"])
+        return None if plan is None else plan["address"]
 
     def run(self, x: torch.Tensor) -> torch.Tensor:
         """Called by the first member: launch the whole group, keep the other members' outputs, return its own."""
         first = self.members[0]
-        inner = first.inner
+        inners = [w._modules["inner"] for w in self.members]   # (nn.Module.__getattr__ takes half a microsecond)
+        inner = inners[0]
         x2d = inner._flatten_input(x)
-        m, dev = x2d.size(0), x2d.device
-        outs = [torch.empty((m, w.inner.out_features), dtype=inner._out_dtype, device=dev) for w in self.members]
+        m, dev, dtype = x2d.size(0), x2d.device, inner._out_dtype
+        outs = [torch.empty((m, lin.out_features), dtype=dtype, device=dev) for lin in inners]
         self._pending.clear()
+        key = _x_key(x)
         if m > 0:
             plan = self._plan(m, dev)
-            grp, ext = plan["grp"], plan["ext"]
-            grp.x, grp.x_stride = x2d.data_ptr(), x2d.stride(0)
-            for i, (w, o) in enumerate(zip(self.members, outs)):
-                on = w.alpha_svd != 0.0 and not w._mismatch
-                w.inner.fill_member(grp.members[i], o, w.A_q if on else None, float(w.alpha_svd) if on else 0.0)
-            nxt = self.next_launcher
-            grp.next = nxt.descriptor_address(m, dev, inner._out_dtype) if nxt is not None else None
-            with torch.cuda.device(dev):
-                grp.stream = torch.cuda.current_stream(dev).cuda_stream
-                ext.check(ext.lib.glowq_w4a16_group_forward(grp), "glowq_w4a16_group_forward")
-                if inner._check_status:
-                    ext.check(ext.lib.glowq_w4a16_read_status(grp.workspace, grp.stream), "device status")
+            if torch.cuda.current_device() == dev.index:
+                self._launch(plan, x2d, inners, outs, m, dev, dtype)
+            else:
+                with torch.cuda.device(dev):
+                    self._launch(plan, x2d, inners, outs, m, dev, dtype)
             self._keep = x2d          # the launch reads x2d asynchronously
-        key = _x_key(x)
-        cache = first.group_cache if first.is_group else None
-        if cache is not None and m > 0:
-            cache.set(self._plans[(m, dev, inner._out_dtype)]["r_buf"], len(self.members) - 1, key)
-        lead = x.shape[:-1]
+            if first.is_group and first.group_cache is not None:
+                first.group_cache.set(plan["r_buf"], len(self.members) - 1, key)
+        flat = x.dim() == 2
         for w, o in zip(self.members[1:], outs[1:]):
-            self._pending[id(w)] = o.reshape(*lead, w.inner.out_features)
+            self._pending[id(w)] = o if flat else o.reshape(*x.shape[:-1], o.size(1))
         self._pending_key = key
-        return outs[0].reshape(*lead, inner.out_features)
+        return outs[0] if flat else outs[0].reshape(*x.shape[:-1], inner.out_features)
+
+    def _launch(self, plan, x2d, inners, outs, m, dev, dtype) -> None:
+        grp, ext = plan["grp"], plan["ext"]
+        grp.x, grp.x_stride = x2d.data_ptr(), x2d.stride(0)
+        at = K.Group.members.offset
+        for w, lin, o in zip(self.members, inners, outs):
+            alpha = float(w.alpha_svd)
+            if alpha != 0.0 and not w._mismatch:
+                fields = lin.pack_member(o, w._buffers["A_q"], alpha)
+            else:
+                fields = lin.pack_member(o)
+            K.PACK_MEMBER.pack_into(grp, at, *fields)
+            at += K.PACK_MEMBER.size
+        nxt = self.next_launcher
+        grp.next = nxt.descriptor_address(m, dev, dtype) if nxt is not None else None
+        grp.stream = stream = K.current_stream_ptr(dev)
+        ext.check(ext.lib.glowq_w4a16_group_forward(grp), "glowq_w4a16_group_forward")
+        if inners[0]._check_status:
+            ext.check(ext.lib.glowq_w4a16_read_status(grp.workspace, stream), "device status")
 
     def forget(self) -> None:
         self._pending.clear()

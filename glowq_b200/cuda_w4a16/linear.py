@@ -175,25 +175,23 @@ class CudaW4A16Linear(nn.Module):
             raise ValueError(f"Input dim mismatch: got {x.shape[-1]}, expected {self.in_features}")
         if not x.is_cuda:
             raise RuntimeError("CudaW4A16Linear runs on CUDA (sm_100) tensors only; there is no CPU path")
-        x2d = x.reshape(-1, x.shape[-1])
+        x2d = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
         if x2d.dtype != torch.float16:
             x2d = x2d.to(torch.float16)
         return x2d.contiguous()
 
-    def fill_member(self, mem: "K.Member", out: torch.Tensor, L: Optional[torch.Tensor] = None, alpha: float = 0.0):
-        mem.qweight = self.qweight_i32.data_ptr()
-        mem.scales = self.scales_f16.data_ptr()
-        mem.qzeros = self.qzeros_i32.data_ptr()
-        mem.bias = self.bias.data_ptr() if self.bias is not None else None
-        mem.L = L.data_ptr() if L is not None else None
-        mem.out = out.data_ptr()
-        mem.OC = self.out_features
-        mem.weight_stride_i32 = self.qweight_i32.stride(0)
-        mem.zero_stride_i32 = self.qzeros_i32.stride(0)
-        mem.scale_stride = self.scales_f16.stride(0)
-        mem.L_stride = L.stride(0) if L is not None else 0
-        mem.out_stride = out.stride(0)
-        mem.alpha = float(alpha)
+    def pack_member(self, out: torch.Tensor, L: Optional[torch.Tensor] = None, alpha: float = 0.0) -> tuple:
+        """The fields of a ``Member`` in order (``kernels.PACK_MEMBER``).  Buffers are looked up in their dictionary:
+        ``nn.Module.__getattr__`` takes half a microsecond each."""
+        bufs = self._buffers
+        try:
+            qw, sc, qz = bufs["qweight_i32"], bufs["scales_f16"], bufs["qzeros_i32"]
+        except KeyError:
+            qw, sc, qz = self.qweight_i32, self.scales_f16, self.qzeros_i32
+        bias = self._parameters["bias"] if "bias" in self._parameters else self.bias
+        return (qw.data_ptr(), sc.data_ptr(), qz.data_ptr(), bias.data_ptr() if bias is not None else 0,
+                L.data_ptr() if L is not None else 0, out.data_ptr(), self.out_features, qw.stride(0), qz.stride(0), sc.stride(0),
+                L.stride(0) if L is not None else 0, out.stride(0), alpha, 0)
 
     def workspace_for(self, m: int, rank: int, device) -> torch.Tensor:
         key = (m, rank, device)
@@ -212,34 +210,35 @@ class CudaW4A16Linear(nn.Module):
         ``glowq_b200.tp.PeerAllReduce`` - a row-split tensor-parallel shard then also stores its result into every
         rank's staging slot of ``push_site`` (complete the sum with ``push.finish(out, push_site)``)."""
         ext = self._get_ext()
-        m = x2d.size(0)
-        out = torch.empty((m, self.out_features), dtype=self._out_dtype, device=x2d.device)
+        m, dev = x2d.size(0), x2d.device
+        out = torch.empty((m, self.out_features), dtype=self._out_dtype, device=dev)
         if m == 0:
             return out
-        rank = 0 if r_mode == K.R_NONE else int(L.size(1))
-        grp = K.Group()
-        grp.x = x2d.data_ptr()
-        grp.M, grp.IC, grp.x_stride = m, self.in_features, x2d.stride(0)
-        grp.group_size = self.group_size
-        grp.rank, grp.r_mode = rank, r_mode
-        if r_mode != K.R_NONE:
-            grp.R = R.data_ptr() if R is not None else None
-            grp.R_stride = R.stride(0) if R is not None else 0
-            grp.r_buf = r_buf.data_ptr()
-        grp.out_dtype = K.OUT_F32 if self._out_dtype == torch.float32 else K.OUT_F16
-        grp.kernel = self.kernel_choice(m)
-        grp.n_members = 1
-        if push is not None:
-            grp.push, grp.push_site = push.descriptor_address(), int(push_site)
-        self.fill_member(grp.members[0], out, L if r_mode != K.R_NONE else None, alpha)
-        with torch.cuda.device(x2d.device):
-            ws = self.workspace_for(m, rank, x2d.device)
-            grp.workspace, grp.workspace_bytes = ws.data_ptr(), ws.numel()
-            grp.stream = torch.cuda.current_stream(x2d.device).cuda_stream
-            ext.check(ext.lib.glowq_w4a16_group_forward(grp), "glowq_w4a16_group_forward")
-            if self._check_status:   # debugging aid: synchronises the stream after every launch
-                ext.check(ext.lib.glowq_w4a16_read_status(grp.workspace, grp.stream), "device status")
+        if torch.cuda.current_device() == dev.index:
+            self._launch(ext, x2d, out, m, dev, L, R, r_buf, r_mode, alpha, push, push_site)
+        else:
+            with torch.cuda.device(dev):
+                self._launch(ext, x2d, out, m, dev, L, R, r_buf, r_mode, alpha, push, push_site)
         return out
+
+    def _launch(self, ext, x2d, out, m, dev, L, R, r_buf, r_mode, alpha, push, push_site) -> None:
+        rank = r_ptr = r_stride = rb_ptr = 0
+        if r_mode != K.R_NONE:
+            rank = int(L.size(1))
+            if R is not None:
+                r_ptr, r_stride = R.data_ptr(), R.stride(0)
+            rb_ptr = r_buf.data_ptr()
+        else:
+            L = None
+        ws = self.workspace_for(m, rank, dev)
+        stream = K.current_stream_ptr(dev)
+        grp = K.PACK_GROUP.pack(
+            x2d.data_ptr(), r_ptr, rb_ptr, ws.data_ptr(), ws.numel(), stream, m, self.in_features, K.int32(x2d.stride(0)), r_stride, rank,
+            self.group_size, r_mode, K.OUT_F32 if self._out_dtype == torch.float32 else K.OUT_F16, self.kernel_choice(m), 1, 0, 0, 0,
+            push.descriptor_address() if push is not None else 0, int(push_site) if push is not None else 0, 0, 0, 0, 0, 0.0, 0)
+        ext.check(ext.group_forward_packed(grp + K.PACK_MEMBER.pack(*self.pack_member(out, L, alpha))), "glowq_w4a16_group_forward")
+        if self._check_status:   # debugging aid: synchronises the stream after every launch
+            ext.check(ext.lib.glowq_w4a16_read_status(ws.data_ptr(), stream), "device status")
 
     # ------------------------------------------------------------------ reference-named entry points
     def _run_cuda_gemv(self, x2d: torch.Tensor) -> torch.Tensor:
@@ -251,9 +250,8 @@ class CudaW4A16Linear(nn.Module):
                                                        int(self.group_size), _env_int("W4A16_SPLIT_K_ITERS", default=1))
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        lead = x.shape[:-1]
         out = self.launch(self._flatten_input(x))
-        return out.reshape(*lead, self.out_features)
+        return out if x.dim() == 2 else out.reshape(*x.shape[:-1], self.out_features)
 
     def _dequant_full_weight_fallback(self) -> torch.Tensor:
         """[OC, in_features] fp16 dequantised weight (bit-exact with linear.py:240-253), on the device."""
