@@ -200,10 +200,13 @@ class _Ext:
         qweight = torch.empty((oc, groups * (group_size // 8)), dtype=torch.int32, device=weight.device)
         qzeros = torch.empty((oc, (groups + 7) // 8), dtype=torch.int32, device=weight.device)
         scales = torch.empty((oc, groups), dtype=torch.float16, device=weight.device)
-        with torch.cuda.device(weight.device):
-            rc = self.lib.glowq_w4a16_quantize(weight.data_ptr(), qweight.data_ptr(), qzeros.data_ptr(), scales.data_ptr(),
-                                               oc, ic, int(group_size), max(weight.stride(0), ic),
-                                               torch.cuda.current_stream(weight.device).cuda_stream)
+        args = (weight.data_ptr(), qweight.data_ptr(), qzeros.data_ptr(), scales.data_ptr(), oc, ic, int(group_size),
+                max(weight.stride(0), ic), current_stream_ptr(weight.device))
+        if torch.cuda.current_device() == weight.device.index:
+            rc = self.lib.glowq_w4a16_quantize(*args)
+        else:
+            with torch.cuda.device(weight.device):
+                rc = self.lib.glowq_w4a16_quantize(*args)
         self.check(rc, "glowq_w4a16_quantize")
         return qweight, qzeros, scales
 

@@ -123,30 +123,28 @@ class CudaW4A16Linear(nn.Module):
 
     def __init__(self, in_features: int, out_features: int, group_size: int = 128, bias: bool = False):
         super().__init__()
-        self.in_features = int(in_features)
-        self.out_features = int(out_features)
-        self.group_size = int(group_size)
-        if self.group_size <= 0 or self.group_size % 8 != 0:
-            raise ValueError("group_size must be > 0 and a multiple of 8 for GlowQ int32 int4 packing")
-        groups = math.ceil(self.in_features / self.group_size)
-        groups_packed = (groups + 7) // 8
+        self._configure(in_features, out_features, group_size)
         self.register_buffer("qweight_i32", torch.empty(self.out_features, (self.in_features + 7) // 8, dtype=torch.int32))
-        self.register_buffer("qzeros_i32", torch.empty(self.out_features, max(1, groups_packed), dtype=torch.int32))
-        self.register_buffer("scales_f16", torch.empty(self.out_features, groups, dtype=torch.float16))
+        self.register_buffer("qzeros_i32", torch.empty(self.out_features, max(1, self.groups_packed), dtype=torch.int32))
+        self.register_buffer("scales_f16", torch.empty(self.out_features, self.groups, dtype=torch.float16))
         self.register_buffer("gid", torch.arange(self.in_features, dtype=torch.long) // self.group_size, persistent=False)
-        self.groups = groups
-        self.groups_packed = groups_packed
         self.bias = nn.Parameter(torch.empty(self.out_features, dtype=torch.float16)) if bias else None
 
-        self._ext = None
-        # -1: the knob is unset and the library's own switch-over applies
-        self._gemv_threshold = _env_int("W4A16_GEMV_M_MAX", "CUDA_MIXED_GEMV_M_MAX", default=-1)
-        self._force_gemm = _env_flag("W4A16_FORCE_GEMM", "CUDA_MIXED_FORCE_GEMM")
-        self._force_gemv = _env_flag("W4A16_FORCE_GEMV", "CUDA_MIXED_FORCE_GEMV") or _env_flag("W4A16_USE_GEMV")
-        self._out_dtype = _get_kernel_out_dtype()
-        self._check_status = _env_flag("GLOWQ_CHECK_STATUS")
-        self._ws: Optional[torch.Tensor] = None      # scratch for plain (uncorrected) calls
-        self._ws_key = None
+    def _configure(self, in_features: int, out_features: int, group_size: int) -> None:
+        """Sizes and knobs.  (Plain values go to the module's dictionary at once: nn.Module.__setattr__ takes microseconds each.)"""
+        in_features, out_features, group_size = int(in_features), int(out_features), int(group_size)
+        if group_size <= 0 or group_size % 8 != 0:
+            raise ValueError("group_size must be > 0 and a multiple of 8 for GlowQ int32 int4 packing")
+        groups = math.ceil(in_features / group_size)
+        self.__dict__.update(
+            in_features=in_features, out_features=out_features, group_size=group_size, groups=groups, groups_packed=(groups + 7) // 8,
+            _ext=None,
+            # -1: the knob is unset and the library's own switch-over applies
+            _gemv_threshold=_env_int("W4A16_GEMV_M_MAX", "CUDA_MIXED_GEMV_M_MAX", default=-1),
+            _force_gemm=_env_flag("W4A16_FORCE_GEMM", "CUDA_MIXED_FORCE_GEMM"),
+            _force_gemv=_env_flag("W4A16_FORCE_GEMV", "CUDA_MIXED_FORCE_GEMV") or _env_flag("W4A16_USE_GEMV"),
+            _out_dtype=_get_kernel_out_dtype(), _check_status=_env_flag("GLOWQ_CHECK_STATUS"),
+            _ws=None, _ws_key=None)      # scratch for plain (uncorrected) calls
 
     def extra_repr(self) -> str:
         return (f"in_features={self.in_features}, out_features={self.out_features}, "
@@ -261,7 +259,23 @@ class CudaW4A16Linear(nn.Module):
     @classmethod
     def from_float(cls, linear_layer: nn.Linear, group_size: int):
         dev = linear_layer.weight.device
-        with torch.device(dev):    # buffers made where they stay: copying empty ones from the host took longer than quantising
+        if cls is CudaW4A16Linear:
+            # The same module without the buffers that the constructor makes only for them to be replaced: made on the host, moved
+            # and replaced they took longer than quantising (140 us a module; 50 so, most of it the launch and the group index).
+            mod = cls.__new__(cls)
+            nn.Module.__init__(mod)
+            mod._configure(linear_layer.in_features, linear_layer.out_features, group_size)
+            qweight, qzeros, scales, _ = _quantize_per_group_w4(linear_layer.weight.data.to(torch.float16), group_size)
+            gid = torch.arange(mod.in_features, dtype=torch.long, device=dev) // mod.group_size
+            mod._buffers.update(qweight_i32=qweight, qzeros_i32=qzeros, scales_f16=scales, gid=gid)
+            mod._non_persistent_buffers_set.add("gid")
+            if linear_layer.bias is None:
+                mod.__dict__["bias"] = None
+            else:
+                mod.bias = nn.Parameter(torch.empty(mod.out_features, dtype=torch.float16, device=dev))
+                mod.bias.data.copy_(linear_layer.bias.data.to(torch.float16))
+            return mod
+        with torch.device(dev):    # a subclass: its constructor
             mod = cls(linear_layer.in_features, linear_layer.out_features, group_size,
                       bias=linear_layer.bias is not None).to(dev)
         mod.qweight_i32, mod.qzeros_i32, mod.scales_f16, _ = _quantize_per_group_w4(
