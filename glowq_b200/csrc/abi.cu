@@ -21,6 +21,7 @@ cudaError_t launch_dequant(const int32_t* qweight, const __half* scales, const i
 cudaError_t launch_quantize(const __half* w, int32_t* qweight, int32_t* qzeros, __half* scales, int OC, int IC,
                             long long w_stride, cudaStream_t stream);
 bool gemm_supported(const glowq_w4a16_group_t& g);
+double gemm_exact_us(const glowq_w4a16_group_t& g, int sms);
 size_t gemm_workspace_bytes(int M, int IC, int OC_total, int rank, int n_members);
 unsigned allreduce_spin_limit();
 int gemm_group_forward(const glowq_w4a16_group_t& g, cudaStream_t stream, cudaError_t* cuda_err);
@@ -38,6 +39,40 @@ namespace glowq {
 int tensor_map_2d_ex(CUtensorMap* out, CUtensorMapDataType dtype, const void* ptr, uint64_t dim0, uint64_t dim1,
                      uint64_t stride_bytes, uint32_t box0, uint32_t box1, int swizzle) {
   return tensor_map_2d(out, dtype, ptr, dim0, dim1, stride_bytes, box0, box1, swizzle);
+}
+
+// L2 prefetch requests for the call that follows on the stream: its right factor, then a prefix of its packed rows in tile order (what
+// its CTAs read first).  Returns their number.
+// Defaults from the Llama-2-13B token step (ms, next-call megabytes / in-launch lookahead): 16/off 2.365, 8/off 2.357, 16/on 2.369,
+// 32/on 2.440, 64/on 2.590, 0/off 2.407 - more than the head of the next call evicts what this one still needs, and the lookahead no
+// longer pays on top of it.
+int plan_prefetch(const glowq_w4a16_group_t& g, const unsigned char** ptr, unsigned* bytes) {
+  static const int mb = [] {
+    const char* v = std::getenv("GLOWQ_GEMV_PREFETCH_MB");
+    return (v && *v) ? std::atoi(v) : 16;
+  }();
+  int n = 0;
+  if (g.next == nullptr || mb <= 0) return 0;
+  const glowq_w4a16_group_t& nx = *g.next;
+  size_t budget = static_cast<size_t>(mb) << 20;
+  auto add = [&](const void* at, size_t size) {
+    size = std::min(size, budget) & ~static_cast<size_t>(15);
+    if (at != nullptr && (reinterpret_cast<uintptr_t>(at) & 15u) == 0 && size >= 16 && n < kMaxPrefetch) {
+      ptr[n] = static_cast<const unsigned char*>(at);
+      bytes[n++] = static_cast<unsigned>(size);
+      budget -= size;
+    }
+  };
+  if (nx.IC > 0 && nx.n_members >= 1 && nx.n_members <= GLOWQ_MAX_MEMBERS) {
+    if (nx.r_mode == GLOWQ_R_COMPUTE && nx.R != nullptr && nx.rank > 0 && nx.R_stride >= nx.IC)
+      add(nx.R, (static_cast<size_t>(nx.rank - 1) * nx.R_stride + nx.IC) * 2);
+    for (int i = 0; i < nx.n_members; ++i) {
+      const auto& m = nx.members[i];
+      const int words = (nx.IC + 7) / 8;
+      if (m.OC > 0 && m.weight_stride_i32 >= words) add(m.qweight, (static_cast<size_t>(m.OC - 1) * m.weight_stride_i32 + words) * 4);
+    }
+  }
+  return n;
 }
 }  // namespace glowq
 
@@ -346,14 +381,37 @@ int n_tiles_of(const glowq_w4a16_group_t& g) {
   return n;
 }
 
-// Up to 8 tokens fit one streaming launch (one MMA N tile), which multiplies the exact integer codes and applies the scales in
-// fp32; the tensor-core kernels round the scaled weights to fp16 first, as the reference does.  So 8 tokens stay here although
-// the tensor-memory kernel is ahead in time by then (a corrected Qwen3-14B layer: 129 us at 8 tokens here, 112 at 16 there).
-// 9 to 16 tokens would take two streaming launches: 47 / 70 / 64 / 33 us for q/k/v, gate/up, down_proj and o_proj of the
-// Llama-2-13B shapes at 16 tokens, corrected, against 23.6 / 36.7 / 22.8 / 15.5.
-bool takes_gemm(const glowq_w4a16_group_t& g) {
-  const bool use_gemm = g.kernel == GLOWQ_KERNEL_GEMM || (g.kernel == GLOWQ_KERNEL_AUTO && g.M > kGemvAutoMaxM);
-  return use_gemm && gemm_supported(g);
+// Microseconds of one streaming launch of 2 to 8 tokens, fitted on B200 to 266 group calls (9 % rms): latency, the rounds of tiles times
+// their chunks of 1024 columns - with one CTA per SM, where the staged activations leave room for no more, a chunk takes two thirds of
+// the time, but there are half as many CTAs - the correction, K slices that meet in memory, a ring too shallow for one CTA.
+double stream_us(const glowq_w4a16_group_t& g, const GemvPlan& pl, int n_tiles, bool corr, int sms) {
+  const int r_ctas = corr && g.r_mode == GLOWQ_R_COMPUTE ? std::min({pl.n_r_tiles * pl.SKr, 96, sms * pl.ctas_per_sm / 3}) : 0;
+  const int rounds = pl.SK == 1 ? ceil_div(n_tiles, sms * pl.ctas_per_sm) : ceil_div(n_tiles * pl.SK, std::max(1, sms * pl.ctas_per_sm - r_ctas));
+  const int chunks = ceil_div(std::min(pl.gps, pl.G), kChunkGroups);
+  return 0.925 + 0.792 * g.M + rounds * chunks * (pl.ctas_per_sm == 2 ? 0.972 : 0.618 + 0.006 * g.M) +
+         (corr ? 1.014 + 0.738 * ceil_div(g.rank, 256) * rounds : 0.0) + (pl.SK > 1 ? 4.5 : 0.0) +
+         (pl.ctas_per_sm == 1 && pl.stages < 4 ? 0.0212 * pl.G : 0.0);
+}
+
+// Which kernel.  Up to 8 tokens fit one streaming launch (one MMA N tile), which multiplies the exact integer codes and applies the
+// scales in fp32; from 2 tokens the tensor-memory kernel's exact form, of the same precision, takes the calls that it is faster on:
+// many tokens and long rows (us streamed / exact: 13B down_proj corrected at 2 and 8 tokens 21.2 / 19.1 and 33.8 / 19.1, 14B gate/up at
+// 2 and 8 tokens 21.7 / 29.2 and 35.1 / 29.3, 3B o_proj corrected at 3 and 8 tokens 7.8 / 9.3 and 10.4 / 9.4).  Above 8 tokens the
+// tensor-core kernels round the scaled weights to fp16 first, as the reference does.  9 to 16 tokens would take two streaming launches:
+// 47 / 70 / 64 / 33 us for q/k/v, gate/up, down_proj and o_proj of the Llama-2-13B shapes at 16 tokens, corrected, against
+// 19.1 / 29.3 / 18.1 / 11.3.
+bool takes_gemm(const glowq_w4a16_group_t& g, int sms) {
+  if (g.kernel == GLOWQ_KERNEL_GEMV) return false;
+  if (g.kernel == GLOWQ_KERNEL_GEMM || g.M > kGemvAutoMaxM) return gemm_supported(g);
+  // (a fused input transform, a push and K slices on request are the streaming kernel's)
+  if (g.M < 2 || g.push != nullptr || g.norm_weight != nullptr || g.split_k > 0 || !gemv_fast_ok(g) || !gemm_supported(g)) return false;
+  const int n_tiles = n_tiles_of(g);
+  const GemvPlan pl = make_plan(g.M, g.IC, n_tiles, g.r_mode != GLOWQ_R_NONE ? g.rank : 0, sms, 0);
+  if (pl.total > g.workspace_bytes) return false;   // (refused there)
+  bool corr = false;
+  for (int i = 0; i < g.n_members && g.r_mode != GLOWQ_R_NONE; ++i) corr = corr || (g.members[i].L && g.members[i].alpha != 0.f);
+  const double exact = gemm_exact_us(g, sms);
+  return exact >= 0.0 && exact < stream_us(g, pl, n_tiles, corr, sms);
 }
 
 int gemv_group_forward(const glowq_w4a16_group_t& g, const DeviceInfo& dev, cudaStream_t stream) {
@@ -484,37 +542,9 @@ int gemv_group_forward(const glowq_w4a16_group_t& g, const DeviceInfo& dev, cuda
                              static_cast<uint64_t>(d.Lstride) * 2, p.l_cols, kTileRows);
         if (rc != GLOWQ_OK) return rc;
       }
-      // L2 prefetch requests for the call that follows on this stream: its right factor, then a prefix of its packed
-      // rows in tile order (what its CTAs read first)
-      // Defaults from the Llama-2-13B token step (ms, next-call megabytes / in-launch lookahead): 16/off 2.365,
-      // 8/off 2.357, 16/on 2.369, 32/on 2.440, 64/on 2.590, 0/off 2.407 - more than the head of the next call evicts
-      // what this one still needs, and the lookahead no longer pays on top of it.
-      static const int pf_mb = env_int("GLOWQ_GEMV_PREFETCH_MB", 16);
       static const int deep_pf = env_int("GLOWQ_GEMV_DEEP_PREFETCH", 0);
       p.deep_prefetch = deep_pf;
-      p.n_pf = 0;
-      if (g.next != nullptr && pf_mb > 0 && m0 + kGemvMaxM >= g.M) {
-        const glowq_w4a16_group_t& nx = *g.next;
-        size_t budget = static_cast<size_t>(pf_mb) << 20;
-        auto add = [&](const void* ptr, size_t bytes) {
-          bytes = std::min(bytes, budget) & ~static_cast<size_t>(15);
-          if (ptr != nullptr && aligned16(ptr) && bytes >= 16 && p.n_pf < kMaxPrefetch) {
-            p.pf_ptr[p.n_pf] = static_cast<const unsigned char*>(ptr);
-            p.pf_bytes[p.n_pf] = static_cast<unsigned>(bytes);
-            ++p.n_pf;
-            budget -= bytes;
-          }
-        };
-        if (nx.IC > 0 && nx.n_members >= 1 && nx.n_members <= GLOWQ_MAX_MEMBERS) {
-          if (nx.r_mode == GLOWQ_R_COMPUTE && nx.R != nullptr && nx.rank > 0 && nx.R_stride >= nx.IC)
-            add(nx.R, (static_cast<size_t>(nx.rank - 1) * nx.R_stride + nx.IC) * 2);
-          for (int i = 0; i < nx.n_members; ++i) {
-            const auto& m = nx.members[i];
-            if (m.OC > 0 && m.weight_stride_i32 >= ceil_div(nx.IC, 8))
-              add(m.qweight, (static_cast<size_t>(m.OC - 1) * m.weight_stride_i32 + ceil_div(nx.IC, 8)) * 4);
-          }
-        }
-      }
+      p.n_pf = m0 + kGemvMaxM >= g.M ? plan_prefetch(g, p.pf_ptr, p.pf_bytes) : 0;
       if (pl.own_ctr && pl.SK > 1) {
         e = cudaMemsetAsync(p.tile_ctr, 0, static_cast<size_t>(n_tiles) * 4, stream);
         if (e != cudaSuccess) return fail_cuda(e);
@@ -611,7 +641,7 @@ int glowq_w4a16_group_forward(const glowq_w4a16_group_t* group) {
   if (rc != GLOWQ_OK) return rc;
   if (g.M == 0) return GLOWQ_OK;
   cudaStream_t stream = static_cast<cudaStream_t>(g.stream);
-  if (takes_gemm(g)) {
+  if (takes_gemm(g, dev->sms)) {
     cudaError_t ce = cudaSuccess;
     rc = gemm_group_forward(g, stream, &ce);
     if (rc == GLOWQ_ERR_CUDA) return fail_cuda(ce);
@@ -629,7 +659,7 @@ int glowq_internal_workspace_map(const glowq_w4a16_group_t* group, int sms, Work
   if (rc != GLOWQ_OK) return rc;
   *map = WorkspaceMap{};
   if (g.M == 0) return GLOWQ_OK;
-  if (takes_gemm(g)) {
+  if (takes_gemm(g, sms)) {
     gemm_workspace_map(g, sms, map);
     return GLOWQ_OK;
   }

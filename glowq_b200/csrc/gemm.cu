@@ -18,11 +18,11 @@ size_t r_product_slot_bytes(int M, int IC, int rank);
 cudaError_t launch_r_product(const __half* x, const __half* R, __half* r_buf, float* slots, uint32_t* ctr, int M, int IC,
                              int rank, int x_stride, int R_stride, cudaStream_t stream);
 size_t gemm_tmem_r_bytes(int M, int IC, int rank);
-int gemm_tmem_forward(const glowq_w4a16_group_t& g, bool compute_r, bool any_corr, bool any_separate, int sms, cudaStream_t stream,
+int gemm_tmem_forward(const glowq_w4a16_group_t& g, bool exact, bool compute_r, bool any_corr, bool any_separate, int sms, cudaStream_t stream,
                       cudaError_t* cuda_err);
 int gemm_pair_forward(const glowq_w4a16_group_t& g, bool compute_r, bool r_only, bool any_corr, bool any_separate, int sms,
                       cudaStream_t stream, cudaError_t* cuda_err);
-void gemm_tmem_workspace_map(const glowq_w4a16_group_t& g, bool compute_r, bool any_corr, bool any_separate, int sms, WorkspaceMap* map);
+void gemm_tmem_workspace_map(const glowq_w4a16_group_t& g, bool exact, bool compute_r, bool any_corr, bool any_separate, int sms, WorkspaceMap* map);
 void gemm_pair_workspace_map(const glowq_w4a16_group_t& g, bool compute_r, bool any_corr, bool any_separate, int sms, WorkspaceMap* map);
 
 namespace {
@@ -74,10 +74,10 @@ size_t gemm_workspace_bytes(int M, int IC, int OC_total, int rank, int n_members
   if (rank > 0 && M <= 128) slots = std::max(slots, r_product_slot_bytes(M, IC, rank));
   // K slices of the one-CTA form, unless whole tiles fill the SMs and the last round of them is nearly full too
   const int tmem_tiles = cdiv(OC_total, 128), tmem_rest = tmem_tiles % kPlanSms;
-  if (M > 8 && M <= kTmemMaxM && !(tmem_tiles >= kPlanSms && tmem_rest * 4 >= 3 * kPlanSms))
-    slots = std::max(slots, static_cast<size_t>(kTmemSlices) * (M <= 32 ? 32 : 64) * 128 * 4);
+  if (M > 1 && M <= kTmemMaxM && !(tmem_tiles >= kPlanSms && tmem_rest * 4 >= 3 * kPlanSms))
+    slots = std::max(slots, static_cast<size_t>(kTmemSlices) * (M <= 8 ? 16 : M <= 32 ? 32 : 64) * 128 * 4);
   if (M > 256) slots = std::max(slots, static_cast<size_t>(kMaxTailSlots) * 4 * kSlotBytes);
-  if (rank > 0 && M > 8 && M <= kTmemMaxM) slots += gemm_tmem_r_bytes(M, IC, rank);
+  if (rank > 0 && M > 1 && M <= kTmemMaxM) slots += gemm_tmem_r_bytes(M, IC, rank);
   if (slots == 0) return kWsHeaderBytes;
   return kWsSlotsOffset + slots + 256;
 }
@@ -86,6 +86,7 @@ namespace {
 // What the routes of a group call hang on.
 struct GemmRoute {
   bool any_corr, any_separate;   // some member is corrected; with a factor other than 1 (an accumulator of its own)
+  bool exact;                    // up to 8 tokens, chosen by the library: integer weights and fp32 scales (gemm_tmem.cu)
   bool tmem, r_in_launch;        // up to 64 tokens (gemm_tmem.cu); r computed by the members' launch
 };
 GemmRoute gemm_route(const glowq_w4a16_group_t& g) {
@@ -95,6 +96,7 @@ GemmRoute gemm_route(const glowq_w4a16_group_t& g) {
     rt.any_corr = rt.any_corr || corr;
     rt.any_separate = rt.any_separate || (corr && g.members[i].alpha != 1.f);
   }
+  rt.exact = g.M <= 8 && g.kernel == GLOWQ_KERNEL_AUTO;
   rt.tmem = g.M <= kTmemMaxM;
   rt.r_in_launch = g.r_mode == GLOWQ_R_COMPUTE &&
                    g.workspace_bytes >= (rt.tmem ? kWsSlotsOffset + gemm_tmem_r_bytes(g.M, g.IC, g.rank) : kWsRllOffset);
@@ -102,10 +104,21 @@ GemmRoute gemm_route(const glowq_w4a16_group_t& g) {
 }
 }  // namespace
 
+double gemm_tmem_us(const glowq_w4a16_group_t& g, bool exact, bool compute_r, bool any_corr, bool any_separate, int sms);
+
+// Microseconds of a call of up to 8 tokens in the exact form, as far as its workspace goes (-1: r would need a launch of its own).  The
+// planner's costs leave out what does not depend on the partition: fitted beside the streaming kernel's on the same 266 calls, where the
+// kernel that the two estimates choose is 1.2 % slower than the better one on average (always the streaming kernel: 14.9 %).
+double gemm_exact_us(const glowq_w4a16_group_t& g, int sms) {
+  const GemmRoute rt = gemm_route(g);
+  if (g.r_mode == GLOWQ_R_COMPUTE && !rt.r_in_launch) return -1.0;
+  return 1.5 + 1.38 * gemm_tmem_us(g, true, rt.r_in_launch, rt.any_corr, rt.any_separate, sms);
+}
+
 // (host arithmetic: see glowq_internal_workspace_map)
 void gemm_workspace_map(const glowq_w4a16_group_t& g, int sms, WorkspaceMap* map) {
   const GemmRoute rt = gemm_route(g);
-  if (rt.tmem) return gemm_tmem_workspace_map(g, rt.r_in_launch, rt.any_corr, rt.any_separate, sms, map);
+  if (rt.tmem) return gemm_tmem_workspace_map(g, rt.exact, rt.r_in_launch, rt.any_corr, rt.any_separate, sms, map);
   gemm_pair_workspace_map(g, rt.r_in_launch, rt.any_corr, rt.any_separate, sms, map);
 }
 
@@ -133,7 +146,7 @@ int gemm_group_forward(const glowq_w4a16_group_t& g, cudaStream_t stream, cudaEr
       return rc;
     }
   }
-  if (rt.tmem) return gemm_tmem_forward(g, rt.r_in_launch, rt.any_corr, rt.any_separate, sms, stream, cuda_err);
+  if (rt.tmem) return gemm_tmem_forward(g, rt.exact, rt.r_in_launch, rt.any_corr, rt.any_separate, sms, stream, cuda_err);
   return gemm_pair_forward(g, rt.r_in_launch, false, rt.any_corr, rt.any_separate, sms, stream, cuda_err);
 }
 

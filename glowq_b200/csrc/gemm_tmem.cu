@@ -42,6 +42,7 @@
 
 namespace glowq {
 
+int plan_prefetch(const glowq_w4a16_group_t& g, const unsigned char** ptr, unsigned* bytes);
 int tensor_map_2d_ex(CUtensorMap* out, CUtensorMapDataType dtype, const void* ptr, uint64_t dim0, uint64_t dim1,
                      uint64_t stride_bytes, uint32_t box0, uint32_t box1, int swizzle);
 
@@ -91,6 +92,10 @@ struct TsParams {
   int ns, np;           // ring depths: stages (an activation tile and a tensor-memory A tile each), packed weights
   int a_col;            // first tensor-memory column of the A tiles
   int ksplit, full_tiles, n_tail, n_x;   // items: full_tiles whole tiles, then n_tail tiles of ksplit K slices each
+  // head of the call that follows (weights of a streaming launch, which starts on them): every CTA asks L2 for its share
+  int n_pf;
+  const unsigned char* pf_ptr[kMaxPrefetch];
+  unsigned pf_bytes[kMaxPrefetch];
   TsMember mem[kMaxMembers];
 };
 struct alignas(64) TsMaps {
@@ -221,6 +226,10 @@ __device__ __noinline__ void add_shares(ShareArgs a, unsigned long long left, in
   for (; left != 0; left &= left - 1) add_share(a, __ffsll(left) - 1, et);
 }
 
+// EXACT (up to 8 tokens): the weights enter the product as the exact integers code - zero, every step has an accumulator of its own per
+// team, and the team that dequantised a step adds scale x accumulator to fp32 sums in registers - the precision of the weight-streaming
+// kernel.  Else they are rounded to fp16 with their scale first, as the reference rounds them.
+template <bool EXACT>
 __global__ void __launch_bounds__(kThreads, 2)
 gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsMaps tm) {
   extern __shared__ unsigned char smem[];
@@ -268,7 +277,8 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
   }
   const TsMember& mb = p.mem[mi];
   const int u0 = r_cta ? 0 : p.G;   // fp16 step it covers columns 64 (it - u0) .. of its operands
-  const bool sep = !r_cta && mb.lr_separate != 0;
+  constexpr int kAccs = EXACT ? kTeams : 1;   // accumulators in front of the correction's own
+  const bool sep = !r_cta && (EXACT || mb.lr_separate != 0);
   const uint32_t cdepth = r_cta ? static_cast<uint32_t>(min(kMaxC, kA16Slots + p.np * kPStage / kA16)) : kA16Slots;
 
   if (threadIdx.x == 0) {
@@ -379,6 +389,11 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
       drain(pfull, p.np, issued);
     }
     __syncwarp();
+    if (EXACT)
+      for (int r = 0; r < p.n_pf; ++r)   // this CTA's copies are all issued
+        for (uint32_t at = (blockIdx.x + lane * gridDim.x) * kPrefetchSlice; at < p.pf_bytes[r]; at += 32 * gridDim.x * kPrefetchSlice)
+          asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p.pf_ptr[r] + at), "r"(min(kPrefetchSlice, p.pf_bytes[r] - at))
+                       : "memory");
   } else if (warp == 1) {
     {   // the whole warp: see umma_ts_step
       Ring b{0, 0}, c{0, 0};
@@ -401,11 +416,12 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
         const uint32_t cur = b.i;
         b.step(1, p.ns);
         ready = g_mbar_test_elected(full + 8 * b.i, b.ph);   // answered while this stage's MMAs are issued
-        umma_ts_step(tmem, tmem + p.a_col + cur * 64, lo0 + cur * ((2 * sub) >> 4), hi, sub >> 4, idesc, acc, empty + 8 * cur);
+        if (EXACT) acc = 0;
+        umma_ts_step(EXACT ? tmem + ((it - it0) & 1) * p.N : tmem, tmem + p.a_col + cur * 64, lo0 + cur * ((2 * sub) >> 4), hi, sub >> 4, idesc, acc, empty + 8 * cur);
         acc = 1;
       }
       if (sep) acc = 0;   // the first MMA overwrites its accumulator
-      const uint32_t d = tmem + (sep ? p.N : 0);
+      const uint32_t d = tmem + (sep ? kAccs * p.N : 0);
       for (int it = nkp; it < nk; ++it) {
         wait_slow(cfull + 8 * c.i, c.ph);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -431,6 +447,9 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
     const bool rvalid = row < mb.OC;
     const uint32_t lane_base = tmem + (static_cast<uint32_t>(q * 32) << 16);
     bool ok = true;
+    float xacc[8];   // EXACT: this row's sums of the team's steps
+#pragma unroll
+    for (int j = 0; j < 8; ++j) xacc[j] = 0.f;
     {
       const __half* srow = mb.scales + static_cast<size_t>(rvalid ? row : 0) * mb.sstride;
       const int32_t* zrow = mb.qzeros + static_cast<size_t>(rvalid ? row : 0) * mb.zstride;
@@ -447,8 +466,22 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
         }
       };
       fetch(it0 + team);
+      // EXACT: the sums of the team's step before (its MMAs are done, or nearly) are added before the next one's may overwrite them
+      Ring before = a;
+      float scale_before = 0.f;
+      auto add_step = [&] {
+        if (!test_bar(empty + 8 * before.i, before.ph)) ok = ok && g_mbar_wait(empty + 8 * before.i, before.ph, abort_flag, p.status);
+        __syncwarp();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        uint32_t d[8];
+        tmem_ld8(lane_base + team * p.N, d);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int j = 0; j < 8; ++j) xacc[j] = fmaf(scale_before, __uint_as_float(d[j]), xacc[j]);
+      };
       for (int it = it0 + team; it < nkp; it += kTeams) {
         const uint32_t s2 = nx_s * 0x00010001u;
+        const float scale = __half2float(__ushort_as_half(static_cast<unsigned short>(nx_s)));
         // -(1024 + z) and -(64 + z): the fp16 ulp is 1 at 1024 and 1/16 at 64
         const uint32_t zc = 0xD400E400u | (nx_z * 0x00100001u);
         // both polls go out together (an answer takes about a hundred clocks); after a failed wait the stores go on:
@@ -472,7 +505,7 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
           uint32_t v[32];
-          dequant_words(v, w, 8 * half, zc, s2);
+          dequant_words<!EXACT>(v, w, 8 * half, zc, s2);
           if (half == 0) {   // the MMAs that read this stage's A tile before are done
             if (!have_e) ok = ok && g_mbar_wait(empty + 8 * a.i, a.ph ^ 1, abort_flag, p.status);
             __syncwarp();
@@ -481,12 +514,35 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
           tmem_st32(dst + half * 32, v);
           if (half == 0 && lane == 0) g_mbar_arrive(pempty + 8 * s.i);   // the packed rows are in registers
         }
+        if (EXACT && it >= it0 + kTeams) add_step();
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) g_mbar_arrive(full + 8 * a.i);
+        if (EXACT) {
+          before = a;
+          scale_before = scale;
+        }
         a.step(kTeams, p.ns);
         s.step(kTeams, p.np);
+      }
+      if (EXACT && it0 + team < nkp) add_step();
+    }
+    if (EXACT && !r_cta) {   // the first team has the tokens: the other's sums go through the packed ring, which is free by now
+      const uint32_t at = pring + rloc * 4;
+      epi_sync();
+      if (team == 1) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + j * (kRows * 4)), "f"(xacc[j]) : "memory");
+      }
+      epi_sync();
+      if (team == 0) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          float v;
+          asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(at + j * (kRows * 4)) : "memory");
+          xacc[j] += v;
+        }
       }
     }
 
@@ -555,11 +611,14 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
         waited = true;
       }
       uint32_t acc[8], lr[8];
-      tmem_ld8(lane_base + t0, acc);
-      if (has_lr) tmem_ld8(lane_base + p.N + t0, lr);
+      if (!EXACT || r_cta) tmem_ld8(lane_base + t0, acc);
+      if (has_lr) tmem_ld8(lane_base + kAccs * p.N + t0, lr);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       if (!ok) continue;
-      if (has_main) {
+      if (EXACT && !r_cta) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) sum[j] += xacc[j];
+      } else if (has_main) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) sum[j] += __uint_as_float(acc[j]);
       }
@@ -659,12 +718,13 @@ inline bool pdl_enabled() {
   return on;
 }
 
+template <bool EXACT>
 cudaError_t launch(const TsParams& p, const TsMaps& tm, int ctas, cudaStream_t stream) {
   static bool attr_done[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr_done[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tmem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(gemm_tmem_kernel<EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     if (e != cudaSuccess) return e;
     attr_done[dev] = true;
   }
@@ -678,7 +738,7 @@ cudaError_t launch(const TsParams& p, const TsMaps& tm, int ctas, cudaStream_t s
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, gemm_tmem_kernel, p, tm);
+  return cudaLaunchKernelEx(&cfg, gemm_tmem_kernel<EXACT>, p, tm);
 }
 
 inline int tile_tokens(int M) { return cdiv(M, 16) * 16; }   // tokens of the one tile (M <= 64)
@@ -699,16 +759,17 @@ struct TmemPlan {
   int n_r, r_slices;           // CTAs of r, K slices of an R tile
   int ksplit, full_tiles, n_tail;
   int nk_min;                  // K steps of the shortest member
+  double us;                   // estimate of what depends on the partition
   size_t off_slots;            // in the workspace: K slices' slots (those of r are at kWsSlotsOffset)
 };
-TmemPlan make_tmem_plan(const glowq_w4a16_group_t& g, bool compute_r, bool any_corr, bool any_separate, int sms) {
+TmemPlan make_tmem_plan(const glowq_w4a16_group_t& g, bool exact, bool compute_r, bool any_corr, bool any_separate, int sms) {
   TmemPlan pl{};
   pl.N = tile_tokens(g.M);
   {
     // stages: what tensor memory leaves beside the accumulators (a correction with its own doubles them), as far as shared
     // memory holds them and a few packed tiles
     const int smem = kSmemBytes - 2048 - kA16Slots * kA16, bst = pl.N * 256;
-    pl.ns = std::min({kMaxS, (kTmemCols - (any_separate ? 2 : 1) * pl.N) / 64, (smem - 3 * kPStage) / bst});
+    pl.ns = std::min({kMaxS, (kTmemCols - (exact ? kTeams + 1 : any_separate ? 2 : 1) * pl.N) / 64, (smem - 3 * kPStage) / bst});
     pl.np = std::min(kMaxP, (smem - pl.ns * bst) / kPStage);
   }
   pl.off_slots = kWsSlotsOffset;
@@ -756,13 +817,18 @@ TmemPlan make_tmem_plan(const glowq_w4a16_group_t& g, bool compute_r, bool any_c
       }
     }
   }
+  pl.us = best;
   return pl;
 }
 }  // namespace
 
+double gemm_tmem_us(const glowq_w4a16_group_t& g, bool exact, bool compute_r, bool any_corr, bool any_separate, int sms) {
+  return make_tmem_plan(g, exact, compute_r, any_corr, any_separate, sms).us;
+}
+
 // (host arithmetic: see glowq_internal_workspace_map)
-void gemm_tmem_workspace_map(const glowq_w4a16_group_t& g, bool compute_r, bool any_corr, bool any_separate, int sms, WorkspaceMap* map) {
-  const TmemPlan pl = make_tmem_plan(g, compute_r, any_corr, any_separate, sms);
+void gemm_tmem_workspace_map(const glowq_w4a16_group_t& g, bool exact, bool compute_r, bool any_corr, bool any_separate, int sms, WorkspaceMap* map) {
+  const TmemPlan pl = make_tmem_plan(g, exact, compute_r, any_corr, any_separate, sms);
   map->kernel = 1;
   map->ksplit = pl.ksplit;
   map->whole_tiles = pl.full_tiles;
@@ -777,10 +843,10 @@ void gemm_tmem_workspace_map(const glowq_w4a16_group_t& g, bool compute_r, bool 
 
 // Members' products and corrections of a group call of up to 64 tokens.  compute_r: r into g.r_buf as well (else it is
 // there); the workspace must hold gemm_tmem_r_bytes for it behind kWsSlotsOffset.
-int gemm_tmem_forward(const glowq_w4a16_group_t& g, bool compute_r, bool any_corr, bool any_separate, int sms, cudaStream_t stream,
+int gemm_tmem_forward(const glowq_w4a16_group_t& g, bool exact, bool compute_r, bool any_corr, bool any_separate, int sms, cudaStream_t stream,
                       cudaError_t* cuda_err) {
   const int G = cdiv(g.IC, kGroup);
-  const TmemPlan pl = make_tmem_plan(g, compute_r, any_corr, any_separate, sms);
+  const TmemPlan pl = make_tmem_plan(g, exact, compute_r, any_corr, any_separate, sms);
   unsigned char* const ws = static_cast<unsigned char*>(g.workspace);
   TsParams p{};
   p.N = pl.N;
@@ -805,6 +871,7 @@ int gemm_tmem_forward(const glowq_w4a16_group_t& g, bool compute_r, bool any_cor
   p.M = g.M;
   p.G = G;
   p.out_fp32 = g.out_dtype == GLOWQ_OUT_F32;
+  p.n_pf = exact ? plan_prefetch(g, p.pf_ptr, p.pf_bytes) : 0;
   p.n_members = g.n_members;
   TsMaps tm;
   std::memset(&tm, 0, sizeof(tm));
@@ -847,7 +914,8 @@ int gemm_tmem_forward(const glowq_w4a16_group_t& g, bool compute_r, bool any_cor
     n_x += cdiv(m.OC, kRows);
   }
   p.n_x = n_x;
-  const cudaError_t e = launch(p, tm, p.n_r + p.full_tiles + p.n_tail * p.ksplit, stream);
+  const int ctas = p.n_r + p.full_tiles + p.n_tail * p.ksplit;
+  const cudaError_t e = exact ? launch<true>(p, tm, ctas, stream) : launch<false>(p, tm, ctas, stream);
   if (e != cudaSuccess) {
     *cuda_err = e;
     return GLOWQ_ERR_CUDA;
