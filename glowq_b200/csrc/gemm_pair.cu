@@ -288,7 +288,84 @@ constexpr uint32_t kBAccEmpty = 272;              // [2] CTA 0: the epilogue war
 constexpr uint32_t kBSFull = 288;                 // each CTA: an item
 constexpr uint32_t kBSEmpty = 320;                // CTA 1: everybody has read it, and the weight producers are nearly through with it
 constexpr uint32_t kBFin = 352;                   // CTA 0: all MMAs done
+constexpr uint32_t kBSumGo = 360;                 // each CTA: an item's accumulators may be merged (see merge)
+constexpr uint32_t kBSumDone = 368;               // each CTA: the dequant warps have merged their part
 constexpr uint32_t kBItem = 384;                  // the item (a Tile)
+
+// The pass over an item's accumulators that comes before the output where K is sliced or the correction has an accumulator of its own:
+// 16 tokens at a time from `first` on, every `step`, the correction's sums and the other slices' slots (in slice order) are added, and
+// the result goes to the slot or back to the accumulator.  The dequant warps, which have nothing to do until the epilogue gives the
+// accumulators back, take two thirds of it: by the four epilogue warps alone the seven slots of a sliced r tile of 224 tokens took 18 us.
+constexpr int kMergers = 1 + kTeams;
+struct Merge {
+  uint32_t d;          // this warp's lanes of the accumulators
+  float4* slot0;       // this thread's row of the tile's first slot
+  size_t slice_v4;
+  int ntok;
+  bool park, has_main, has_lr;
+  float alpha;
+  __device__ __forceinline__ Merge(const PtParams& p, const Tile& t, uint32_t lane_base, uint32_t buf, int rank, int rloc) {
+    const bool is_r = t.is_r();
+    const size_t slot_floats = static_cast<size_t>(p.N) * (2 * kRows);
+    d = lane_base + buf * static_cast<uint32_t>(p.N);
+    slot0 = reinterpret_cast<float4*>(is_r ? p.r_slots + static_cast<size_t>(t.ctr) * slot_floats
+                                           : p.slots + static_cast<size_t>(t.ctr - p.ctr_base) * slot_floats) +
+            rank * kRows + rloc;
+    slice_v4 = (is_r ? static_cast<size_t>(p.r_tiles) : static_cast<size_t>(p.n_tail)) * (slot_floats / 4);
+    ntok = min(p.N, p.M - t.m0);
+    park = t.z < t.ks - 1;
+    has_main = t.it0 < p.G || !p.sep;
+    has_lr = p.sep && !is_r && t.corr() && t.nk > p.G;
+    alpha = p.mem[t.mi()].alpha;
+  }
+};
+__device__ __forceinline__ void merge(const PtParams& p, const Tile& t, const Merge& m, int part) {
+  for (int t0 = 16 * part; t0 < m.ntok; t0 += 16 * kMergers) {
+    uint32_t v[16];
+    tmem_ld16p(m.d + t0, v);
+    if (m.has_lr) {
+      uint32_t lr[16];
+      tmem_ld16p(m.d + p.N + t0, lr);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+      for (int k = 0; k < 16; ++k)
+        v[k] = __float_as_uint(fmaf(m.alpha, __uint_as_float(lr[k]), m.has_main ? __uint_as_float(v[k]) : 0.f));
+    } else {
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      if (!m.has_main) {
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[k] = 0u;
+      }
+    }
+    float4* const at = m.slot0 + static_cast<size_t>(t0 / 4) * (2 * kRows);
+    if (m.park) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        __stcg(at + t.z * m.slice_v4 + k * (2 * kRows), make_float4(__uint_as_float(v[4 * k]), __uint_as_float(v[4 * k + 1]),
+                                                                    __uint_as_float(v[4 * k + 2]), __uint_as_float(v[4 * k + 3])));
+      continue;
+    }
+    for (int z = 0; z < t.ks - 1; z += 3) {   // three slots in flight
+      float4 u[3][4];
+#pragma unroll
+      for (int y = 0; y < 3; ++y)
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          u[y][k] = z + y < t.ks - 1 ? __ldcg(at + (z + y) * m.slice_v4 + k * (2 * kRows)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int y = 0; y < 3; ++y)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          v[4 * k] = __float_as_uint(__uint_as_float(v[4 * k]) + u[y][k].x);
+          v[4 * k + 1] = __float_as_uint(__uint_as_float(v[4 * k + 1]) + u[y][k].y);
+          v[4 * k + 2] = __float_as_uint(__uint_as_float(v[4 * k + 2]) + u[y][k].z);
+          v[4 * k + 3] = __float_as_uint(__uint_as_float(v[4 * k + 3]) + u[y][k].w);
+        }
+    }
+    tmem_st16p(m.d + t0, v);
+  }
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ PtParams p, const __grid_constant__ PtMaps tm) {
@@ -320,6 +397,8 @@ gemm_pair_kernel(const __grid_constant__ PtParams p, const __grid_constant__ PtM
     g_mbar_init(smem0 + kBSFull, 1);
     g_mbar_init(smem0 + kBSEmpty, kConsumers);
     g_mbar_init(smem0 + kBFin, 1);
+    g_mbar_init(smem0 + kBSumGo, 1);
+    g_mbar_init(smem0 + kBSumDone, 4 * kTeams);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -604,9 +683,11 @@ gemm_pair_kernel(const __grid_constant__ PtParams p, const __grid_constant__ PtM
     uint32_t jn = team, ai = team % na;
     const uint32_t e0 = team + 4 * nb - na;
     Ring s{0, 0}, d{team % nb, (team / nb) & 1u}, e{e0 % nb, (e0 / nb) & 1u};
-    uint32_t jbase = 0;
+    uint32_t jbase = 0, n = 0, mph = 0;
     bool ok = true;
     while (ok && next_item(t, false, true)) {
+      const uint32_t buf = p.nbuf == 2 ? n & 1 : 0;
+      ++n;
       const uint32_t jend = jbase + static_cast<uint32_t>(t.nk - t.it0);
       for (; jn < jend; jn += kTeams) {
         const int it = t.it0 + static_cast<int>(jn - jbase);
@@ -672,15 +753,24 @@ gemm_pair_kernel(const __grid_constant__ PtParams p, const __grid_constant__ PtM
         }
       }
       jbase = jend;
+      if (ok && (p.sep || t.ks > 1)) {
+        ok = await(kBSumGo, mph);
+        mph ^= 1;
+        if (!__all_sync(0xffffffffu, ok)) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        merge(p, t, Merge(p, t, tmem + (static_cast<uint32_t>(q * 32) << 16), buf, rank, rloc), 1 + team);
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) g_mbar_arrive(smem0 + kBSumDone);
+      }
     }
   } else {
     // ================================================================ epilogue warps
     const int q = warp & 3, rloc = q * 32 + lane, et = static_cast<int>(threadIdx.x) - 128;
     const uint32_t lane_base = tmem + (static_cast<uint32_t>(q * 32) << 16);
     const uint32_t accempty0 = map_to_cta(smem0 + kBAccEmpty, 0);
-    const size_t slot_floats = static_cast<size_t>(p.N) * (2 * kRows);
     const uint32_t ow = ostage + static_cast<uint32_t>(q * p.no) * kOStage;
-    uint32_t n = 0, ob = 0;
+    uint32_t n = 0, ob = 0, mph = 0;
     // Output stages, each warp its own, handed to the copy engine two at a time (the fence takes some hundred clocks).  Behind the
     // stores the oldest ones have been read, so that the next two stages are free: a stage has a group of its own, an empty one where
     // the warp's columns lie past the end, so that the groups still to be waited for are the last stages written.
@@ -726,14 +816,8 @@ gemm_pair_kernel(const __grid_constant__ PtParams p, const __grid_constant__ PtM
         const int c = frag ? col0 + 8 * m + (lane >> 2) : row;
         bias[m] = (go && !is_r && mb.bias && c < mb.OC) ? __half2float(mb.bias[c]) : 0.f;
       }
-      const float alpha = mb.alpha;
       const bool park = t.z < t.ks - 1, finish = t.ks > 1 && !park;
       uint32_t* const tctr = p.tile_ctr + 2 * t.ctr + rank;
-      float4* const slot0 = reinterpret_cast<float4*>(is_r ? p.r_slots + static_cast<size_t>(t.ctr) * slot_floats
-                                                           : p.slots + static_cast<size_t>(t.ctr - p.ctr_base) * slot_floats) +
-                            rank * kRows + rloc;
-      const size_t slice_v4 = (is_r ? static_cast<size_t>(p.r_tiles) : static_cast<size_t>(p.n_tail)) * (slot_floats / 4);
-      const bool has_main = t.it0 < p.G || !p.sep, has_lr = p.sep && !is_r && t.corr() && t.nk > p.G;
       go = go && await(kBAccFull + 8 * buf, use & 1);
       if (!epi_vote(go)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -754,53 +838,12 @@ gemm_pair_kernel(const __grid_constant__ PtParams p, const __grid_constant__ PtM
       const CUtensorMap* const om = is_r ? &tm.r_out : &tm.out[t.mi()];
       const bool inside = col0 < (is_r ? p.rank : mb.OC);
       if (p.sep || t.ks > 1) {
-        // Sixteen tokens at a time: the correction from its own accumulator, the other slices' partial sums in slice order; the
-        // result goes to the slot or back to the accumulator.
-        for (int t0 = 0; t0 < ntok; t0 += 16) {
-          uint32_t v[16];
-          tmem_ld16p(d + t0, v);
-          if (has_lr) {
-            uint32_t lr[16];
-            tmem_ld16p(d + p.N + t0, lr);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-            for (int k = 0; k < 16; ++k)
-              v[k] = __float_as_uint(fmaf(alpha, __uint_as_float(lr[k]), has_main ? __uint_as_float(v[k]) : 0.f));
-          } else {
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (!has_main) {
-#pragma unroll
-              for (int k = 0; k < 16; ++k) v[k] = 0u;
-            }
-          }
-          float4* const at = slot0 + static_cast<size_t>(t0 / 4) * (2 * kRows);
-          if (park) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-              __stcg(at + t.z * slice_v4 + k * (2 * kRows), make_float4(__uint_as_float(v[4 * k]), __uint_as_float(v[4 * k + 1]),
-                                                                        __uint_as_float(v[4 * k + 2]), __uint_as_float(v[4 * k + 3])));
-            continue;
-          }
-          for (int z = 0; z < t.ks - 1; z += 3) {   // three slots in flight
-            float4 u[3][4];
-#pragma unroll
-            for (int y = 0; y < 3; ++y)
-#pragma unroll
-              for (int k = 0; k < 4; ++k)
-                u[y][k] = z + y < t.ks - 1 ? __ldcg(at + (z + y) * slice_v4 + k * (2 * kRows)) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int y = 0; y < 3; ++y)
-#pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                v[4 * k] = __float_as_uint(__uint_as_float(v[4 * k]) + u[y][k].x);
-                v[4 * k + 1] = __float_as_uint(__uint_as_float(v[4 * k + 1]) + u[y][k].y);
-                v[4 * k + 2] = __float_as_uint(__uint_as_float(v[4 * k + 2]) + u[y][k].z);
-                v[4 * k + 3] = __float_as_uint(__uint_as_float(v[4 * k + 3]) + u[y][k].w);
-              }
-          }
-          tmem_st16p(d + t0, v);
-        }
-        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        if (et == 0) g_mbar_arrive(smem0 + kBSumGo);
+        merge(p, t, Merge(p, t, lane_base, buf, rank, rloc), 0);
+        const bool merged = await(kBSumDone, mph);
+        mph ^= 1;
+        if (!epi_vote(merged)) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       }
       int pending = 0;
       for (int t0 = 0; t0 < (park ? 0 : ntok); t0 += 32) {
