@@ -981,19 +981,20 @@ struct PairPlan {
   size_t off_slots, end;       // in the workspace: slots of the K slices (those of r at kWsSlotsOffset), end of all slots
 };
 
-// Microseconds of a launch's parts, fitted on B200 to 638 group calls of 65 to 4096 tokens with some twenty plans each: the plans that
-// the fit takes are 1 % slower than the best ones on average, 12 % at worst.
+// Microseconds of a launch's parts, fitted on B200 to 288 group calls of 65 to 4096 tokens with some twenty plans each: the plans that
+// the planner takes are 0.8 % slower than the best ones on average, 12 % at worst.
 // A step of N tokens (tensor-memory writes and the chain from a stage's release to its next MMAs bound narrow tiles, the MMAs the
 // widest; slower the more pairs are busy); what a tile costs beside its steps; an item of r, whose fp16 rows come through four weight
-// stages a step; adding up K slices, three slots of 16 tokens a trip to memory.
-inline double step_us(int N, double busy) { return (N <= 192 ? 0.366 + 0.0004 * N : 0.00183 * N) * (1.0 + 0.366 * busy); }
-inline double tile_us(int N, bool two) { return two ? 4.25 : 4.2 + 0.004 * N; }
-inline double r_item_us(int N, double steps) { return 0.3 + steps * (0.834 + 0.0034 * N); }
-inline double r_sum_us(int N, int ks) { return ks > 1 ? 0.7 + (0.0216 * cdiv(ks - 1, 3) + 0.0018 * (ks - 1)) * N : 0.0; }
+// stages a step; adding up K slices, three slots of 48 tokens a trip to memory.
+inline double step_us(int N, double busy) { return (N <= 192 ? 0.363 + 0.0003 * N : 0.00191 * N) * (1.0 + 0.32 * busy); }
+inline double tile_us(int N, bool two) { return two ? 3.44 : 3.2 + 0.0048 * N; }
+inline double r_item_us(int N, double steps) { return 0.1 + steps * (0.815 + 0.0032 * N); }
+inline double r_sum_us(int N, int ks) { return ks > 1 ? 0.9 + (0.0116 * cdiv(ks - 1, 3) + 0.0009 * (ks - 1)) * N : 0.0; }
 inline double sum_us(int N, int ks, bool whole_before) {
-  return ks > 1 ? (whole_before ? 3.4 : 1.4) + (0.0349 * cdiv(ks - 1, 3) + 0.0003 * (ks - 1)) * N : 0.0;
+  return ks > 1 ? (whole_before ? 2.2 : 0.7) + (0.0187 * cdiv(ks - 1, 3) + 0.0023 * (ks - 1)) * N : 0.0;
 }
-constexpr double kTicketUs = 3.2;   // the first item by ticket: nothing of it runs ahead of the kernel before
+constexpr int kMaxRSlices = 16;
+constexpr double kTicketUs = 5.0;   // the first item by ticket: nothing of it runs ahead of the kernel before
 // When `items` of d microseconds each, taken in order, are done: n[i] pairs are through with their first at e[i].
 double rounds_us(int items, const int (&n)[4], const double (&e)[4], double d) {
   double lo = 1e300, hi = 0.0, t = 0.0;
@@ -1060,7 +1061,7 @@ PairPlan make_pair_plan(const glowq_w4a16_group_t& g, bool compute_r, bool any_c
       pl.r_x = cdiv(g.rank, 2 * kRows);
       pl.r_tiles = pl.r_x * pl.n_y;
     }
-    for (int rks = 1; rks <= (compute_r ? std::max(1, std::min({8, pairs / pl.r_tiles, G / 4})) : 1); ++rks) {   // K slices of r
+    for (int rks = 1; rks <= (compute_r ? std::max(1, std::min({kMaxRSlices, pairs / pl.r_tiles, G / 4})) : 1); ++rks) {   // K slices of r
       const size_t r_bytes = rks > 1 ? tile_bytes * pl.r_tiles * rks : 0;
       if (rks > 1 && (2 * pl.r_tiles > kTileCtrWords || r_bytes > room)) break;
       const int n_r = pl.r_tiles * rks, ctr_room = kTileCtrWords / 2 - (rks > 1 ? pl.r_tiles : 0);
@@ -1094,7 +1095,8 @@ PairPlan make_pair_plan(const glowq_w4a16_group_t& g, bool compute_r, bool any_c
           } else {
             cost = std::max(tile, with_r) + (f - 1) * tile + cdiv(tail * ks + static_cast<int>(r_pairs * r_item / slice), pairs) * slice;
           }
-          cost += sum_us(pl.N, ks, f > 0) + (items > pairs ? kTicketUs : 0.0);
+          // (where r is not what the launch waits for, it had better be ready early all the same: the plans differ by a few per cent)
+          cost += 0.04 * r_ready + sum_us(pl.N, ks, f > 0) + (items > pairs ? kTicketUs : 0.0) + (two ? 0.003 * pl.N : 0.0);   // (the last epilogue)
           if (cost < best_cost) {
             best_cost = cost;
             best = pl;
