@@ -981,20 +981,20 @@ struct PairPlan {
   size_t off_slots, end;       // in the workspace: slots of the K slices (those of r at kWsSlotsOffset), end of all slots
 };
 
-// Microseconds of a launch's parts, fitted on B200 to 288 group calls of 65 to 4096 tokens with some twenty plans each: the plans that
-// the planner takes are 0.8 % slower than the best ones on average, 12 % at worst.
+// Microseconds of a launch's parts, fitted on B200 to 438 group calls of 65 to 4096 tokens with some twenty plans each: the plans that
+// the planner takes are 0.8 % slower than the best ones on average, 11 % at worst.
 // A step of N tokens (tensor-memory writes and the chain from a stage's release to its next MMAs bound narrow tiles, the MMAs the
 // widest; slower the more pairs are busy); what a tile costs beside its steps; an item of r, whose fp16 rows come through four weight
 // stages a step; adding up K slices, three slots of 48 tokens a trip to memory.
-inline double step_us(int N, double busy) { return (N <= 192 ? 0.363 + 0.0003 * N : 0.00191 * N) * (1.0 + 0.32 * busy); }
-inline double tile_us(int N, bool two) { return two ? 3.44 : 3.2 + 0.0048 * N; }
-inline double r_item_us(int N, double steps) { return 0.1 + steps * (0.815 + 0.0032 * N); }
-inline double r_sum_us(int N, int ks) { return ks > 1 ? 0.9 + (0.0116 * cdiv(ks - 1, 3) + 0.0009 * (ks - 1)) * N : 0.0; }
+inline double step_us(int N, double busy) { return (N <= 192 ? 0.3571 + 0.00032 * N : 0.00189 * N) * (1.0 + 0.345 * busy); }
+inline double tile_us(int N, bool two) { return two ? 3.35 : 2.83 + 0.0063 * N; }
+inline double r_item_us(int N, double steps) { return 0.05 + steps * (0.816 + 0.0032 * N); }
+inline double r_sum_us(int N, int ks) { return ks > 1 ? 1.27 + (0.0117 * cdiv(ks - 1, 3) + 0.0003 * (ks - 1)) * N : 0.0; }
 inline double sum_us(int N, int ks, bool whole_before) {
-  return ks > 1 ? (whole_before ? 2.2 : 0.7) + (0.0187 * cdiv(ks - 1, 3) + 0.0023 * (ks - 1)) * N : 0.0;
+  return ks > 1 ? (whole_before ? 1.7 : 2.03) + (0.0173 * cdiv(ks - 1, 3) + 0.0025 * (ks - 1)) * N : 0.0;
 }
 constexpr int kMaxRSlices = 16;
-constexpr double kTicketUs = 5.0;   // the first item by ticket: nothing of it runs ahead of the kernel before
+constexpr double kTicketUs = 5.6;   // the first item by ticket: nothing of it runs ahead of the kernel before
 // When `items` of d microseconds each, taken in order, are done: n[i] pairs are through with their first at e[i].
 double rounds_us(int items, const int (&n)[4], const double (&e)[4], double d) {
   double lo = 1e300, hi = 0.0, t = 0.0;
@@ -1092,11 +1092,17 @@ PairPlan make_pair_plan(const glowq_w4a16_group_t& g, bool compute_r, bool any_c
             cost = std::max(with_r, rounds_us(tail * ks, {others - last, last, r_pairs - r_last, r_last},
                                               {slice, std::max(slice, with_r), r_item + slice, r_free + slice}, slice));
             if (r_last > 0 && tail * ks > others) cost = std::max(cost, r_free + slice);
+            cost += sum_us(pl.N, ks, false);
           } else {
-            cost = std::max(tile, with_r) + (f - 1) * tile + cdiv(tail * ks + static_cast<int>(r_pairs * r_item / slice), pairs) * slice;
+            // (slices are added up while pairs that began with r are in their tiles; short ones help where both are through together)
+            const double first = std::max(tile, with_r), after_r = std::max(r_item + tile, with_r), last_r = std::max(r_free + tile, with_r);
+            cost = (f - 1) * tile + 0.05 * slice +
+                   std::max(r_last > 0 ? last_r : first,
+                            rounds_us(tail * ks, {others, r_pairs - r_last, r_last, 0},
+                                      {first + slice, after_r + slice, last_r + slice, 0.0}, slice) + sum_us(pl.N, ks, true));
           }
           // (where r is not what the launch waits for, it had better be ready early all the same: the plans differ by a few per cent)
-          cost += 0.04 * r_ready + sum_us(pl.N, ks, f > 0) + (items > pairs ? kTicketUs : 0.0) + (two ? 0.003 * pl.N : 0.0);   // (the last epilogue)
+          cost += 0.04 * r_ready + (items > pairs ? kTicketUs : 0.0) + (two ? 0.0026 * pl.N : 0.0);   // (the last epilogue)
           if (cost < best_cost) {
             best_cost = cost;
             best = pl;
