@@ -236,7 +236,44 @@ size_t plan_smem(const GemvPlan& pl, int Mc, int stages) {
   return gemv_smem_layout_bytes(stages, pl.meta_gp, pl.meta_gw, pl.gps, pl.NT, Mc, pl.xs_stride);
 }
 
-GemvPlan make_plan(int M, int IC, int n_tiles, int rank, int sms, int split_k) {
+// CTAs that a launch of `cap` CTA slots sets apart for the R units.
+int gemv_r_ctas(const GemvPlan& pl, int n_tiles, int units, int cap) {
+  static const int max_r_ctas = env_int("GLOWQ_GEMV_R_CTAS", 96);
+  int want = std::min(units, max_r_ctas);
+  if (pl.SK > 1) {
+    // K slices: the R CTAs take no row tiles afterwards, so give them the CTA slots that do not add a round
+    // of tiles to the slices (at least a few, or r would arrive long after the first tiles are done)
+    const int rounds = ceil_div(n_tiles * pl.SK, cap);
+    const int spare = cap - pl.SK * ceil_div(n_tiles, rounds);
+    want = std::min(units, std::max(std::min(spare, max_r_ctas), std::min(max_r_ctas, 16)));
+  }
+  want = std::min(want, cap / 3);
+  if (pl.SK == 1 && n_tiles <= cap && want > cap - n_tiles && cap - n_tiles >= 8) {
+    // Every tile has a slot of its own: fewer R CTAs (2.65 us a unit), unless a tile after a unit or two (0.5 us a chunk) is sooner
+    // done.  3584 x 18944, rank 128, two tokens 31.6 -> 20.5 us; 4096 x 15360, rank 64, one token 16.8 -> 13.6.
+    const int spare = cap - n_tiles;
+    if (2.65 * (ceil_div(units, spare) - ceil_div(units, want)) < 0.5 * ceil_div(pl.G, kChunkGroups)) want = spare;
+  }
+  return std::max(0, want);
+}
+
+// Microseconds of a one-token launch on long rows, fitted on B200 to 1000 calls of 48 to 288 tiles, 96 to 148 groups and ranks 0 to 256
+// with 1 to 6 slices each (the plans taken are 0.9 % slower than the best ones on average, 13 % at worst; 12 % and 46 % by a fixed rule).  Unsliced, a launch is as long
+// as a CTA's tiles or as r; a tile that follows R units begins when they are done.  Sliced, every round of tiles pays the combine.
+double one_token_us(const GemvPlan& pl, int n_tiles, int rank, int units, int sms) {
+  const int cap = sms * pl.ctas_per_sm, r_ctas = gemv_r_ctas(pl, n_tiles, units, cap);
+  const int chunks = ceil_div(pl.G, kChunkGroups), ch = ceil_div(std::min(pl.gps, pl.G), kChunkGroups);
+  if (pl.SK == 1) {
+    const double tile = 3.027 + (0.35 + 0.00193 * n_tiles + (n_tiles > cap ? 0.221 : 0.0)) * ch + 0.0237 * rank;
+    if (units == 0) return tile;
+    return std::max(tile, 2.247 + 3.448 * ceil_div(units, std::max(1, r_ctas)) + (n_tiles > cap - r_ctas ? 0.591 * ch : 0.0));
+  }
+  const int rounds = ceil_div(n_tiles * pl.SK, std::max(1, (cap - r_ctas) / pl.SK * pl.SK));
+  return 4.267 + (1.95 + 0.101 * ch) * rounds + 0.00253 * n_tiles * chunks + (pl.ctas_per_sm == 1 ? 0.648 : 0.0) + 0.079 * pl.SK +
+         (rank > 0 ? 0.874 + (0.0252 / pl.SK + 0.0169) * units : 0.0);
+}
+
+GemvPlan make_plan(int M, int IC, int n_tiles, int rank, bool compute_r, int sms, int split_k) {
   static const int forced_stages = env_int("GLOWQ_GEMV_STAGES", 0);       // tuning overrides
   static const int forced_ctas = env_int("GLOWQ_GEMV_CTAS_PER_SM", 0);
   GemvPlan pl{};
@@ -247,25 +284,18 @@ GemvPlan make_plan(int M, int IC, int n_tiles, int rank, int sms, int split_k) {
   const int chunks = ceil_div(pl.G, kChunkGroups);
   // K is sliced across CTAs on request, when an unsliced CTA does not fit shared memory (long rows with several
   // tokens: the staged activations and the converted scale pairs grow with the slice length), and for ONE token on
-  // long rows with few tiles (down_proj of the 7B - 14B shapes, K >= 12288): there the slice length is also chosen so
-  // that two CTAs per SM with four ring stages fit.  Measured, microseconds sliced / unsliced: Llama-2-13B down_proj
-  // 19.7 / 20.0, Qwen3-14B 29.6 / 32.5, Qwen2.5-7B 20.0 / 27.2 - but Llama-3.2-3B down_proj (K = 8192) 11.2 / 9.0, and
-  // at two tokens q/k/v of the 13B shape 28.4 / 16.3, its o_proj 15.8 / 9.7, its down_proj 25.3 / 22.2: the combine
-  // of the partial tiles (fence, counter, re-read) costs more than a somewhat shorter K walk saves.
+  // long rows with few tiles (down_proj of the 7B - 14B shapes, K >= 12288), where it shares the rows among idle CTAs
+  // or leaves room for two CTAs per SM.  Not below (us sliced / unsliced): Llama-3.2-3B down_proj (K = 8192) 11.2 / 9.0,
+  // and at two tokens q/k/v of the 13B shape 28.4 / 16.3, its o_proj 15.8 / 9.7: the combine of the partial tiles
+  // (fence, counter, re-read) costs more than a somewhat shorter K walk saves.
   const bool slice_long_rows = split_k <= 0 && Mc == 1 && n_tiles < 2 * sms && chunks >= 12;
-  int sk = 1;
-  if (split_k > 0) {
-    sk = std::min(split_k, chunks);
-  } else if (slice_long_rows) {
-    sk = std::max(1, std::min(ceil_div(2 * sms, std::max(1, n_tiles)), chunks / 4));
-  }
-  for (;; ++sk) {
+  const auto cut = [&](int sk) {
     pl.gps = ceil_div(chunks, sk) * kChunkGroups;   // whole pipeline stages per slice
     pl.SK = ceil_div(pl.G, pl.gps);
     pl.meta_gp = (std::min(pl.gps, pl.G) + 1) & ~1;
     pl.meta_gw = ceil_div(pl.gps, 8);
     pl.xs_stride = pl.gps * 256 + 64;
-    // deepest ring that fits, preferring two CTAs per SM (16 consumer warps per SM) when that leaves >= 4 stages
+    // deepest ring that fits, preferring two CTAs per SM (16 consumer warps per SM) when that leaves >= 3 stages
     pl.ctas_per_sm = (pl.NT <= 2) ? 2 : 1;
     if (forced_ctas > 0) pl.ctas_per_sm = std::min(forced_ctas, pl.ctas_per_sm);
     pl.stages = 0;
@@ -278,14 +308,41 @@ GemvPlan make_plan(int M, int IC, int n_tiles, int rank, int sms, int split_k) {
           break;
         }
     }
+  };
+  int sk = 1;
+  if (split_k > 0) {
+    sk = std::min(split_k, chunks);
+  } else if (slice_long_rows) {
+    sk = std::max(1, std::min(ceil_div(2 * sms, std::max(1, n_tiles)), chunks / 4));
+  }
+  for (;; ++sk) {
+    cut(sk);
     if (pl.gps == kChunkGroups) break;  // K cannot be sliced any finer
     const bool want_two = slice_long_rows && sk < 8 && n_tiles * (sk + 1) <= 8 * sms;
     if (pl.stages > 0 && ((pl.ctas_per_sm == 2 && pl.stages >= 4) || !want_two)) break;
   }
-  if (forced_stages > 0 && pl.stages > 0) pl.stages = std::max(2, std::min(forced_stages, pl.stages));
-  pl.smem = plan_smem(pl, Mc, pl.stages);
   pl.n_r_tiles = ceil_div(std::max(rank, 0), kRTileRows);
   pl.SKr = chunks;   // one quantisation group per warp and R unit: a single round of loads per unit
+  const int max_sk = pl.SK;   // (the scratch that a call needs is that of so many slices, also where it takes fewer)
+  if (slice_long_rows && pl.stages > 0) {
+    // Of the slice counts up to there the one with the least cost: 14B down_proj 20.6 -> 16.4 us (4 slices -> 3), corrected 29.2 -> 24.4;
+    // 3584 x 13824 14.2 -> 10.7 (3 -> none), 7168 x 12288 corrected 24.3 -> 17.5 (3 -> none).
+    const int units = compute_r ? pl.n_r_tiles * ceil_div(pl.G, ceil_div(pl.G, pl.SKr)) : 0;
+    int best = sk;
+    double best_us = 0.96 * one_token_us(pl, n_tiles, rank, units, sms);   // (less than that is within the estimate's error)
+    for (int s = sk - 1; s >= 1; --s) {
+      cut(s);
+      if (pl.stages == 0) break;
+      const double us = one_token_us(pl, n_tiles, rank, units, sms);
+      if (us < best_us) {
+        best = s;
+        best_us = us;
+      }
+    }
+    cut(best);
+  }
+  if (forced_stages > 0 && pl.stages > 0) pl.stages = std::max(2, std::min(forced_stages, pl.stages));
+  pl.smem = plan_smem(pl, Mc, pl.stages);
   const size_t tile_elems = static_cast<size_t>(kRowTiles) * pl.NT * 128;
   // (room for counters among the slots whether or not K is sliced: the size a call needs grows with its rows, as the callers'
   // checks against their scratch expect)
@@ -298,7 +355,7 @@ GemvPlan make_plan(int M, int IC, int n_tiles, int rank, int sms, int split_k) {
   pl.SKr = ceil_div(pl.G, pl.gpr);
   off = align_up(off + static_cast<size_t>(pl.n_r_tiles) * pl.SKr * pl.NT * 128 * 4, 256);
   pl.off_sk_partial = off;
-  off = align_up(off + (pl.SK > 1 ? static_cast<size_t>(n_tiles) * pl.SK * tile_elems * 4 : 0), 256);
+  off = align_up(off + (max_sk > 1 ? static_cast<size_t>(n_tiles) * max_sk * tile_elems * 4 : 0), 256);
   pl.off_r32 = off;
   off = align_up(off + static_cast<size_t>(Mc) * std::max(rank, 0) * 4, 256);
   pl.total = off;
@@ -406,7 +463,7 @@ bool takes_gemm(const glowq_w4a16_group_t& g, int sms) {
   // (a fused input transform, a push and K slices on request are the streaming kernel's)
   if (g.M < 2 || g.push != nullptr || g.norm_weight != nullptr || g.split_k > 0 || !gemv_fast_ok(g) || !gemm_supported(g)) return false;
   const int n_tiles = n_tiles_of(g);
-  const GemvPlan pl = make_plan(g.M, g.IC, n_tiles, g.r_mode != GLOWQ_R_NONE ? g.rank : 0, sms, 0);
+  const GemvPlan pl = make_plan(g.M, g.IC, n_tiles, g.r_mode != GLOWQ_R_NONE ? g.rank : 0, g.r_mode == GLOWQ_R_COMPUTE, sms, 0);
   if (pl.total > g.workspace_bytes) return false;   // (refused there)
   bool corr = false;
   for (int i = 0; i < g.n_members && g.r_mode != GLOWQ_R_NONE; ++i) corr = corr || (g.members[i].L && g.members[i].alpha != 0.f);
@@ -419,7 +476,7 @@ int gemv_group_forward(const glowq_w4a16_group_t& g, const DeviceInfo& dev, cuda
   const int n_tiles = n_tiles_of(g);
   for (int m0 = 0; m0 < g.M; m0 += kGemvMaxM) {
     const int Mc = std::min(kGemvMaxM, g.M - m0);
-    const GemvPlan pl = make_plan(Mc, g.IC, n_tiles, g.r_mode != GLOWQ_R_NONE ? g.rank : 0, dev.sms, g.split_k);
+    const GemvPlan pl = make_plan(Mc, g.IC, n_tiles, g.r_mode != GLOWQ_R_NONE ? g.rank : 0, g.r_mode == GLOWQ_R_COMPUTE, dev.sms, g.split_k);
     if (pl.total > g.workspace_bytes) return GLOWQ_ERR_WORKSPACE_TOO_SMALL;
     unsigned char* ws = static_cast<unsigned char*>(g.workspace);
     const __half* x = static_cast<const __half*>(g.x) + static_cast<size_t>(m0) * g.x_stride;
@@ -510,20 +567,9 @@ int gemv_group_forward(const glowq_w4a16_group_t& g, const DeviceInfo& dev, cuda
       // persistent grid: every CTA resident at once, a whole number of CTAs per K slice
       // R units run on dedicated CTAs (the lowest block indices; several units each when there are many), so that the
       // r chain (R loads, MMAs, slot, release counter) overlaps the other CTAs' x staging and weight streaming
-      static const int max_r_ctas = env_int("GLOWQ_GEMV_R_CTAS", 96);
       // (the epoch word of the workspace counts the consumer warps of a grid in kEpochShift bits)
       const int cap = std::min(dev.sms * pl.ctas_per_sm, static_cast<int>(kEpochReaderMask) / kConsumerWarps);
-      {
-        int want = std::min(p.n_r_units, max_r_ctas);
-        if (pl.SK > 1) {
-          // K slices: the R CTAs take no row tiles afterwards, so give them the CTA slots that do not add a round
-          // of tiles to the slices (at least a few, or r would arrive long after the first tiles are done)
-          const int rounds = ceil_div(n_tiles * pl.SK, cap);
-          const int spare = cap - pl.SK * ceil_div(n_tiles, rounds);
-          want = std::min(p.n_r_units, std::max(std::min(spare, max_r_ctas), std::min(max_r_ctas, 16)));
-        }
-        p.n_r_ctas = std::max(0, std::min(want, cap / 3));
-      }
+      p.n_r_ctas = gemv_r_ctas(pl, n_tiles, p.n_r_units, cap);
       int grid = std::min(cap - p.n_r_ctas, n_tiles * pl.SK);
       grid = std::max(pl.SK, grid / pl.SK * pl.SK) + p.n_r_ctas;
       p.l_cols = std::min(std::max(p.rank, 8), 256);
@@ -625,7 +671,7 @@ size_t glowq_w4a16_workspace_bytes(int M, int IC, int OC_total, int rank, int n_
   n_members = std::max(1, std::min(n_members, GLOWQ_MAX_MEMBERS));
   const int n_tiles = ceil_div(OC_total, kTileRows) + n_members;
   // planned for more SMs than any device has, which bounds the split-K partial-sum area from above
-  const GemvPlan pl = make_plan(M, IC, n_tiles, rank, 1024, 0);
+  const GemvPlan pl = make_plan(M, IC, n_tiles, rank, rank > 0, 1024, 0);
   size_t need = pl.total;
   need = std::max(need, gemm_workspace_bytes(M, IC, OC_total, rank, n_members));
   return align_up(need, 256);
@@ -664,7 +710,7 @@ int glowq_internal_workspace_map(const glowq_w4a16_group_t* group, int sms, Work
     return GLOWQ_OK;
   }
   const int n_tiles = n_tiles_of(g);
-  const GemvPlan pl = make_plan(std::min(g.M, kGemvMaxM), g.IC, n_tiles, g.r_mode != GLOWQ_R_NONE ? g.rank : 0, sms, g.split_k);
+  const GemvPlan pl = make_plan(std::min(g.M, kGemvMaxM), g.IC, n_tiles, g.r_mode != GLOWQ_R_NONE ? g.rank : 0, g.r_mode == GLOWQ_R_COMPUTE, sms, g.split_k);
   if (pl.total > g.workspace_bytes) return GLOWQ_ERR_WORKSPACE_TOO_SMALL;
   map->kernel = 0;
   if (pl.SK > 1 && !pl.own_ctr) {
@@ -783,7 +829,7 @@ int glowq_w4a16_gemv_forward_static(const void* x, const int32_t* qweight, const
   if (rc != GLOWQ_OK) return rc;
   // The scratch this launch would use, from the same planner the launch itself runs.
   const int n_tiles = ceil_div(OC, kTileRows);
-  const GemvPlan pl = make_plan(std::max(M, 1), IC, n_tiles, 0, dev->sms, 0);
+  const GemvPlan pl = make_plan(std::max(M, 1), IC, n_tiles, 0, false, dev->sms, 0);
   if (pl.total > GLOWQ_W4A16_STATIC_SCRATCH_BYTES) return GLOWQ_ERR_TOO_LARGE;
   void* scratch = nullptr;
   rc = static_scratch_address(&scratch);

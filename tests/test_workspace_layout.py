@@ -100,3 +100,34 @@ def test_the_plans_have_slices_that_start_behind_the_weights(M, oc, ic, rank, r_
     m = workspace_map(M, ic, [oc], rank, alphas=[0.5], nbytes=nbytes, r_mode=r_mode)
     groups, steps = -(-ic // 128), -(-ic // 128) + -(-rank // 128)
     assert m.kernel == 2 and m.ksplit > 1 and steps * (m.ksplit - 1) // m.ksplit > groups
+
+
+@pytest.mark.parametrize("M", [2, 3, 5, 8])
+def test_what_the_exact_form_takes_and_what_stays_with_the_streaming_kernel(M):
+    """Only calls that the streaming kernel would take as well (its scratch, its layouts), and none that ask for something of its own."""
+    for ocs, ic, rank in itertools.product(([128], [72, 130], [5120], [3584, 512, 512], [18944] * 2), (128, 2048, 8200, 18944), (0, 64, 264)):
+        m = workspace_map(M, ic, ocs, rank)
+        assert m.kernel in (0, 1)
+        assert workspace_map(M, ic, ocs, rank, kernel=K.KERNEL_GEMV).kernel == 0
+        assert workspace_map(M, ic, ocs, rank, split_k=2).kernel == 0
+        e = K.load_w4a16_extension()
+        need = e.workspace_bytes(M, ic, sum(ocs), rank, len(ocs))
+        exact = workspace_map(M, ic, ocs, rank, nbytes=need)
+        assert (exact.kernel, exact.ksplit, exact.slots_end <= need) == (m.kernel, m.ksplit, True)
+        stream = workspace_map(M, ic, ocs, rank, kernel=K.KERNEL_GEMV)
+        if stream.slots_end > 38144:
+            workspace_map(M, ic, ocs, rank, nbytes=stream.slots_end - 1, rc=4)
+    assert workspace_map(8, 18944, [3584], 128).kernel == 1 and workspace_map(1, 18944, [3584], 128).kernel == 0
+
+
+def test_one_token_on_long_rows_takes_no_more_scratch_than_its_most_slices():
+    """The cost of a one-token launch may choose fewer slices than fit; the scratch asked for does not depend on the choice."""
+    seen = set()
+    for oc, ic, rank in itertools.product((32, 1536, 2048, 3584, 5120, 7168, 9216, 9472), (12288, 13824, 17408, 18944, 32768, 65536), (0, 16, 128, 1024)):
+        m = workspace_map(1, ic, [oc], rank)
+        seen.add(m.ksplit)
+        assert m.kernel == 0 and m.slots_end >= m.slots_begin + m.sliced_tiles * m.ksplit * 1024
+        workspace_map(1, ic, [oc], rank, nbytes=m.slots_end - 1, rc=4)
+        need = K.load_w4a16_extension().workspace_bytes(1, ic, oc, rank, 1)
+        assert workspace_map(1, ic, [oc], rank, nbytes=need).ksplit == m.ksplit
+    assert {1, 2, 3, 4} <= seen
