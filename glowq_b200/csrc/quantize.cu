@@ -4,15 +4,19 @@
 //   scale = (max - min) / 15, zero = clamp(rint(-min / scale), 0, 15), code = clamp(rint(w / scale + zero), 0, 15)
 // per (row, 128-column group); columns past IC count as zero; zero-point nibbles past the last group hold 8.
 //
-// Bound: HBM (2.6 bytes per weight).  A half warp holds one group in registers (16 lanes x 8 columns = one 16-byte load
-// and one packed word per lane), a warp takes the eight groups of one zero-point word: four loads in flight per lane,
-// the minimum and maximum travel as ONE half2 {-min, max} through four shuffles, and codes, scales and the zero word
-// leave as whole segments.  The weight is read once and nothing intermediate is written (the torch expression is about
-// thirty elementwise kernels).  Measured on B200: 13824 x 5120 in 66 us (2.8 TB/s), 5120 x 5120 in 29 us (2.4 TB/s): the
-// arithmetic (two conversions, a quotient and a rounding per weight) is what is left above the copy's 28 us.
+// Bound: HBM (2.6 bytes per weight), then issue slots.  A half warp holds one group in registers (16 lanes x 8 columns = one 16-byte
+// load and one packed word per lane), a warp takes the eight groups of one zero-point word: four loads in flight per lane, the minimum
+// and maximum travel as ONE half2 {-min, max}, and codes, scales and the zero word leave as whole segments.  The weight is read once
+// and nothing intermediate is written (the torch expression is about thirty elementwise kernels).
+// A warp's eight groups are divided once, a group per quad of lanes, and the quotients of its weights are paired fp32 operations; with
+// every half warp dividing for each of its four groups in turn, and for groups past the end of a row too, 13824 x 5120 took 64 us and
+// 18944 x 3584 (28 groups) 89; now 42 (3.9 TB/s; a copy's 28) and 46.  5120 x 5120: 26 -> 18.  Six blocks an SM: a few bytes of spill
+// in the path that divides, 43 us where five without took 45.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -25,6 +29,11 @@ constexpr int kQIters = 4;      // passes of two groups: the eight groups of a z
 __device__ __forceinline__ uint32_t hmax2_nan(uint32_t a, uint32_t b) {
   uint32_t r;
   asm("max.NaN.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ uint32_t hmin2_nan(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("min.NaN.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
   return r;
 }
 __device__ __forceinline__ uint32_t hadd2(uint32_t a, uint32_t b) {
@@ -40,18 +49,43 @@ __device__ __forceinline__ uint32_t code_bits(uint32_t x) {
   asm("min.f16x2 %0, %1, %2;" : "=r"(r) : "r"(r), "r"(0x4B804B80u));
   return hadd2(r, 0x64006400u);
 }
+// code_bits(q + z) where neither is NaN: the sum as a fused multiply-add by one that takes the lower clamp along.
+__device__ __forceinline__ uint32_t sum_code_bits(uint32_t q, uint32_t z) {
+  uint32_t r;
+  asm("fma.rn.relu.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(q), "r"(0x3C003C00u), "r"(z));
+  asm("min.f16x2 %0, %1, %2;" : "=r"(r) : "r"(r), "r"(0x4B804B80u));
+  return hadd2(r, 0x64006400u);
+}
+// Two products or fused multiply-adds in one instruction, each rounded like the single one.
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z, w;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+      "fma.rn.f32x2 w, x, y, z;\n\tmov.b64 {%0, %1}, w;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   const __half2 h = __floats2half2_rn(lo, hi);
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-__global__ void __launch_bounds__(kQThreads) quantize_kernel(const __half* __restrict__ w, int32_t* __restrict__ qweight,
+__global__ void __launch_bounds__(kQThreads, 6) quantize_kernel(const __half* __restrict__ w, int32_t* __restrict__ qweight,
                                                              int32_t* __restrict__ qzeros, __half* __restrict__ scales, int OC,
                                                              int IC, int G, int words, long long w_stride, int vec_ok) {
   const int lane = threadIdx.x & 31, hsel = lane >> 4, s16 = lane & 15;
-  const long long item = static_cast<long long>(blockIdx.x) * (kQThreads / 32) + (threadIdx.x >> 5);
-  if (item >= static_cast<long long>(OC) * words) return;   // whole warps leave together
-  const int row = static_cast<int>(item / words), zw_i = static_cast<int>(item - static_cast<long long>(row) * words);
+  // (32 bits: an item is 1024 weights, or one row; the launch refuses more than 2^31 blocks of eight)
+  const uint32_t item = blockIdx.x * (kQThreads / 32) + (threadIdx.x >> 5);
+  const uint32_t row_u = item / static_cast<uint32_t>(words);
+  if (row_u >= static_cast<uint32_t>(OC)) return;   // whole warps leave together
+  const int row = static_cast<int>(row_u), zw_i = static_cast<int>(item - row_u * static_cast<uint32_t>(words));
   const __half* wrow = w + static_cast<size_t>(row) * w_stride;
   uint4 v[kQIters];
 #pragma unroll
@@ -67,57 +101,74 @@ __global__ void __launch_bounds__(kQThreads) quantize_kernel(const __half* __res
       v[i] = *reinterpret_cast<const uint4*>(t);
     }
   }
-  uint32_t zword = 0, my_scale = 0;
+  // {-min, max} of the eight groups as one half2 each: a half warp's four passes change places while they are reduced (five shuffles,
+  // not sixteen), after which the four lanes of a quad hold one group, pass `mine` of their half warp.
+  uint32_t mm[kQIters];
 #pragma unroll
   for (int i = 0; i < kQIters; ++i) {
-    const int g = zw_i * 8 + 2 * i + hsel;
-    // {-min, max} of the group as one half2
     const uint32_t hi2 = hmax2_nan(hmax2_nan(v[i].x, v[i].y), hmax2_nan(v[i].z, v[i].w));
-    constexpr uint32_t kSign = 0x80008000u;
-    const uint32_t lo2 = hmax2_nan(hmax2_nan(v[i].x ^ kSign, v[i].y ^ kSign), hmax2_nan(v[i].z ^ kSign, v[i].w ^ kSign));
-    uint32_t mm = hmax2_nan(prmt(lo2, hi2, 0x5410), prmt(lo2, hi2, 0x7632));
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) mm = hmax2_nan(mm, __shfl_xor_sync(0xffffffffu, mm, o));
-    const float2 mf = __half22float2(*reinterpret_cast<const __half2*>(&mm));   // {-min, max}
-    const float diff = __half2float(__float2half_rn(mf.y + mf.x));
-    // (the lower clamp of the scale, 1e-8, rounds to zero in fp16: it only turns -0 into +0)
-    const uint32_t sbits = __half_as_ushort(__float2half_rn(__fdiv_rn(diff, 15.f))) & (diff == 0.f ? 0u : 0xFFFFu);
-    const float sc = __half2float(__ushort_as_half(static_cast<unsigned short>(sbits)));
-    const uint32_t zq = pack2(__fdiv_rn(mf.x, sc), 0.f);
-    const uint32_t z = code_bits(zq) & 0xFu;
-    zword |= (g < G ? z : 8u) << (4 * (2 * i + hsel));
-    // w / scale rounded to fp32 and then to fp16, as the division of two halves is.  With r the correctly rounded
-    // reciprocal, one residual step on w * r gives the correctly rounded quotient (Markstein, IBM J. Res. Dev. 34,
-    // 1990); a scale of zero, infinity or NaN divides.
-    // (the zero point that is added keeps a NaN, 0 / 0, although the stored one is 0)
-    const uint32_t zh = (zq & 0x7FFFu) > 0x7C00u ? 0x7FFFu : static_cast<uint32_t>(__half_as_ushort(__uint2half_rn(z)));
-    const uint32_t z2 = zh * 0x00010001u;
-    const float r = __frcp_rn(sc);
-    const bool plain = sbits != 0u && sbits < 0x7C00u;   // the same for the half warp's 16 lanes
-    const uint32_t* vw = &v[i].x;
-    uint32_t word = 0;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(vw + e));
-      uint32_t q;
-      if (plain) {
-        const float q0 = f.x * r, q1 = f.y * r;
-        q = pack2(fmaf(fmaf(-q0, sc, f.x), r, q0), fmaf(fmaf(-q1, sc, f.y), r, q1));
-      } else {
-        q = pack2(__fdiv_rn(f.x, sc), __fdiv_rn(f.y, sc));
-      }
-      const uint32_t c = code_bits(hadd2(q, z2));          // bits 0..3: column 2e, bits 16..19: column 2e + 1
-      word |= ((c & 0xFu) | ((c >> 12) & 0xF0u)) << (8 * e);
-    }
-    if (g < G) qweight[static_cast<size_t>(row) * (static_cast<size_t>(G) * 16) + g * 16 + s16] = static_cast<int32_t>(word);
-    // lane l < 8 keeps the scale of group l of the word (group 2 i + h comes from half warp h)
-    const uint32_t from = __shfl_sync(0xffffffffu, sbits, (lane & 1) * 16);
-    if ((lane >> 1) == i) my_scale = from;
+    const uint32_t lo2 = hmin2_nan(hmin2_nan(v[i].x, v[i].y), hmin2_nan(v[i].z, v[i].w));
+    mm[i] = hmax2_nan(prmt(lo2, hi2, 0x5410) ^ 0x8000u, prmt(lo2, hi2, 0x7632) ^ 0x8000u);
   }
-  zword |= __shfl_xor_sync(0xffffffffu, zword, 16);
+  const bool b3 = lane & 8, b2 = lane & 4;
+  const int mine = (b2 ? 2 : 0) + (b3 ? 1 : 0);
+  const uint32_t m01 = hmax2_nan(b3 ? mm[1] : mm[0], __shfl_xor_sync(0xffffffffu, b3 ? mm[0] : mm[1], 8));
+  const uint32_t m23 = hmax2_nan(b3 ? mm[3] : mm[2], __shfl_xor_sync(0xffffffffu, b3 ? mm[2] : mm[3], 8));
+  uint32_t m = hmax2_nan(b2 ? m23 : m01, __shfl_xor_sync(0xffffffffu, b2 ? m01 : m23, 4));
+  m = hmax2_nan(m, __shfl_xor_sync(0xffffffffu, m, 2));
+  m = hmax2_nan(m, __shfl_xor_sync(0xffffffffu, m, 1));
+  const int gl = 2 * mine + hsel, g_own = zw_i * 8 + gl;
+  const float2 mf = __half22float2(*reinterpret_cast<const __half2*>(&m));   // {-min, max}
+  const float diff = __half2float(__float2half_rn(mf.y + mf.x));
+  // (the lower clamp of the scale, 1e-8, rounds to zero in fp16: it only turns -0 into +0)
+  const uint32_t sbits = __half_as_ushort(__float2half_rn(__fdiv_rn(diff, 15.f))) & (diff == 0.f ? 0u : 0xFFFFu);
+  const float sc_own = __half2float(__ushort_as_half(static_cast<unsigned short>(sbits)));
+  const uint32_t zq = pack2(__fdiv_rn(mf.x, sc_own), 0.f);
+  const uint32_t z = code_bits(zq) & 0xFu;
+  // (the zero point that is added keeps a NaN, 0 / 0, although the stored one is 0)
+  const uint32_t zh = (zq & 0x7FFFu) > 0x7C00u ? 0x7FFFu : static_cast<uint32_t>(__half_as_ushort(__uint2half_rn(z)));
+  const uint32_t own = sbits | (zh << 16);
+  const float r_own = __frcp_rn(sc_own);
+  // w / scale rounded to fp32 and then to fp16, as the division of two halves is.  With r the correctly rounded
+  // reciprocal, one residual step on w * r gives the correctly rounded quotient (Markstein, IBM J. Res. Dev. 34,
+  // 1990); where a group's scale is zero, infinity or NaN the warp divides.  (Not for groups past the end, which are not stored.)
+  const auto codes = [&](auto plain) {
+#pragma unroll
+    for (int i = 0; i < kQIters; ++i) {
+      const int g = zw_i * 8 + 2 * i + hsel, from = hsel * 16 + (i & 1) * 8 + (i >> 1) * 4;
+      const uint32_t sz = __shfl_sync(0xffffffffu, own, from);
+      const float sc = __half2float(__ushort_as_half(static_cast<unsigned short>(sz & 0xFFFFu)));
+      const uint32_t z2 = prmt(sz, sz, 0x3232);
+      const uint32_t* vw = &v[i].x;
+      uint32_t c[4];
+      if constexpr (plain.value) {
+        const float r = __shfl_sync(0xffffffffu, r_own, from);
+        const float2 rr = make_float2(r, r), ss = make_float2(-sc, -sc);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 f = __half22float2(*reinterpret_cast<const __half2*>(vw + e));
+          const float2 q0 = mul2(f, rr), q1 = fma2(fma2(q0, ss, f), rr, q0);
+          c[e] = sum_code_bits(pack2(q1.x, q1.y), z2);   // byte 0: column 2e, byte 2: column 2e + 1 (in its low four bits)
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 f = __half22float2(*reinterpret_cast<const __half2*>(vw + e));
+          c[e] = code_bits(hadd2(pack2(__fdiv_rn(f.x, sc), __fdiv_rn(f.y, sc)), z2));
+        }
+      }
+      const uint32_t c01 = prmt(c[0], c[1], 0x6240), c23 = prmt(c[2], c[3], 0x6240);
+      const uint32_t word = prmt(c01, c23, 0x5410) | (prmt(c01, c23, 0x7632) << 4);
+      if (g < G) qweight[static_cast<size_t>(row) * (static_cast<size_t>(G) * 16) + g * 16 + s16] = static_cast<int32_t>(word);
+    }
+  };
+  if (__all_sync(0xffffffffu, (sbits != 0u && sbits < 0x7C00u) || g_own >= G))
+    codes(std::true_type{});
+  else
+    codes(std::false_type{});
+  const uint32_t zword = __reduce_or_sync(0xffffffffu, (g_own < G ? z : 8u) << (4 * gl));
   if (lane == 0) qzeros[static_cast<size_t>(row) * words + zw_i] = static_cast<int32_t>(zword);
-  const int gs = zw_i * 8 + lane;
-  if (lane < 8 && gs < G) scales[static_cast<size_t>(row) * G + gs] = __ushort_as_half(static_cast<unsigned short>(my_scale));
+  if ((lane & 3) == 0 && g_own < G) scales[static_cast<size_t>(row) * G + g_own] = __ushort_as_half(static_cast<unsigned short>(sbits));
 }
 
 }  // namespace
