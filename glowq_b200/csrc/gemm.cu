@@ -2,7 +2,7 @@
 //
 //   Y[M, OC] = X[M, IC] . dequant(Q)^T  +  alpha * r[M, rank] . L[OC, rank]^T  (+ bias),     r = X . R^T
 //
-// Up to 64 tokens one CTA per 128 output columns (gemm_tmem.cu), above a CTA pair per 256 (gemm_pair.cu).  Both keep the
+// Up to 64 tokens one CTA per 128 output columns (gemm_tmem.cu; up to 8 in its exact form), above a CTA pair per 256 (gemm_pair.cu).  Both keep the
 // dequantised weights in tensor memory, and both compute r inside the group launch.  The line lies where the first ends: two CTAs
 // share an SM's tensor memory there, which leaves an accumulator 64 tokens (13B gate/up 45 us at 64 tokens; the pair form, whose
 // tiles have 64 tokens at least, takes 14B gate/up at 65 tokens from 67 to 63 us).
@@ -59,9 +59,9 @@ inline size_t r_slot_bytes(int M, int IC, int rank) {
   const int ks = std::max(1, std::min({16, cdiv(IC, 64) / 4, 128 / tiles}));
   return ks > 1 ? static_cast<size_t>(ks) * tiles * kSlotBytes : 0;
 }
-// Slots of the members' K slices where the tiles do not fill the SMs (9 to 256 tokens).
+// Slots of the members' K slices where the tiles do not fill the SMs (9 to 256 tokens; the one-CTA form's are counted below).
 inline size_t main_slot_bytes(int M, int OC_total, int n_members) {
-  // (up to 8 tokens the automatic choice never comes here; a forced call then runs without slicing)
+  // (up to 8 tokens only the one-CTA form comes here)
   const int m_tiles = cdiv(M, 128);
   if (M <= 8 || M > 256 || cdiv(OC_total, 256) * m_tiles * 2 > kPlanSms) return 0;
   const int tiles = (cdiv(OC_total, 128) + n_members) * m_tiles;

@@ -1,4 +1,4 @@
-// Corrected W4A16 product for decode batches (9 to 64 tokens; fewer on request) with the dequantised weights in TENSOR MEMORY.
+// Corrected W4A16 product for decode batches (9 to 64 tokens; 2 to 8 in an exact form, see EXACT) with the dequantised weights in TENSOR MEMORY.
 //
 //   D[128 output columns, N tokens] += W[128, 128 k] . X[N, 128 k]^T      (one quantisation group of K per step)
 //
@@ -27,10 +27,11 @@
 // gets through on any number of SMs.  Every wait is bounded; on expiry a status word is set, and the CTA drains and frees its
 // tensor memory.
 //
-// Measured (B200, corrected group calls of the 13B shapes, microseconds at 16 / 32 / 64 tokens; before: weights through
-// shared memory, r and slot sum as launches of their own): q/k/v 38.7 / 39.4 / 44.5 -> 23.6 / 24.3 / 28.7, o_proj 22.2 /
-// 22.9 / 25.0 -> 15.5 / 16.1 / 21.6, gate/up 58.1 / 58.6 / 60.5 -> 36.7 / 37.5 / 42.3 (1.9 TB/s of packed weights), down_proj
-// 38.8 / 38.1 / 40.7 -> 22.8 / 23.7 / 29.0.  Left: about 8 microseconds of dependent chain per launch, and 0.33 per step and SM.
+// Measured (B200, corrected group calls of the 13B shapes, microseconds at 16 / 32 / 64 tokens; before: MMAs issued by a lane that
+// had waited alone, an epilogue of one token at a time, two slots in flight): q/k/v 19.2 / 20.5 / 23.3 (23.6 / 24.3 / 28.7), o_proj
+// 11.2 / 12.3 / 16.1 (15.5 / 16.1 / 21.6), gate/up 29.5 / 30.1 / 33.8 (36.7 / 37.5 / 42.3), down_proj 18.1 / 19.8 / 23.7 (22.8 /
+// 23.7 / 29.0).  Left: five to six microseconds of dependent chain per launch, and 0.3 to 0.4 per step and SM for the
+// issue slots of the dequant warps, where the packed bytes alone would take 0.19 at the measured copy rate.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>

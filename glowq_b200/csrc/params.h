@@ -49,7 +49,7 @@ constexpr uint32_t kEpochReaderMask = (1u << kEpochShift) - 1u;
 constexpr uint32_t kEpochMask = (1u << 20) - 1u;
 constexpr size_t kWsHeaderBytes = WS_HEADER_WORDS * 4;
 constexpr int kMaxRTiles = 64;      // rank <= 1024
-// After the header: 1 KB of counters for r = x . R^T (of the stand-alone product, or of the CTAs of a 9 to 64 token launch that
+// After the header: 1 KB of counters for r = x . R^T (of the stand-alone product, or of the CTAs of a 2 to 64 token launch that
 // compute it), then r of the running streaming launch as its row tiles read it - 8-byte words
 // {half2(r[tok][2j], r[tok][2j+1]), launch epoch}, up to 8 tokens x rank 1024 - then the tile counters.  All of this lies at
 // the same place whatever a call's sizes are, and every slot and partial buffer of every kernel lies behind it
@@ -70,7 +70,7 @@ constexpr unsigned kPrefetchSlice = 16u << 10;  // bytes per L2 prefetch request
 
 // Byte ranges of the workspace that a launch uses besides the fixed areas in front of the tile counters, and its partition.
 struct WorkspaceMap {
-  int kernel;                       // 0 weight streaming, 1 one CTA per tile (9 to 64 tokens), 2 CTA pairs
+  int kernel;                       // 0 weight streaming, 1 one CTA per tile (2 to 64 tokens), 2 CTA pairs
   int ksplit, whole_tiles, sliced_tiles, r_ctas, shortest;   // shortest: K steps of the member with the fewest
   unsigned long long ctr_begin, ctr_end;       // tile counters, zero between launches
   unsigned long long slots_begin, slots_end;   // partial results: any bits before and after a launch

@@ -1,4 +1,4 @@
-// r = x . R^T (the shared right factor applied to the activations) for 9 to 64 tokens, as ONE small launch in front of a group
+// r = x . R^T (the shared right factor applied to the activations) for up to 64 tokens, as ONE small launch in front of a group
 // launch whose workspace has no room to compute r itself.
 // The [M, rank] result is a handful of tiles, so the work is cut along K as well:
 // CTA (unit, by) multiplies 16 rows of R with one 1024-column slice of K for 64 tokens (one 8-token block per warp,

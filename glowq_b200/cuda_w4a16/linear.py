@@ -7,7 +7,7 @@ Differences from the reference, all on the host side of the same interface:
 * the kernel choice knobs W4A16_KERNEL_OUT_DTYPE / W4A16_GEMV_M_MAX / W4A16_FORCE_GEMM / W4A16_FORCE_GEMV are
   read once when the module is built (the reference re-reads the environment on every call, linear.py:172-177);
   W4A16_GEMV_M_MAX has no built-in default of 128 here: unset, the library switches kernels where it measured the
-  cross-over (8 tokens);
+  cross-over (2 to 8 tokens by an estimate of both, tensor cores above);
   the dequant-cache / chunk / JIT knobs belong to fallbacks that do not exist here;
 * output and scratch buffers are caller-side torch tensors; the library allocates nothing.
 """
@@ -81,7 +81,7 @@ def _kernel_quantises(weight: torch.Tensor, group_size: int) -> bool:
     """The one-launch quantiser takes what a conversion hands over: a plain fp16 matrix on an sm_100 device in groups of
     128.  Everything else (CPU tensors, other types, group sizes and devices, no library) is the torch expression, the same bits.
     Measured for the seven linears of a Llama-2-13B layer: 29.1 ms with the torch expression and the buffers of the
-    module made on the host, 1.0 ms with this launch (0.32 ms on the GPU, the rest builds the modules)."""
+    module made on the host, 0.38 ms with this launch (0.31 ms of it on the GPU; the modules are built around its buffers)."""
     return (group_size == 128 and weight.is_cuda and weight.dtype == torch.float16 and type(weight) is torch.Tensor
             and not weight.requires_grad and weight.numel() > 0 and weight.stride(1) == 1
             and weight.stride(0) >= weight.shape[1] and _device_quantises(weight.device))
@@ -159,7 +159,7 @@ class CudaW4A16Linear(nn.Module):
     def kernel_choice(self, m: int) -> int:
         """Which kernel a call with ``m`` tokens asks for (linear.py:172-181): a FORCE knob wins; otherwise an
         explicitly set W4A16_GEMV_M_MAX sends ``m <= W4A16_GEMV_M_MAX`` to the weight-streaming kernel and anything
-        larger to the tensor-core kernel; with the knob unset the library's own switch-over (8 tokens) applies."""
+        larger to the tensor-core kernel; with the knob unset the library's own switch-over (2 to 8 tokens) applies."""
         if self._force_gemm:
             return K.KERNEL_GEMM
         if self._force_gemv:
