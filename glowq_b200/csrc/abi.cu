@@ -18,7 +18,7 @@ cudaError_t launch_generic(const __half* x, const MemberDev& mb, const float* r3
                            int group_size, int x_stride, cudaStream_t stream);
 cudaError_t launch_dequant(const int32_t* qweight, const __half* scales, const int32_t* qzeros, __half* out, int OC, int IC,
                            int group_size, int wstride, int zstride, int sstride, cudaStream_t stream);
-cudaError_t launch_quantize(const __half* w, int32_t* qweight, int32_t* qzeros, __half* scales, int OC, int IC,
+cudaError_t launch_quantize(const __half* w, int32_t* qweight, int32_t* qzeros, __half* scales, int64_t* gid, int OC, int IC,
                             long long w_stride, cudaStream_t stream);
 bool gemm_supported(const glowq_w4a16_group_t& g);
 double gemm_exact_us(const glowq_w4a16_group_t& g, int sms);
@@ -654,6 +654,11 @@ int glowq_w4a16_dequant(const int32_t* qweight, const void* scales, const int32_
 
 int glowq_w4a16_quantize(const void* weight, int32_t* qweight, int32_t* qzeros, void* scales, int OC, int IC, int group_size,
                          long long weight_stride, void* stream) {
+  return glowq_w4a16_quantize_indexed(weight, qweight, qzeros, scales, nullptr, OC, IC, group_size, weight_stride, stream);
+}
+
+int glowq_w4a16_quantize_indexed(const void* weight, int32_t* qweight, int32_t* qzeros, void* scales, int64_t* group_index, int OC, int IC,
+                                 int group_size, long long weight_stride, void* stream) {
   if (!weight || !qweight || !qzeros || !scales || OC <= 0 || IC <= 0) return GLOWQ_ERR_BAD_ARGUMENT;
   if (group_size <= 0 || group_size % 8 != 0) return GLOWQ_ERR_BAD_GROUP_SIZE;
   if (group_size != kGroup) return GLOWQ_ERR_UNSUPPORTED_SHAPE;
@@ -661,8 +666,8 @@ int glowq_w4a16_quantize(const void* weight, int32_t* qweight, int32_t* qzeros, 
   const DeviceInfo* dev = nullptr;
   int rc = device_info(&dev);
   if (rc != GLOWQ_OK) return rc;
-  const cudaError_t e = launch_quantize(static_cast<const __half*>(weight), qweight, qzeros, static_cast<__half*>(scales), OC, IC,
-                                        weight_stride, static_cast<cudaStream_t>(stream));
+  const cudaError_t e = launch_quantize(static_cast<const __half*>(weight), qweight, qzeros, static_cast<__half*>(scales), group_index, OC,
+                                        IC, weight_stride, static_cast<cudaStream_t>(stream));
   return e == cudaSuccess ? GLOWQ_OK : fail_cuda(e);
 }
 

@@ -79,7 +79,8 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 
 __global__ void __launch_bounds__(kQThreads, 6) quantize_kernel(const __half* __restrict__ w, int32_t* __restrict__ qweight,
                                                              int32_t* __restrict__ qzeros, __half* __restrict__ scales, int OC,
-                                                             int IC, int G, int words, long long w_stride, int vec_ok) {
+                                                             int IC, int G, int words, long long w_stride, int vec_ok,
+                                                             int64_t* __restrict__ gid) {
   const int lane = threadIdx.x & 31, hsel = lane >> 4, s16 = lane & 15;
   // (32 bits: an item is 1024 weights, or one row; the launch refuses more than 2^31 blocks of eight)
   const uint32_t item = blockIdx.x * (kQThreads / 32) + (threadIdx.x >> 5);
@@ -166,6 +167,9 @@ __global__ void __launch_bounds__(kQThreads, 6) quantize_kernel(const __half* __
     codes(std::true_type{});
   else
     codes(std::false_type{});
+  if (gid != nullptr && row == 0) {   // the module's group index of every column: a launch or two less than made on their own
+    for (int k = zw_i * 1024 + lane; k < min(IC, zw_i * 1024 + 1024); k += 32) gid[k] = k >> 7;
+  }
   const uint32_t zword = __reduce_or_sync(0xffffffffu, (g_own < G ? z : 8u) << (4 * gl));
   if (lane == 0) qzeros[static_cast<size_t>(row) * words + zw_i] = static_cast<int32_t>(zword);
   if ((lane & 3) == 0 && g_own < G) scales[static_cast<size_t>(row) * G + g_own] = __ushort_as_half(static_cast<unsigned short>(sbits));
@@ -173,7 +177,7 @@ __global__ void __launch_bounds__(kQThreads, 6) quantize_kernel(const __half* __
 
 }  // namespace
 
-cudaError_t launch_quantize(const __half* w, int32_t* qweight, int32_t* qzeros, __half* scales, int OC, int IC,
+cudaError_t launch_quantize(const __half* w, int32_t* qweight, int32_t* qzeros, __half* scales, int64_t* gid, int OC, int IC,
                             long long w_stride, cudaStream_t stream) {
   const int G = (IC + 127) / 128, words = (G + 7) / 8;
   const long long items = static_cast<long long>(OC) * words;
@@ -181,7 +185,7 @@ cudaError_t launch_quantize(const __half* w, int32_t* qweight, int32_t* qzeros, 
   if (blocks > 0x7FFFFFFFll) return cudaErrorInvalidValue;
   const int vec_ok = (IC & 7) == 0 && (w_stride & 7) == 0 && (reinterpret_cast<uintptr_t>(w) & 15u) == 0;
   quantize_kernel<<<static_cast<unsigned>(blocks), kQThreads, 0, stream>>>(w, qweight, qzeros, scales, OC, IC, G, words, w_stride,
-                                                                          vec_ok);
+                                                                          vec_ok, gid);
   return cudaGetLastError();
 }
 

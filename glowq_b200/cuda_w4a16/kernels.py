@@ -65,7 +65,7 @@ EXPORTS = ("glowq_w4a16_version", "glowq_w4a16_strerror", "glowq_w4a16_last_cuda
            "glowq_w4a16_gemv_forward", "glowq_w4a16_gemm_forward", "glowq_w4a16_group_forward",
            "glowq_w4a16_group_forward_many", "glowq_w4a16_group_forward_host", "glowq_w4a16_workspace_bytes",
            "glowq_w4a16_read_status", "glowq_w4a16_gemv_forward_static", "glowq_w4a16_allreduce_f16",
-           "glowq_w4a16_allreduce_finish_f16", "glowq_w4a16_quantize")
+           "glowq_w4a16_allreduce_finish_f16", "glowq_w4a16_quantize", "glowq_w4a16_quantize_indexed")
 
 
 def library_path() -> str:
@@ -92,6 +92,7 @@ class _Ext:
         lib.glowq_w4a16_last_cuda_error.restype = i32
         lib.glowq_w4a16_dequant.argtypes = [vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, vp]
         lib.glowq_w4a16_quantize.argtypes = [vp, vp, vp, vp, i32, i32, i32, ctypes.c_longlong, vp]
+        lib.glowq_w4a16_quantize_indexed.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, ctypes.c_longlong, vp]
         lib.glowq_w4a16_gemv_forward.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp, sz, vp]
         lib.glowq_w4a16_gemm_forward.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32, vp, sz, vp]
         lib.glowq_w4a16_group_forward.argtypes = [ctypes.POINTER(Group)]
@@ -195,20 +196,25 @@ class _Ext:
 
     def quantize(self, weight, group_size: int):
         """(qweight_i32, qzeros_i32, scales_f16) of a [OC, IC] fp16 weight with unit column stride, in one launch."""
+        return self.quantize_indexed(weight, group_size, False)[:3]
+
+    def quantize_indexed(self, weight, group_size: int, index: bool = True):
+        """``quantize`` and the group index of every column (int64 [IC]; None unless asked for), in the same launch."""
         oc, ic = weight.shape
         groups = -(-ic // group_size)
         qweight = torch.empty((oc, groups * (group_size // 8)), dtype=torch.int32, device=weight.device)
         qzeros = torch.empty((oc, (groups + 7) // 8), dtype=torch.int32, device=weight.device)
         scales = torch.empty((oc, groups), dtype=torch.float16, device=weight.device)
-        args = (weight.data_ptr(), qweight.data_ptr(), qzeros.data_ptr(), scales.data_ptr(), oc, ic, int(group_size),
-                max(weight.stride(0), ic), current_stream_ptr(weight.device))
+        gid = torch.empty(ic, dtype=torch.int64, device=weight.device) if index else None
+        args = (weight.data_ptr(), qweight.data_ptr(), qzeros.data_ptr(), scales.data_ptr(),
+                gid.data_ptr() if index else None, oc, ic, int(group_size), max(weight.stride(0), ic), current_stream_ptr(weight.device))
         if torch.cuda.current_device() == weight.device.index:
-            rc = self.lib.glowq_w4a16_quantize(*args)
+            rc = self.lib.glowq_w4a16_quantize_indexed(*args)
         else:
             with torch.cuda.device(weight.device):
-                rc = self.lib.glowq_w4a16_quantize(*args)
+                rc = self.lib.glowq_w4a16_quantize_indexed(*args)
         self.check(rc, "glowq_w4a16_quantize")
-        return qweight, qzeros, scales
+        return qweight, qzeros, scales, gid
 
 
 def int32(v: int) -> int:

@@ -153,6 +153,10 @@ int glowq_w4a16_dequant(const int32_t* qweight, const void* scales, const int32_
 int glowq_w4a16_quantize(const void* weight, int32_t* qweight, int32_t* qzeros, void* scales, int OC, int IC,
                          int group_size, long long weight_stride, void* stream);
 
+/* The same, and group_index[IC] (int64, NULL = not wanted): k / 128 of every column k, the module's `gid` buffer. */
+int glowq_w4a16_quantize_indexed(const void* weight, int32_t* qweight, int32_t* qzeros, void* scales, int64_t* group_index, int OC,
+                                 int IC, int group_size, long long weight_stride, void* stream);
+
 /* Plain W4A16 product out[M, OC] (fp16) = x[M, IC] . dequant(Q)^T with the weight-streaming kernel.
  * Replaces w4a16_gemv_forward_cuda / gemv_w4a16_asym (csrc/gemv_w4a16.cu:146-214, csrc/pybind.cpp:19-34).
  * The caller allocates `out`; `workspace` as for a group call. */

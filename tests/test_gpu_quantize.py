@@ -69,3 +69,20 @@ def test_from_float_without_a_library(monkeypatch):
     got = L.CudaW4A16Linear.from_float(lin, 128)
     for name, t in want.state_dict().items():
         assert torch.equal(got.state_dict()[name], t), name
+
+
+class _Sub(L.CudaW4A16Linear):
+    """A subclass goes through its constructor: buffers of its own, replaced and moved."""
+
+
+@pytest.mark.parametrize("oc,ic,bias", [(1, 1, True), (3, 128, False), (24, 200, True), (7, 1032, True), (40, 2047, False), (9, 5000, False)])
+def test_a_conversion_makes_the_module_that_the_constructor_makes(oc, ic, bias):
+    lin = torch.nn.Linear(ic, oc, bias=bias, device="cuda", dtype=torch.float16)
+    got, want = L.CudaW4A16Linear.from_float(lin, 128), _Sub.from_float(lin, 128)
+    assert [n for n, _ in got.named_buffers()] == [n for n, _ in want.named_buffers()]
+    for (n, a), (_, b) in zip(got.named_buffers(), want.named_buffers()):
+        assert a.dtype == b.dtype and a.device == b.device and a.stride() == b.stride() and torch.equal(a, b), n
+    assert set(got.state_dict()) == set(want.state_dict()) and (got.bias is None) == (want.bias is None) == (not bias)
+    assert not bias or torch.equal(got.bias, want.bias) and got.bias.requires_grad == want.bias.requires_grad
+    x = torch.randn(3, ic, device="cuda", dtype=torch.float16)
+    assert ic % 8 or torch.equal(got(x), want(x))
