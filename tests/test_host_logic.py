@@ -1,4 +1,5 @@
 """Host side of the drop-in (quantiser, conversion pass, wrappers, patchers, C-ABI exports) on CPU."""
+import ctypes
 import json
 import os
 import re
@@ -237,3 +238,22 @@ def test_workspace_covers_every_k_sliced_plan():
                         need = max(need, ks * tiles * nn * rows * 128 * 4)
                 have = wb(m, ic, sum(ocs), 0, len(ocs))
                 assert have >= need + 256, (ocs, ic, m, have, need)
+
+
+def test_a_packed_descriptor_has_the_fields_of_the_struct():
+    """Every field in its place: the packed form of a call with as many values as fields, read back through the struct."""
+    group_fields = [n for n, _ in K.Group._fields_ if n != "members"]
+    member_fields = [n for n, _ in K.Member._fields_]
+    group = dict(zip(group_fields, range(1, len(group_fields) + 1)))
+    members = [dict(zip(member_fields, range(100 * (i + 1), 100 * (i + 1) + len(member_fields)))) for i in range(4)]
+    raw = K.PACK_GROUP.pack(*group.values()) + b"".join(K.PACK_MEMBER.pack(*m.values()) for m in members)
+    got = K.Group.from_buffer_copy(raw)
+
+    def value(struct, name):
+        v = getattr(struct, name)
+        return v if isinstance(v, (int, float)) else ctypes.cast(v, ctypes.c_void_p).value
+
+    assert {n: value(got, n) for n in group_fields} == group
+    for i, m in enumerate(members):
+        assert {n: value(got.members[i], n) for n in member_fields} == m
+    assert K.int32(2**31 + 5) == 5 - 2**31 and K.int32(-7) == -7 and K.int32(2**31 - 1) == 2**31 - 1
