@@ -12,14 +12,15 @@
 //   warp 2      weight producer (one thread): TMA of 128 rows x 64 B of packed codes, or of 32 columns of an fp16 operand (L, R)
 //   warp 3      scales and zero points: from memory into shared memory beside the packed stage, in the form the arithmetic takes
 //   warps 4-7   epilogue: accumulators as MMA fragments, transposed by stmatrix, stored by the copy engine
-//   warps 8-15  dequantise, in two teams of four warps that take alternate steps (a thread owns one weight row)
+//   warps 8-15  dequantise, in two teams of four warps that take alternate steps (a thread owns one weight row); two thirds of the pass
+//               that adds K slices' slots or the correction's accumulator are theirs as well
 // r = X . R^T is the first items of the launch: R in the place of the weights (fp16 rows go to tensor memory as they are), the
 // output goes to r_buf; the producers wait for the count of finished r tiles before their first correction step.
 //   What bounds it: 256 tokens, the MMAs (1024 clocks a step; measured 1030) and the epilogue that only the next steps' dequantisation
-// runs under; narrower tiles, tensor memory's writes and the chain from a stage's release to its next MMAs (about 1100 clocks a step
+// runs under; narrower tiles, tensor memory's writes and the chain from a stage's release to its next MMAs (about 1000 clocks a step
 // whatever the width, also with four teams).  Long runs are bound by the 1 kW limit.  Corrected group calls at 211, 2048 and
-// 4096 tokens, us (behind the stroke the form with fp16 weight tiles in shared memory, r and the slot sum as launches): 14B gate/up 70,
-// 551, 1083 / 90, 690, 1328; 14B down_proj 61, 298, 562 / 95, 374, 749; 3B q/k/v 21, 72, 117 / 37, 85, 143.
+// 4096 tokens, us (behind the stroke before the elected waits, the dequantisation in place, the shared sums and the fitted plans, same
+// minute): 14B gate/up 69, 601, 1217 / 72, 641, 1244; 14B down_proj 49, 310, 640 / 64, 351, 657; 3B q/k/v 25, 69, 123 / 28, 75, 136.
 //   Items are taken in order from a ticket (or are the clusters themselves where they are few): a CTA waits for items in front of
 // its own only, so a launch gets through on any number of SMs.  K may be sliced; the CTAs of a tile's last slice add the other
 // slices' fp32 slots in slice order (deterministic).  Every wait is bounded; on expiry a status word is set and the CTAs drain.
