@@ -8,6 +8,7 @@ from __future__ import annotations
 import ctypes
 import os
 import struct
+import threading
 from typing import Optional
 
 import torch
@@ -106,7 +107,8 @@ class _Ext:
         lib.glowq_w4a16_allreduce_finish_f16.argtypes = [ctypes.POINTER(Peers), vp, i32, i32, vp]
         if lib.glowq_w4a16_version() != ABI_VERSION:
             raise RuntimeError("libglowq_w4a16.so ABI version mismatch; rebuild with `python -m glowq_b200.build`")
-        self._ws = {}
+        self._ws = {}               # per device: the piece that the last plain call worked in
+        self._pieces = Scratch()
         # the group call on a descriptor that struct.pack made (bytes)
         self.group_forward_packed = ctypes.CFUNCTYPE(i32, ctypes.c_char_p)(("glowq_w4a16_group_forward", lib))
 
@@ -126,11 +128,7 @@ class _Ext:
         return torch.zeros(max(int(nbytes), 256), dtype=torch.uint8, device=device)
 
     def _scratch(self, device, nbytes: int) -> torch.Tensor:
-        key = (device.type, device.index)
-        ws = self._ws.get(key)
-        if ws is None or ws.numel() < nbytes:
-            ws = self.new_workspace(nbytes, device)
-            self._ws[key] = ws
+        ws = self._ws[device.type, device.index] = self._pieces.get(nbytes, device, current_stream_ptr(device))
         return ws
 
     @staticmethod
@@ -162,12 +160,12 @@ class _Ext:
         if M == 0:
             return out
         with torch.cuda.device(x.device):
-            ws = self._scratch(x.device, self.workspace_bytes(M, IC, OC, 0, 1))
+            need = self.workspace_bytes(M, IC, OC, 0, 1)
+            ws = self._scratch(x.device, need)
             stream = torch.cuda.current_stream(x.device).cuda_stream
             fn = getattr(self.lib, fn_name)
             rc = fn(x.data_ptr(), qweight.data_ptr(), scales.data_ptr(), qzeros.data_ptr(), out.data_ptr(), M, IC, OC,
-                    int(group_size), *extra, qweight.size(1), qzeros.size(1), scales.size(1), ws.data_ptr(), ws.numel(),
-                    stream)
+                    int(group_size), *extra, qweight.size(1), qzeros.size(1), scales.size(1), ws.data_ptr(), need, stream)
         self.check(rc, fn_name)
         return out
 
@@ -230,6 +228,63 @@ def current_stream_ptr(device: torch.device) -> int:
     if _raw_stream is not None:
         return _raw_stream(device.index)
     return torch.cuda.current_stream(device).cuda_stream
+
+
+_is_capturing = getattr(torch._C, "_cuda_isCurrentStreamCapturing", torch.cuda.is_current_stream_capturing)
+
+
+class Scratch:
+    """Zeroed device memory that one module's launches work in: counters, which every launch leaves at zero, and partial sums.
+
+    Launches on one stream take turns on one piece, whatever their sizes; every stream has a piece of its own.  A CUDA graph
+    keeps the addresses it was captured with, so what a capture has used belongs to the captures of that stream from then on
+    and is held as long as this object, and other calls get another piece.  A capture takes over a piece that its thread's
+    calls have used before (the warm-up), whose counters are zero; where there is none, a captured launch gets memory of the
+    graph's own, which the graph zeroes.  Graphs captured on one stream share a piece: they are not to be replayed at the same time."""
+
+    __slots__ = ("_pieces", "_makers", "_kept", "_largest")
+    MAX_STREAMS = 8      # streams that keep a piece; beyond, the oldest is given back (its memory is freed in its stream's order)
+
+    def __init__(self):
+        self._pieces = {}      # (device, stream, capturing): uint8 tensor
+        self._makers = {}      # the same keys: the thread that asked for the piece
+        self._kept = []        # pieces of captures that later ones outgrew
+        self._largest = 0
+
+    def __reduce__(self):      # a copied or loaded module starts without any
+        return Scratch, ()
+
+    def get(self, nbytes: int, device: torch.device, stream: int) -> torch.Tensor:
+        """At least ``nbytes`` for a launch on ``stream``, the current stream of ``device``, which is the current device."""
+        key = (device.index, stream, stream != 0 and _is_capturing())   # (the default stream, 0, cannot be captured)
+        piece = self._pieces.get(key)
+        if piece is None or piece.numel() < nbytes:
+            piece = self._more(nbytes, device, key)
+        return piece
+
+    def _more(self, nbytes: int, device: torch.device, key) -> torch.Tensor:
+        pieces, me = self._pieces, threading.get_ident()
+        if key[2]:
+            mine = [k for k, p in list(pieces.items())
+                    if not k[2] and k[0] == key[0] and p.numel() >= nbytes and self._makers.get(k) == me]
+            mine.sort(key=lambda k: k[1] != key[1])
+            piece = pieces.pop(mine[0], None) if mine else None
+            if piece is None:
+                return torch.zeros(nbytes, dtype=torch.uint8, device=device)
+            if key in pieces:
+                self._kept.append(pieces[key])
+        else:
+            # (sizes that outgrow one another grow by half at least, so that what captures hold on to is a few times the largest)
+            size = max(nbytes, 256)
+            if size > self._largest:
+                self._largest = size = max(size, self._largest * 3 // 2)
+            piece = torch.zeros(size, dtype=torch.uint8, device=device)
+            streams = [k for k in list(pieces) if not k[2] and k != key]
+            if len(streams) >= self.MAX_STREAMS:
+                pieces.pop(streams[0], None)
+        self._makers[key] = me
+        pieces[key] = piece
+        return piece
 
 
 _ext: Optional[_Ext] = None

@@ -143,8 +143,7 @@ class CudaW4A16Linear(nn.Module):
             _gemv_threshold=_env_int("W4A16_GEMV_M_MAX", "CUDA_MIXED_GEMV_M_MAX", default=-1),
             _force_gemm=_env_flag("W4A16_FORCE_GEMM", "CUDA_MIXED_FORCE_GEMM"),
             _force_gemv=_env_flag("W4A16_FORCE_GEMV", "CUDA_MIXED_FORCE_GEMV") or _env_flag("W4A16_USE_GEMV"),
-            _out_dtype=_get_kernel_out_dtype(), _check_status=_env_flag("GLOWQ_CHECK_STATUS"),
-            _ws=None, _ws_key=None)      # scratch for plain (uncorrected) calls
+            _out_dtype=_get_kernel_out_dtype(), _check_status=_env_flag("GLOWQ_CHECK_STATUS"))
 
     def extra_repr(self) -> str:
         return (f"in_features={self.in_features}, out_features={self.out_features}, "
@@ -191,16 +190,25 @@ class CudaW4A16Linear(nn.Module):
                 L.data_ptr() if L is not None else 0, out.data_ptr(), self.out_features, qw.stride(0), qz.stride(0), sc.stride(0),
                 L.stride(0) if L is not None else 0, out.stride(0), alpha, 0)
 
+    def _work(self, m: int, rank: int, device, stream: int):
+        """What a call on ``stream`` works in, and how much of it is this call's: the slices of K follow from the size, so that a
+        larger call before leaves the results as they are."""
+        own = self.__dict__
+        needs = own.get("_needs")
+        if needs is None:
+            needs = own.setdefault("_needs", {})
+        need = needs.get((m, rank))
+        if need is None:
+            if len(needs) > 4096:
+                needs.clear()
+            need = needs[m, rank] = self._get_ext().workspace_bytes(m, self.in_features, self.out_features, rank, 1)
+        scratch = own.get("_scratch")
+        if scratch is None:
+            scratch = own.setdefault("_scratch", K.Scratch())
+        return scratch.get(need, device, stream), need
+
     def workspace_for(self, m: int, rank: int, device) -> torch.Tensor:
-        key = (m, rank, device)
-        if self._ws is None or self._ws_key != key:
-            ext = self._get_ext()
-            have = 0 if self._ws is None or self._ws.device != device else self._ws.numel()
-            need = ext.workspace_bytes(m, self.in_features, self.out_features, rank, 1)
-            if need > have:
-                self._ws = ext.new_workspace(need, device)
-            self._ws_key = key
-        return self._ws
+        return self._work(m, rank, device, K.current_stream_ptr(device))[0]
 
     def launch(self, x2d: torch.Tensor, *, L=None, R=None, r_buf=None, r_mode=K.R_NONE, alpha=0.0, push=None,
                push_site: int = 0) -> torch.Tensor:
@@ -228,10 +236,10 @@ class CudaW4A16Linear(nn.Module):
             rb_ptr = r_buf.data_ptr()
         else:
             L = None
-        ws = self.workspace_for(m, rank, dev)
         stream = K.current_stream_ptr(dev)
+        ws, need = self._work(m, rank, dev, stream)
         grp = K.PACK_GROUP.pack(
-            x2d.data_ptr(), r_ptr, rb_ptr, ws.data_ptr(), ws.numel(), stream, m, self.in_features, K.int32(x2d.stride(0)), r_stride, rank,
+            x2d.data_ptr(), r_ptr, rb_ptr, ws.data_ptr(), need, stream, m, self.in_features, K.int32(x2d.stride(0)), r_stride, rank,
             self.group_size, r_mode, K.OUT_F32 if self._out_dtype == torch.float32 else K.OUT_F16, self.kernel_choice(m), 1, 0, 0, 0,
             push.descriptor_address() if push is not None else 0, int(push_site) if push is not None else 0, 0, 0, 0, 0, 0.0, 0)
         ext.check(ext.group_forward_packed(grp + K.PACK_MEMBER.pack(*self.pack_member(out, L, alpha))), "glowq_w4a16_group_forward")
