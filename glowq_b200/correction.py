@@ -43,6 +43,18 @@ def _x_key(x: torch.Tensor):
     return (x.data_ptr(), tuple(x.shape), x.dtype, x._version)
 
 
+def _inner(w: "AddSVDCorrection") -> CudaW4A16Linear:
+    """``w.inner`` (``nn.Module.__getattr__`` takes half a microsecond)."""
+    inner = w._modules.get("inner")
+    return w.inner if inner is None else inner
+
+
+def _factor(w: "AddSVDCorrection", name: str) -> torch.Tensor:
+    """``w.A_q`` or ``w.B_q``, a buffer unless somebody made it a parameter."""
+    t = w._buffers.get(name)
+    return getattr(w, name) if t is None else t
+
+
 class MiniGroupCache:
     """Hand-off of r = B_shared . x between the members of a group (src/step3_eval_dataset.py:417-444):
     the producer (q / gate) calls ``set(r, uses)``; each consumer (k, v / up) calls ``consume()`` and gets
@@ -117,7 +129,7 @@ class GroupLauncher:
 
     def _plan(self, m: int, device) -> dict:
         first = self.members[0]
-        key = (m, device, first._modules["inner"]._out_dtype)
+        key = (m, device, _inner(first)._out_dtype)
         plan = self._plans.get(key)
         if plan is None:
             ext = first.inner._get_ext()
@@ -147,7 +159,7 @@ class GroupLauncher:
     def run(self, x: torch.Tensor) -> torch.Tensor:
         """Called by the first member: launch the whole group, keep the other members' outputs, return its own."""
         first = self.members[0]
-        inners = [w._modules["inner"] for w in self.members]   # (nn.Module.__getattr__ takes half a microsecond)
+        inners = [_inner(w) for w in self.members]
         inner = inners[0]
         x2d = inner._flatten_input(x)
         m, dev, dtype = x2d.size(0), x2d.device, inner._out_dtype
@@ -177,7 +189,7 @@ class GroupLauncher:
         for w, lin, o in zip(self.members, inners, outs):
             alpha = float(w.alpha_svd)
             if alpha != 0.0 and not w._mismatch:
-                fields = lin.pack_member(o, w._buffers["A_q"], alpha)
+                fields = lin.pack_member(o, _factor(w, "A_q"), alpha)
             else:
                 fields = lin.pack_member(o)
             K.PACK_MEMBER.pack_into(grp, at, *fields)

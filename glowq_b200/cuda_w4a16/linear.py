@@ -177,6 +177,10 @@ class CudaW4A16Linear(nn.Module):
             x2d = x2d.to(torch.float16)
         return x2d.contiguous()
 
+    def fill_member(self, mem: "K.Member", out: torch.Tensor, L: Optional[torch.Tensor] = None, alpha: float = 0.0):
+        """Fill a descriptor's ``Member`` in place."""
+        K.PACK_MEMBER.pack_into(mem, 0, *self.pack_member(out, L, float(alpha)))
+
     def pack_member(self, out: torch.Tensor, L: Optional[torch.Tensor] = None, alpha: float = 0.0) -> tuple:
         """The fields of a ``Member`` in order (``kernels.PACK_MEMBER``).  Buffers are looked up in their dictionary:
         ``nn.Module.__getattr__`` takes half a microsecond each."""
@@ -267,7 +271,7 @@ class CudaW4A16Linear(nn.Module):
     @classmethod
     def from_float(cls, linear_layer: nn.Linear, group_size: int):
         dev = linear_layer.weight.device
-        if cls is CudaW4A16Linear:
+        if cls is CudaW4A16Linear and cls.__init__ is _CONSTRUCTOR:
             # The same module without the buffers that the constructor makes only for them to be replaced: made on the host, moved
             # and replaced they took longer than quantising (140 us a module; 37 so, with the group index from the quantiser's launch).
             mod = cls.__new__(cls)
@@ -279,15 +283,20 @@ class CudaW4A16Linear(nn.Module):
             else:
                 qweight, qzeros, scales, _ = _quantize_per_group_w4(weight, group_size)
                 gid = torch.arange(mod.in_features, dtype=torch.long, device=dev) // mod.group_size
-            mod._buffers.update(qweight_i32=qweight, qzeros_i32=qzeros, scales_f16=scales, gid=gid)
-            mod._non_persistent_buffers_set.add("gid")
+            if _BUFFER_HOOKS is not None and not _BUFFER_HOOKS:
+                mod._buffers.update(qweight_i32=qweight, qzeros_i32=qzeros, scales_f16=scales, gid=gid)
+                mod._non_persistent_buffers_set.add("gid")
+            else:
+                for name, t in (("qweight_i32", qweight), ("qzeros_i32", qzeros), ("scales_f16", scales)):
+                    mod.register_buffer(name, t)
+                mod.register_buffer("gid", gid, persistent=False)
             if linear_layer.bias is None:
                 mod.__dict__["bias"] = None
             else:
                 mod.bias = nn.Parameter(torch.empty(mod.out_features, dtype=torch.float16, device=dev))
                 mod.bias.data.copy_(linear_layer.bias.data.to(torch.float16))
             return mod
-        with torch.device(dev):    # a subclass: its constructor
+        with torch.device(dev):    # a subclass, or a constructor put in the place of this one
             mod = cls(linear_layer.in_features, linear_layer.out_features, group_size,
                       bias=linear_layer.bias is not None).to(dev)
         mod.qweight_i32, mod.qzeros_i32, mod.scales_f16, _ = _quantize_per_group_w4(
@@ -295,6 +304,10 @@ class CudaW4A16Linear(nn.Module):
         if linear_layer.bias is not None:
             mod.bias.data.copy_(linear_layer.bias.data.to(torch.float16))
         return mod
+
+
+_CONSTRUCTOR = CudaW4A16Linear.__init__
+_BUFFER_HOOKS = getattr(nn.modules.module, "_global_buffer_registration_hooks", None)   # of register_module_buffer_registration_hook
 
 
 def convert_to_cuda_w4a16(model: nn.Module, group_size: int = 128) -> nn.Module:

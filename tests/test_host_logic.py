@@ -257,3 +257,29 @@ def test_a_packed_descriptor_has_the_fields_of_the_struct():
     for i, m in enumerate(members):
         assert {n: value(got.members[i], n) for n in member_fields} == m
     assert K.int32(2**31 + 5) == 5 - 2**31 and K.int32(-7) == -7 and K.int32(2**31 - 1) == 2**31 - 1
+
+
+def test_a_conversion_passes_by_neither_buffer_hooks_nor_a_constructor_in_the_place_of_the_class_s(monkeypatch):
+    lin = torch.nn.Linear(200, 24, dtype=torch.float16)
+    want = CudaW4A16Linear.from_float(lin, 128)
+    names = []
+    hook = torch.nn.modules.module.register_module_buffer_registration_hook(lambda mod, name, buf: names.append(name))
+    try:
+        hooked = CudaW4A16Linear.from_float(lin, 128)
+    finally:
+        hook.remove()
+    init, made = CudaW4A16Linear.__init__, []
+    monkeypatch.setattr(CudaW4A16Linear, "__init__", lambda self, *a, **k: (init(self, *a, **k), made.append(self))[0])
+    replaced = CudaW4A16Linear.from_float(lin, 128)
+    assert sorted(names) == sorted(n for n, _ in want.named_buffers()) and made == [replaced]
+    for got in (hooked, replaced):
+        assert set(got.state_dict()) == set(want.state_dict()) and "gid" not in got.state_dict()
+        assert all(torch.equal(a, b) for (_, a), (_, b) in zip(got.named_buffers(), want.named_buffers()))
+
+
+def test_a_member_filled_in_place_has_the_packed_fields():
+    lin = CudaW4A16Linear.from_float(torch.nn.Linear(256, 16, bias=True, dtype=torch.float16), 128)
+    out, L, mem = torch.empty(3, 16), torch.empty(16, 8, dtype=torch.float16), K.Member()
+    lin.fill_member(mem, out, L, 0.5)
+    assert (mem.qweight, mem.bias, mem.L, mem.out) == tuple(t.data_ptr() for t in (lin.qweight_i32, lin.bias, L, out))
+    assert (mem.OC, mem.weight_stride_i32, mem.L_stride, mem.out_stride, mem.alpha) == (16, 32, 8, 16, 0.5)
