@@ -49,10 +49,10 @@ def _inner(w: "AddSVDCorrection") -> CudaW4A16Linear:
     return w.inner if inner is None else inner
 
 
-def _factor(w: "AddSVDCorrection", name: str) -> torch.Tensor:
-    """``w.A_q`` or ``w.B_q``, a buffer unless somebody made it a parameter."""
-    t = w._buffers.get(name)
-    return getattr(w, name) if t is None else t
+def _buffer(mod: nn.Module, name: str) -> torch.Tensor:
+    """The module's tensor of that name: a buffer, unless somebody made it a parameter."""
+    t = mod._buffers.get(name)
+    return getattr(mod, name) if t is None else t
 
 
 class MiniGroupCache:
@@ -138,7 +138,6 @@ class GroupLauncher:
             grp.M, grp.IC = m, first.inner.in_features
             grp.group_size = first.inner.group_size
             grp.rank, grp.r_mode = rank, K.R_COMPUTE
-            grp.R, grp.R_stride = first.B_q.data_ptr(), first.B_q.stride(0)
             grp.out_dtype = K.OUT_F32 if first.inner._out_dtype == torch.float32 else K.OUT_F16
             grp.kernel = first.inner.kernel_choice(m)
             grp.n_members = len(self.members)
@@ -148,13 +147,19 @@ class GroupLauncher:
             oc_total = sum(w.inner.out_features for w in self.members)
             ws = ext.new_workspace(ext.workspace_bytes(m, grp.IC, oc_total, rank, len(self.members)), device)
             grp.workspace, grp.workspace_bytes = ws.data_ptr(), ws.numel()
-            plan = {"grp": grp, "r_buf": r_buf, "ws": ws, "ext": ext, "address": ctypes.addressof(grp)}
+            plan = {"grp": grp, "r_buf": r_buf, "ws": ws, "ext": ext, "address": ctypes.addressof(grp), "weights": None}
             self._plans[key] = plan
         return plan
 
+    def _weights(self) -> list:
+        """Where the right factor and the packed weights are now."""
+        return [_buffer(self.members[0], "B_q").data_ptr()] + [_buffer(_inner(w), "qweight_i32").data_ptr() for w in self.members]
+
     def descriptor_address(self, m: int, device, dtype) -> Optional[int]:
+        """The descriptor of the last launch for so many tokens, for the ``next`` hint of the launch in front.  None where there was
+        none, or where the weights have moved since: what the descriptor points to may be unmapped by now."""
         plan = self._plans.get((m, device, dtype))
-        return None if plan is None else plan["address"]
+        return None if plan is None or plan["weights"] != self._weights() else plan["address"]
 
     def run(self, x: torch.Tensor) -> torch.Tensor:
         """Called by the first member: launch the whole group, keep the other members' outputs, return its own."""
@@ -184,12 +189,17 @@ class GroupLauncher:
 
     def _launch(self, plan, x2d, inners, outs, m, dev, dtype) -> None:
         grp, ext = plan["grp"], plan["ext"]
+        R = _buffer(self.members[0], "B_q")
+        if R.size(0) != grp.rank:
+            raise RuntimeError(f"the right factor has rank {R.size(0)}, the group {grp.rank}")
+        plan["weights"] = self._weights()
+        grp.R, grp.R_stride = R.data_ptr(), R.stride(0)
         grp.x, grp.x_stride = x2d.data_ptr(), x2d.stride(0)
         at = K.Group.members.offset
         for w, lin, o in zip(self.members, inners, outs):
             alpha = float(w.alpha_svd)
             if alpha != 0.0 and not w._mismatch:
-                fields = lin.pack_member(o, _factor(w, "A_q"), alpha)
+                fields = lin.pack_member(o, _buffer(w, "A_q"), alpha)
             else:
                 fields = lin.pack_member(o)
             K.PACK_MEMBER.pack_into(grp, at, *fields)

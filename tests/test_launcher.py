@@ -42,3 +42,44 @@ def test_left_factors_that_are_parameters(m):
                 w.A_q = nn.Parameter(t, requires_grad=False)
         for y, z in zip(want, forward(model, *x)):
             assert torch.equal(y, z)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [1, 5, 20, 70])
+def test_factors_and_weights_that_move(m):
+    """A right factor replaced (by a parameter, by other values) and a model that leaves the device and comes back: every call reads
+    what is there now, and no launch names the places of before to the one in front of it."""
+    model, x = patched("cuda"), inputs(m)
+    other = patched("cuda", seed=5)
+    dev = x[0].device
+    with torch.no_grad():
+        want = [y.clone() for y in forward(model, *x)]
+        forward(model, *x)                                 # (with the hints of the pass before)
+        launchers = [model.proj(li, p).group_launcher for li in range(2) for p in ("self_attn.q_proj", "mlp.down_proj")]
+        assert all(g.descriptor_address(m, dev, torch.float32) for g in launchers)
+        for g in launchers:
+            t = g.members[0].B_q
+            del g.members[0].B_q
+            g.members[0].B_q = nn.Parameter(t.clone(), requires_grad=False)
+            del t
+        junk = [torch.full((64, 1024), 9.0, dtype=torch.float16, device="cuda") for _ in range(64)]     # over the old ones
+        assert not any(g.descriptor_address(m, dev, torch.float32) for g in launchers)
+        assert all(torch.equal(y, z) for y, z in zip(forward(model, *x), want))
+        assert all(g.descriptor_address(m, dev, torch.float32) for g in launchers)
+        model.cpu()
+        assert not any(g.descriptor_address(m, dev, torch.float32) for g in launchers)
+        del junk
+        torch.cuda.empty_cache()
+        keep = torch.empty(1 << 20, device="cuda")
+        model.cuda()
+        assert all(torch.equal(y, z) for y, z in zip(forward(model, *x), want))
+        for li in range(2):
+            for p in ToyDecoder.PROJ:
+                new = other.proj(li, p).B_q * 2
+                w = model.proj(li, p)
+                w.B_q = nn.Parameter(new, requires_grad=False) if "B_q" in w._parameters else new
+        assert not any(torch.equal(y, z) for y, z in zip(forward(model, *x), want))
+        model.proj(0, "self_attn.o_proj").B_q = torch.zeros(8, 256, dtype=torch.float16, device="cuda")
+        with pytest.raises(RuntimeError):
+            forward(model, *x)
+        del keep
