@@ -40,7 +40,7 @@ def clear_group_cache() -> None:
 
 
 def _x_key(x: torch.Tensor):
-    return (x.data_ptr(), tuple(x.shape), x.dtype, x._version)
+    return (x.data_ptr(), x.shape, x.dtype, x._version)
 
 
 def _inner(w: "AddSVDCorrection") -> CudaW4A16Linear:
@@ -109,15 +109,20 @@ class GroupLauncher:
     reference's cache relies on (src/step3_eval_dataset.py:481-504).  The patchers therefore give every group a
     launcher: the FIRST member's forward issues ONE ``glowq_w4a16_group_forward`` for all members and keeps the other
     members' outputs; their forwards return them when they are called with the same tensor (identity, shape, dtype and
-    version), and fall back to a launch of their own otherwise.  The filled call descriptor, the r buffer and the
-    workspace are cached per (tokens, device, output dtype), so a decode step does no descriptor building beyond a few
-    pointer stores; outputs are fresh tensors on every call, as in the reference.  ``next_launcher`` (set by the
-    patchers in model order) names the launch that follows, for the library's ``next`` hint."""
+    version), and fall back to a launch of their own otherwise.  Outputs are fresh tensors on every call, as in the
+    reference.  The workspace and r are one piece of scratch (``kernels.Scratch``) that launches of all token counts share:
+    a piece for each of them would be 17 MB a group and prompt length.  ``next_launcher`` (set by the patchers in model
+    order) names the launch that follows, for the library's ``next`` hint."""
 
     def __init__(self, members):
         self.members = list(members)          # AddSVDCorrection wrappers, first = producer (q / gate / solo)
         self.next_launcher: Optional["GroupLauncher"] = None
-        self._plans: Dict[tuple, dict] = {}
+        self._scratch = K.Scratch()
+        self._sizes: Dict[tuple, tuple] = {}  # by (tokens, device, rank): the workspace's bytes, and those with r's behind them
+        self._call: Optional[K.Group] = None  # the descriptor of the last launch, which the launch in front names as the one that follows
+        self._call_key: Optional[tuple] = None
+        self._call_r: Optional[tuple] = None
+        self._call_weights: list = []         # the members' buffers and where it found the packed weights
         self._pending: Dict[int, torch.Tensor] = {}
         self._pending_key = None
         first = self.members[0]
@@ -127,39 +132,37 @@ class GroupLauncher:
             and w.inner._out_dtype == inner0._out_dtype and w.B_q.shape == first.B_q.shape
             and w.A_q.size(1) == first.A_q.size(1) for w in self.members) and len(self.members) <= K.MAX_MEMBERS
 
-    def _plan(self, m: int, device) -> dict:
-        first = self.members[0]
-        key = (m, device, _inner(first)._out_dtype)
-        plan = self._plans.get(key)
-        if plan is None:
-            ext = first.inner._get_ext()
-            rank = first.A_q.size(1)
-            grp = K.Group()
-            grp.M, grp.IC = m, first.inner.in_features
-            grp.group_size = first.inner.group_size
-            grp.rank, grp.r_mode = rank, K.R_COMPUTE
-            grp.out_dtype = K.OUT_F32 if first.inner._out_dtype == torch.float32 else K.OUT_F16
-            grp.kernel = first.inner.kernel_choice(m)
-            grp.n_members = len(self.members)
-            cache = first.group_cache if first.is_group else None
-            r_buf = cache.buffer(m, rank, device) if cache is not None else first._private_r(m, rank, device)
-            grp.r_buf = r_buf.data_ptr()
-            oc_total = sum(w.inner.out_features for w in self.members)
-            ws = ext.new_workspace(ext.workspace_bytes(m, grp.IC, oc_total, rank, len(self.members)), device)
-            grp.workspace, grp.workspace_bytes = ws.data_ptr(), ws.numel()
-            plan = {"grp": grp, "r_buf": r_buf, "ws": ws, "ext": ext, "address": ctypes.addressof(grp), "weights": None}
-            self._plans[key] = plan
-        return plan
+    def _describe(self, key: tuple, inners) -> None:
+        """What calls of one size have in common: the descriptor's fixed fields."""
+        m, dev, rank, dtype, kernel = key
+        if self._call is None:
+            call = K.Group()
+            self._call_at = ctypes.addressof(call)
+            self._call = call
+        grp, lin = self._call, inners[0]
+        grp.M, grp.IC, grp.rank, grp.group_size = m, lin.in_features, rank, lin.group_size
+        grp.r_mode, grp.kernel, grp.n_members = K.R_COMPUTE, kernel, len(inners)
+        grp.out_dtype = K.OUT_F32 if dtype == torch.float32 else K.OUT_F16
+        if (m, dev, rank) not in self._sizes:
+            if len(self._sizes) > 4096:
+                self._sizes.clear()
+            need = lin._get_ext().workspace_bytes(m, lin.in_features, sum(i.out_features for i in inners), rank, len(inners))
+            self._sizes[m, dev, rank] = need, need + 2 * m * rank     # (a workspace is a multiple of 256 bytes)
+        self._call_key = key
 
-    def _weights(self) -> list:
-        """Where the right factor and the packed weights are now."""
-        return [_buffer(self.members[0], "B_q").data_ptr()] + [_buffer(_inner(w), "qweight_i32").data_ptr() for w in self.members]
-
-    def descriptor_address(self, m: int, device, dtype) -> Optional[int]:
-        """The descriptor of the last launch for so many tokens, for the ``next`` hint of the launch in front.  None where there was
-        none, or where the weights have moved since: what the descriptor points to may be unmapped by now."""
-        plan = self._plans.get((m, device, dtype))
-        return None if plan is None or plan["weights"] != self._weights() else plan["address"]
+    def descriptor_address(self, m: int, device, dtype=None) -> Optional[int]:
+        """The descriptor of the last launch, for the ``next`` hint of the one in front.  None before a launch of so many tokens, and
+        where the weights have moved since: what the descriptor points to may be unmapped by now."""
+        grp, dev = self._call, device.index
+        if grp is None or self._call_key[1] != dev or (m, dev, grp.rank) not in self._sizes:
+            return None
+        if _buffer(self.members[0], "B_q").data_ptr() != grp.R:
+            return None
+        for buffers, at in self._call_weights:
+            t = buffers.get("qweight_i32")
+            if t is None or t.data_ptr() != at:
+                return None
+        return self._call_at
 
     def run(self, x: torch.Tensor) -> torch.Tensor:
         """Called by the first member: launch the whole group, keep the other members' outputs, return its own."""
@@ -167,49 +170,66 @@ class GroupLauncher:
         inners = [_inner(w) for w in self.members]
         inner = inners[0]
         x2d = inner._flatten_input(x)
-        m, dev, dtype = x2d.size(0), x2d.device, inner._out_dtype
-        outs = [torch.empty((m, lin.out_features), dtype=dtype, device=dev) for lin in inners]
+        m, dev, dtype = x2d.shape[0], x2d.device, inner._out_dtype
+        outs = [torch.empty(m, lin.out_features, dtype=dtype, device=dev) for lin in inners]
         self._pending.clear()
         key = _x_key(x)
         if m > 0:
-            plan = self._plan(m, dev)
             if torch.cuda.current_device() == dev.index:
-                self._launch(plan, x2d, inners, outs, m, dev, dtype)
+                r = self._launch(x2d, inners, outs, m, dev, dtype)
             else:
                 with torch.cuda.device(dev):
-                    self._launch(plan, x2d, inners, outs, m, dev, dtype)
+                    r = self._launch(x2d, inners, outs, m, dev, dtype)
             self._keep = x2d          # the launch reads x2d asynchronously
-            if first.is_group and first.group_cache is not None:
-                first.group_cache.set(plan["r_buf"], len(self.members) - 1, key)
+            if r is not None:
+                first.group_cache.set(r, len(self.members) - 1, key)
         flat = x.dim() == 2
         for w, o in zip(self.members[1:], outs[1:]):
             self._pending[id(w)] = o if flat else o.reshape(*x.shape[:-1], o.size(1))
         self._pending_key = key
         return outs[0] if flat else outs[0].reshape(*x.shape[:-1], inner.out_features)
 
-    def _launch(self, plan, x2d, inners, outs, m, dev, dtype) -> None:
-        grp, ext = plan["grp"], plan["ext"]
-        R = _buffer(self.members[0], "B_q")
-        if R.size(0) != grp.rank:
-            raise RuntimeError(f"the right factor has rank {R.size(0)}, the group {grp.rank}")
-        plan["weights"] = self._weights()
-        grp.R, grp.R_stride = R.data_ptr(), R.stride(0)
-        grp.x, grp.x_stride = x2d.data_ptr(), x2d.stride(0)
-        at = K.Group.members.offset
+    def _launch(self, x2d, inners, outs, m, dev, dtype) -> Optional[torch.Tensor]:
+        """The launch; r, where the members' cache hands it on."""
+        first, inner, index = self.members[0], inners[0], dev.index
+        R = _buffer(first, "B_q")
+        rank = R.shape[0]
+        key = (m, index, rank, dtype, inner.kernel_choice(m))
+        if key != self._call_key:
+            self._describe(key, inners)
+        need, total = self._sizes[m, index, rank]
+        grp, ext = self._call, inner._get_ext()
+        stream = K.current_stream_ptr(dev)
+        piece = self._scratch.get(total, dev, stream)
+        at = piece.data_ptr()
+        grp.x, grp.x_stride = x2d.data_ptr(), x2d.stride()[0]
+        grp.R, grp.R_stride = R.data_ptr(), R.stride()[0]
+        grp.workspace, grp.workspace_bytes, grp.r_buf, grp.stream = at, need, at + need, stream
+        weights, place = [], K.Group.members.offset
         for w, lin, o in zip(self.members, inners, outs):
             alpha = float(w.alpha_svd)
             if alpha != 0.0 and not w._mismatch:
-                fields = lin.pack_member(o, _buffer(w, "A_q"), alpha)
+                L = _buffer(w, "A_q")
+                fields = lin.pack_member(o, L, alpha)
+                if fields[10] != rank and L.shape[1] != rank:      # (the row stride: other than the rank in a part of a larger factor)
+                    raise RuntimeError(f"a left factor has rank {L.shape[1]}, the group's right factor {rank}")
             else:
                 fields = lin.pack_member(o)
-            K.PACK_MEMBER.pack_into(grp, at, *fields)
-            at += K.PACK_MEMBER.size
+            K.PACK_MEMBER.pack_into(grp, place, *fields)
+            place += K.PACK_MEMBER.size
+            weights.append((lin._buffers, fields[0]))
+        self._call_weights = weights
         nxt = self.next_launcher
-        grp.next = nxt.descriptor_address(m, dev, dtype) if nxt is not None else None
-        grp.stream = stream = K.current_stream_ptr(dev)
+        grp.next = nxt.descriptor_address(m, dev) if nxt is not None else None
         ext.check(ext.lib.glowq_w4a16_group_forward(grp), "glowq_w4a16_group_forward")
-        if inners[0]._check_status:
-            ext.check(ext.lib.glowq_w4a16_read_status(grp.workspace, stream), "device status")
+        if inner._check_status:
+            ext.check(ext.lib.glowq_w4a16_read_status(at, stream), "device status")
+        if not first.is_group or first.group_cache is None:
+            return None
+        r = self._call_r
+        if r is None or r[0] is not piece or r[1] != key:
+            self._call_r = r = (piece, key, piece[need:total].view(torch.float16).view(m, rank))
+        return r[2]
 
     def forget(self) -> None:
         self._pending.clear()
@@ -260,8 +280,9 @@ class AddSVDCorrection(nn.Module):
         gl = self.group_launcher
         if gl is not None and gl.usable and x.is_cuda:
             if gl.members[0] is self:
-                if any(w.alpha_svd != 0.0 and not w._mismatch for w in gl.members):
-                    return gl.run(x)
+                for w in gl.members:
+                    if w.alpha_svd != 0.0 and not w._mismatch:
+                        return gl.run(x)
                 gl.forget()      # nothing to correct in this group: outputs kept from an earlier call must not be served
             else:
                 out = gl.take(self, x)

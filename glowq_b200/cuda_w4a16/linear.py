@@ -190,9 +190,10 @@ class CudaW4A16Linear(nn.Module):
         except KeyError:
             qw, sc, qz = self.qweight_i32, self.scales_f16, self.qzeros_i32
         bias = self._parameters["bias"] if "bias" in self._parameters else self.bias
+        # (stride()[0]: half the time of stride(0))
         return (qw.data_ptr(), sc.data_ptr(), qz.data_ptr(), bias.data_ptr() if bias is not None else 0,
-                L.data_ptr() if L is not None else 0, out.data_ptr(), self.out_features, qw.stride(0), qz.stride(0), sc.stride(0),
-                L.stride(0) if L is not None else 0, out.stride(0), alpha, 0)
+                L.data_ptr() if L is not None else 0, out.data_ptr(), self.out_features, qw.stride()[0], qz.stride()[0],
+                sc.stride()[0], L.stride()[0] if L is not None else 0, out.stride()[0], alpha, 0)
 
     def _work(self, m: int, rank: int, device, stream: int):
         """What a call on ``stream`` works in, and how much of it is this call's: the slices of K follow from the size, so that a
@@ -221,7 +222,7 @@ class CudaW4A16Linear(nn.Module):
         rank's staging slot of ``push_site`` (complete the sum with ``push.finish(out, push_site)``)."""
         ext = self._get_ext()
         m, dev = x2d.size(0), x2d.device
-        out = torch.empty((m, self.out_features), dtype=self._out_dtype, device=dev)
+        out = torch.empty(m, self.out_features, dtype=self._out_dtype, device=dev)
         if m == 0:
             return out
         if torch.cuda.current_device() == dev.index:

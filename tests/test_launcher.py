@@ -83,3 +83,59 @@ def test_factors_and_weights_that_move(m):
         with pytest.raises(RuntimeError):
             forward(model, *x)
         del keep
+
+
+def pieces(launcher):
+    return list(launcher._scratch._pieces.values()) + launcher._scratch._kept
+
+
+@pytest.mark.gpu
+def test_token_counts_share_a_piece():
+    """Prompts of many lengths, decode in between: one piece a launcher, of the largest call's size, and results without a history."""
+    model = patched("cuda")
+    x = {m: inputs(m, seed=m) for m in (1, 3, 8, 20, 64, 70, 257, 300, 411, 700)}
+    with torch.no_grad():
+        want = {m: forward(patched("cuda"), *x[m]) for m in x}
+        for m in (700, 1, 8, 300, 3, 64, 20, 411, 1, 257, 70, 8, 700, 1):
+            assert all(torch.equal(y, z) for y, z in zip(forward(model, *x[m]), want[m])), m
+    for li in range(2):
+        for p in ("self_attn.q_proj", "self_attn.o_proj", "mlp.gate_proj", "mlp.down_proj"):
+            (piece,) = pieces(model.proj(li, p).group_launcher)
+            assert piece.numel() < 18 << 20
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [1, 5, 20, 100])
+def test_a_captured_step_beside_other_calls(m):
+    """A step in a graph, replayed on one stream while calls of other sizes, and of its own, run on another."""
+    sizes = dict(hidden=2048, kv=512, inter=8192)
+    model, x = patched("cuda", rank=64, **sizes), inputs(m, 2048, 8192)
+    other = {n: inputs(n, 2048, 8192, seed=n) for n in (m, 3, 33, 300)}
+    with torch.no_grad():
+        fresh = patched("cuda", rank=64, **sizes)
+        want = [y.clone() for y in forward(fresh, *x)]
+        want_other = {n: [y.clone() for y in forward(fresh, *other[n])] for n in other}
+        for _ in range(2):
+            forward(model, *x)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            outs = forward(model, *x)
+        forward(model, *other[300])
+        torch.cuda.synchronize()
+        side, got = torch.cuda.Stream(), []
+        for rep in range(6):
+            for o in outs:
+                o.fill_(float("nan"))
+            side.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(side):
+                graph.replay()
+            for n in other:
+                got.append((n, forward(model, *other[n])))
+            torch.cuda.current_stream().wait_stream(side)
+            assert all(torch.equal(y, z) for y, z in zip(outs, want)), rep
+        assert all(torch.equal(y, z) for n, ys in got for y, z in zip(ys, want_other[n]))
+    ext = model.proj(0, "self_attn.q_proj").inner._get_ext()
+    status = ext.lib.glowq_w4a16_read_status
+    stream = torch.cuda.current_stream().cuda_stream
+    assert {status(p.data_ptr(), stream) for li in range(2) for q in ToyDecoder.PROJ for p in pieces(model.proj(li, q).group_launcher)} == {0}
