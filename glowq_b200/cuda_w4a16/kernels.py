@@ -287,6 +287,27 @@ class Scratch:
         return piece
 
 
+class RRows:
+    """Room for r = B x, [tokens, rank] fp16, as ``Scratch`` gives it: by streams, and a captured graph's own."""
+
+    __slots__ = ("_scratch", "_last")
+
+    def __init__(self):
+        self._scratch = Scratch()
+        self._last = None
+
+    def __reduce__(self):
+        return RRows, ()
+
+    def rows(self, m: int, rank: int, device: torch.device) -> torch.Tensor:
+        stream = current_stream_ptr(device) if device.type == "cuda" else 0
+        piece = self._scratch.get(2 * max(m, 16) * rank, device, stream)
+        last = self._last
+        if last is None or last[0] is not piece or last[1] != (m, rank):
+            self._last = last = (piece, (m, rank), piece[:2 * m * rank].view(torch.float16).view(m, rank))
+        return last[2]
+
+
 _ext: Optional[_Ext] = None
 
 

@@ -1,9 +1,12 @@
 """The group launchers: what they look up on every call and what they hold."""
+from types import SimpleNamespace
+
 import pytest
 import torch
 import torch.nn as nn
 
-from glowq_b200.correction import patch_svd_correction_wrappers_cumulative
+from glowq_b200.correction import MiniGroupCache, patch_svd_correction_wrappers_cumulative
+from glowq_b200.cuda_w4a16 import kernels as K
 from glowq_b200.cuda_w4a16.linear import CudaW4A16Linear
 from toy_model import ToyDecoder, make_artifacts
 
@@ -86,7 +89,8 @@ def test_factors_and_weights_that_move(m):
 
 
 def pieces(launcher):
-    return list(launcher._scratch._pieces.values()) + launcher._scratch._kept
+    scratch = getattr(launcher, "_scratch", None)
+    return [] if scratch is None else list(scratch._pieces.values()) + scratch._kept
 
 
 @pytest.mark.gpu
@@ -104,10 +108,31 @@ def test_token_counts_share_a_piece():
             assert piece.numel() < 18 << 20
 
 
+def test_room_for_r_that_a_graph_was_captured_with_stays(monkeypatch):
+    capturing = [False]
+    monkeypatch.setattr(K, "_is_capturing", lambda: capturing[0])
+    monkeypatch.setattr(K, "current_stream_ptr", lambda device: 7)
+    device = SimpleNamespace(type="cuda", index=0)
+    monkeypatch.setattr(K.torch, "zeros", lambda n, dtype, device, zeros=torch.zeros: zeros(n, dtype=dtype))
+    for room in (MiniGroupCache().buffer, patched().proj(0, "mlp.down_proj")._private_r):
+        warm = room(5, 16, device)
+        assert warm.shape == (5, 16) and warm.dtype == torch.float16 and room(5, 16, device) is warm
+        capturing[0] = True
+        captured = room(5, 16, device)
+        capturing[0] = False
+        assert captured.data_ptr() == warm.data_ptr()
+        at = {room(m, 16, device).data_ptr() for m in (5, 16, 17, 300)}
+        capturing[0] = True
+        assert room(5, 16, device).data_ptr() == warm.data_ptr() not in at
+        capturing[0] = False
+
+
 @pytest.mark.gpu
+@pytest.mark.parametrize("fuse", ["1", "0"])
 @pytest.mark.parametrize("m", [1, 5, 20, 100])
-def test_a_captured_step_beside_other_calls(m):
+def test_a_captured_step_beside_other_calls(m, fuse, monkeypatch):
     """A step in a graph, replayed on one stream while calls of other sizes, and of its own, run on another."""
+    monkeypatch.setenv("GLOWQ_FUSE_GROUPS", fuse)
     sizes = dict(hidden=2048, kv=512, inter=8192)
     model, x = patched("cuda", rank=64, **sizes), inputs(m, 2048, 8192)
     other = {n: inputs(n, 2048, 8192, seed=n) for n in (m, 3, 33, 300)}
@@ -138,4 +163,6 @@ def test_a_captured_step_beside_other_calls(m):
     ext = model.proj(0, "self_attn.q_proj").inner._get_ext()
     status = ext.lib.glowq_w4a16_read_status
     stream = torch.cuda.current_stream().cuda_stream
-    assert {status(p.data_ptr(), stream) for li in range(2) for q in ToyDecoder.PROJ for p in pieces(model.proj(li, q).group_launcher)} == {0}
+    mods = [model.proj(li, p) for li in range(2) for p in ToyDecoder.PROJ]
+    used = [piece for w in mods for piece in pieces(w.group_launcher) + pieces(w.inner)]
+    assert used and {status(piece.data_ptr(), stream) for piece in used} == {0}
