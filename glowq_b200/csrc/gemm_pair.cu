@@ -56,6 +56,8 @@ constexpr int kConsumers = 2 * (1 + 1 + 1 + 4 * kTeams + 4) + 1;   // arrivals t
 constexpr int kAhead = 12;                 // the next item is asked for when this many steps of one are still to be loaded
 constexpr int kSmemMax = 227 * 1024 - 512;
 constexpr unsigned kCountSpin = 1u << 22;  // polls of a count of finished CTAs (seconds)
+constexpr unsigned kSumGoSpin = 1u << 25;  // polls for the end of such a wait, longer than it: 8 s at a quarter of a microsecond
+static_assert(kSumGoSpin >= 8 * kCountSpin, "a poll of a count is a trip to memory, up to eight times a poll of a barrier");
 constexpr unsigned kDrainSpin = 1u << 18;  // polls for one of this CTA's own copies or MMAs
 enum : int { kCTicket = 72, kCFlag = 73, kCExit = 74 };   // words of the counters in front of the slots, zero between launches
 
@@ -755,7 +757,8 @@ gemm_pair_kernel(const __grid_constant__ PtParams p, const __grid_constant__ PtM
       }
       jbase = jend;
       if (ok && (p.sep || t.ks > 1)) {
-        ok = await(kBSumGo, mph);
+        // (the epilogue may be waiting for the other slices, whose CTAs another stream's kernel may keep from their SMs)
+        ok = g_mbar_wait<kSumGoSpin>(smem0 + kBSumGo, mph, abort_flag, p.status);
         mph ^= 1;
         if (!__all_sync(0xffffffffu, ok)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

@@ -22,6 +22,7 @@ __device__ __forceinline__ void g_mbar_arrive(uint32_t a) {
 __device__ __forceinline__ void g_mbar_expect_tx(uint32_t a, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a), "r"(bytes) : "memory");
 }
+template <uint32_t kLimit = kGemmSpin>
 __device__ __forceinline__ bool g_mbar_wait(uint32_t a, uint32_t parity, volatile int* abort_flag, uint32_t* status) {
   uint32_t spins = 0;
   for (;;) {
@@ -32,7 +33,7 @@ __device__ __forceinline__ bool g_mbar_wait(uint32_t a, uint32_t parity, volatil
                  : "memory");
     if (ok) return true;
     if ((++spins & 63u) == 0 && *abort_flag) return false;
-    if (spins > kGemmSpin) {
+    if (spins > kLimit) {
       *abort_flag = 1;
       atomicExch(status, 3u);
       return false;
