@@ -663,6 +663,8 @@ int glowq_w4a16_quantize_indexed(const void* weight, int32_t* qweight, int32_t* 
   if (group_size <= 0 || group_size % 8 != 0) return GLOWQ_ERR_BAD_GROUP_SIZE;
   if (group_size != kGroup) return GLOWQ_ERR_UNSUPPORTED_SHAPE;
   if (weight_stride < IC) return GLOWQ_ERR_BAD_STRIDE;
+  // (the kernel numbers its warps, eight a block and eight groups of a row each, in 32 bits)
+  if ((static_cast<long long>(IC) + 8 * kGroup - 1) / (8 * kGroup) * OC > 0xFFFFFFF8ll) return GLOWQ_ERR_TOO_LARGE;
   const DeviceInfo* dev = nullptr;
   int rc = device_info(&dev);
   if (rc != GLOWQ_OK) return rc;

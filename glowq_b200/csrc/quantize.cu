@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(kQThreads, 6) quantize_kernel(const __half* __
                                                              int IC, int G, int words, long long w_stride, int vec_ok,
                                                              int64_t* __restrict__ gid) {
   const int lane = threadIdx.x & 31, hsel = lane >> 4, s16 = lane & 15;
-  // (32 bits: an item is 1024 weights, or one row; the launch refuses more than 2^31 blocks of eight)
+  // (32 bits: the entry point refuses more than 2^32 - 8 items, so that the last block's eight fit as well)
   const uint32_t item = blockIdx.x * (kQThreads / 32) + (threadIdx.x >> 5);
   const uint32_t row_u = item / static_cast<uint32_t>(words);
   if (row_u >= static_cast<uint32_t>(OC)) return;   // whole warps leave together
@@ -179,10 +179,9 @@ __global__ void __launch_bounds__(kQThreads, 6) quantize_kernel(const __half* __
 
 cudaError_t launch_quantize(const __half* w, int32_t* qweight, int32_t* qzeros, __half* scales, int64_t* gid, int OC, int IC,
                             long long w_stride, cudaStream_t stream) {
-  const int G = (IC + 127) / 128, words = (G + 7) / 8;
+  const int G = (IC - 1) / 128 + 1, words = (G + 7) / 8;
   const long long items = static_cast<long long>(OC) * words;
   const long long blocks = (items + kQThreads / 32 - 1) / (kQThreads / 32);
-  if (blocks > 0x7FFFFFFFll) return cudaErrorInvalidValue;
   const int vec_ok = (IC & 7) == 0 && (w_stride & 7) == 0 && (reinterpret_cast<uintptr_t>(w) & 15u) == 0;
   quantize_kernel<<<static_cast<unsigned>(blocks), kQThreads, 0, stream>>>(w, qweight, qzeros, scales, OC, IC, G, words, w_stride,
                                                                           vec_ok, gid);

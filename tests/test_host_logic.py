@@ -283,3 +283,10 @@ def test_a_member_filled_in_place_has_the_packed_fields():
     lin.fill_member(mem, out, L, 0.5)
     assert (mem.qweight, mem.bias, mem.L, mem.out) == tuple(t.data_ptr() for t in (lin.qweight_i32, lin.bias, L, out))
     assert (mem.OC, mem.weight_stride_i32, mem.L_stride, mem.out_stride, mem.alpha) == (16, 32, 8, 16, 0.5)
+
+
+def test_the_quantiser_refuses_more_items_than_it_can_number():
+    """Rows times zero-point words above 2^32 - 8, whatever the device (refused before anything is launched)."""
+    fn = K.load_w4a16_extension().lib.glowq_w4a16_quantize
+    for oc, ic in ((2**31 - 1, 1025), (2**31 - 1, 2**31 - 1), (2**31 - 3, 2048)):
+        assert fn(4096, 4096, 4096, 4096, oc, ic, 128, ic, None) == 9, (oc, ic)
