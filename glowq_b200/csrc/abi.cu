@@ -438,25 +438,46 @@ int n_tiles_of(const glowq_w4a16_group_t& g) {
   return n;
 }
 
-// Microseconds of one streaming launch of 2 to 8 tokens, fitted on B200 to 266 group calls (9 % rms): latency, the rounds of tiles times
-// their chunks of 1024 columns - with one CTA per SM, where the staged activations leave room for no more, a chunk takes two thirds of
-// the time, but there are half as many CTAs - the correction, K slices that meet in memory, a ring too shallow for one CTA.
+// CTA slots of a streaming launch (the epoch word of the workspace counts the consumer warps of a grid in kEpochShift bits).
+int gemv_slots(const GemvPlan& pl, int sms) {
+  return std::min(sms * pl.ctas_per_sm, static_cast<int>(kEpochReaderMask) / kConsumerWarps);
+}
+
+// Microseconds of one streaming launch of 2 to 8 tokens: latency, the rounds of tiles times their chunks of 1024 columns (a last round
+// that is not full is shorter, but not as much), the correction of a tile, the CTAs that begin with R units, K slices that meet in
+// memory.
 double stream_us(const glowq_w4a16_group_t& g, const GemvPlan& pl, int n_tiles, bool corr, int sms) {
-  const int r_ctas = corr && g.r_mode == GLOWQ_R_COMPUTE ? std::min({pl.n_r_tiles * pl.SKr, 96, sms * pl.ctas_per_sm / 3}) : 0;
-  const int rounds = pl.SK == 1 ? ceil_div(n_tiles, sms * pl.ctas_per_sm) : ceil_div(n_tiles * pl.SK, std::max(1, sms * pl.ctas_per_sm - r_ctas));
-  const int chunks = ceil_div(std::min(pl.gps, pl.G), kChunkGroups);
-  return 0.925 + 0.792 * g.M + rounds * chunks * (pl.ctas_per_sm == 2 ? 0.972 : 0.618 + 0.006 * g.M) +
-         (corr ? 1.014 + 0.738 * ceil_div(g.rank, 256) * rounds : 0.0) + (pl.SK > 1 ? 4.5 : 0.0) +
-         (pl.ctas_per_sm == 1 && pl.stages < 4 ? 0.0212 * pl.G : 0.0);
+  const int cap = gemv_slots(pl, sms), units = g.r_mode == GLOWQ_R_COMPUTE ? pl.n_r_tiles * pl.SKr : 0;
+  const int r_ctas = gemv_r_ctas(pl, n_tiles, units, cap), unit_rounds = units > 0 ? ceil_div(units, std::max(1, r_ctas)) : 0;
+  const int groups = std::min(pl.gps, pl.G);
+  const double chunk = pl.ctas_per_sm == 2 ? 0.672 : 0.259 + 0.878 / pl.stages;
+  const double tile = chunk * (0.444 * ceil_div(groups, kChunkGroups) + 0.556 * groups / kChunkGroups);
+  const double latency = 1.667 + 0.953 * g.M, ranks = corr ? g.rank / 64.0 : 0.0;
+  if (pl.SK > 1) {
+    const int rounds = ceil_div(n_tiles * pl.SK, std::max(1, (cap - r_ctas) / pl.SK * pl.SK));
+    return latency - 1.672 + rounds * (1.359 * tile + 1.739 + 0.546 * ranks) + 0.45 * pl.SK + 0.317 * units / std::max(1, r_ctas);
+  }
+  const int rounds = ceil_div(n_tiles, cap);
+  const double last = static_cast<double>(n_tiles) / cap - (rounds - 1), each = corr ? 0.326 + 0.072 * ranks : 0.0;
+  const double all = latency + tile * (rounds - 1 + last + (rounds == 1 ? 0.345 : 0.181) * (1.0 - last)) + 0.672 * (rounds - 1) +
+                     each * rounds;
+  if (units == 0) return all;
+  const int behind = n_tiles > cap - r_ctas ? ceil_div(n_tiles - (cap - r_ctas), cap) : 0;   // tiles of a CTA after its R units
+  return std::max(all, 0.802 * latency - 0.257 + 1.675 * unit_rounds + 1.218 * behind * tile + each * std::max(behind, 1));
 }
 
 // Which kernel.  Up to 8 tokens fit one streaming launch (one MMA N tile), which multiplies the exact integer codes and applies the
 // scales in fp32; from 2 tokens the tensor-memory kernel's exact form, of the same precision, takes the calls that it is faster on:
 // many tokens and long rows (us streamed / exact: 13B down_proj corrected at 2 and 8 tokens 21.2 / 19.1 and 33.8 / 19.1, 14B gate/up at
-// 2 and 8 tokens 21.7 / 29.2 and 35.1 / 29.3, 3B o_proj corrected at 3 and 8 tokens 7.8 / 9.3 and 10.4 / 9.4).  Above 8 tokens the
-// tensor-core kernels round the scaled weights to fp16 first, as the reference does.  9 to 16 tokens would take two streaming launches:
-// 47 / 70 / 64 / 33 us for q/k/v, gate/up, down_proj and o_proj of the Llama-2-13B shapes at 16 tokens, corrected, against
-// 19.1 / 29.3 / 18.1 / 11.3.
+// 2 and 8 tokens 21.7 / 29.2 and 35.1 / 29.3, 3B o_proj corrected at 3 and 8 tokens 7.8 / 9.3 and 10.4 / 9.4).
+// Both estimates are fitted on B200 to the calls of 3920 layers (280 shapes, groups corrected or their members one by one), each call
+// streamed and exact among the others: a change of kernel from one call to the next costs 0.8 us more, which a call repeated alone does
+// not show.  On shapes left out of the fit the layers are 0.7 % slower than with the best choice for every call, 13 % at worst.  Layers
+// that are more than 1 % slower than all streamed: 5 % of 1470 on other shapes still, 15 % at worst; on average they are 10 % faster.
+// (By the estimates before, fitted to calls alone and to another rule for R CTAs: 10 % of them, 17 % at worst, 9 % faster.)
+// Above 8 tokens the tensor-core kernels round the scaled weights to fp16 first, as the reference does.  9 to 16 tokens would take two
+// streaming launches: 47 / 70 / 64 / 33 us for q/k/v, gate/up, down_proj and o_proj of the Llama-2-13B shapes at 16 tokens, corrected,
+// against 19.1 / 29.3 / 18.1 / 11.3.
 bool takes_gemm(const glowq_w4a16_group_t& g, int sms) {
   if (g.kernel == GLOWQ_KERNEL_GEMV) return false;
   if (g.kernel == GLOWQ_KERNEL_GEMM || g.M > kGemvAutoMaxM) return gemm_supported(g);
@@ -468,7 +489,7 @@ bool takes_gemm(const glowq_w4a16_group_t& g, int sms) {
   bool corr = false;
   for (int i = 0; i < g.n_members && g.r_mode != GLOWQ_R_NONE; ++i) corr = corr || (g.members[i].L && g.members[i].alpha != 0.f);
   const double exact = gemm_exact_us(g, sms);
-  return exact >= 0.0 && exact < stream_us(g, pl, n_tiles, corr, sms);
+  return exact >= 0.0 && exact < stream_us(g, pl, n_tiles, corr, sms) - 0.15;   // (level: the calls around are streamed more often)
 }
 
 int gemv_group_forward(const glowq_w4a16_group_t& g, const DeviceInfo& dev, cudaStream_t stream) {
@@ -567,8 +588,7 @@ int gemv_group_forward(const glowq_w4a16_group_t& g, const DeviceInfo& dev, cuda
       // persistent grid: every CTA resident at once, a whole number of CTAs per K slice
       // R units run on dedicated CTAs (the lowest block indices; several units each when there are many), so that the
       // r chain (R loads, MMAs, slot, release counter) overlaps the other CTAs' x staging and weight streaming
-      // (the epoch word of the workspace counts the consumer warps of a grid in kEpochShift bits)
-      const int cap = std::min(dev.sms * pl.ctas_per_sm, static_cast<int>(kEpochReaderMask) / kConsumerWarps);
+      const int cap = gemv_slots(pl, dev.sms);
       p.n_r_ctas = gemv_r_ctas(pl, n_tiles, p.n_r_units, cap);
       int grid = std::min(cap - p.n_r_ctas, n_tiles * pl.SK);
       grid = std::max(pl.SK, grid / pl.SK * pl.SK) + p.n_r_ctas;

@@ -104,15 +104,13 @@ GemmRoute gemm_route(const glowq_w4a16_group_t& g) {
 }
 }  // namespace
 
-double gemm_tmem_us(const glowq_w4a16_group_t& g, bool exact, bool compute_r, bool any_corr, bool any_separate, int sms);
+double gemm_tmem_exact_us(const glowq_w4a16_group_t& g, bool compute_r, bool any_corr, int sms);
 
-// Microseconds of a call of up to 8 tokens in the exact form, as far as its workspace goes (-1: r would need a launch of its own).  The
-// planner's costs leave out what does not depend on the partition: fitted beside the streaming kernel's on the same 266 calls, where the
-// kernel that the two estimates choose is 1.2 % slower than the better one on average (always the streaming kernel: 14.9 %).
+// Microseconds of a call of up to 8 tokens in the exact form, as far as its workspace goes (-1: r would need a launch of its own).
 double gemm_exact_us(const glowq_w4a16_group_t& g, int sms) {
   const GemmRoute rt = gemm_route(g);
   if (g.r_mode == GLOWQ_R_COMPUTE && !rt.r_in_launch) return -1.0;
-  return 1.5 + 1.38 * gemm_tmem_us(g, true, rt.r_in_launch, rt.any_corr, rt.any_separate, sms);
+  return gemm_tmem_exact_us(g, rt.r_in_launch, rt.any_corr, sms);
 }
 
 // (host arithmetic: see glowq_internal_workspace_map)

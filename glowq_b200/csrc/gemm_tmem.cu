@@ -760,7 +760,7 @@ struct TmemPlan {
   int n_r, r_slices;           // CTAs of r, K slices of an R tile
   int ksplit, full_tiles, n_tail;
   int nk_min;                  // K steps of the shortest member
-  double us;                   // estimate of what depends on the partition
+  int total, nk;               // tiles, K steps of the longest member
   size_t off_slots;            // in the workspace: K slices' slots (those of r are at kWsSlotsOffset)
 };
 TmemPlan make_tmem_plan(const glowq_w4a16_group_t& g, bool exact, bool compute_r, bool any_corr, bool any_separate, int sms) {
@@ -789,12 +789,14 @@ TmemPlan make_tmem_plan(const glowq_w4a16_group_t& g, bool exact, bool compute_r
     nk_min = std::min(nk_min, steps);
   }
   pl.nk_min = nk_min;
+  pl.nk = nk;
+  pl.total = total;
   const int units = sms, resident = 2 * sms;
   const size_t item_bytes = static_cast<size_t>(pl.N) * kRows * 4;
   // Work partition: f rounds of whole tiles, the rest cut into ks slices of K.  Microseconds, fitted on B200 to every partition of 108
   // group calls (the one taken is 1.2 % slower than the best on average): a step of an SM while two CTAs share it, or of a CTA alone; r,
   // which the last steps wait for; a second wave of items (the CTAs of r take slots, but are gone before a whole tile is done); the
-  // slices of a tile, which go through memory.
+  // slices of a tile, which go through memory.  (The exact form's partitions of 808 calls: 1.0 % slower than the best, 21 % at worst.)
   const double r_us = compute_r ? 3.9 + 0.052 * pl.N : 0.0;
   pl.full_tiles = total;
   pl.n_tail = 0;
@@ -818,13 +820,34 @@ TmemPlan make_tmem_plan(const glowq_w4a16_group_t& g, bool exact, bool compute_r
       }
     }
   }
-  pl.us = best;
   return pl;
 }
 }  // namespace
 
-double gemm_tmem_us(const glowq_w4a16_group_t& g, bool exact, bool compute_r, bool any_corr, bool any_separate, int sms) {
-  return make_tmem_plan(g, exact, compute_r, any_corr, any_separate, sms).us;
+// Microseconds of a call of 2 to 8 tokens in the exact form, as its partition has it.  Fitted on B200 together with the streaming
+// kernel's estimate (see takes_gemm): a step of an SM that two CTAs share, of a CTA alone; r; a second wave; K slices.
+double gemm_tmem_exact_us(const glowq_w4a16_group_t& g, bool compute_r, bool any_corr, int sms) {
+  const TmemPlan pl = make_tmem_plan(g, true, compute_r, any_corr, false, sms);
+  constexpr double kShared = 0.226, kAlone = 0.356;
+  const int ks = pl.ksplit, f = ks > 1 ? pl.full_tiles / sms : 0, slices = ks > 1 ? pl.n_tail * ks : pl.total;
+  const int per_sm = cdiv(slices, sms), items = f * sms + slices;
+  const double steps = static_cast<double>(pl.nk) / ks;   // of an item that is not a whole tile beside slices
+  double body;
+  if (f == 0) {
+    body = per_sm / 2 * 2 * steps * kShared + per_sm % 2 * steps * kAlone;
+  } else {   // whole tiles in pairs, an odd one beside the slices
+    const double cut = per_sm * steps, nk = pl.nk;
+    body = f / 2 * 2 * nk * kShared;
+    if (f % 2 == 0)
+      body += cut * kShared;
+    else
+      body += cut < nk ? 2 * cut * kShared + (nk - cut) * kAlone : (nk + cut) * kShared;
+  }
+  const double slots = ks > 1 ? 0.455 : 0.0, start = 3.898;
+  double us = start + std::max(body, compute_r ? 3.258 : 0.0) + slots + (ks > 1 ? 0.869 * slices / sms : 0.0) +
+              2.196 * (cdiv(items, f > 0 ? 2 * sms : std::max(sms, 2 * sms - pl.n_r)) - 1);
+  if (compute_r && items + pl.n_r > 2 * sms) us = std::max(us, start + 0.304 + 1.77 * steps * kShared + slots);   // items behind r's CTAs
+  return us;
 }
 
 // (host arithmetic: see glowq_internal_workspace_map)

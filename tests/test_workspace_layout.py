@@ -131,3 +131,17 @@ def test_one_token_on_long_rows_takes_no_more_scratch_than_its_most_slices():
         need = K.load_w4a16_extension().workspace_bytes(1, ic, oc, rank, 1)
         assert workspace_map(1, ic, [oc], rank, nbytes=need).ksplit == m.ksplit
     assert {1, 2, 3, 4} <= seen
+
+
+# tokens, columns, K, rank (0: no correction), microseconds streamed and in the exact form on B200, call after call
+MEASURED = [(4, [4224], 12416, 256, 33.6, 16.0), (6, [4480], 4992, 256, 17.7, 11.6), (7, [16768, 16768], 4992, 0, 40.8, 28.5),
+            (5, [3840], 3840, 256, 15.1, 11.1), (4, [2048], 9600, 0, 12.3, 9.5), (5, [13696, 13696], 3456, 0, 24.3, 18.9),
+            (7, [1920, 1408, 1408], 2304, 128, 12.3, 9.8), (3, [9856, 9856], 4608, 128, 20.6, 26.7),
+            (3, [12544, 12544], 2432, 64, 13.9, 17.0), (2, [3840] * 3, 3328, 256, 11.3, 13.8), (2, [3584] * 3, 2560, 128, 9.6, 11.0),
+            (3, [10624, 10624], 4736, 64, 23.4, 26.5)]
+
+
+@pytest.mark.parametrize("M,ocs,ic,rank,stream,exact", MEASURED)
+def test_two_to_eight_tokens_take_the_kernel_that_was_measured_faster(M, ocs, ic, rank, stream, exact):
+    nbytes = K.load_w4a16_extension().workspace_bytes(M, ic, sum(ocs), rank, len(ocs))
+    assert workspace_map(M, ic, ocs, rank, nbytes=nbytes).kernel == (1 if exact < stream else 0)
