@@ -18,6 +18,7 @@ size_t r_product_slot_bytes(int M, int IC, int rank);
 cudaError_t launch_r_product(const __half* x, const __half* R, __half* r_buf, float* slots, uint32_t* ctr, int M, int IC,
                              int rank, int x_stride, int R_stride, cudaStream_t stream);
 size_t gemm_tmem_r_bytes(int M, int IC, int rank);
+size_t gemm_tmem_slot_bytes(int M, int IC, int OC_total, int rank, int n_members, int sms);
 int gemm_tmem_forward(const glowq_w4a16_group_t& g, bool exact, bool compute_r, bool any_corr, bool any_separate, int sms, cudaStream_t stream,
                       cudaError_t* cuda_err);
 int gemm_pair_forward(const glowq_w4a16_group_t& g, bool compute_r, bool r_only, bool any_corr, bool any_separate, int sms,
@@ -72,10 +73,13 @@ size_t gemm_workspace_bytes(int M, int IC, int OC_total, int rank, int n_members
   size_t slots = std::max(rank > 0 ? r_slot_bytes(M, IC, rank) : 0, main_slot_bytes(M, OC_total, n_members));
   // r in a launch of its own (up to 64 tokens); up to 128 the room serves the pairs' slots, which for long rows it lets slice K finer
   if (rank > 0 && M <= 128) slots = std::max(slots, r_product_slot_bytes(M, IC, rank));
-  // K slices of the one-CTA form, unless whole tiles fill the SMs and the last round of them is nearly full too
+  // K slices of the one-CTA form: what its plan takes up to 8 tokens (304 slots for every call were 11.0 MB for a layer of the 13B shapes,
+  // now 8.8); above, unless whole tiles fill the SMs and the last round of them is nearly full too
   const int tmem_tiles = cdiv(OC_total, 128), tmem_rest = tmem_tiles % kPlanSms;
-  if (M > 1 && M <= kTmemMaxM && !(tmem_tiles >= kPlanSms && tmem_rest * 4 >= 3 * kPlanSms))
-    slots = std::max(slots, static_cast<size_t>(kTmemSlices) * (M <= 8 ? 16 : M <= 32 ? 32 : 64) * 128 * 4);
+  if (M > 1 && M <= 8)
+    slots = std::max(slots, gemm_tmem_slot_bytes(M, IC, OC_total, rank, n_members, kPlanSms));
+  else if (M > 8 && M <= kTmemMaxM && !(tmem_tiles >= kPlanSms && tmem_rest * 4 >= 3 * kPlanSms))
+    slots = std::max(slots, static_cast<size_t>(kTmemSlices) * (M <= 32 ? 32 : 64) * 128 * 4);
   if (M > 256) slots = std::max(slots, static_cast<size_t>(kMaxTailSlots) * 4 * kSlotBytes);
   if (rank > 0 && M > 1 && M <= kTmemMaxM) slots += gemm_tmem_r_bytes(M, IC, rank);
   if (slots == 0) return kWsHeaderBytes;

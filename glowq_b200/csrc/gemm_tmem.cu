@@ -824,6 +824,30 @@ TmemPlan make_tmem_plan(const glowq_w4a16_group_t& g, bool exact, bool compute_r
 }
 }  // namespace
 
+// The K slices' slots that a call takes where it has the room: any members of so many columns in all, with and without a correction
+// (and r), planned for `sms` SMs.
+size_t gemm_tmem_slot_bytes(int M, int IC, int OC_total, int rank, int n_members, int sms) {
+  size_t most = 0;
+  glowq_w4a16_group_t g{};
+  g.M = M;
+  g.IC = IC;
+  g.workspace_bytes = ~static_cast<size_t>(0);
+  g.n_members = std::min(n_members, OC_total);
+  for (int narrow = 0; narrow < g.n_members; ++narrow) {   // members that end within a tile: one tile more each
+    for (int i = 0; i < g.n_members; ++i) {
+      g.members[i].OC = i == 0 ? OC_total - narrow : i <= narrow ? 1 : 0;
+      g.members[i].L = &g;
+      g.members[i].alpha = 1.f;
+    }
+    for (int corr = 0; corr <= (rank > 0 ? 2 : 0); ++corr) {   // none, r at hand, r of this launch
+      g.rank = corr ? rank : 0;
+      const TmemPlan pl = make_tmem_plan(g, true, corr == 2, corr > 0, false, sms);
+      most = std::max(most, static_cast<size_t>(pl.n_tail) * pl.ksplit * pl.N * kRows * 4);
+    }
+  }
+  return most;
+}
+
 // Microseconds of a call of 2 to 8 tokens in the exact form, as its partition has it.  Fitted on B200 together with the streaming
 // kernel's estimate (see takes_gemm): a step of an SM that two CTAs share, of a CTA alone; r; a second wave; K slices.
 double gemm_tmem_exact_us(const glowq_w4a16_group_t& g, bool compute_r, bool any_corr, int sms) {

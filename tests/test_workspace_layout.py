@@ -145,3 +145,19 @@ MEASURED = [(4, [4224], 12416, 256, 33.6, 16.0), (6, [4480], 4992, 256, 17.7, 11
 def test_two_to_eight_tokens_take_the_kernel_that_was_measured_faster(M, ocs, ic, rank, stream, exact):
     nbytes = K.load_w4a16_extension().workspace_bytes(M, ic, sum(ocs), rank, len(ocs))
     assert workspace_map(M, ic, ocs, rank, nbytes=nbytes).kernel == (1 if exact < stream else 0)
+
+
+def test_two_to_eight_tokens_ask_for_the_slices_they_take():
+    """With the reported bytes a call is cut as with any amount, in the form the library chooses and in the one asked for, whatever
+    its members' sizes; and it is not asked for much more."""
+    e, layer = K.load_w4a16_extension(), 0
+    groups = [([5120] * 3, 5120), ([5120], 5120), ([13824] * 2, 5120), ([5120], 13824)]
+    others = [([3000, 500, 501, 1], 2176), ([129, 127], 18944), ([1], 640), ([9856] * 2, 4608), ([200, 200, 200, 200], 8200)]
+    for (ocs, ic), rank, kernel in itertools.product(groups + others, (0, 16, 128, 1024), (K.KERNEL_AUTO, K.KERNEL_GEMM)):
+        need = e.workspace_bytes(6, ic, sum(ocs), rank, len(ocs))
+        for r_mode in (K.R_COMPUTE, K.R_LOAD):
+            a, b = (workspace_map(6, ic, ocs, rank, nbytes=n, kernel=kernel, r_mode=r_mode) for n in (need, 1 << 28))
+            assert (a.kernel, a.ksplit, a.whole_tiles, a.sliced_tiles) == (b.kernel, b.ksplit, b.whole_tiles, b.sliced_tiles)
+    for ocs, ic in groups:
+        layer += e.workspace_bytes(8, ic, sum(ocs), 128, len(ocs))
+    assert layer < 9e6
