@@ -112,8 +112,20 @@ class GroupLauncher:
     order) names the launch that follows, for the library's ``next`` hint."""
 
     def __init__(self, members):
-        self.members = list(members)          # AddSVDCorrection wrappers, first = producer (q / gate / solo)
-        self.next_launcher: Optional["GroupLauncher"] = None
+        members = list(members)               # AddSVDCorrection wrappers, first = producer (q / gate / solo)
+        first = members[0]
+        inner0 = first.inner
+        self._reset(members, None, len(members) <= K.MAX_MEMBERS and all(
+            w.inner.in_features == inner0.in_features and w.inner.group_size == inner0.group_size
+            and w.inner._out_dtype == inner0._out_dtype and w.B_q.shape == first.B_q.shape
+            and w.A_q.size(1) == first.A_q.size(1) for w in members))
+
+    def _reset(self, members, next_launcher, usable: bool) -> None:
+        # The wrappers hold their launcher, and it names them and its successor weakly: a model that is dropped gives its memory back
+        # then and there, not when the cycle collector runs.
+        self._refs = [weakref.ref(w) for w in members]
+        self.next_launcher = next_launcher
+        self.usable = usable
         self._scratch = K.Scratch()
         self._sizes: Dict[tuple, tuple] = {}  # by (tokens, device, rank): the workspace's bytes, and those with r's behind them
         self._call: Optional[K.Group] = None  # the descriptor of the last launch, which the launch in front names as the one that follows
@@ -122,12 +134,27 @@ class GroupLauncher:
         self._call_weights: list = []         # the members' buffers and where it found the packed weights
         self._pending: Dict[int, torch.Tensor] = {}
         self._pending_key = None
-        first = self.members[0]
-        inner0 = first.inner
-        self.usable = all(
-            w.inner.in_features == inner0.in_features and w.inner.group_size == inner0.group_size
-            and w.inner._out_dtype == inner0._out_dtype and w.B_q.shape == first.B_q.shape
-            and w.A_q.size(1) == first.A_q.size(1) for w in self.members) and len(self.members) <= K.MAX_MEMBERS
+
+    @property
+    def members(self) -> list:
+        """The wrappers that are alive, the producer first."""
+        return [w for w in (ref() for ref in self._refs) if w is not None]
+
+    @property
+    def next_launcher(self) -> Optional["GroupLauncher"]:
+        return None if self._next is None else self._next()
+
+    @next_launcher.setter
+    def next_launcher(self, launcher: Optional["GroupLauncher"]) -> None:
+        self._next = None if launcher is None else weakref.ref(launcher)
+
+    def __getstate__(self):      # a copied or saved launcher has the same place in its model, and nothing of its launches
+        return self.members, self.next_launcher, self.usable and len(self.members) == len(self._refs)
+
+    def __setstate__(self, state):
+        if isinstance(state, dict):      # saved when launchers named their members strongly
+            state = state["members"], state["next_launcher"], state["usable"]
+        self._reset(*state)
 
     def _describe(self, key: tuple, inners) -> None:
         """What calls of one size have in common: the descriptor's fixed fields."""
@@ -153,7 +180,8 @@ class GroupLauncher:
         grp, dev = self._call, device.index
         if grp is None or self._call_key[1] != dev or (m, dev, grp.rank) not in self._sizes:
             return None
-        if _buffer(self.members[0], "B_q").data_ptr() != grp.R:
+        first = self._refs[0]()
+        if first is None or _buffer(first, "B_q").data_ptr() != grp.R:
             return None
         for buffers, at in self._call_weights:
             t = buffers.get("qweight_i32")
@@ -161,10 +189,11 @@ class GroupLauncher:
                 return None
         return self._call_at
 
-    def run(self, x: torch.Tensor) -> torch.Tensor:
+    def run(self, x: torch.Tensor, members: Optional[list] = None) -> torch.Tensor:
         """Called by the first member: launch the whole group, keep the other members' outputs, return its own."""
-        first = self.members[0]
-        inners = [_inner(w) for w in self.members]
+        members = members or self.members
+        first = members[0]
+        inners = [_inner(w) for w in members]
         inner = inners[0]
         x2d = inner._flatten_input(x)
         m, dev, dtype = x2d.shape[0], x2d.device, inner._out_dtype
@@ -172,23 +201,23 @@ class GroupLauncher:
         self._pending.clear()
         key = _x_key(x)
         if m > 0:
-            if torch.cuda.current_device() == dev.index:
-                r = self._launch(x2d, inners, outs, m, dev, dtype)
+            if K.current_device() == dev.index:
+                r = self._launch(x2d, members, inners, outs, m, dev, dtype)
             else:
                 with torch.cuda.device(dev):
-                    r = self._launch(x2d, inners, outs, m, dev, dtype)
+                    r = self._launch(x2d, members, inners, outs, m, dev, dtype)
             self._keep = x2d          # the launch reads x2d asynchronously
             if r is not None:
-                first.group_cache.set(r, len(self.members) - 1, key)
+                first.group_cache.set(r, len(members) - 1, key)
         flat = x.dim() == 2
-        for w, o in zip(self.members[1:], outs[1:]):
+        for w, o in zip(members[1:], outs[1:]):
             self._pending[id(w)] = o if flat else o.reshape(*x.shape[:-1], o.size(1))
         self._pending_key = key
         return outs[0] if flat else outs[0].reshape(*x.shape[:-1], inner.out_features)
 
-    def _launch(self, x2d, inners, outs, m, dev, dtype) -> Optional[torch.Tensor]:
+    def _launch(self, x2d, members, inners, outs, m, dev, dtype) -> Optional[torch.Tensor]:
         """The launch; r, where the members' cache hands it on."""
-        first, inner, index = self.members[0], inners[0], dev.index
+        first, inner, index = members[0], inners[0], dev.index
         R = _buffer(first, "B_q")
         rank = R.shape[0]
         key = (m, index, rank, dtype, inner.kernel_choice(m))
@@ -203,10 +232,12 @@ class GroupLauncher:
         grp.R, grp.R_stride = R.data_ptr(), R.stride()[0]
         grp.workspace, grp.workspace_bytes, grp.r_buf, grp.stream = at, need, at + need, stream
         weights, place = [], K.Group.members.offset
-        for w, lin, o in zip(self.members, inners, outs):
+        for w, lin, o in zip(members, inners, outs):
             alpha = float(w.alpha_svd)
             if alpha != 0.0 and not w._mismatch:
-                L = _buffer(w, "A_q")
+                L = w._buffers.get("A_q")
+                if L is None:
+                    L = w.A_q
                 fields = lin.pack_member(o, L, alpha)
                 if fields[10] != rank and L.shape[1] != rank:      # (the row stride: other than the rank in a part of a larger factor)
                     raise RuntimeError(f"a left factor has rank {L.shape[1]}, the group's right factor {rank}")
@@ -216,9 +247,11 @@ class GroupLauncher:
             place += K.PACK_MEMBER.size
             weights.append((lin._buffers, fields[0]))
         self._call_weights = weights
-        nxt = self.next_launcher
+        nxt = self._next and self._next()
         grp.next = nxt.descriptor_address(m, dev) if nxt is not None else None
-        ext.check(ext.lib.glowq_w4a16_group_forward(grp), "glowq_w4a16_group_forward")
+        rc = ext.lib.glowq_w4a16_group_forward(grp)
+        if rc:
+            ext.check(rc, "glowq_w4a16_group_forward")
         if inner._check_status:
             ext.check(ext.lib.glowq_w4a16_read_status(at, stream), "device status")
         if not first.is_group or first.group_cache is None:
@@ -273,10 +306,12 @@ class AddSVDCorrection(nn.Module):
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         gl = self.group_launcher
         if gl is not None and gl.usable and x.is_cuda:
-            if gl.members[0] is self:
-                for w in gl.members:
-                    if w.alpha_svd != 0.0 and not w._mismatch:
-                        return gl.run(x)
+            if gl._refs[0]() is self:
+                members = [ref() for ref in gl._refs]
+                if None not in members:      # (of a group of which only some are left, each launches for itself)
+                    for w in members:
+                        if w.alpha_svd != 0.0 and not w._mismatch:
+                            return gl.run(x, members)
                 gl.forget()      # nothing to correct in this group: outputs kept from an earlier call must not be served
             else:
                 out = gl.take(self, x)

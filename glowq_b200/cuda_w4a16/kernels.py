@@ -206,7 +206,7 @@ class _Ext:
         gid = torch.empty(ic, dtype=torch.int64, device=weight.device) if index else None
         args = (weight.data_ptr(), qweight.data_ptr(), qzeros.data_ptr(), scales.data_ptr(),
                 gid.data_ptr() if index else None, oc, ic, int(group_size), max(weight.stride(0), ic), current_stream_ptr(weight.device))
-        if torch.cuda.current_device() == weight.device.index:
+        if current_device() == weight.device.index:
             rc = self.lib.glowq_w4a16_quantize_indexed(*args)
         else:
             with torch.cuda.device(weight.device):
@@ -230,6 +230,7 @@ def current_stream_ptr(device: torch.device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
 
 
+current_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)   # (where CUDA is in use already)
 _is_capturing = getattr(torch._C, "_cuda_isCurrentStreamCapturing", torch.cuda.is_current_stream_capturing)
 
 

@@ -225,7 +225,7 @@ class CudaW4A16Linear(nn.Module):
         out = torch.empty(m, self.out_features, dtype=self._out_dtype, device=dev)
         if m == 0:
             return out
-        if torch.cuda.current_device() == dev.index:
+        if K.current_device() == dev.index:
             self._launch(ext, x2d, out, m, dev, L, R, r_buf, r_mode, alpha, push, push_site)
         else:
             with torch.cuda.device(dev):

@@ -1,4 +1,8 @@
 """The group launchers: what they look up on every call and what they hold."""
+import copy
+import gc
+import pickle
+import weakref
 from types import SimpleNamespace
 
 import pytest
@@ -108,6 +112,39 @@ def test_token_counts_share_a_piece():
             assert piece.numel() < 18 << 20
 
 
+def test_a_dropped_model_is_gone_at_once():
+    gc.collect()
+    gc.disable()
+    try:
+        model = patched()
+        refs = [weakref.ref(o) for li in range(2) for p in ToyDecoder.PROJ for w in [model.proj(li, p)]
+                for o in (w, w.inner, w.group_launcher, w.inner.qweight_i32)]
+        part = model.proj(0, "self_attn.k_proj")
+        launcher = part.group_launcher
+        del model
+        alive = [r() for r in refs if r() is not None]
+        assert {id(o) for o in alive} == {id(o) for o in (part, part.inner, launcher, part.inner.qweight_i32)}
+        assert launcher.members == [part] and launcher.next_launcher is None
+    finally:
+        gc.enable()
+
+
+@pytest.mark.parametrize("make", [copy.deepcopy, lambda m: pickle.loads(pickle.dumps(m))])
+def test_a_copied_model_has_launchers_of_its_own(make):
+    model = patched()
+    other = make(model)
+    del model
+    launchers = []
+    for li in range(2):
+        for p in ToyDecoder.PROJ:
+            w = other.proj(li, p)
+            gl = w.group_launcher
+            assert gl.usable and any(m is w for m in gl.members) and gl._sizes == {}
+            if gl.members[0] is w:
+                launchers.append(gl)
+    assert len(launchers) == 8 and all(a.next_launcher is b for a, b in zip(launchers, launchers[1:] + launchers[:1]))
+
+
 def test_room_for_r_that_a_graph_was_captured_with_stays(monkeypatch):
     capturing = [False]
     monkeypatch.setattr(K, "_is_capturing", lambda: capturing[0])
@@ -166,3 +203,18 @@ def test_a_captured_step_beside_other_calls(m, fuse, monkeypatch):
     mods = [model.proj(li, p) for li in range(2) for p in ToyDecoder.PROJ]
     used = [piece for w in mods for piece in pieces(w.group_launcher) + pieces(w.inner)]
     assert used and {status(piece.data_ptr(), stream) for piece in used} == {0}
+
+
+@pytest.mark.gpu
+def test_what_is_left_of_a_group(m=5):
+    """A member whose wrapper is gone: the others launch for themselves, the producer first."""
+    model, x = patched("cuda"), inputs(m)
+    with torch.no_grad():
+        want = [y.clone() for y in forward(model, *x)]
+        model.model.layers[0].self_attn.k_proj = nn.Identity()
+        model.model.layers[1].self_attn.q_proj = nn.Identity()
+        got = forward(model, *x)
+    for li in range(2):
+        for i, p in enumerate(ToyDecoder.PROJ):
+            if not isinstance(model.proj(li, p), nn.Identity):
+                torch.testing.assert_close(got[7 * li + i], want[7 * li + i], rtol=1e-4, atol=1e-4)
