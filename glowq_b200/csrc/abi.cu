@@ -257,20 +257,30 @@ int gemv_r_ctas(const GemvPlan& pl, int n_tiles, int units, int cap) {
   return std::max(0, want);
 }
 
-// Microseconds of a one-token launch on long rows, fitted on B200 to 1000 calls of 48 to 288 tiles, 96 to 148 groups and ranks 0 to 256
-// with 1 to 6 slices each (the plans taken are 0.9 % slower than the best ones on average, 13 % at worst; 12 % and 46 % by a fixed rule).  Unsliced, a launch is as long
-// as a CTA's tiles or as r; a tile that follows R units begins when they are done.  Sliced, every round of tiles pays the combine.
+// Microseconds of a one-token launch on long rows: chunks of 1024 columns with two CTAs or one per SM (an odd number of groups arrives
+// without the swizzle, see tensor_map_w3d: its chunks take a tenth to a half longer), the rounds of tiles - a last one that is not full
+// is shorter, but not as much -, the correction of a tile, and r.  Unsliced, a launch is as long as a CTA's tiles or as R units and the
+// tiles behind them; sliced, every round pays the combine.  Fitted on B200 to 1300 calls of 48 to 288 tiles, 96 to 150 groups and ranks
+// 0 to 256 with 1 to 6 slices each; of those left out of the fit the plans taken are 0.4 % slower than the best ones on average, 14 % at
+// worst.  (By costs without the parity 2.5 % and 42 %: 2304 x 14208, rank 40, 15.3 us in one slice instead of 12.2.)
 double one_token_us(const GemvPlan& pl, int n_tiles, int rank, int units, int sms) {
   const int cap = sms * pl.ctas_per_sm, r_ctas = gemv_r_ctas(pl, n_tiles, units, cap);
-  const int chunks = ceil_div(pl.G, kChunkGroups), ch = ceil_div(std::min(pl.gps, pl.G), kChunkGroups);
-  if (pl.SK == 1) {
-    const double tile = 3.027 + (0.35 + 0.00193 * n_tiles + (n_tiles > cap ? 0.221 : 0.0)) * ch + 0.0237 * rank;
-    if (units == 0) return tile;
-    return std::max(tile, 2.247 + 3.448 * ceil_div(units, std::max(1, r_ctas)) + (n_tiles > cap - r_ctas ? 0.591 * ch : 0.0));
+  const bool odd = pl.G & 1;
+  const double chunk = pl.ctas_per_sm == 2 ? (odd ? 0.860 : 0.785) : (0.418 + 0.564 / pl.stages) * (odd ? 1.439 : 1.0);
+  const double tile = chunk * std::min(pl.gps, pl.G) / kChunkGroups, ranks = rank / 64.0;
+  const int unit_rounds = units > 0 ? ceil_div(units, std::max(1, r_ctas)) : 0;
+  if (pl.SK > 1) {
+    const int slots = std::max(1, (cap - r_ctas) / pl.SK * pl.SK), rounds = ceil_div(n_tiles * pl.SK, slots);
+    const double last = static_cast<double>(n_tiles) * pl.SK / slots - (rounds - 1), load = rounds - 1 + last + 0.586 * (1.0 - last);
+    return 5.614 + load * (0.686 * tile + 1.548) - 0.223 * pl.SK + 0.072e-6 * n_tiles * kTileRows * (66.5 * pl.G) +
+           (rank > 0 ? 0.677 + 0.514 * ranks * load : 0.0) + 0.09 * unit_rounds;
   }
-  const int rounds = ceil_div(n_tiles * pl.SK, std::max(1, (cap - r_ctas) / pl.SK * pl.SK));
-  return 4.267 + (1.95 + 0.101 * ch) * rounds + 0.00253 * n_tiles * chunks + (pl.ctas_per_sm == 1 ? 0.648 : 0.0) + 0.079 * pl.SK +
-         (rank > 0 ? 0.874 + (0.0252 / pl.SK + 0.0169) * units : 0.0);
+  const int rounds = ceil_div(n_tiles, cap);
+  const double last = static_cast<double>(n_tiles) / cap - (rounds - 1), load = rounds - 1 + last + (rounds == 1 ? 0.249 : 0.375) * (1.0 - last);
+  const double each = rank > 0 ? 1.059 + 0.526 * ranks : 0.0, all = 5.663 + tile * load + each * rounds;
+  if (units == 0) return all;
+  const int behind = n_tiles > cap - r_ctas ? ceil_div(n_tiles - (cap - r_ctas), cap) : 0;   // tiles of a CTA after its R units
+  return std::max(all, 3.191 + 2.696 * unit_rounds + 0.933 * behind * tile + each * std::max(behind, 1));
 }
 
 GemvPlan make_plan(int M, int IC, int n_tiles, int rank, bool compute_r, int sms, int split_k) {
@@ -329,7 +339,7 @@ GemvPlan make_plan(int M, int IC, int n_tiles, int rank, bool compute_r, int sms
     // 3584 x 13824 14.2 -> 10.7 (3 -> none), 7168 x 12288 corrected 24.3 -> 17.5 (3 -> none).
     const int units = compute_r ? pl.n_r_tiles * ceil_div(pl.G, ceil_div(pl.G, pl.SKr)) : 0;
     int best = sk;
-    double best_us = 0.96 * one_token_us(pl, n_tiles, rank, units, sms);   // (less than that is within the estimate's error)
+    double best_us = one_token_us(pl, n_tiles, rank, units, sms);
     for (int s = sk - 1; s >= 1; --s) {
       cut(s);
       if (pl.stages == 0) break;

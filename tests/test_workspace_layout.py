@@ -161,3 +161,15 @@ def test_two_to_eight_tokens_ask_for_the_slices_they_take():
     for ocs, ic in groups:
         layer += e.workspace_bytes(8, ic, sum(ocs), 128, len(ocs))
     assert layer < 9e6
+
+
+# outputs, K, rank (0: no correction), the number of slices that was fastest on B200, its microseconds and those of another number
+SLICES = [(2304, 14208, 40, 3, 12.2, 15.3), (2944, 16256, 40, 3, 14.3, 22.2), (5760, 16256, 64, 3, 21.1, 27.7),
+          (4992, 13440, 40, 3, 17.4, 19.2), (3584, 16256, 0, 4, 14.2, 18.9), (3584, 17920, 128, 1, 15.7, 17.6), (3584, 13824, 0, 1, 10.8, 14.2),
+          (7168, 12288, 64, 1, 17.3, 22.6), (5120, 17408, 256, 3, 24.4, 29.2)]
+
+
+@pytest.mark.parametrize("oc,ic,rank,slices,us,other", SLICES)
+def test_one_token_on_long_rows_takes_the_slices_that_were_measured_fastest(oc, ic, rank, slices, us, other):
+    nbytes = K.load_w4a16_extension().workspace_bytes(1, ic, oc, rank, 1)
+    assert us < other and workspace_map(1, ic, [oc], rank, nbytes=nbytes).ksplit == slices
