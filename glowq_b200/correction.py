@@ -26,6 +26,8 @@ except Exception:  # noqa: BLE001
     def _tqdm(it, **_):
         return it
 
+_pack_member_into, _MEMBER_BYTES, _MEMBERS_AT = K.PACK_MEMBER.pack_into, K.PACK_MEMBER.size, K.Group.members.offset
+
 _ALL_CACHES: "weakref.WeakSet[MiniGroupCache]" = weakref.WeakSet()
 
 
@@ -47,12 +49,6 @@ def _inner(w: "AddSVDCorrection") -> CudaW4A16Linear:
     """``w.inner`` (``nn.Module.__getattr__`` takes half a microsecond)."""
     inner = w._modules.get("inner")
     return w.inner if inner is None else inner
-
-
-def _buffer(mod: nn.Module, name: str) -> torch.Tensor:
-    """The module's tensor of that name: a buffer, unless somebody made it a parameter."""
-    t = mod._buffers.get(name)
-    return getattr(mod, name) if t is None else t
 
 
 class MiniGroupCache:
@@ -127,11 +123,11 @@ class GroupLauncher:
         self.next_launcher = next_launcher
         self.usable = usable
         self._scratch = K.Scratch()
-        self._sizes: Dict[tuple, tuple] = {}  # by (tokens, device, rank): the workspace's bytes, and those with r's behind them
+        self._sizes: Dict[tuple, int] = {}    # the workspace's bytes by (tokens, device, rank)
         self._call: Optional[K.Group] = None  # the descriptor of the last launch, which the launch in front names as the one that follows
         self._call_key: Optional[tuple] = None
         self._call_r: Optional[tuple] = None
-        self._call_weights: list = []         # the members' buffers and where it found the packed weights
+        self._call_weights: list = []         # (buffers, name, address) of the right factor and the packed weights
         self._pending: Dict[int, torch.Tensor] = {}
         self._pending_key = None
 
@@ -158,33 +154,31 @@ class GroupLauncher:
 
     def _describe(self, key: tuple, inners) -> None:
         """What calls of one size have in common: the descriptor's fixed fields."""
-        m, dev, rank, dtype, kernel = key
+        m, dev, rank, dtype = key
         if self._call is None:
             call = K.Group()
             self._call_at = ctypes.addressof(call)
             self._call = call
         grp, lin = self._call, inners[0]
         grp.M, grp.IC, grp.rank, grp.group_size = m, lin.in_features, rank, lin.group_size
-        grp.r_mode, grp.kernel, grp.n_members = K.R_COMPUTE, kernel, len(inners)
+        grp.r_mode, grp.kernel, grp.n_members = K.R_COMPUTE, lin.kernel_choice(m), len(inners)
         grp.out_dtype = K.OUT_F32 if dtype == torch.float32 else K.OUT_F16
-        if (m, dev, rank) not in self._sizes:
+        need = self._sizes.get((m, dev, rank))
+        if need is None:
             if len(self._sizes) > 4096:
                 self._sizes.clear()
             need = lin._get_ext().workspace_bytes(m, lin.in_features, sum(i.out_features for i in inners), rank, len(inners))
-            self._sizes[m, dev, rank] = need, need + 2 * m * rank     # (a workspace is a multiple of 256 bytes)
-        self._call_key = key
+            self._sizes[m, dev, rank] = need
+        self._call_key, self._call_need, self._call_total = key, need, need + 2 * m * rank   # (a multiple of 256 bytes, and r)
 
     def descriptor_address(self, m: int, device, dtype=None) -> Optional[int]:
         """The descriptor of the last launch, for the ``next`` hint of the one in front.  None before a launch of so many tokens, and
         where the weights have moved since: what the descriptor points to may be unmapped by now."""
-        grp, dev = self._call, device.index
-        if grp is None or self._call_key[1] != dev or (m, dev, grp.rank) not in self._sizes:
+        key = self._call_key
+        if key is None or key[1] != device.index or (m, key[1], key[2]) not in self._sizes:
             return None
-        first = self._refs[0]()
-        if first is None or _buffer(first, "B_q").data_ptr() != grp.R:
-            return None
-        for buffers, at in self._call_weights:
-            t = buffers.get("qweight_i32")
+        for buffers, name, at in self._call_weights:
+            t = buffers.get(name)
             if t is None or t.data_ptr() != at:
                 return None
         return self._call_at
@@ -217,21 +211,23 @@ class GroupLauncher:
 
     def _launch(self, x2d, members, inners, outs, m, dev, dtype) -> Optional[torch.Tensor]:
         """The launch; r, where the members' cache hands it on."""
-        first, inner, index = members[0], inners[0], dev.index
-        R = _buffer(first, "B_q")
+        first, inner = members[0], inners[0]
+        factors, name = first._buffers, "B_q"
+        R = factors.get(name)
+        if R is None:
+            factors, R = first._parameters, first.B_q
         rank = R.shape[0]
-        key = (m, index, rank, dtype, inner.kernel_choice(m))
+        key = (m, dev.index, rank, dtype)
         if key != self._call_key:
             self._describe(key, inners)
-        need, total = self._sizes[m, index, rank]
         grp, ext = self._call, inner._get_ext()
         stream = K.current_stream_ptr(dev)
-        piece = self._scratch.get(total, dev, stream)
-        at = piece.data_ptr()
+        piece = self._scratch.get(self._call_total, dev, stream)
+        at, R_at = piece.data_ptr(), R.data_ptr()
         grp.x, grp.x_stride = x2d.data_ptr(), x2d.stride()[0]
-        grp.R, grp.R_stride = R.data_ptr(), R.stride()[0]
-        grp.workspace, grp.workspace_bytes, grp.r_buf, grp.stream = at, need, at + need, stream
-        weights, place = [], K.Group.members.offset
+        grp.R, grp.R_stride = R_at, R.stride()[0]
+        grp.workspace, grp.workspace_bytes, grp.r_buf, grp.stream = at, self._call_need, at + self._call_need, stream
+        weights, place = [(factors, name, R_at)], _MEMBERS_AT
         for w, lin, o in zip(members, inners, outs):
             alpha = float(w.alpha_svd)
             if alpha != 0.0 and not w._mismatch:
@@ -243,9 +239,9 @@ class GroupLauncher:
                     raise RuntimeError(f"a left factor has rank {L.shape[1]}, the group's right factor {rank}")
             else:
                 fields = lin.pack_member(o)
-            K.PACK_MEMBER.pack_into(grp, place, *fields)
-            place += K.PACK_MEMBER.size
-            weights.append((lin._buffers, fields[0]))
+            _pack_member_into(grp, place, *fields)
+            place += _MEMBER_BYTES
+            weights.append((lin._buffers, "qweight_i32", fields[0]))
         self._call_weights = weights
         nxt = self._next and self._next()
         grp.next = nxt.descriptor_address(m, dev) if nxt is not None else None
@@ -257,8 +253,9 @@ class GroupLauncher:
         if not first.is_group or first.group_cache is None:
             return None
         r = self._call_r
-        if r is None or r[0] is not piece or r[1] != key:
-            self._call_r = r = (piece, key, piece[need:total].view(torch.float16).view(m, rank))
+        if r is None or r[0] is not piece or r[1] is not self._call_key:
+            need, total = self._call_need, self._call_total
+            self._call_r = r = (piece, self._call_key, piece[need:total].view(torch.float16).view(m, rank))
         return r[2]
 
     def forget(self) -> None:
