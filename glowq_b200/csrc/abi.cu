@@ -276,7 +276,8 @@ double one_token_us(const GemvPlan& pl, int n_tiles, int rank, int units, int sm
            (rank > 0 ? 0.677 + 0.514 * ranks * load : 0.0) + 0.09 * unit_rounds;
   }
   const int rounds = ceil_div(n_tiles, cap);
-  const double last = static_cast<double>(n_tiles) / cap - (rounds - 1), load = rounds - 1 + last + (rounds == 1 ? 0.249 : 0.375) * (1.0 - last);
+  const double last = static_cast<double>(n_tiles) / cap - (rounds - 1);
+  const double load = rounds - 1 + last + (rounds == 1 ? 0.249 : 0.375) * (1.0 - last);
   const double each = rank > 0 ? 1.059 + 0.526 * ranks : 0.0, all = 5.663 + tile * load + each * rounds;
   if (units == 0) return all;
   const int behind = n_tiles > cap - r_ctas ? ceil_div(n_tiles - (cap - r_ctas), cap) : 0;   // tiles of a CTA after its R units
@@ -507,7 +508,8 @@ int gemv_group_forward(const glowq_w4a16_group_t& g, const DeviceInfo& dev, cuda
   const int n_tiles = n_tiles_of(g);
   for (int m0 = 0; m0 < g.M; m0 += kGemvMaxM) {
     const int Mc = std::min(kGemvMaxM, g.M - m0);
-    const GemvPlan pl = make_plan(Mc, g.IC, n_tiles, g.r_mode != GLOWQ_R_NONE ? g.rank : 0, g.r_mode == GLOWQ_R_COMPUTE, dev.sms, g.split_k);
+    const GemvPlan pl = make_plan(Mc, g.IC, n_tiles, g.r_mode != GLOWQ_R_NONE ? g.rank : 0, g.r_mode == GLOWQ_R_COMPUTE, dev.sms,
+                                  g.split_k);
     if (pl.total > g.workspace_bytes) return GLOWQ_ERR_WORKSPACE_TOO_SMALL;
     unsigned char* ws = static_cast<unsigned char*>(g.workspace);
     const __half* x = static_cast<const __half*>(g.x) + static_cast<size_t>(m0) * g.x_stride;
@@ -747,7 +749,8 @@ int glowq_internal_workspace_map(const glowq_w4a16_group_t* group, int sms, Work
     return GLOWQ_OK;
   }
   const int n_tiles = n_tiles_of(g);
-  const GemvPlan pl = make_plan(std::min(g.M, kGemvMaxM), g.IC, n_tiles, g.r_mode != GLOWQ_R_NONE ? g.rank : 0, g.r_mode == GLOWQ_R_COMPUTE, sms, g.split_k);
+  const GemvPlan pl = make_plan(std::min(g.M, kGemvMaxM), g.IC, n_tiles, g.r_mode != GLOWQ_R_NONE ? g.rank : 0,
+                                g.r_mode == GLOWQ_R_COMPUTE, sms, g.split_k);
   if (pl.total > g.workspace_bytes) return GLOWQ_ERR_WORKSPACE_TOO_SMALL;
   map->kernel = 0;
   if (pl.SK > 1 && !pl.own_ctr) {

@@ -2,8 +2,8 @@
 //
 //   Y[M, OC] = X[M, IC] . dequant(Q)^T  +  alpha * r[M, rank] . L[OC, rank]^T  (+ bias),     r = X . R^T
 //
-// Up to 64 tokens one CTA per 128 output columns (gemm_tmem.cu; up to 8 in its exact form), above a CTA pair per 256 (gemm_pair.cu).  Both keep the
-// dequantised weights in tensor memory, and both compute r inside the group launch.  The line lies where the first ends: two CTAs
+// Up to 64 tokens one CTA per 128 output columns (gemm_tmem.cu; up to 8 in its exact form), above a CTA pair per 256 (gemm_pair.cu).
+// Both keep the dequantised weights in tensor memory, and both compute r inside the group launch.  The line lies where the first ends: two CTAs
 // share an SM's tensor memory there, which leaves an accumulator 64 tokens (13B gate/up 45 us at 64 tokens; the pair form, whose
 // tiles have 64 tokens at least, takes 14B gate/up at 65 tokens from 67 to 63 us).
 #include <algorithm>
@@ -19,11 +19,12 @@ cudaError_t launch_r_product(const __half* x, const __half* R, __half* r_buf, fl
                              int rank, int x_stride, int R_stride, cudaStream_t stream);
 size_t gemm_tmem_r_bytes(int M, int IC, int rank);
 size_t gemm_tmem_slot_bytes(int M, int IC, int OC_total, int rank, int n_members, int sms);
-int gemm_tmem_forward(const glowq_w4a16_group_t& g, bool exact, bool compute_r, bool any_corr, bool any_separate, int sms, cudaStream_t stream,
-                      cudaError_t* cuda_err);
+int gemm_tmem_forward(const glowq_w4a16_group_t& g, bool exact, bool compute_r, bool any_corr, bool any_separate, int sms,
+                      cudaStream_t stream, cudaError_t* cuda_err);
 int gemm_pair_forward(const glowq_w4a16_group_t& g, bool compute_r, bool r_only, bool any_corr, bool any_separate, int sms,
                       cudaStream_t stream, cudaError_t* cuda_err);
-void gemm_tmem_workspace_map(const glowq_w4a16_group_t& g, bool exact, bool compute_r, bool any_corr, bool any_separate, int sms, WorkspaceMap* map);
+void gemm_tmem_workspace_map(const glowq_w4a16_group_t& g, bool exact, bool compute_r, bool any_corr, bool any_separate, int sms,
+                             WorkspaceMap* map);
 void gemm_pair_workspace_map(const glowq_w4a16_group_t& g, bool compute_r, bool any_corr, bool any_separate, int sms, WorkspaceMap* map);
 
 namespace {

@@ -191,7 +191,7 @@ __device__ __forceinline__ void lds_v4(uint32_t* w, uint32_t addr) {
 }
 
 // The MMAs of one step (eight of 16 columns, or the first four) and the commit that releases its stages in both CTAs, issued by
-// one elected lane of a converged warp: as one block, so that descriptors and addresses stay in uniform registers.
+// one elected lane of a converged warp, as one block (see umma_ts_step of the one-CTA form, where it was measured).
 #define GLOWQ_PT_MMA(E, A, B, P) "@" E " tcgen05.mma.cta_group::2.kind::f16 [%0], " A ", " B ", %5, " P ";\n\t"
 __device__ __forceinline__ void pair_step(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t b_hi, uint32_t sub16, uint32_t idesc,
                                           uint32_t accumulate, uint32_t both_halves, uint32_t bar) {
@@ -625,7 +625,7 @@ gemm_pair_kernel(const __grid_constant__ PtParams p, const __grid_constant__ PtM
         if (!(ok = g_mbar_wait_warp<false>(smem0 + kBAccEmpty + 8 * buf, (use & 1) ^ 1, abort_flag, p.status))) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         uint32_t d = tmem + buf * static_cast<uint32_t>(p.N), acc = 0;
-        // (what was read from shared memory is the same in all lanes: the compiler learns it from a reduction)
+        // (what was read from shared memory is the same in all lanes: a reduction says so in the source)
         const uint32_t it0 = __reduce_or_sync(0xffffffffu, t.it0), nk = __reduce_or_sync(0xffffffffu, t.nk);
         const uint32_t last = G + ((p.rank + 127) >> 7) - 1, last_both = (p.rank & 127) == 0 || (p.rank & 127) > 64;
         const uint32_t sep_at = p.sep ? G : 0xFFFFFFFFu;
@@ -1099,7 +1099,8 @@ PairPlan make_pair_plan(const glowq_w4a16_group_t& g, bool compute_r, bool any_c
             cost += sum_us(pl.N, ks, false);
           } else {
             // (slices are added up while pairs that began with r are in their tiles; short ones help where both are through together)
-            const double first = std::max(tile, with_r), after_r = std::max(r_item + tile, with_r), last_r = std::max(r_free + tile, with_r);
+            const double first = std::max(tile, with_r), after_r = std::max(r_item + tile, with_r);
+            const double last_r = std::max(r_free + tile, with_r);
             cost = (f - 1) * tile + 0.05 * slice +
                    std::max(r_last > 0 ? last_r : first,
                             rounds_us(tail * ks, {others, r_pairs - r_last, r_last, 0},

@@ -1,4 +1,5 @@
-// Corrected W4A16 product for decode batches (9 to 64 tokens; 2 to 8 in an exact form, see EXACT) with the dequantised weights in TENSOR MEMORY.
+// Corrected W4A16 product for decode batches (9 to 64 tokens; 2 to 8 in an exact form, see EXACT) with the dequantised weights in
+// TENSOR MEMORY.
 //
 //   D[128 output columns, N tokens] += W[128, 128 k] . X[N, 128 k]^T      (one quantisation group of K per step)
 //
@@ -121,9 +122,9 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
 }
 
 // The MMAs of one step and the commit that releases its stage, issued by one elected lane of a converged warp.  The whole
-// warp runs the issuing loop, and the step is one block, so that descriptors and addresses stay in uniform registers,
-// which these instructions read: a loop under `lane == 0` moves every operand of every MMA over first (the gate/up launch
-// of the 13B shapes at 16 tokens: 38.6 us so, 34.4 with an elected lane per MMA, 33.0 with the step as one block).
+// warp runs the issuing loop, and the step is one block, meant to leave descriptors and addresses where these instructions read
+// them.  The gate/up launch of the 13B shapes at 16 tokens: 38.6 us with a loop under `lane == 0`, 34.4 with an elected lane per
+// MMA, 33.0 with the step as one block.
 // `bar`: the stage's release.  b_lo / b_hi: descriptor words of the activation tile, whose second 64 columns lie `sub16`
 // further; accumulate 0: the first MMA overwrites D.
 #define GLOWQ_TS_MMA(A, B, P) "@e tcgen05.mma.cta_group::1.kind::f16 [%0], " A ", " B ", %5, " P ";\n\t"
@@ -221,15 +222,16 @@ __device__ __forceinline__ void add_share(const ShareArgs& a, int share, int et)
     }
   }
 }
-// The shares of the CTAs in `left`, which could not wait.  Rare, and out of line: with this loop in the kernel the code that the
-// compiler makes of the main loop is slower (the half-corrected Qwen2.5-7B step at 64 tokens: 548 us so, 514 with the call).
+// The shares of the CTAs in `left`, which could not wait.  Rare, and out of line: with this loop in the kernel the half-corrected
+// Qwen2.5-7B step at 64 tokens took 548 us, 514 with the call.
 __device__ __noinline__ void add_shares(ShareArgs a, unsigned long long left, int et) {
   for (; left != 0; left &= left - 1) add_share(a, __ffsll(left) - 1, et);
 }
 
 // EXACT (up to 8 tokens): the weights enter the product as the exact integers code - zero, every step has an accumulator of its own per
 // team, and the team that dequantised a step adds scale x accumulator to fp32 sums in registers - the precision of the weight-streaming
-// kernel.  Else they are rounded to fp16 with their scale first, as the reference rounds them.
+// kernel.  Else they are rounded to fp16 with their scale first, as the reference rounds them.  The exact form spills: 48 bytes a
+// thread, 46 thousand of 16.1 million instructions in the launch of the 13B gate/up shape at 8 tokens (29.6 us).
 template <bool EXACT>
 __global__ void __launch_bounds__(kThreads, 2)
 gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsMaps tm) {
@@ -418,7 +420,8 @@ gemm_tmem_kernel(const __grid_constant__ TsParams p, const __grid_constant__ TsM
         b.step(1, p.ns);
         ready = g_mbar_test_elected(full + 8 * b.i, b.ph);   // answered while this stage's MMAs are issued
         if (EXACT) acc = 0;
-        umma_ts_step(EXACT ? tmem + ((it - it0) & 1) * p.N : tmem, tmem + p.a_col + cur * 64, lo0 + cur * ((2 * sub) >> 4), hi, sub >> 4, idesc, acc, empty + 8 * cur);
+        umma_ts_step(EXACT ? tmem + ((it - it0) & 1) * p.N : tmem, tmem + p.a_col + cur * 64, lo0 + cur * ((2 * sub) >> 4), hi, sub >> 4,
+                     idesc, acc, empty + 8 * cur);
         acc = 1;
       }
       if (sep) acc = 0;   // the first MMA overwrites its accumulator
@@ -875,7 +878,8 @@ double gemm_tmem_exact_us(const glowq_w4a16_group_t& g, bool compute_r, bool any
 }
 
 // (host arithmetic: see glowq_internal_workspace_map)
-void gemm_tmem_workspace_map(const glowq_w4a16_group_t& g, bool exact, bool compute_r, bool any_corr, bool any_separate, int sms, WorkspaceMap* map) {
+void gemm_tmem_workspace_map(const glowq_w4a16_group_t& g, bool exact, bool compute_r, bool any_corr, bool any_separate, int sms,
+                             WorkspaceMap* map) {
   const TmemPlan pl = make_tmem_plan(g, exact, compute_r, any_corr, any_separate, sms);
   map->kernel = 1;
   map->ksplit = pl.ksplit;
@@ -891,8 +895,8 @@ void gemm_tmem_workspace_map(const glowq_w4a16_group_t& g, bool exact, bool comp
 
 // Members' products and corrections of a group call of up to 64 tokens.  compute_r: r into g.r_buf as well (else it is
 // there); the workspace must hold gemm_tmem_r_bytes for it behind kWsSlotsOffset.
-int gemm_tmem_forward(const glowq_w4a16_group_t& g, bool exact, bool compute_r, bool any_corr, bool any_separate, int sms, cudaStream_t stream,
-                      cudaError_t* cuda_err) {
+int gemm_tmem_forward(const glowq_w4a16_group_t& g, bool exact, bool compute_r, bool any_corr, bool any_separate, int sms,
+                      cudaStream_t stream, cudaError_t* cuda_err) {
   const int G = cdiv(g.IC, kGroup);
   const TmemPlan pl = make_tmem_plan(g, exact, compute_r, any_corr, any_separate, sms);
   unsigned char* const ws = static_cast<unsigned char*>(g.workspace);

@@ -10,7 +10,7 @@
 // and nothing intermediate is written (the torch expression is about thirty elementwise kernels).
 // A warp's eight groups are divided once, a group per quad of lanes, and the quotients of its weights are paired fp32 operations; with
 // every half warp dividing for each of its four groups in turn, and for groups past the end of a row too, 13824 x 5120 took 64 us and
-// 18944 x 3584 (28 groups) 89; now 42 (3.9 TB/s; a copy's 28) and 46.  5120 x 5120: 26 -> 18.  Six blocks an SM: a few bytes of spill
+// 18944 x 3584 (28 groups) 89; now 42 (4.2 TB/s; a copy's 28) and 46.  5120 x 5120: 26 -> 18.  Six blocks an SM: a few bytes of spill
 // in the path that divides, 43 us where five without took 45.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>

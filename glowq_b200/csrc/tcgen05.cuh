@@ -83,10 +83,9 @@ __device__ __forceinline__ bool g_mbar_try_once(uint32_t a, uint32_t parity) {
                : "memory");
   return ok != 0;
 }
-// Waits of a whole warp that issues tcgen05.mma: one elected lane asks, and a vote gives the answer to all.  Every branch is then
-// uniform to the compiler as well.  Behind a branch or a loop that it takes to be divergent - a wait under `lane == 0` - it no longer
-// keeps the operands of the MMAs in uniform registers, and a step of eight MMAs takes 506 clocks to issue instead of 171 (N = 16, one
-// warp per SM, barriers open; 78 without any wait).
+// Waits of a whole warp that issues tcgen05.mma: one elected lane asks, and a vote gives the answer to all, so that every branch is
+// uniform in the source.  With the wait under `lane == 0` a step of eight MMAs takes 506 clocks to issue, so 171 (N = 16, one warp per
+// SM, barriers open; 78 without any wait).  Supposed reason: behind a branch that may diverge the MMAs' operands are not kept uniform.
 __device__ __forceinline__ uint32_t g_mbar_test_elected(uint32_t a, uint32_t parity) {   // does not suspend
   uint32_t r;
   asm volatile(
@@ -152,9 +151,9 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
 // Eight packed words -> 64 fp16 weights half_rn((n - z) * scale) in the order of K.  Byte i of a word holds codes 2i, 2i + 1: as the low
 // bytes of two halves with exponent byte 0x64 and the other nibble masked off they are (1024 + n, 1024 + 16 n'), in the order the MMA
 // wants them; one FMA with zc = (-(1024 + z), -(64 + z)) leaves the exact (n - z, n' - z), and the product with the scale (s2: twice)
-// rounds once.  In three passes over all 32 registers: as one expression per register the compiler computes beside the block of
-// consecutive registers that tcgen05.st takes, and moves each result over (19.3 instead of 17.1 million instructions in the launch of
-// the 13B gate/up shape at 16 tokens, 31.2 us instead of 29.3).
+// rounds once.  In three passes over all 32 registers: as one expression per register the launch of the 13B gate/up shape at 16 tokens
+// executes 19.3 million instructions instead of 17.1 and takes 31.2 us instead of 29.3 (supposedly moves into the consecutive registers
+// that tcgen05.st takes).
 // SCALED false: the exact integers n - z.
 template <bool SCALED = true>
 __device__ __forceinline__ void dequant_words(uint32_t (&v)[32], const uint32_t (&w)[16], int first, uint32_t zc, uint32_t s2) {
