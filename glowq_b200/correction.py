@@ -69,6 +69,8 @@ class MiniGroupCache:
         _ALL_CACHES.add(self)
 
     def buffer(self, m: int, rank: int, device) -> torch.Tensor:
+        if not isinstance(self._buf, K.RRows):      # loaded from a file of an earlier form
+            self._buf = K.RRows()
         return self._buf.rows(m, rank, device)
 
     def set(self, r: torch.Tensor, uses: int, key=None):
@@ -298,6 +300,8 @@ class AddSVDCorrection(nn.Module):
                           f"linear {inner.in_features}->{inner.out_features}; correction disabled for this module")
 
     def _private_r(self, m: int, rank: int, device) -> torch.Tensor:
+        if not isinstance(self._own_r, K.RRows):
+            self._own_r = K.RRows()
         return self._own_r.rows(m, rank, device)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:

@@ -301,7 +301,12 @@ class RRows:
         return RRows, ()
 
     def rows(self, m: int, rank: int, device: torch.device) -> torch.Tensor:
-        stream = current_stream_ptr(device) if device.type == "cuda" else 0
+        stream = 0
+        if device.type == "cuda":
+            if current_device() != device.index:     # (whether the stream captures is asked of the current device)
+                with torch.cuda.device(device):
+                    return self.rows(m, rank, device)
+            stream = current_stream_ptr(device)
         piece = self._scratch.get(2 * max(m, 16) * rank, device, stream)
         last = self._last
         if last is None or last[0] is not piece or last[1] != (m, rank):

@@ -149,9 +149,12 @@ def test_room_for_r_that_a_graph_was_captured_with_stays(monkeypatch):
     capturing = [False]
     monkeypatch.setattr(K, "_is_capturing", lambda: capturing[0])
     monkeypatch.setattr(K, "current_stream_ptr", lambda device: 7)
+    monkeypatch.setattr(K, "current_device", lambda: 0)
     device = SimpleNamespace(type="cuda", index=0)
     monkeypatch.setattr(K.torch, "zeros", lambda n, dtype, device, zeros=torch.zeros: zeros(n, dtype=dtype))
-    for room in (MiniGroupCache().buffer, patched().proj(0, "mlp.down_proj")._private_r):
+    cache, model = MiniGroupCache(), patched()
+    cache._buf = model.proj(0, "mlp.down_proj")._own_r = None      # as a file of an earlier form has them
+    for room in (cache.buffer, model.proj(0, "mlp.down_proj")._private_r):
         warm = room(5, 16, device)
         assert warm.shape == (5, 16) and warm.dtype == torch.float16 and room(5, 16, device) is warm
         capturing[0] = True
